@@ -39,28 +39,55 @@ struct HnswDev {
   size_t n;
 };
 
-template <bool IS_L2>
-__global__ void __launch_bounds__(256, 4)
-    hnsw_search_kernel(HnswDev g, const float* __restrict__ queries, const uint32_t* __restrict__ qids, size_t nq, int k,
-                       int ef, int log2slots, uint32_t* __restrict__ global_tables, u64* __restrict__ out_keys,
-                       uint32_t* __restrict__ overflow, unsigned long long* __restrict__ work,
-                       unsigned int* __restrict__ next_query) {
-  unsigned char* smem_raw = dyn_smem();
-  const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int slots = 1 << log2slots;
-  const size_t list_bytes = ((size_t(ef) * 8 + 15) & ~size_t(15)) + TIED_CAP * 4;
-  const size_t per_warp = size_t(g.pd) * 4 + list_bytes + (global_tables ? 0 : size_t(slots) * 4);
-  unsigned char* mine = smem_raw + size_t(w) * per_warp;
-  float* sq = reinterpret_cast<float*>(mine);
-  u64* best = reinterpret_cast<u64*>(mine + size_t(g.pd) * 4);
-  uint32_t* tied = reinterpret_cast<uint32_t*>(mine + size_t(g.pd) * 4 + list_bytes - TIED_CAP * 4);
-  const size_t gw = size_t(blockIdx.x) * W + w;
-  uint32_t* table = global_tables ? global_tables + gw * size_t(slots)
-                                  : reinterpret_cast<uint32_t*>(mine + size_t(g.pd) * 4 + list_bytes);
-  unsigned long long n_dist = 0, n_exp = 0, n_tie_lost = 0;
+// Shared memory of one search, in bytes: the query, the visited set's first part, the tie list, a run of rows and
+// their distances, the team's job, and the beam where it is not in registers.
+static constexpr int SEARCH_BLOCKS_PER_SM = 3;  // of 256 threads
+template <int R>
+__host__ __device__ __forceinline__ size_t search_smem(int pd, int ef, int sbits) {
+  return size_t(pd) * 4 + (size_t(4) << sbits) + (TIED_CAP + 32 + 32) * 4 + sizeof(TeamJob) +
+         (R == 0 ? ((size_t(ef) * 8 + 15) & ~size_t(15)) : 0);
+}
 
-  // Queries are drawn from a counter (zero at launch): a batch gives every resident warp two or three of them and
-  // they differ in length, so a fixed deal leaves the warps that drew three long ones running alone at the end.
+// Bound by the latency of a chain: link row, visited set, rows, insertions, about 65 times per query at ef 64, and by the
+// longest of a batch's queries (twice the average) at its end.  24 warps of 80 registers per SM hold a lane's 16
+// pieces of a row in flight: 2.02 ms per 10,000 queries at 200k x 128, ef 64 (32 warps of 64 registers, where the
+// loads are issued a few at a time: 2.46; 16 warps of 128: 2.28; before, with a row per lane, the beam in shared
+// memory and the visited set in L2: 2.35).
+// work: distances, expansions, queries whose tie list overflowed, queries whose visited set overflowed (marked in
+// overflow[] and left for a re-run).  NW = 1: one warp per query, blockDim / 32 queries per block; NW > 1: a query
+// per block (Team in hnsw.cuh).
+template <bool IS_L2, int R, int NW>
+__global__ void __launch_bounds__(256, SEARCH_BLOCKS_PER_SM)
+    hnsw_search_kernel(HnswDev g, const float* __restrict__ queries, const uint32_t* __restrict__ qids, size_t nq, int k,
+                       int ef, int sbits, int log2slots, uint32_t* __restrict__ tables, fv_neighbor* __restrict__ out,
+                       uint32_t* __restrict__ counts, uint32_t* __restrict__ overflow,
+                       unsigned long long* __restrict__ work, unsigned int* __restrict__ next_query) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int searcher = NW == 1 ? w : 0, per_block = NW == 1 ? int(blockDim.x >> 5) : 1;
+  unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, ef, sbits);
+  float* sq = reinterpret_cast<float*>(mine);
+  uint32_t* small = reinterpret_cast<uint32_t*>(sq + g.pd);
+  uint32_t* tied = small + (size_t(1) << sbits);
+  Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + 32),
+                reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64)};
+  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + sizeof(TeamJob));
+  if (NW > 1 && w > 0) {
+    team_serve<IS_L2, NW>(team);
+    return;
+  }
+  const size_t gw = size_t(blockIdx.x) * per_block + searcher;
+  VisitSet seen;
+  visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
+  unsigned long long n_dist = 0, n_exp = 0, n_tie_lost = 0, n_over = 0;
+  auto upper = [&](uint32_t x, int layer) {
+    size_t p = g.upper_off[x];
+    for (int s = 1; s < layer; ++s) p += 1 + g.upper_flat[p];
+    return g.upper_flat + p;
+  };
+  auto layer0 = [&](uint32_t x) { return g.links0 + size_t(x) * (g.m0 + 1); };
+
+  // Queries are drawn from a counter (zero at launch): a batch gives every resident searcher two or three of them and
+  // they differ in length, so a fixed deal leaves the ones that drew three long ones running alone at the end.
   for (;;) {
     size_t qi = 0;
     if (lane == 0) qi = atomicAdd(next_query, 1u);
@@ -69,187 +96,46 @@ __global__ void __launch_bounds__(256, 4)
     const size_t qsrc = qids ? size_t(qids[qi]) : qi;
     const unsigned long long n_dist0 = n_dist, n_exp0 = n_exp;  // a query that overflows its table is re-run: its work counts once
     for (int c = lane; c < g.pd; c += 32) sq[c] = queries[qsrc * size_t(g.pd) + c];
-    for (int s = lane * 4; s < slots; s += 128) *reinterpret_cast<uint4*>(table + s) = make_uint4(~0u, ~0u, ~0u, ~0u);
-    warp_list_init(best, ef);
+    visit_clear(seen, lane, 32);
 
     // entry point and greedy descent (hnsw.rs:329-347)
     uint32_t cur = g.ep;
-    float curd = exact_distance<IS_L2>(sq, g.data + size_t(cur) * g.pd, g.pd);
+    if (lane == 0) team.ids[0] = cur;
+    team_eval<IS_L2, NW>(team, sq, 1);
+    float curd = team.out[0];
     n_dist += 1;
-    for (int layer = g.top; layer >= 1; --layer) {
-      bool changed = true;
-      while (changed) {
-        changed = false;
-        size_t p = g.upper_off[cur];
-        for (int s = 1; s < layer; ++s) p += 1 + g.upper_flat[p];
-        const int cnt = int(g.upper_flat[p]);
-        n_exp += 1;
-        for (int c0 = 0; c0 < cnt; c0 += 32) {
-          const int i = c0 + lane;
-          uint32_t x = 0;
-          float d = INFINITY;
-          if (i < cnt) {
-            x = g.upper_flat[p + 1 + i];
-            const char* rowp = reinterpret_cast<const char*>(g.data + size_t(x) * g.pd);
-            for (int b = 0; b < g.pd * 4; b += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(rowp + b));
-            d = exact_distance<IS_L2>(sq, g.data + size_t(x) * g.pd, g.pd);
-          }
-          n_dist += __popc(__ballot_sync(FV_FULL, i < cnt));
-          // first minimum of the chunk, taken only if strictly below the current distance
-          const unsigned better = __ballot_sync(FV_FULL, i < cnt && d < curd);
-          if (better) {
-            float md = d < curd ? d : INFINITY;
-            for (int o = 16; o > 0; o >>= 1) md = fminf(md, __shfl_xor_sync(FV_FULL, md, o));
-            const unsigned at = __ballot_sync(FV_FULL, i < cnt && d == md);
-            const int src = __ffs(at) - 1;
-            cur = __shfl_sync(FV_FULL, x, src);
-            curd = md;
-            changed = true;
-          }
-        }
-      }
-    }
+    greedy_descent<IS_L2, NW>(team, g.n, upper, g.m0, sq, g.top, 0, cur, curd, n_dist, n_exp);
 
-    // layer 0 (hnsw.rs:179-226 with ef = max(ef, k)).  This is beam_search of hnsw.cuh (which the graph construction
-    // uses on every layer) written out for one entry point and layer 0's fixed-stride rows: through the shared
-    // function this kernel measured 2.3 % slower (7.78 against 7.61 ms per 10,000 queries on 1M nodes).
-    warp_list_insert(best, ef, beam_key(curd, cur));
-    if (lane == 0) visit(table, log2slots, cur);
-    __syncwarp();
-    int filled = 1;          // entries of `best` in use
-    int visited = 1;
+    // layer 0 (hnsw.rs:179-226 with ef = max(ef, k))
+    Beam<R> best;
+    best.init(ef, list);
+    best.insert(beam_key(curd, cur));
+    visit_warp(seen, lane == 0, cur);
     bool over = false, tie_lost = false;
-    int cursor = 0;          // first entry that may be unexpanded
-    int ntied = 0;           // pushed-out entries still tied with the worst kept distance
-    for (;;) {
-      // next unexpanded entry at or after `cursor`
-      int pos = -1;
-      for (int e0 = cursor & ~31; e0 < filled; e0 += 32) {
-        const int e = e0 + lane;
-        const bool open = e >= cursor && e < filled && !(best[e] & 1ull);
-        const unsigned mk = __ballot_sync(FV_FULL, open);
-        if (mk) {
-          pos = e0 + __ffs(mk) - 1;
-          break;
-        }
-      }
-      uint32_t c = 0;
-      if (ntied > 0) {
-        // the smallest id among the tied entries; it goes first if the beam has nothing open or only a larger key
-        uint32_t tmin = 0xFFFFFFFFu;
-        for (int t = lane; t < ntied; t += 32) tmin = min(tmin, tied[t]);
-        for (int o = 16; o > 0; o >>= 1) tmin = min(tmin, __shfl_xor_sync(FV_FULL, tmin, o));
-        const u64 tkey = (best[ef - 1] & 0xFFFFFFFF00000000ull) | (u64(tmin) << 1);
-        if (pos < 0 || tkey < best[pos]) {
-          __syncwarp();
-          for (int t = lane; t < ntied; t += 32)
-            if (tied[t] == tmin) tied[t] = tied[ntied - 1];  // ids are unique: one match
-          __syncwarp();
-          ntied--;
-          pos = -2;
-          c = tmin;
-        }
-      }
-      if (pos == -1) break;
-      if (pos >= 0) {
-        const u64 ck = best[pos];
-        __syncwarp();
-        if (lane == 0) best[pos] = ck | 1ull;
-        __syncwarp();
-        cursor = pos + 1;
-        c = uint32_t(ck >> 1) & 0x7FFFFFFFu;
-      }
-      if (!FV_IDX_OK(c, g.n, 1)) break;
-      const uint32_t* row = g.links0 + size_t(c) * (g.m0 + 1);
-      // the first 32 links are requested together with the count: one round trip, not two
-      const uint32_t x_first = lane < g.m0 ? __ldg(row + 1 + lane) : 0u;
-      const int cnt = int(__ldg(row));
-      n_exp += 1;
-      for (int c0 = 0; c0 < cnt; c0 += 32) {
-        const int i = c0 + lane;
-        u64 key = FV_EMPTY_KEY;
-        bool fresh = false;
-        uint32_t x = 0;
-        if (i < cnt) {
-          x = c0 == 0 ? x_first : row[1 + i];
-          fresh = FV_IDX_OK(x, g.n, 2) && visit(table, log2slots, x);
-        }
-        const int nfresh = __popc(__ballot_sync(FV_FULL, fresh));
-        visited += nfresh;
-        n_dist += nfresh;
-        if (fresh) {
-          // all lines of the row are requested before the dependent FMA chains start, so the gather costs one
-          // memory round trip instead of one per unrolled group of loads
-          const char* rowp = reinterpret_cast<const char*>(g.data + size_t(x) * g.pd);
-          for (int b = 0; b < g.pd * 4; b += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(rowp + b));
-          key = beam_key(exact_distance<IS_L2>(sq, g.data + size_t(x) * g.pd, g.pd), x);
-        }
-        // offer in stored order: admitted while the list is not full, or on a strictly smaller distance
-        u64 bound = best[ef - 1];
-        unsigned pending = __ballot_sync(FV_FULL, fresh);
-        while (pending) {
-          const int src = __ffs(pending) - 1;
-          pending &= pending - 1;
-          const u64 kk = __shfl_sync(FV_FULL, key, src);
-          if ((kk >> 32) < (bound >> 32)) {
-            // position of the new entry = number of entries below it
-            int below = 0;
-            for (int e0 = 0; e0 < filled; e0 += 32) {
-              const int e = e0 + lane;
-              below += __popc(__ballot_sync(FV_FULL, e < filled && best[e] < kk));
-            }
-            __syncwarp();
-            const bool was_full = filled == ef;
-            warp_list_insert(best, ef, kk);
-            if (filled < ef) filled++;
-            if (below < cursor) cursor = below;
-            const u64 pushed = bound;  // the entry that fell off the end, if the beam was full
-            bound = best[ef - 1];
-            if (was_full) {
-              if ((bound >> 32) < (pushed >> 32)) {
-                ntied = 0;  // the worst distance went down: nothing pushed out so far can tie with it any more
-              } else if (!(pushed & 1ull)) {
-                if (ntied < TIED_CAP) {
-                  __syncwarp();
-                  if (lane == 0) tied[ntied] = uint32_t(pushed >> 1) & 0x7FFFFFFFu;
-                  __syncwarp();
-                  ntied++;
-                } else {
-                  tie_lost = true;
-                }
-              }
-            }
-          }
-        }
-      }
-      if (visited > (slots >> 1)) {
-        over = true;
-        break;
-      }
-    }
-    __syncwarp();
+    beam_search<IS_L2, R, NW>(team, g.n, layer0, g.m0, sq, best, tied, seen, over, tie_lost, n_dist, n_exp);
     if (tie_lost && !over) n_tie_lost += 1;
+    if (lane == 0) overflow[qi] = over ? 1 : 0;
     if (over) {
-      if (lane == 0) overflow[qi] = 1;
+      n_over += 1;
       n_dist = n_dist0;
       n_exp = n_exp0;
     } else {
-      if (lane == 0) overflow[qi] = 0;
-      for (int e = lane; e < k; e += 32) {
-        u64 v = FV_EMPTY_KEY;
-        if (e < filled) {
-          const u64 b = best[e];
-          v = (b & 0xFFFFFFFF00000000ull) | u64(uint32_t(b >> 1) & 0x7FFFFFFFu);
-        }
-        out_keys[qsrc * size_t(k) + e] = v;
-      }
+      const int found = min(best.filled(), k);
+      fv_neighbor* dst = out + qsrc * size_t(k);
+      best.each([&](int e, u64 b) {
+        if (e < k) dst[e] = fv_neighbor{beam_id(b), beam_distance(b)};
+      });
+      for (int e = found + lane; e < k; e += 32) dst[e] = fv_neighbor{0xFFFFFFFFu, INFINITY};
+      if (lane == 0 && counts) counts[qsrc] = uint32_t(found);
     }
     __syncwarp();
   }
-  if (work && lane == 0) {
+  team_dismiss(team);
+  if (lane == 0) {
     atomicAdd(work, n_dist);
     atomicAdd(work + 1, n_exp);
     if (n_tie_lost) atomicAdd(work + 2, n_tie_lost);
+    if (n_over) atomicAdd(work + 3, n_over);
   }
 }
 
@@ -478,6 +364,59 @@ struct Builder {
   }
 };
 
+// ---- launch shape of a search
+// A team of TEAM_WARPS warps per query while the batch is small, a warp per query beyond.  Measured (us a batch, team /
+// warp): 200k x 128, ef 64: 1 query 193 / 279, 592 queries 516 / 1,300, 2,368 queries 1,070 / 1,500, 10,000 queries
+// 3,850 / 2,020; 5,183 x 384, ef 64: 1 query 267 / 680, 2,368 queries 1,240 / 1,700, 5,000 queries 2,350 / 2,370; the
+// lines meet near 16 queries per SM at ef 16 and 200 too.
+typedef void (*SearchKernel)(HnswDev, const float*, const uint32_t*, size_t, int, int, int, int, uint32_t*, fv_neighbor*,
+                             uint32_t*, uint32_t*, unsigned long long*, unsigned int*);
+struct SearchShape {
+  SearchKernel kern;
+  size_t blocks, searchers, smem;  // searchers per block
+  int threads, sbits;
+};
+
+template <int NW>
+static SearchKernel pick_search(bool is_l2, int R) {
+  switch (R) {
+    case 1: return is_l2 ? hnsw_search_kernel<true, 1, NW> : hnsw_search_kernel<false, 1, NW>;
+    case 2: return is_l2 ? hnsw_search_kernel<true, 2, NW> : hnsw_search_kernel<false, 2, NW>;
+    case 4: return is_l2 ? hnsw_search_kernel<true, 4, NW> : hnsw_search_kernel<false, 4, NW>;
+    case 8: return is_l2 ? hnsw_search_kernel<true, 8, NW> : hnsw_search_kernel<false, 8, NW>;
+    default: return is_l2 ? hnsw_search_kernel<true, 0, NW> : hnsw_search_kernel<false, 0, NW>;
+  }
+}
+
+static int search_shape(fv_ctx* ctx, bool is_l2, int pd, int ef, size_t active, SearchShape* s) {
+  const int R = ef <= 32 ? 1 : ef <= 64 ? 2 : ef <= 128 ? 4 : ef <= 256 ? 8 : 0;
+  const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
+  const bool team = active <= size_t(ctx->sm_count) * TEAM_SEARCHES_PER_SM;
+  s->sbits = visit_sbits(ef, team ? 13 : 11);
+  size_t per = R == 0 ? search_smem<0>(pd, ef, s->sbits) : search_smem<1>(pd, ef, s->sbits);
+  int W = 8;
+  if (team) {
+    s->searchers = 1;
+    s->threads = TEAM_WARPS * 32;
+  } else {
+    while (W > 1 && per * W > budget / 2) W >>= 1;
+    s->searchers = size_t(W);
+    s->threads = W * 32;
+  }
+  while (s->sbits > 7 && per * s->searchers > budget) {
+    per -= size_t(2) << s->sbits;
+    s->sbits--;
+  }
+  s->smem = per * s->searchers;
+  if (s->smem > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "dimension and ef too large for shared memory");
+  const size_t by_warps = 8 * SEARCH_BLOCKS_PER_SM / (s->threads / 32);
+  const size_t per_sm = std::max<size_t>(1, std::min(size_t(227 * 1024) / (s->smem + 1024), by_warps));
+  s->blocks = std::min<size_t>((active + s->searchers - 1) / s->searchers, size_t(ctx->sm_count) * per_sm);
+  s->kern = team ? pick_search<TEAM_WARPS>(is_l2, R) : pick_search<1>(is_l2, R);
+  if (s->smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(s->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s->smem)));
+  return FV_OK;
+}
+
 // scratch slots: 0 padded queries, 1 keys, 5 overflow flags, 6 retry ids, 7 global tables
 static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t k, size_t ef_in, fv_neighbor* d_out,
                            uint32_t* d_counts) {
@@ -486,9 +425,9 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   if (nq == 0) return FV_OK;
   ctx->stats = fv_stats{};
   const size_t n = h->n();
-  FV_TRY(ctx->scratch[1].reserve(nq * k * sizeof(u64)));
-  u64* keys = ctx->scratch[1].as<u64>();
   if (n == 0) {  // hnsw.rs:324-326: an empty index finds nothing
+    FV_TRY(ctx->scratch[1].reserve(nq * k * sizeof(u64)));
+    u64* keys = ctx->scratch[1].as<u64>();
     FV_CUDA(cudaMemsetAsync(keys, 0xFF, nq * k * sizeof(u64), ctx->stream));
     FV_TRY(keys_to_neighbors(ctx, keys, nq, int(k), int(k), d_out, d_counts));
     FV_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -507,8 +446,9 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   }
   FV_TRY(ctx->scratch[5].reserve(nq * sizeof(uint32_t)));
   uint32_t* d_over = ctx->scratch[5].as<uint32_t>();
+  // words 16..23: the four counters; word 24: the next query
   unsigned long long* d_work = reinterpret_cast<unsigned long long*>(ctx->d_flags + 16);
-  FV_CUDA(cudaMemsetAsync(d_work, 0, 3 * sizeof(unsigned long long), ctx->stream));
+  unsigned int* d_next = reinterpret_cast<unsigned int*>(ctx->d_flags + 24);
   HnswDev g{};
   g.data = h->d_data.as<float>();
   g.links0 = h->d_links0.as<uint32_t>();
@@ -520,61 +460,42 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   g.top = int(h->top);
   g.ep = h->ep;
   g.n = n;
-  // visited-table size: room for the nodes a beam of width ef usually touches, doubled
+  // second part of the visited set: 48 * ef slots to begin with (it may fill to one half); the overflow path
+  // quadruples it for the queries that need more
   int log2slots = 11;
-  // visited-table size: a beam of width ef evaluates a few dozen nodes per entry kept; start at 48 * ef slots
-  // (the table may fill to one half) and let the overflow path quadruple it for the queries that need more
-  const char* menv = getenv("FV_HNSW_SLOTS_PER_EF");  // tuning knob
-  const size_t per_ef = menv ? size_t(atoi(menv)) : 48;
-  while ((size_t(1) << log2slots) < ef * per_ef && log2slots < 26) log2slots++;
+  while ((size_t(1) << log2slots) < ef * 48 && log2slots < 26) log2slots++;
   const uint32_t* d_qids = nullptr;
   size_t active = nq;
-  std::vector<uint32_t> h_over(nq), retry;
-  for (int attempt = 0; attempt < 8; ++attempt) {
-    const size_t slots = size_t(1) << log2slots;
-    const size_t base_bytes = size_t(pd) * 4 + ((ef * 8 + 15) & ~size_t(15)) + TIED_CAP * 4;
-    const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
-    int W = 8;
-    bool use_global = false;
-    // Tables in shared memory cap the resident warps (latency-bound kernel); in global memory they are
-    // L2-resident and 32 warps fit per SM (64 registers each: the kernel spills about 40 words, which costs less
-    // than the eight extra warps bring -- measured 4.85 against 5.30 ms per 10,000 queries with 24 warps of 80
-    // registers, and 5.26 ms with 40 warps of 48).
-    const char* genv = getenv("FV_HNSW_TABLES");  // tuning knob: "smem" or "global"
-    use_global = genv ? genv[0] == 'g' : true;
-    if (base_bytes + slots * 4 > budget / 2) use_global = true;
-    const size_t per_warp = base_bytes + (use_global ? 0 : slots * 4);
-    while (W > 1 && per_warp * W > budget) W >>= 1;
-    if (per_warp * W > budget) return fail(FV_ERR_UNSUPPORTED, "dimension and ef too large for shared memory");
-    int blocks_per_sm = int(std::max<size_t>(1, std::min<size_t>(budget / (per_warp * W), 32 / W)));
-    size_t blocks = std::min<size_t>((active + W - 1) / W, size_t(ctx->sm_count) * blocks_per_sm);
-    uint32_t* tables = nullptr;
-    if (use_global) {
-      FV_TRY(ctx->scratch[7].reserve(blocks * W * slots * 4));
-      tables = ctx->scratch[7].as<uint32_t>();
-    }
-    auto kern = h->metric == FV_L2 ? hnsw_search_kernel<true> : hnsw_search_kernel<false>;
-    const size_t smem = per_warp * W;
-    if (smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    unsigned int* d_next = reinterpret_cast<unsigned int*>(ctx->d_flags + 32);
-    FV_CUDA(cudaMemsetAsync(d_next, 0, sizeof(unsigned int), ctx->stream));
-    kern<<<unsigned(blocks), W * 32, smem, ctx->stream>>>(g, q, d_qids, active, int(k), int(ef), log2slots, tables, keys,
-                                                         d_over, d_work, d_next);
+  std::vector<uint32_t> h_over, retry;
+  unsigned long long wk[4] = {0, 0, 0, 0}, total[3] = {0, 0, 0};
+  for (int attempt = 0; attempt < 8 && active; ++attempt) {
+    SearchShape sh{};
+    FV_TRY(search_shape(ctx, h->metric == FV_L2, pd, int(ef), active, &sh));
+    const size_t tables = sh.blocks * sh.searchers;
+    FV_TRY(ctx->scratch[7].reserve((tables << log2slots) * 4));
+    FV_CUDA(cudaMemsetAsync(d_work, 0, 4 * sizeof(unsigned long long) + sizeof(unsigned int), ctx->stream));
+    sh.kern<<<unsigned(sh.blocks), sh.threads, sh.smem, ctx->stream>>>(g, q, d_qids, active, int(k), int(ef), sh.sbits, log2slots,
+                                                                       ctx->scratch[7].as<uint32_t>(), d_out, d_counts, d_over,
+                                                                       d_work, d_next);
     ctx->stats.launches++;
     FV_CUDA(cudaGetLastError());
+    FV_CUDA(cudaMemcpyAsync(wk, d_work, sizeof(wk), cudaMemcpyDeviceToHost, ctx->stream));
+    FV_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (int i = 0; i < 3; ++i) total[i] += wk[i];
+    if (wk[3] == 0) {
+      active = 0;
+      break;
+    }
+    h_over.resize(active);
     FV_CUDA(cudaMemcpyAsync(h_over.data(), d_over, active * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     FV_CUDA(cudaStreamSynchronize(ctx->stream));
     std::vector<uint32_t> next;
     for (size_t i = 0; i < active; i++)
       if (h_over[i]) next.push_back(d_qids ? retry[i] : uint32_t(i));
-    if (next.empty()) {
-      active = 0;
-      break;
-    }
     ctx->stats.regrown += next.size();
     retry = next;
     active = retry.size();
-    FV_TRY(ctx->scratch[6].reserve(active * sizeof(uint32_t)));
+    FV_TRY(ctx->scratch[6].reserve(active * sizeof(uint32_t) + 4));
     FV_CUDA(cudaMemcpyAsync(ctx->scratch[6].p, retry.data(), active * sizeof(uint32_t), cudaMemcpyHostToDevice,
                             ctx->stream));
     d_qids = ctx->scratch[6].as<uint32_t>();
@@ -582,13 +503,10 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   }
   if (active) return fail(FV_ERR_OVERFLOW, "visited table overflow after regrowing");
   stage_mark(ctx);
-  FV_TRY(keys_to_neighbors(ctx, keys, nq, int(k), int(k), d_out, d_counts));
-  unsigned long long wk[3] = {0, 0, 0};
-  FV_CUDA(cudaMemcpyAsync(wk, d_work, sizeof(wk), cudaMemcpyDeviceToHost, ctx->stream));
+  ctx->stats.dist_evals = total[0];
+  ctx->stats.expansions = total[1];
+  ctx->stats.uncertified = total[2];  // queries whose list of tied, pushed-out entries overflowed (see TIED_CAP)
   FV_CUDA(cudaStreamSynchronize(ctx->stream));
-  ctx->stats.dist_evals = wk[0];
-  ctx->stats.expansions = wk[1];
-  ctx->stats.uncertified = wk[2];  // queries whose list of tied, pushed-out entries overflowed (see TIED_CAP)
   stage_end(ctx);
   return bounds_report_hnsw();
 }

@@ -43,6 +43,11 @@ int upload_graph(fv_hnsw* h, bool with_data = true);
 // distance) and take their turn in (distance, id) order; the list is dropped as soon as the worst distance goes down.
 static constexpr int TIED_CAP = 64;
 
+// Searches of one launch are run by teams of TEAM_WARPS warps up to this many per SM, by single warps beyond (the
+// figures are at search_shape in hnsw.cu).
+static constexpr int TEAM_WARPS = 8;
+static constexpr int TEAM_SEARCHES_PER_SM = 16;
+
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t hash_slot(uint32_t x, int log2slots) { return (x * 2654435761u) >> (32 - log2slots); }
 
@@ -64,54 +69,444 @@ __device__ __forceinline__ u64 beam_key(float d, uint32_t id) { return (u64(orde
 __device__ __forceinline__ uint32_t beam_id(u64 key) { return uint32_t(key >> 1) & 0x7FFFFFFFu; }
 __device__ __forceinline__ float beam_distance(u64 key) { return order_bits_to_float(uint32_t(key >> 32)); }
 
-// search_layer (hnsw.rs:179-226) by one warp, from the entries best[0..filled) (sorted, at most ef).  `rows(c)` is the
-// link block of node c on the searched layer (count, then at most `width` ids; width + 1 words are readable).  The
-// reference's pair of heaps is ONE sorted list of ef entries with an "expanded" bit each: a candidate that has been
-// evicted from `best` can only be popped after every entry of `best` has been expanded, and then it trips the stop
-// test (hnsw.rs:203-205) unless its distance ties the current worst exactly -- see TIED_CAP.  Neighbours of the
-// expanded node are evaluated one per lane and offered to the list in stored order, so the admission test
-// (hnsw.rs:214) sees the same evolving bound as the sequential loop.  The visited set is an exact open-addressing
-// hash table of 2^log2slots words owned by the warp; a search that fills more than half of it stops with `over`.
-// On return best[0..filled) is the reference's result, nearest first; n_dist and n_exp have grown by the distances
-// evaluated and the nodes expanded.
-template <bool IS_L2, class Rows>
-__device__ __forceinline__ void beam_search(const float* __restrict__ data, int pd, size_t n, Rows rows, int width,
-                                            const float* sq, u64* best, int ef, uint32_t* tied, uint32_t* table,
-                                            int log2slots, int& filled, bool& over, bool& tie_lost,
-                                            unsigned long long& n_dist, unsigned long long& n_exp) {
-  const int lane = lane_id();
-  const int slots = 1 << log2slots;
-  for (int s = lane * 4; s < slots; s += 128) *reinterpret_cast<uint4*>(table + s) = make_uint4(~0u, ~0u, ~0u, ~0u);
-  __syncwarp();
-  for (int e = lane; e < filled; e += 32) {
-    const u64 b = best[e] & ~1ull;
-    best[e] = b;
-    visit(table, log2slots, beam_id(b));
-  }
-  __syncwarp();
-  int visited = filled, cursor = 0, ntied = 0;
-  over = false;
-  for (;;) {
-    int pos = -1;
-    for (int e0 = cursor & ~31; e0 < filled; e0 += 32) {
-      const int e = e0 + lane;
-      const bool open = e >= cursor && e < filled && !(best[e] & 1ull);
-      const unsigned mk = __ballot_sync(FV_FULL, open);
-      if (mk) {
-        pos = e0 + __ffs(mk) - 1;
+// ---- visited set: exact, in two parts.
+// The first part is a small table in shared memory with two 16-bit entries per word.  x -> x * odd (mod 2^b, b bits
+// holding every id) is a bijection; the high bits of the image name the home bucket, so an entry needs only the low
+// `rb` bits and how many buckets it sits behind its home.  An id that finds all of its `probes` buckets full goes to
+// the second part, an open-addressing table of whole ids in global memory that is cleared by the first id it gets.
+// Nothing is ever removed, so a bucket that was full when an id passed it is full whenever the id comes back.
+// With the whole set in global memory, as it was, an expansion spent 2,100 of 10,600 cycles in atomics on L2.
+struct VisitSet {
+  uint32_t* small;    // shared memory: 2^sbits words
+  uint32_t* big;      // global memory: 2^log2slots words
+  int sbits, rb, probes, log2slots;
+  uint32_t idmask;
+  int in_big;         // ids in `big`, the same in every lane; -1: not cleared yet
+};
+
+// Words of the shared part for a beam of ef entries: about 12 ids are visited per entry of the beam on the benchmark's
+// graphs, and 32 * ef places keep the table below half full.
+__host__ __device__ __forceinline__ int visit_sbits(int ef, int max_bits) {
+  int s = 7;
+  while (s < max_bits && (1 << s) < ef * 16) ++s;
+  return s;
+}
+
+__device__ __forceinline__ void visit_setup(VisitSet& v, uint32_t* small, int sbits, uint32_t* big, int log2slots,
+                                            size_t n) {
+  int b = 1;
+  while (b < 32 && (size_t(1) << b) < n) ++b;
+  v.small = small;
+  v.big = big;
+  v.sbits = sbits;
+  v.rb = b > sbits ? b - sbits : 0;
+  v.probes = min(32, int(0xFFFFu >> min(v.rb, 16)));  // (the largest displacement must leave 0xFFFF, "empty", unused)
+  v.idmask = b == 32 ? 0xFFFFFFFFu : (1u << b) - 1u;
+  v.log2slots = log2slots;
+  v.in_big = -1;
+}
+
+// empties the set; `nthreads` threads (of which this is `tid`) share the work, and the caller lines them up afterwards
+__device__ __forceinline__ void visit_clear(VisitSet& v, int tid, int nthreads) {
+  for (int i = tid * 4; i < (1 << v.sbits); i += nthreads * 4) *reinterpret_cast<uint4*>(v.small + i) = make_uint4(~0u, ~0u, ~0u, ~0u);
+  v.in_big = -1;
+}
+
+// called by a whole warp: true in the lanes whose x (on && x < n) was not in the set and is now.
+// The usual case -- the home bucket holds x, or has room and no other lane wants it -- is straight-line code: a branch
+// costs a warp here about as much as a trip to shared memory.
+__device__ __forceinline__ bool visit_warp(VisitSet& v, bool on, uint32_t x) {
+  const uint32_t h = (x * 0x9E3779B1u) & v.idmask;
+  const uint32_t bucket = h >> v.rb, rem = h & ((1u << v.rb) - 1u);
+  uint32_t* p = v.small + bucket;
+  uint32_t w = *reinterpret_cast<volatile uint32_t*>(p);
+  const bool lo_free = (w & 0xFFFFu) == 0xFFFFu, hi_free = (w >> 16) == 0xFFFFu;
+  const bool seen = (w & 0xFFFFu) == rem || (w >> 16) == rem;
+  const bool want = on && !seen && (lo_free || hi_free) && v.probes > 0;
+  const uint32_t nw = lo_free ? ((w & 0xFFFF0000u) | rem) : ((w & 0xFFFFu) | (rem << 16));
+  uint32_t old = ~w;
+  if (want) old = atomicCAS(p, w, nw);
+  bool fresh = want && old == w;
+  bool open = on && !fresh && (!seen || v.probes <= 0);  // another lane was quicker, or the bucket is full
+  if (!__any_sync(FV_FULL, open)) return fresh;
+  bool full = open;
+  const uint32_t smask = (1u << v.sbits) - 1u;
+  for (int d = 0; d < v.probes && full; ++d) {
+    const uint32_t val = (uint32_t(d) << v.rb) | rem;
+    p = v.small + ((bucket + uint32_t(d)) & smask);
+    w = *reinterpret_cast<volatile uint32_t*>(p);
+    for (;;) {  // (a word fills up after two insertions: at most three turns)
+      const uint32_t lo = w & 0xFFFFu, hi = w >> 16;
+      if (lo == val || hi == val) {
+        full = false;
         break;
       }
+      uint32_t nv;
+      if (lo == 0xFFFFu) nv = (w & 0xFFFF0000u) | val;
+      else if (hi == 0xFFFFu) nv = (w & 0xFFFFu) | (val << 16);
+      else break;
+      const uint32_t was = atomicCAS(p, w, nv);
+      if (was == w) {
+        full = false;
+        fresh = true;
+        break;
+      }
+      w = was;
     }
-    uint32_t c = 0;
-    if (ntied > 0) {
-      uint32_t tmin = 0xFFFFFFFFu;
-      for (int t = lane; t < ntied; t += 32) tmin = min(tmin, tied[t]);
-      for (int o = 16; o > 0; o >>= 1) tmin = min(tmin, __shfl_xor_sync(FV_FULL, tmin, o));
-      const u64 tkey = (best[ef - 1] & 0xFFFFFFFF00000000ull) | (u64(tmin) << 1);
-      if (pos < 0 || tkey < best[pos]) {
+  }
+  if (__any_sync(FV_FULL, full)) {
+    const int lane = lane_id();
+    if (v.in_big < 0) {
+      for (int s = lane * 4; s < (1 << v.log2slots); s += 128) *reinterpret_cast<uint4*>(v.big + s) = make_uint4(~0u, ~0u, ~0u, ~0u);
+      v.in_big = 0;
+      __syncwarp();
+    }
+    if (full) fresh = visit(v.big, v.log2slots, x);
+    v.in_big += __popc(__ballot_sync(FV_FULL, full && fresh));
+  }
+  return fresh;
+}
+__device__ __forceinline__ bool visit_overflow(const VisitSet& v) { return v.in_big > (1 << (v.log2slots - 1)); }
+
+// ---- the beam: the ef nearest entries seen so far, ascending, each with its "expanded" bit.
+// R > 0: in registers, place 32 r + lane in e[r] (ef <= 32 R): an insertion is one compare and one shuffle per 32
+// entries, without the shared-memory round trips and barriers of the list below.  The list ends at the last place, so
+// that its last entry is found and dropped without knowing ef; the `off` places before it hold a key below every
+// other.  That key and FV_EMPTY_KEY, the unused entry, both read "expanded" in their lowest bit.
+template <int R>
+struct Beam {
+  u64 e[R];
+  int off;
+  __device__ __forceinline__ void init(int ef, u64*) {
+    off = 32 * R - ef;
+#pragma unroll
+    for (int r = 0; r < R; ++r) e[r] = r * 32 + lane_id() < off ? 1ull : FV_EMPTY_KEY;
+  }
+  __device__ __forceinline__ u64 last() const { return __shfl_sync(FV_FULL, e[R - 1], 31); }
+  __device__ __forceinline__ int last_pos() const { return 32 * R - 1; }
+  __device__ __forceinline__ void insert(u64 key) {  // key < last()
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r) {
+      u64 prev = __shfl_up_sync(FV_FULL, e[r], 1);
+      const u64 carry = r > 0 ? __shfl_sync(FV_FULL, e[r > 0 ? r - 1 : 0], 31) : 0ull;
+      if (lane_id() == 0) prev = carry;
+      if (!(e[r] < key)) e[r] = prev < key ? key : prev;
+    }
+  }
+  // the first entry that is not expanded: its position (-1: none) and key
+  __device__ __forceinline__ int first_open(u64& key) const {
+    int pos = -1;
+    u64 v = 0;
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r) {
+      const unsigned mk = __ballot_sync(FV_FULL, !(e[r] & 1ull));
+      pos = mk ? r * 32 + __ffs(mk) - 1 : pos;
+      v = mk ? e[r] : v;
+    }
+    key = __shfl_sync(FV_FULL, v, pos & 31);
+    return pos;
+  }
+  __device__ __forceinline__ void mark(int pos) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (pos == r * 32 + lane_id()) e[r] |= 1ull;
+  }
+  __device__ __forceinline__ int filled() const {
+    int c = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) c += __popc(__ballot_sync(FV_FULL, e[r] != FV_EMPTY_KEY));
+    return c - off;
+  }
+  // fn(position, entry) for every entry in use, entries spread over the lanes
+  template <class Fn>
+  __device__ __forceinline__ void each(Fn fn) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (e[r] != FV_EMPTY_KEY && r * 32 + lane_id() >= off) fn(r * 32 + lane_id() - off, e[r]);
+  }
+  // takes the "expanded" marks off; fn(in use, id) is called by the whole warp, 32 entries at a time
+  template <class Fn>
+  __device__ __forceinline__ void reopen(Fn fn) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool on = e[r] != FV_EMPTY_KEY && r * 32 + lane_id() >= off;
+      if (on) e[r] &= ~1ull;
+      fn(on, beam_id(e[r]));
+    }
+  }
+};
+// R = 0: in shared memory, any ef
+template <>
+struct Beam<0> {
+  u64* e;
+  int ef, n, cursor;  // entries in use; the first entry that may be open
+  __device__ __forceinline__ void init(int ef_, u64* smem) {
+    e = smem;
+    ef = ef_;
+    n = 0;
+    cursor = 0;
+    warp_list_init(e, ef);
+  }
+  __device__ __forceinline__ u64 last() const { return e[ef - 1]; }
+  __device__ __forceinline__ int last_pos() const { return ef - 1; }
+  __device__ __forceinline__ void insert(u64 key) {
+    int below = 0;
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      const int i = e0 + lane_id();
+      below += __popc(__ballot_sync(FV_FULL, i < n && e[i] < key));
+    }
+    __syncwarp();
+    warp_list_insert(e, ef, key);
+    __syncwarp();
+    if (n < ef) n++;
+    if (below < cursor) cursor = below;
+  }
+  __device__ __forceinline__ int first_open(u64& key) const {
+    for (int e0 = cursor & ~31; e0 < n; e0 += 32) {
+      const int i = e0 + lane_id();
+      const unsigned mk = __ballot_sync(FV_FULL, i >= cursor && i < n && !(e[i] & 1ull));
+      if (mk) {
+        key = e[e0 + __ffs(mk) - 1];
+        return e0 + __ffs(mk) - 1;
+      }
+    }
+    return -1;
+  }
+  __device__ __forceinline__ void mark(int pos) {
+    __syncwarp();
+    if (lane_id() == 0) e[pos] |= 1ull;
+    cursor = pos + 1;
+    __syncwarp();
+  }
+  __device__ __forceinline__ int filled() const { return n; }
+  template <class Fn>
+  __device__ __forceinline__ void each(Fn fn) {
+    __syncwarp();
+    for (int i = lane_id(); i < n; i += 32) fn(i, e[i]);
+    __syncwarp();
+  }
+  template <class Fn>
+  __device__ __forceinline__ void reopen(Fn fn) {
+    __syncwarp();
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      const int i = e0 + lane_id();
+      const bool on = i < n;
+      if (on) e[i] &= ~1ull;
+      fn(on, on ? beam_id(e[i]) : 0u);
+    }
+    cursor = 0;
+    __syncwarp();
+  }
+};
+
+// ---- distances of a run of gathered rows, by LPR lanes per row (32 / LPR rows at a time).  A lane owns 8 / LPR of
+// the reference's eight chains (src/kernels.rs:200-231) and the lane sums are added in its pairwise order, so the
+// bits are exact_distance's.  A node has about ten unvisited links: with one row per lane, as it was, two thirds of
+// the lanes idle through 320 instructions per 128 dimensions and every load touches as many lines as there are rows.
+// What bounds a search is the trips to L2 in its chain (about 700 cycles each), so a lane requests U = 16 pieces (128
+// dimensions of its row) before it works on the first; what is left of the row goes in halves.
+template <bool IS_L2, int LPR, int U>
+__device__ __forceinline__ void group_chunk(const float* __restrict__ a, const float* __restrict__ row, int t, float& c0,
+                                            float& c1) {
+  if (LPR == 8) {
+    float b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) b[u] = __ldg(row + t + 8 * u);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (IS_L2) {
+        const float d = __fsub_rn(a[t + 8 * u], b[u]);
+        c0 = __fmaf_rn(d, d, c0);
+      } else {
+        c0 = __fmaf_rn(a[t + 8 * u], b[u], c0);
+      }
+    }
+  } else {
+    float2 b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) b[u] = __ldg(reinterpret_cast<const float2*>(row + t + 8 * u));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float2 x = *reinterpret_cast<const float2*>(a + t + 8 * u);
+      if (IS_L2) {
+        const float d0 = __fsub_rn(x.x, b[u].x), d1 = __fsub_rn(x.y, b[u].y);
+        c0 = __fmaf_rn(d0, d0, c0);
+        c1 = __fmaf_rn(d1, d1, c1);
+      } else {
+        c0 = __fmaf_rn(x.x, b[u].x, c0);
+        c1 = __fmaf_rn(x.y, b[u].y, c1);
+      }
+    }
+  }
+}
+template <bool IS_L2, int LPR>
+__device__ __forceinline__ float group_distance(const float* __restrict__ a, const float* __restrict__ row, int pd) {
+  const int j = lane_id() & (LPR - 1);
+  a += LPR == 8 ? j : 2 * j;
+  row += LPR == 8 ? j : 2 * j;
+  float c0 = 0.f, c1 = 0.f;
+  int t = 0;
+  for (; t + 128 <= pd; t += 128) group_chunk<IS_L2, LPR, 16>(a, row, t, c0, c1);
+  if (pd & 64) {
+    group_chunk<IS_L2, LPR, 8>(a, row, t, c0, c1);
+    t += 64;
+  }
+  if (pd & 32) {
+    group_chunk<IS_L2, LPR, 4>(a, row, t, c0, c1);
+    t += 32;
+  }
+  for (; t < pd; t += 8) group_chunk<IS_L2, LPR, 1>(a, row, t, c0, c1);
+  if (LPR == 8) {
+    float s = __fadd_rn(c0, __shfl_xor_sync(FV_FULL, c0, 4));
+    s = __fadd_rn(s, __shfl_xor_sync(FV_FULL, s, 2));
+    s = __fadd_rn(s, __shfl_xor_sync(FV_FULL, s, 1));
+    return IS_L2 ? s : -s;
+  }
+  // lanes hold (l0,l1) (l2,l3) (l4,l5) (l6,l7): ((l0 + l4) + (l2 + l6)) + ((l1 + l5) + (l3 + l7))
+  float s0 = __fadd_rn(c0, __shfl_xor_sync(FV_FULL, c0, 2)), s1 = __fadd_rn(c1, __shfl_xor_sync(FV_FULL, c1, 2));
+  s0 = __fadd_rn(s0, __shfl_xor_sync(FV_FULL, s0, 1));
+  s1 = __fadd_rn(s1, __shfl_xor_sync(FV_FULL, s1, 1));
+  const float s = __fadd_rn(s0, s1);
+  return IS_L2 ? s : -s;
+}
+
+// Who computes a run of distances.  NW = 1: the warp itself.  NW > 1: the block's NW warps together; warp 0 runs the
+// search and posts each run (team_eval), the others wait for it in team_serve.  A single search is a chain of memory
+// trips, and when there are fewer searches than warps the rest of the SM can only help by shortening each link.
+struct TeamJob {
+  const float* from;  // shared memory: the vector the distances are from
+  int count;          // rows; -1: no more work
+};
+template <int NW>
+struct Team {
+  const float* data;
+  int pd;
+  uint32_t* ids;  // shared memory: the rows of a run ...
+  float* out;     // ... and their distances
+  TeamJob* job;   // NW > 1
+};
+template <bool IS_L2, int LPR>
+__device__ __forceinline__ void team_rows(const float* __restrict__ data, int pd, const uint32_t* ids, float* out,
+                                          const float* from, int count, int first, int step) {
+  const int sub = lane_id() & (LPR - 1), g = lane_id() / LPR;
+  for (int i0 = first; i0 < count; i0 += step) {
+    const int i = i0 + g;
+    const float* row = data + size_t(ids[min(i, count - 1)]) * pd;  // (rows past the end: the last one again)
+    const float d = group_distance<IS_L2, LPR>(from, row, pd);
+    if (sub == 0 && i < count) out[i] = d;
+  }
+}
+template <bool IS_L2, int NW>
+__device__ __forceinline__ void team_eval(const Team<NW>& t, const float* from, int count) {
+  __syncwarp();
+  if (NW == 1) {
+    team_rows<IS_L2, 4>(t.data, t.pd, t.ids, t.out, from, count, 0, 8);
+    __syncwarp();
+  } else if (count <= 4) {  // one step of this warp: not worth the two barriers
+    team_rows<IS_L2, 8>(t.data, t.pd, t.ids, t.out, from, count, 0, 4);
+    __syncwarp();
+  } else {
+    if (lane_id() == 0) {
+      t.job->from = from;
+      t.job->count = count;
+    }
+    __syncthreads();
+    team_rows<IS_L2, 8>(t.data, t.pd, t.ids, t.out, from, count, 0, 4 * NW);
+    __syncthreads();
+  }
+}
+template <bool IS_L2, int NW>
+__device__ __forceinline__ void team_serve(const Team<NW>& t) {  // warps 1 .. NW - 1
+  for (;;) {
+    __syncthreads();
+    const int count = t.job->count;
+    if (count < 0) return;
+    team_rows<IS_L2, 8>(t.data, t.pd, t.ids, t.out, t.job->from, count, 4 * int(threadIdx.x >> 5), 4 * NW);
+    __syncthreads();
+  }
+}
+template <int NW>
+__device__ __forceinline__ void team_dismiss(const Team<NW>& t) {
+  if (NW > 1) {
+    __syncwarp();
+    if (lane_id() == 0) t.job->count = -1;
+    __syncthreads();
+  }
+}
+
+// The greedy descent through layers top .. bottom + 1 (hnsw.rs:254-268, :334-347).  `rows(c, layer)` is a node's link
+// block on a layer (count, then at most `width` ids).
+template <bool IS_L2, int NW, class Rows>
+__device__ __forceinline__ void greedy_descent(const Team<NW>& t, size_t n, Rows rows, int width, const float* sq, int top,
+                                               int bottom, uint32_t& cur, float& curd, unsigned long long& n_dist,
+                                               unsigned long long& n_exp) {
+  const int lane = lane_id();
+  for (int layer = top; layer > bottom; --layer) {
+    bool changed = true;
+    while (changed) {
+      changed = false;
+      const uint32_t* row = rows(cur, layer);
+      const int cnt = min(int(row[0]), width);
+      n_exp += 1;
+      for (int c0 = 0; c0 < cnt; c0 += 32) {
+        const int i = c0 + lane, m = min(32, cnt - c0);
+        uint32_t x = 0;
+        bool on = i < cnt;
+        if (on) {
+          x = row[1 + i];
+          on = FV_IDX_OK(x, n, 4);
+        }
         __syncwarp();
-        for (int t = lane; t < ntied; t += 32)
-          if (tied[t] == tmin) tied[t] = tied[ntied - 1];
+        if (i < cnt) t.ids[lane] = on ? x : cur;
+        team_eval<IS_L2, NW>(t, sq, m);
+        const float d = on ? t.out[lane] : INFINITY;
+        n_dist += __popc(__ballot_sync(FV_FULL, on));
+        // first minimum of the chunk, taken only if strictly below the current distance
+        const unsigned better = __ballot_sync(FV_FULL, on && d < curd);
+        if (better) {
+          float md = d < curd ? d : INFINITY;
+          for (int o = 16; o > 0; o >>= 1) md = fminf(md, __shfl_xor_sync(FV_FULL, md, o));
+          const unsigned at = __ballot_sync(FV_FULL, on && d == md);
+          cur = __shfl_sync(FV_FULL, x, __ffs(at) - 1);
+          curd = md;
+          changed = true;
+        }
+      }
+    }
+  }
+}
+
+// search_layer (hnsw.rs:179-226) from the entries of `best`, all of them not expanded and already in `seen`.
+// `rows(c)` is the link block of node c on the searched layer (count, then at most `width` ids; width + 1 words are
+// readable).  The reference's pair of heaps is ONE sorted list of ef entries with an "expanded" bit each: a candidate
+// that has been evicted from `best` can only be popped after every entry of `best` has been expanded, and then it
+// trips the stop test (hnsw.rs:203-205) unless its distance ties the current worst exactly -- see TIED_CAP.
+// The unvisited neighbours of the expanded node are offered to the list in stored order, so the admission test
+// (hnsw.rs:214) sees the same evolving bound as the sequential loop.  A search that fills more than half of the
+// visited set's second part stops with `over`.  n_dist and n_exp grow by the distances evaluated and the nodes
+// expanded.
+template <bool IS_L2, int R, int NW, class Rows>
+__device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows rows, int width, const float* sq, Beam<R>& best,
+                                            uint32_t* tied, VisitSet& seen, bool& over, bool& tie_lost,
+                                            unsigned long long& n_dist, unsigned long long& n_exp) {
+  const int lane = lane_id();
+  int ntied = 0;  // pushed-out entries still tied with the worst kept distance
+  over = false;
+  u64 bound = best.last();
+  for (;;) {
+    u64 ck = 0;
+    int pos = best.first_open(ck);
+    uint32_t c = beam_id(ck);
+    if (ntied > 0) {
+      // the smallest id among the tied entries; it goes first if the beam has nothing open or only a larger key
+      uint32_t tmin = 0xFFFFFFFFu;
+      for (int i = lane; i < ntied; i += 32) tmin = min(tmin, tied[i]);
+      tmin = __reduce_min_sync(FV_FULL, tmin);
+      const u64 tkey = (bound & 0xFFFFFFFF00000000ull) | (u64(tmin) << 1);
+      if (pos < 0 || tkey < ck) {
+        __syncwarp();
+        for (int i = lane; i < ntied; i += 32)
+          if (tied[i] == tmin) tied[i] = tied[ntied - 1];  // ids are unique: one match
         __syncwarp();
         ntied--;
         pos = -2;
@@ -120,12 +515,8 @@ __device__ __forceinline__ void beam_search(const float* __restrict__ data, int 
     }
     if (pos == -1) break;
     if (pos >= 0) {
-      const u64 ck = best[pos];
-      __syncwarp();
-      if (lane == 0) best[pos] = ck | 1ull;
-      __syncwarp();
-      cursor = pos + 1;
-      c = beam_id(ck);
+      best.mark(pos);
+      if (pos == best.last_pos()) bound |= 1ull;
     }
     if (!FV_IDX_OK(c, n, 1)) break;
     const uint32_t* row = rows(c);
@@ -134,63 +525,52 @@ __device__ __forceinline__ void beam_search(const float* __restrict__ data, int 
     const uint32_t x_first = lane < width ? __ldg(row + 1 + lane) : 0u;
     const int cnt = min(int(__ldg(row)), width);
     n_exp += 1;
+    {
+      // the entry that is next in line now is expanded next unless a nearer one is found: its links are on their way
+      u64 nk = 0;
+      if (best.first_open(nk) >= 0) {
+        const uint32_t* nrow = rows(beam_id(nk));
+        if (lane * 32 <= width) asm volatile("prefetch.global.L1 [%0];" ::"l"(nrow + min(lane * 32, width)));
+      }
+    }
     for (int c0 = 0; c0 < cnt; c0 += 32) {
       const int i = c0 + lane;
-      u64 key = FV_EMPTY_KEY;
-      bool fresh = false;
       uint32_t x = 0;
-      if (i < cnt) {
-        x = c0 == 0 ? x_first : __ldg(row + 1 + i);
-        fresh = FV_IDX_OK(x, n, 2) && visit(table, log2slots, x);
-      }
-      const int nfresh = __popc(__ballot_sync(FV_FULL, fresh));
-      visited += nfresh;
+      if (i < cnt) x = c0 == 0 ? x_first : __ldg(row + 1 + i);
+      const bool fresh = visit_warp(seen, i < cnt && FV_IDX_OK(x, n, 2), x);
+      const unsigned fmask = __ballot_sync(FV_FULL, fresh);
+      const int nfresh = __popc(fmask);
+      if (nfresh == 0) continue;
       n_dist += nfresh;
-      if (fresh) {
-        // all lines of the row are requested before the dependent FMA chains start, so the gather costs one
-        // memory round trip instead of one per unrolled group of loads
-        const char* rowp = reinterpret_cast<const char*>(data + size_t(x) * pd);
-        for (int b = 0; b < pd * 4; b += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(rowp + b));
-        key = beam_key(exact_distance<IS_L2>(sq, data + size_t(x) * pd, pd), x);
-      }
+      if (fresh) t.ids[__popc(fmask & ((1u << lane) - 1u))] = x;  // stored order
+      team_eval<IS_L2, NW>(t, sq, nfresh);
       // offered in stored order: admitted while the list is not full, or on a strictly smaller distance
-      u64 bound = best[ef - 1];
-      unsigned pending = __ballot_sync(FV_FULL, fresh);
+      const u64 key = lane < nfresh ? beam_key(t.out[lane], t.ids[lane]) : FV_EMPTY_KEY;
+      __syncwarp();
+      const uint32_t hi = uint32_t(key >> 32);
+      unsigned pending = __ballot_sync(FV_FULL, lane < nfresh && hi < uint32_t(bound >> 32));
       while (pending) {
         const int src = __ffs(pending) - 1;
-        pending &= pending - 1;
-        const u64 kk = __shfl_sync(FV_FULL, key, src);
-        if ((kk >> 32) < (bound >> 32)) {
-          int below = 0;
-          for (int e0 = 0; e0 < filled; e0 += 32) {
-            const int e = e0 + lane;
-            below += __popc(__ballot_sync(FV_FULL, e < filled && best[e] < kk));
-          }
-          __syncwarp();
-          const bool was_full = filled == ef;
-          warp_list_insert(best, ef, kk);
-          if (filled < ef) filled++;
-          if (below < cursor) cursor = below;
-          const u64 pushed = bound;
-          bound = best[ef - 1];
-          if (was_full) {
-            if ((bound >> 32) < (pushed >> 32)) {
-              ntied = 0;
-            } else if (!(pushed & 1ull)) {
-              if (ntied < TIED_CAP) {
-                __syncwarp();
-                if (lane == 0) tied[ntied] = beam_id(pushed);
-                __syncwarp();
-                ntied++;
-              } else {
-                tie_lost = true;
-              }
-            }
+        const u64 pushed = bound;  // the entry that falls off the end, if the beam is full
+        best.insert(__shfl_sync(FV_FULL, key, src));
+        bound = best.last();
+        pending = __ballot_sync(FV_FULL, lane > src && lane < nfresh && hi < uint32_t(bound >> 32));
+        // once the worst distance has gone down, nothing pushed out so far can tie with it any more
+        const bool lower = uint32_t(bound >> 32) < uint32_t(pushed >> 32);
+        ntied = lower ? 0 : ntied;
+        if (!lower && !(pushed & 1ull)) {  // (an unused entry reads "expanded")
+          if (ntied < TIED_CAP) {
+            __syncwarp();
+            if (lane == 0) tied[ntied] = beam_id(pushed);
+            __syncwarp();
+            ntied++;
+          } else {
+            tie_lost = true;
           }
         }
       }
     }
-    if (visited > (slots >> 1)) {
+    if (visit_overflow(seen)) {
       over = true;
       break;
     }

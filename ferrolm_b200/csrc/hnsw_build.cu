@@ -49,60 +49,113 @@ __device__ __forceinline__ uint32_t head_slot(const BuildDev& g, uint32_t x, int
   return layer == 0 ? x : g.n + g.up_blk[x] + uint32_t(layer - 1);
 }
 
+// rows of one run of distances: what a search's beam can hold, up to SELECT_RUN
+static constexpr int SELECT_RUN = 512;
+__host__ __device__ __forceinline__ int run_rows(int ncand) { return ncand < SELECT_RUN ? (ncand + 31) & ~31 : SELECT_RUN; }
+
 // select (hnsw.rs:230-242): from candidates sorted nearest first (keys: order bits of the distance above, id at
-// `id_shift` below), keep those farther from every kept one than from the base, up to cap.  `sc` stages the
-// candidate's row.  Returns the number kept (ids in sel[]).
-template <bool IS_L2>
-__device__ __forceinline__ int select_links(const BuildDev& g, const u64* cand, int ncand, int id_shift, int cap,
-                                            float* sc, uint32_t* sel) {
+// `id_shift` below), keep those farther from every kept one than from the base, up to cap.  Worked from the kept
+// side: the first candidate nobody has ruled out is kept, and its distances to all the ones still standing behind it
+// (one run, team_eval) rule out those nearer to it than to the base.  A distance has the same bits from either end, so
+// the choice is the reference's.  (Candidate by candidate, as it was, each of up to ef candidates took a load of its
+// row and a run of at most 32 distances: 200 dependent steps where there are now as many as links kept.)
+// `cand`, `gone` (a bit per candidate) and `sc` (the kept row) are shared memory of the warp; the runs of `t` hold
+// run_rows(ncand) rows.
+// Returns the number kept (ids in sel[]).
+template <bool IS_L2, int NW>
+__device__ __forceinline__ int select_links(const BuildDev& g, const Team<NW>& t, const u64* cand, int ncand, int id_shift,
+                                            int cap, float* sc, uint32_t* gone, uint32_t* sel) {
   const int lane = lane_id();
-  int nsel = 0;
-  for (int i = 0; i < ncand && nsel < cap; ++i) {
-    const u64 ck = cand[i];
-    const uint32_t cid = uint32_t((ck & 0xFFFFFFFFull) >> id_shift);
-    const float cd = order_bits_to_float(uint32_t(ck >> 32));
-    if (!FV_IDX_OK(cid, g.n, 3)) continue;
-    bool bad = false;
-    if (nsel > 0) {
+  for (int i = lane; i * 32 < ncand; i += 32) gone[i] = ncand - i * 32 >= 32 ? 0u : ~0u << (ncand - i * 32);
+  __syncwarp();
+  int nsel = 0, word = 0;
+  while (nsel < cap) {
+    while (word * 32 < ncand && gone[word] == 0xFFFFFFFFu) ++word;  // the same in every lane
+    if (word * 32 >= ncand) break;
+    const int i = word * 32 + __ffs(~gone[word]) - 1;
+    const uint32_t cid = uint32_t((cand[i] & 0xFFFFFFFFull) >> id_shift);
+    __syncwarp();
+    if (lane == 0) gone[word] |= 1u << (i & 31);
+    if (!FV_IDX_OK(cid, g.n, 3)) {
       __syncwarp();
-      for (int c = lane; c < g.pd; c += 32) sc[c] = g.data[size_t(cid) * g.pd + c];
-      __syncwarp();
-      for (int s0 = 0; s0 < nsel && !bad; s0 += 32) {
-        const int s = s0 + lane;
-        bool b = false;
-        if (s < nsel) b = !(exact_distance<IS_L2>(sc, g.data + size_t(sel[s]) * g.pd, g.pd) > cd);
-        bad = __any_sync(FV_FULL, b);
+      continue;
+    }
+    if (lane == 0) sel[nsel] = cid;
+    nsel++;
+    __syncwarp();
+    if (nsel == cap) break;
+    for (int c = lane; c < g.pd; c += 32) sc[c] = g.data[size_t(cid) * g.pd + c];
+    // the candidates still standing, in order, up to SELECT_RUN places at a time
+    for (int w0 = word; w0 * 32 < ncand; w0 += SELECT_RUN / 32) {
+      const int w1 = min(w0 + SELECT_RUN / 32, (ncand + 31) / 32);
+      int m = 0;
+      for (int w = w0; w < w1; ++w) {
+        const unsigned left = ~gone[w];
+        if ((left >> lane) & 1u) {
+          const uint32_t x = uint32_t((cand[w * 32 + lane] & 0xFFFFFFFFull) >> id_shift);
+          t.ids[m + __popc(left & ((1u << lane) - 1u))] = x < g.n ? x : cid;
+        }
+        m += __popc(left);
+      }
+      if (m == 0) continue;
+      team_eval<IS_L2, NW>(t, sc, m);
+      m = 0;
+      for (int w = w0; w < w1; ++w) {
+        const unsigned left = ~gone[w];
+        bool out = false;
+        if ((left >> lane) & 1u) {
+          const float cd = order_bits_to_float(uint32_t(cand[w * 32 + lane] >> 32));
+          out = !(t.out[m + __popc(left & ((1u << lane) - 1u))] > cd);
+        }
+        const unsigned om = __ballot_sync(FV_FULL, out);
+        m += __popc(left);
+        __syncwarp();
+        if (lane == 0) gone[w] |= om;
+        __syncwarp();
       }
     }
-    if (!bad) {
-      __syncwarp();
-      if (lane == 0) sel[nsel] = cid;
-      nsel++;
-      __syncwarp();
-    }
   }
+  __syncwarp();
   return nsel;
 }
 
+// Shared memory of one insertion: the node's row and a kept candidate's, the visited set's first part, the tie list,
+// a run of rows and
+// their distances, the chosen links, the bits of select_links, the team's job, the
+// found list.
+__host__ __device__ __forceinline__ size_t insert_smem(int pd, int m0, int ef, int sbits) {
+  const size_t run = size_t(run_rows(ef));
+  return size_t(pd) * 8 + (size_t(4) << sbits) + (TIED_CAP + 2 * run + ((m0 + 3) & ~3) + 128) * 4 + sizeof(TeamJob) +
+         ((size_t(ef) * 8 + 15) & ~size_t(15));
+}
+
 // flags: [0] visited-table overflows, [1] tie lists that overflowed, [2] edges that did not fit
-template <bool IS_L2>
+template <bool IS_L2, int R, int NW>
 __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
-    hnsw_insert_kernel(BuildDev g, uint32_t lo, uint32_t hi, uint32_t ep, int top, int ef, int log2slots,
+    hnsw_insert_kernel(BuildDev g, uint32_t lo, uint32_t hi, uint32_t ep, int top, int ef, int sbits, int log2slots,
                        uint32_t* __restrict__ tables, Edge* __restrict__ edges, uint32_t* __restrict__ edge_cnt,
                        uint32_t* __restrict__ next_node, uint32_t edge_cap, uint32_t* __restrict__ head,
                        unsigned long long* __restrict__ flags) {
-  unsigned char* smem_raw = dyn_smem();
-  const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t list_bytes = (size_t(ef) * 8 + 15) & ~size_t(15);
-  const size_t per_warp = size_t(g.pd) * 8 + list_bytes + TIED_CAP * 4 + size_t(g.m0) * 4;
-  unsigned char* mine = smem_raw + size_t(w) * per_warp;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int searcher = NW == 1 ? w : 0, per_block = NW == 1 ? int(blockDim.x >> 5) : 1;
+  const int run = run_rows(ef);
+  unsigned char* mine = dyn_smem() + size_t(searcher) * insert_smem(g.pd, g.m0, ef, sbits);
   float* sq = reinterpret_cast<float*>(mine);
   float* sc = sq + g.pd;
-  u64* best = reinterpret_cast<u64*>(mine + size_t(g.pd) * 8);
-  uint32_t* tied = reinterpret_cast<uint32_t*>(mine + size_t(g.pd) * 8 + list_bytes);
-  uint32_t* sel = tied + TIED_CAP;
-  const uint32_t gw = blockIdx.x * W + w;
-  uint32_t* table = tables + (size_t(gw) << log2slots);
+  uint32_t* small = reinterpret_cast<uint32_t*>(sc + g.pd);
+  uint32_t* tied = small + (size_t(1) << sbits);
+  uint32_t* sel = tied + TIED_CAP + 2 * run;
+  uint32_t* gone = sel + ((g.m0 + 3) & ~3);
+  Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + run),
+                reinterpret_cast<TeamJob*>(gone + 128)};
+  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + sizeof(TeamJob));
+  if (NW > 1 && w > 0) {
+    team_serve<IS_L2, NW>(team);
+    return;
+  }
+  const size_t gw = size_t(blockIdx.x) * per_block + searcher;
+  VisitSet seen;
+  visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
 
   // nodes are drawn from a counter: a search takes anything from a few to a few hundred expansions, and which warp
   // inserts which node changes nothing in the result
@@ -114,54 +167,36 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
     const int level = g.levels[id];
     __syncwarp();
     for (int c = lane; c < g.pd; c += 32) sq[c] = g.data[size_t(id) * g.pd + c];
-    warp_list_init(best, ef);
 
     // greedy descent through the layers above the node's own (hnsw.rs:254-268)
     uint32_t cur = ep;
-    float curd = exact_distance<IS_L2>(sq, g.data + size_t(cur) * g.pd, g.pd);
-    for (int layer = top; layer > level; --layer) {
-      bool changed = true;
-      while (changed) {
-        changed = false;
-        const uint32_t* row = link_row(g, cur, layer);
-        const int cnt = min(int(row[0]), g.m);
-        for (int c0 = 0; c0 < cnt; c0 += 32) {
-          const int i = c0 + lane;
-          uint32_t x = 0;
-          float d = INFINITY;
-          const bool on = i < cnt && FV_IDX_OK(row[1 + i], g.n, 4);
-          if (on) {
-            x = row[1 + i];
-            d = exact_distance<IS_L2>(sq, g.data + size_t(x) * g.pd, g.pd);
-          }
-          const unsigned better = __ballot_sync(FV_FULL, on && d < curd);
-          if (better) {
-            float md = d < curd ? d : INFINITY;
-            for (int o = 16; o > 0; o >>= 1) md = fminf(md, __shfl_xor_sync(FV_FULL, md, o));
-            const unsigned at = __ballot_sync(FV_FULL, on && d == md);
-            cur = __shfl_sync(FV_FULL, x, __ffs(at) - 1);
-            curd = md;
-            changed = true;
-          }
-        }
-      }
-    }
+    if (lane == 0) team.ids[0] = cur;
+    team_eval<IS_L2, NW>(team, sq, 1);
+    float curd = team.out[0];
+    unsigned long long n_dist = 0, n_exp = 0;  // (not reported by the build)
+    greedy_descent<IS_L2, NW>(team, g.n, [&](uint32_t x, int layer) { return (const uint32_t*)link_row(g, x, layer); }, g.m,
+                              sq, top, level, cur, curd, n_dist, n_exp);
 
-    warp_list_insert(best, ef, beam_key(curd, cur));
-    int filled = 1;
+    Beam<R> best;
+    best.init(ef, list);
+    best.insert(beam_key(curd, cur));
     bool tie_lost = false;
     for (int layer = min(level, top); layer >= 0; --layer) {
+      // search_layer starts from everything the layer above found (hnsw.rs:181-193), none of it expanded
+      visit_clear(seen, lane, 32);
+      __syncwarp();
+      best.reopen([&](bool on, uint32_t x) { visit_warp(seen, on, x); });
       bool over = false;
-      unsigned long long n_dist = 0, n_exp = 0;  // (not reported by the build)
-      beam_search<IS_L2>(g.data, g.pd, g.n, [&](uint32_t c) { return (const uint32_t*)link_row(g, c, layer); },
-                         layer == 0 ? g.m0 : g.m, sq, best, ef, tied, table, log2slots, filled, over, tie_lost, n_dist,
-                         n_exp);
+      beam_search<IS_L2, R, NW>(team, g.n, [&](uint32_t c) { return (const uint32_t*)link_row(g, c, layer); },
+                                layer == 0 ? g.m0 : g.m, sq, best, tied, seen, over, tie_lost, n_dist, n_exp);
       if (over) {
         if (lane == 0) atomicAdd(flags, 1ull);
         break;
       }
+      const int filled = best.filled();
+      if (R > 0) best.each([&](int e, u64 b) { list[e] = b; });
       const int cap = layer == 0 ? g.m0 : g.m;
-      const int nsel = select_links<IS_L2>(g, best, filled, 1, cap, sc, sel);
+      const int nsel = select_links<IS_L2, NW>(g, team, list, filled, 1, cap, sc, gone, sel);
       // the node's own list: it is new, so add_links(id, layer, chosen) finds it empty (hnsw.rs:277)
       uint32_t* own = link_row(g, id, layer);
       for (int i = lane; i < nsel; i += 32) own[1 + i] = sel[i];
@@ -189,6 +224,14 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
     }
     if (tie_lost && lane == 0) atomicAdd(flags + 1, 1ull);
   }
+  team_dismiss(team);
+}
+
+// Shared memory of one chain: the target's row and a kept candidate's, two arrays of up to m0 + 1 keys, the list, the
+// chosen links, the sources as chained and sorted, the bits of select_links, a run of rows and their distances.
+__host__ __device__ __forceinline__ size_t link_smem(int pd, int m0) {
+  const size_t nc = size_t(m0) + 1, keys_bytes = (nc * 8 + 15) & ~size_t(15);
+  return (size_t(pd) * 8 + 2 * keys_bytes + (nc + m0 + 2 * SRC_CAP + 8 + 2 * run_rows(m0 + 1)) * 4 + 15) & ~size_t(15);
 }
 
 // add_links(target, layer, [source]) (hnsw.rs:294-320) for every edge of the batch.  The warp whose edge was the
@@ -201,8 +244,7 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
   const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cap_max = g.m0, nc = cap_max + 1;
   const size_t keys_bytes = (size_t(nc) * 8 + 15) & ~size_t(15);
-  const size_t per_warp = size_t(g.pd) * 8 + 2 * keys_bytes + size_t(nc + cap_max + 2 * SRC_CAP + 1) * 4;
-  unsigned char* mine = smem_raw + size_t(w) * ((per_warp + 15) & ~size_t(15));
+  unsigned char* mine = smem_raw + size_t(w) * link_smem(g.pd, g.m0);
   float* sb = reinterpret_cast<float*>(mine);
   float* sc = sb + g.pd;
   u64* keys = reinterpret_cast<u64*>(mine + size_t(g.pd) * 8);
@@ -211,6 +253,8 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
   uint32_t* sel = ids + nc;
   uint32_t* srcs = sel + cap_max;
   uint32_t* srcs_sorted = srcs + SRC_CAP;
+  uint32_t* gone = srcs_sorted + SRC_CAP;
+  const Team<1> team{g.data, g.pd, gone + 8, reinterpret_cast<float*>(gone + 8 + run_rows(nc)), nullptr};
   const uint32_t count = min(*edge_cnt, edge_cap);
   const uint32_t gw = blockIdx.x * W + w, total_warps = gridDim.x * W;
 
@@ -285,8 +329,9 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
       __syncwarp();
       if (cnt > cap) {
         // distances from the base, sorted by (distance, id), chosen again (hnsw.rs:307-318)
-        for (int i = lane; i < cnt; i += 32)
-          keys[i] = make_key(exact_distance<IS_L2>(sb, g.data + size_t(ids[i]) * g.pd, g.pd), ids[i]);
+        for (int i = lane; i < cnt; i += 32) team.ids[i] = ids[i];
+        team_eval<IS_L2, 1>(team, sb, cnt);
+        for (int i = lane; i < cnt; i += 32) keys[i] = make_key(team.out[i], ids[i]);
         __syncwarp();
         for (int i = lane; i < cnt; i += 32) {
           const u64 v = keys[i];
@@ -295,7 +340,7 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
           sorted[r] = v;
         }
         __syncwarp();
-        const int nsel = select_links<IS_L2>(g, sorted, cnt, 0, cap, sc, sel);
+        const int nsel = select_links<IS_L2, 1>(g, team, sorted, cnt, 0, cap, sc, gone, sel);
         for (int i = lane; i < nsel; i += 32) {
           ids[i] = sel[i];
           row[1 + i] = sel[i];
@@ -325,6 +370,18 @@ static size_t next_batch(const std::vector<uint8_t>& levels, size_t inserted, si
   for (size_t j = 1; j < b; j++)
     if (levels[inserted + j] > top) return j;
   return b;
+}
+
+typedef void (*InsertKernel)(BuildDev, uint32_t, uint32_t, uint32_t, int, int, int, int, uint32_t*, Edge*, uint32_t*, uint32_t*,
+                             uint32_t, uint32_t*, unsigned long long*);
+template <int NW>
+static InsertKernel pick_insert(bool is_l2, int R) {
+  switch (R) {
+    case 2: return is_l2 ? hnsw_insert_kernel<true, 2, NW> : hnsw_insert_kernel<false, 2, NW>;
+    case 4: return is_l2 ? hnsw_insert_kernel<true, 4, NW> : hnsw_insert_kernel<false, 4, NW>;
+    case 8: return is_l2 ? hnsw_insert_kernel<true, 8, NW> : hnsw_insert_kernel<false, 8, NW>;
+    default: return is_l2 ? hnsw_insert_kernel<true, 0, NW> : hnsw_insert_kernel<false, 0, NW>;
+  }
 }
 
 static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divisor) {
@@ -381,27 +438,34 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
   g.m0 = int(m0);
   g.n = uint32_t(n);
 
-  // launch shapes: shared memory per warp, warps per block, resident warps
-  const size_t list_bytes = (ef * 8 + 15) & ~size_t(15);
-  const size_t ins_warp = size_t(pd) * 8 + list_bytes + TIED_CAP * 4 + m0 * 4;
-  const size_t nc = m0 + 1;
-  const size_t keys_bytes = (nc * 8 + 15) & ~size_t(15);
-  const size_t link_warp = ((size_t(pd) * 8 + 2 * keys_bytes + (nc + m0 + 2 * SRC_CAP + 1) * 4) + 15) & ~size_t(15);
+  // launch shapes: shared memory per searcher, searchers per block, resident blocks
+  const int R = ef <= 64 ? 2 : ef <= 128 ? 4 : ef <= 256 ? 8 : 0;
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
-  int W = 8;
-  while (W > 1 && std::max(ins_warp, link_warp) * W > budget / BUILD_BLOCKS_PER_SM) W >>= 1;
-  if (std::max(ins_warp, link_warp) * W > budget) return fail(FV_ERR_UNSUPPORTED, "dimension and ef_construction too large for shared memory");
+  const bool is_l2 = h->metric == FV_L2;
+  const size_t link_warp = link_smem(pd, int(m0));
+  int sbits = visit_sbits(int(ef), 11), team_sbits = visit_sbits(int(ef), 13), W = 8, LW = 8;
+  auto ins_bytes = [&](int bits) { return insert_smem(pd, int(m0), int(ef), bits); };
+  while (W > 1 && ins_bytes(sbits) * W > budget / BUILD_BLOCKS_PER_SM) W >>= 1;
+  while (LW > 1 && link_warp * LW > budget / BUILD_BLOCKS_PER_SM) LW >>= 1;
+  while (sbits > 7 && ins_bytes(sbits) * W > ctx->smem_optin) sbits--;
+  while (team_sbits > 7 && ins_bytes(team_sbits) > ctx->smem_optin) team_sbits--;
+  if (std::max(ins_bytes(sbits) * W, link_warp * LW) > ctx->smem_optin)
+    return fail(FV_ERR_UNSUPPORTED, "dimension and ef_construction too large for shared memory");
   const size_t resident_blocks = size_t(ctx->sm_count) * BUILD_BLOCKS_PER_SM;
-  const size_t ins_blocks_max = std::min<size_t>(resident_blocks, (widest + W - 1) / W);
-  auto ins = h->metric == FV_L2 ? hnsw_insert_kernel<true> : hnsw_insert_kernel<false>;
-  auto lnk = h->metric == FV_L2 ? hnsw_link_kernel<true> : hnsw_link_kernel<false>;
-  if (ins_warp * W > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(ins, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ins_warp * W)));
-  if (link_warp * W > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(lnk, cudaFuncAttributeMaxDynamicSharedMemorySize, int(link_warp * W)));
+  const size_t searchers_max = std::min(resident_blocks * W, std::max<size_t>(widest, 1));  // (a team is one searcher)
+  InsertKernel ins = pick_insert<1>(is_l2, R), ins_team = pick_insert<TEAM_WARPS>(is_l2, R);
+  auto lnk = is_l2 ? hnsw_link_kernel<true> : hnsw_link_kernel<false>;
+  auto allow = [&](auto kern, size_t bytes) {
+    return bytes > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) : cudaSuccess;
+  };
+  FV_CUDA(allow(ins, ins_bytes(sbits) * W));
+  FV_CUDA(allow(ins_team, ins_bytes(team_sbits)));
+  FV_CUDA(allow(lnk, link_warp * LW));
 
   int log2slots = 11;
   while ((size_t(1) << log2slots) < ef * 128 && log2slots < 24) log2slots++;
   for (int attempt = 0; attempt < 3; ++attempt, log2slots += 2) {
-    FV_TRY(d_tables.reserve((ins_blocks_max * W << log2slots) * 4 + 16));
+    FV_TRY(d_tables.reserve((((searchers_max + W - 1) / W * W) << log2slots) * 4 + 16));
     FV_CUDA(cudaMemsetAsync(h->d_links0.p, 0, h->links0.size() * 4, st));
     FV_CUDA(cudaMemsetAsync(d_up.p, 0, nblk * (m + 1) * 4, st));
     FV_CUDA(cudaMemsetAsync(d_head.p, 0xFF, (n + nblk) * 4, st));
@@ -413,16 +477,19 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
     while (inserted < n) {
       const size_t b = next_batch(h->levels, inserted, top, max_batch, divisor);
       FV_CUDA(cudaMemsetAsync(d_edge_cnt, 0, 8, st));  // and the node counter
-      const size_t ins_blocks = std::min<size_t>(ins_blocks_max, (b + W - 1) / W);
-      ins<<<unsigned(ins_blocks), W * 32, ins_warp * W, st>>>(g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top),
-                                                               int(ef), log2slots, d_tables.as<uint32_t>(),
-                                                               d_edges.as<Edge>(), d_edge_cnt, d_next_node, uint32_t(edge_cap),
-                                                               d_head.as<uint32_t>(), d_flags);
+      if (b <= size_t(ctx->sm_count) * TEAM_SEARCHES_PER_SM)
+        ins_team<<<unsigned(std::min(b, resident_blocks)), TEAM_WARPS * 32, ins_bytes(team_sbits), st>>>(
+            g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), team_sbits, log2slots, d_tables.as<uint32_t>(),
+            d_edges.as<Edge>(), d_edge_cnt, d_next_node, uint32_t(edge_cap), d_head.as<uint32_t>(), d_flags);
+      else
+        ins<<<unsigned(std::min(resident_blocks, (b + W - 1) / W)), W * 32, ins_bytes(sbits) * W, st>>>(
+            g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), sbits, log2slots, d_tables.as<uint32_t>(),
+            d_edges.as<Edge>(), d_edge_cnt, d_next_node, uint32_t(edge_cap), d_head.as<uint32_t>(), d_flags);
       FV_CUDA(cudaGetLastError());
       size_t e_max = 0;
       for (size_t j = 0; j < b; j++) e_max += m0 + std::min<size_t>(h->levels[inserted + j], top) * m;
-      const size_t lnk_blocks = std::max<size_t>(1, std::min<size_t>(resident_blocks, (e_max + W - 1) / W));
-      lnk<<<unsigned(lnk_blocks), W * 32, link_warp * W, st>>>(g, d_edges.as<Edge>(), d_edge_cnt, uint32_t(edge_cap),
+      const size_t lnk_blocks = std::max<size_t>(1, std::min<size_t>(resident_blocks, (e_max + LW - 1) / LW));
+      lnk<<<unsigned(lnk_blocks), LW * 32, link_warp * LW, st>>>(g, d_edges.as<Edge>(), d_edge_cnt, uint32_t(edge_cap),
                                                               d_head.as<uint32_t>());
       FV_CUDA(cudaGetLastError());
       ctx->stats.launches += 2;
