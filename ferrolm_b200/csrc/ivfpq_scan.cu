@@ -84,6 +84,11 @@ struct ScanArgs {
   // order bits (0xFFFFFFFF when they hold fewer than keep rows): an upper bound for the list-major passes.
   uint32_t row_budget;
   uint32_t* bound_out;
+  // Split mode (splits > 1, grid nq x splits): block (q, s) scans the probed lists s, s + splits, ... and leaves its
+  // best `keep` keys in parts[q][s]; the last block of a query to arrive (tickets[q], zero at launch) merges them.
+  int splits;
+  u64* parts;
+  uint32_t* tickets;
 };
 
 // The query's part of the lookup tables for a whole batch (ivfpq.rs:236-238 inner product, :241-251 L2 with
@@ -132,6 +137,24 @@ __device__ __forceinline__ float lut_entry(uint32_t w, uint32_t lut_s) {
   float t;
   asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(t) : "r"(addr), "n"(J * 1024));
   return t;
+}
+
+// CW words of a code, aligned to 4 * CW bytes
+template <int CW>
+__device__ __forceinline__ void load_code(const uint8_t* __restrict__ src, uint32_t* w) {
+  if (CW == 4) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+    w[0] = v.x;
+    w[1] = v.y;
+    w[2] = v.z;
+    w[3] = v.w;
+  } else if (CW == 2) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+    w[0] = v.x;
+    w[1] = v.y;
+  } else {
+    w[0] = __ldg(reinterpret_cast<const uint32_t*>(src));
+  }
 }
 
 // What follows the scan of a query, for both kernels: `cand` holds the query's best a.keep keys by (compressed
@@ -202,7 +225,11 @@ __device__ __forceinline__ void scan_tail(const ScanArgs& a, size_t q, const u64
   }
 }
 
-template <bool M16, int R>
+// CW: 32-bit words of a row's code that one load brings (0: single bytes, for m not a multiple of 4); M16: m is 16 and
+// the one load of four words is the whole code.  R rows per lane and step.  With a byte per load, as it was for every
+// m but 16, the loads of the codes took longer than the lookups: 1,000 queries, 16 probes of 390 rows, m = 48: 428 us,
+// 248 us with words.
+template <bool M16, int CW, int R>
 __global__ void __launch_bounds__(256, 4) ivfpq_scan_kernel(ScanArgs a) {
   unsigned char* smem_raw = dyn_smem();
   const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
@@ -272,7 +299,7 @@ __global__ void __launch_bounds__(256, 4) ivfpq_scan_kernel(ScanArgs a) {
   // the next probed cell this block scans (a list-sharded index skips the other shards' lists), or -1
   uint32_t budget_used = 0;  // bound mode: rows of the lists taken so far (the same in every thread)
   auto next_probe = [&](int p) {
-    for (++p; p < a.nprobe; ++p) {
+    for (p += a.splits; p < a.nprobe; p += a.splits) {
       const u64 c = a.cells[q * size_t(a.nprobe) + p];
       if (c == FV_EMPTY_KEY) return -1;
       if (a.shard_world > 1 && int(key_id(c) % uint32_t(a.shard_world)) != a.shard_rank) continue;
@@ -297,7 +324,7 @@ __global__ void __launch_bounds__(256, 4) ivfpq_scan_kernel(ScanArgs a) {
     }
   };
 
-  int p = next_probe(-1);
+  int p = next_probe(int(blockIdx.y) - a.splits);
   int cur = 0;  // which table the scan reads
   if (use_pre && p >= 0) {
     build_pre(lut0, key_id(a.cells[q * size_t(a.nprobe) + p]), tid, int(blockDim.x));
@@ -373,6 +400,24 @@ __global__ void __launch_bounds__(256, 4) ivfpq_scan_kernel(ScanArgs a) {
             FV_ADC_STEP(6) FV_ADC_STEP(7) FV_ADC_STEP(8) FV_ADC_STEP(9) FV_ADC_STEP(10) FV_ADC_STEP(11)
             FV_ADC_STEP(12) FV_ADC_STEP(13) FV_ADC_STEP(14) FV_ADC_STEP(15)
 #undef FV_ADC_STEP
+          } else if (CW > 0) {
+            for (int j0 = 0; j0 < a.m; j0 += 4 * CW) {
+#pragma unroll
+              for (int i = 0; i < R; ++i) {
+                const int r = min(r0 + i * 32 + lane, end - 1);  // (a lane past the end repeats the last row)
+                load_code<CW>(a.codes + (off + r) * size_t(a.m) + j0, cws[i]);
+              }
+              const uint32_t base_s = lut_s + uint32_t(j0) * 1024u;
+#define FV_ADC_STEP(J)                                                              \
+  _Pragma("unroll") for (int i = 0; i < R; ++i) d[i] = __fadd_rn(d[i], lut_entry<J>(cws[i][(J) >> 2], base_s));
+              FV_ADC_STEP(0) FV_ADC_STEP(1) FV_ADC_STEP(2) FV_ADC_STEP(3)
+              if (CW > 1) { FV_ADC_STEP(4) FV_ADC_STEP(5) FV_ADC_STEP(6) FV_ADC_STEP(7) }
+              if (CW > 2) {
+                FV_ADC_STEP(8) FV_ADC_STEP(9) FV_ADC_STEP(10) FV_ADC_STEP(11)
+                FV_ADC_STEP(12) FV_ADC_STEP(13) FV_ADC_STEP(14) FV_ADC_STEP(15)
+              }
+#undef FV_ADC_STEP
+            }
           } else {
 #pragma unroll
             for (int i = 0; i < R; ++i) {
@@ -421,6 +466,24 @@ __global__ void __launch_bounds__(256, 4) ivfpq_scan_kernel(ScanArgs a) {
   cnt_ub = compact();  // the best `keep` by (compressed distance, id), ascending, at the front of the buffer
   for (int e = cnt_ub + tid; e < a.keep; e += blockDim.x) lists[e] = FV_EMPTY_KEY;
   __syncthreads();
+  if (a.splits > 1) {
+    u64* mine = a.parts + (q * a.splits + blockIdx.y) * size_t(a.keep);
+    for (int e = tid; e < a.keep; e += blockDim.x) mine[e] = lists[e];
+    __threadfence();
+    __syncthreads();
+    __shared__ uint32_t arrived;
+    if (tid == 0) arrived = atomicAdd(a.tickets + q, 1u);
+    __syncthreads();
+    if (arrived != uint32_t(a.splits - 1)) return;
+    __threadfence();
+    const u64* all = a.parts + q * size_t(a.splits) * a.keep;
+    const int total = a.splits * a.keep;  // at most a.cap
+    int n = 32;
+    while (n < total) n <<= 1;
+    for (int e = tid; e < n; e += blockDim.x) lists[e] = e < total ? __ldcg(all + e) : FV_EMPTY_KEY;
+    __syncthreads();
+    block_sort(lists, n);
+  }
   scan_tail(a, q, lists, rerank, sq);
 }
 
@@ -1403,14 +1466,33 @@ __global__ void __launch_bounds__(128) rescore_kernel(RescoreArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------
-static int launch_block_scan(fv_ctx* ctx, const ScanArgs& a, size_t nblocks, bool use_pre) {
+// scratch slot 6 holds the parts of a split search
+static int launch_block_scan(fv_ctx* ctx, ScanArgs a, size_t nblocks, bool use_pre) {
   const size_t tab = size_t(a.m) * KSUB;
   const size_t smem = (2 * size_t(a.pd) + tab * (use_pre ? 2 : 1)) * sizeof(float) +
                       (size_t(a.cap) + size_t(a.keep) + size_t(a.k)) * sizeof(u64);
   if (smem + 256 > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "m, k * refine too large for shared memory");
-  auto kern = a.m == 16 ? ivfpq_scan_kernel<true, 2> : ivfpq_scan_kernel<false, 1>;
+  auto kern = a.m == 16       ? ivfpq_scan_kernel<true, 4, 2>
+              : a.m % 16 == 0 ? ivfpq_scan_kernel<false, 4, 2>
+              : a.m % 8 == 0  ? ivfpq_scan_kernel<false, 2, 2>
+              : a.m % 4 == 0  ? ivfpq_scan_kernel<false, 1, 2>
+                              : ivfpq_scan_kernel<false, 0, 1>;
+  // A batch that leaves SMs without a block: each query's lists are dealt to several blocks, as long as one block can
+  // sort what they leave (32 queries, 16 probes of 590 rows, m = 16: 89 us with a block per query, 35 us with 16).
+  a.splits = 1;
+  if (!a.row_budget && !a.qids) {
+    const size_t room = size_t(ctx->sm_count) * 4 / nblocks;
+    a.splits = int(std::max<size_t>(1, std::min({room, size_t(a.nprobe), size_t(a.cap / a.keep)})));
+  }
+  if (a.splits > 1) {
+    const size_t part_bytes = nblocks * size_t(a.splits) * a.keep * sizeof(u64);
+    FV_TRY(ctx->scratch[6].reserve(part_bytes + nblocks * sizeof(uint32_t)));
+    a.parts = ctx->scratch[6].as<u64>();
+    a.tickets = reinterpret_cast<uint32_t*>(ctx->scratch[6].as<unsigned char>() + part_bytes);
+    FV_CUDA(cudaMemsetAsync(a.tickets, 0, nblocks * sizeof(uint32_t), ctx->stream));
+  }
   if (smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  kern<<<unsigned(nblocks), 256, smem, ctx->stream>>>(a);
+  kern<<<dim3(unsigned(nblocks), unsigned(a.splits)), 256, smem, ctx->stream>>>(a);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   return FV_OK;
