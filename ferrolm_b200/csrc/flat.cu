@@ -308,21 +308,31 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
   if (need(QT, W) > budget) QT = 2;
   if (need(QT, W) > budget)
     return fail(FV_ERR_UNSUPPORTED, "dimension and k too large for the shared-memory budget of the scan");
-  // Long lists over few rows (the coarse quantizer: 64 of 1024 cells): keeping a sorted list per query costs more
-  // than the distances.  Write every key instead and let one block per query sort them.
-  if (L >= 32 && n <= 4096 && nq >= 64 && !d_query_ids) {
+  // Few rows and more than one result per query (the coarse quantizer: 16 of 256 cells, 64 of 1024): keeping a sorted
+  // list per query costs more than the distances, and whole queries are too few pieces of work to fill the GPU.  Write
+  // every key, split by rows down to one tile, and let a warp or a block per query select.  Measured against the lists
+  // (both launches): 1,000 queries, 16 of 256 cells x 384: 67 us against 205; 32 queries, 16 of 512 cells x 128: 15 us
+  // against 45; 10,000 queries, 64 of 1,024 cells x 128: 218 us, with the lists over 1,000.
+  // (not where the keys of a very large batch would take more than 1 GB that the lists do without)
+  if (L >= 2 && n > 0 && n <= 4096 && !d_query_ids && size_t(8) * (size_t(pd) * 4 + 8) <= budget &&
+      (L >= 32 || nq * n * sizeof(u64) <= size_t(1) << 30)) {
     int npow2 = 32;
     while (size_t(npow2) < n) npow2 <<= 1;
     FV_TRY(ctx->scratch[scratch_slot].reserve(nq * n * sizeof(u64)));
     u64* dense = ctx->scratch[scratch_slot].as<u64>();
     const int w4 = 4;
-    const size_t groups = (nq + size_t(QT) * w4 - 1) / (size_t(QT) * w4);
-    size_t S = std::max<size_t>(1, std::min<size_t>(n / 128, (size_t(ctx->sm_count) * 8 + groups - 1) / groups));
+    const size_t row_bytes = size_t(pd) * 4 + 8;
+    // two queries per warp where eight would leave SMs idle or pass the shared memory of a block
+    int DQ = 8;
+    const size_t most_splits = std::max<size_t>(1, n / 32);
+    if ((nq + 31) / 32 * most_splits < size_t(ctx->sm_count) * 4 || size_t(w4) * 8 * row_bytes > budget) DQ = 2;
+    const size_t groups = (nq + size_t(DQ) * w4 - 1) / (size_t(DQ) * w4);
+    size_t S = std::max<size_t>(1, std::min(most_splits, (size_t(ctx->sm_count) * 8 + groups - 1) / groups));
     size_t rps = ((n + S - 1) / S + 31) / 32 * 32;
     S = (n + rps - 1) / rps;
     const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(S));
-    const size_t smem = size_t(w4) * QT * (size_t(pd) * 4 + 8);
-    if (QT == 8)
+    const size_t smem = size_t(w4) * DQ * row_bytes;
+    if (DQ == 8)
       FV_TRY(launch_scan<8>(ctx, metric == FV_L2, grid, w4 * 32, smem, d_rows, n, pd, d_queries, q_stride, nullptr, nq, 1,
                             prefilter_inf, id_base, rps, nullptr, dense, n));
     else
