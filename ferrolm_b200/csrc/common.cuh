@@ -317,6 +317,104 @@ __device__ __forceinline__ float quad_distances(const float* sq, const float* __
   return d;
 }
 
+// The L best keys in a warp's registers (32 * KR places, L <= 32 * KR).
+template <int KR>
+struct TopList {  // ascending; the last of the L entries sits in the last place, the places before the first hold 0
+  u64 e[KR];
+  __device__ __forceinline__ void init(int L) {
+#pragma unroll
+    for (int r = 0; r < KR; ++r) e[r] = r * 32 + lane_id() < 32 * KR - L ? 0ull : FV_EMPTY_KEY;
+  }
+  __device__ __forceinline__ u64 last() const { return __shfl_sync(FV_FULL, e[KR - 1], 31); }
+  __device__ __forceinline__ void offer(u64 key, u64& bound) {  // a key per lane, FV_EMPTY_KEY for none
+    unsigned pending = __ballot_sync(FV_FULL, key < bound);
+    while (pending) {
+      const int src = __ffs(pending) - 1;
+      const u64 k = __shfl_sync(FV_FULL, key, src);
+#pragma unroll
+      for (int r = KR - 1; r >= 0; --r) {
+        u64 prev = __shfl_up_sync(FV_FULL, e[r], 1);
+        const u64 carry = r > 0 ? __shfl_sync(FV_FULL, e[r > 0 ? r - 1 : 0], 31) : 0ull;
+        if (lane_id() == 0) prev = carry;
+        if (!(e[r] < k)) e[r] = prev < k ? k : prev;
+      }
+      bound = last();
+      pending = __ballot_sync(FV_FULL, lane_id() > src && key < bound);
+    }
+  }
+};
+
+// ---- distances of a run of gathered rows, by LPR lanes per row (32 / LPR rows at a time).  A lane owns 8 / LPR of
+// the reference's eight chains (src/kernels.rs:200-231) and the lane sums are added in its pairwise order, so the
+// bits are exact_distance's.  With one row per lane every load touches as many lines as there are rows, and a short
+// run (the ten unvisited links of a graph node) leaves most lanes idle.  What bounds such a run is its trips to memory
+// (about 700 cycles each to L2), so a lane requests U = 16 pieces (128 dimensions of its row) before it works on the
+// first; what is left of the row goes in halves.
+template <bool IS_L2, int LPR, int U>
+__device__ __forceinline__ void group_chunk(const float* __restrict__ a, const float* __restrict__ row, int t, float& c0,
+                                            float& c1) {
+  if (LPR == 8) {
+    float b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) b[u] = __ldg(row + t + 8 * u);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (IS_L2) {
+        const float d = __fsub_rn(a[t + 8 * u], b[u]);
+        c0 = __fmaf_rn(d, d, c0);
+      } else {
+        c0 = __fmaf_rn(a[t + 8 * u], b[u], c0);
+      }
+    }
+  } else {
+    float2 b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) b[u] = __ldg(reinterpret_cast<const float2*>(row + t + 8 * u));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float2 x = *reinterpret_cast<const float2*>(a + t + 8 * u);
+      if (IS_L2) {
+        const float d0 = __fsub_rn(x.x, b[u].x), d1 = __fsub_rn(x.y, b[u].y);
+        c0 = __fmaf_rn(d0, d0, c0);
+        c1 = __fmaf_rn(d1, d1, c1);
+      } else {
+        c0 = __fmaf_rn(x.x, b[u].x, c0);
+        c1 = __fmaf_rn(x.y, b[u].y, c1);
+      }
+    }
+  }
+}
+template <bool IS_L2, int LPR>
+__device__ __forceinline__ float group_distance(const float* __restrict__ a, const float* __restrict__ row, int pd) {
+  const int j = lane_id() & (LPR - 1);
+  a += LPR == 8 ? j : 2 * j;
+  row += LPR == 8 ? j : 2 * j;
+  float c0 = 0.f, c1 = 0.f;
+  int t = 0;
+  for (; t + 128 <= pd; t += 128) group_chunk<IS_L2, LPR, 16>(a, row, t, c0, c1);
+  if (pd & 64) {
+    group_chunk<IS_L2, LPR, 8>(a, row, t, c0, c1);
+    t += 64;
+  }
+  if (pd & 32) {
+    group_chunk<IS_L2, LPR, 4>(a, row, t, c0, c1);
+    t += 32;
+  }
+  for (; t < pd; t += 8) group_chunk<IS_L2, LPR, 1>(a, row, t, c0, c1);
+  if (LPR == 8) {
+    float s = __fadd_rn(c0, __shfl_xor_sync(FV_FULL, c0, 4));
+    s = __fadd_rn(s, __shfl_xor_sync(FV_FULL, s, 2));
+    s = __fadd_rn(s, __shfl_xor_sync(FV_FULL, s, 1));
+    return IS_L2 ? s : -s;
+  }
+  // lanes hold (l0,l1) (l2,l3) (l4,l5) (l6,l7): ((l0 + l4) + (l2 + l6)) + ((l1 + l5) + (l3 + l7))
+  float s0 = __fadd_rn(c0, __shfl_xor_sync(FV_FULL, c0, 2)), s1 = __fadd_rn(c1, __shfl_xor_sync(FV_FULL, c1, 2));
+  s0 = __fadd_rn(s0, __shfl_xor_sync(FV_FULL, s0, 1));
+  s1 = __fadd_rn(s1, __shfl_xor_sync(FV_FULL, s1, 1));
+  const float s = __fadd_rn(s0, s1);
+  return IS_L2 ? s : -s;
+}
+
 __device__ __forceinline__ float exact_distance(int metric, const float* a, const float* b, int pd) {
   return metric == FV_L2 ? exact_distance<true>(a, b, pd) : exact_distance<false>(a, b, pd);
 }

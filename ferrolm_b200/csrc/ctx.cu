@@ -130,12 +130,12 @@ int fv_ctx_create(int device, fv_ctx** out) {
     return fv::fail(FV_ERR_CUDA, "cudaStreamCreate failed");
   }
   for (auto& ev : ctx->ev) cudaEventCreate(&ev);
-  if (cudaMalloc(&ctx->d_flags, 64 * sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&ctx->d_flags, FV_NFLAGS * sizeof(int)) != cudaSuccess) {
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return fv::fail(FV_ERR_NOMEM, "cudaMalloc failed");
   }
-  cudaMemset(ctx->d_flags, 0, 64 * sizeof(int));
+  cudaMemsetAsync(ctx->d_flags, 0, FV_NFLAGS * sizeof(int), ctx->stream);
   *out = ctx;
   return FV_OK;
 }

@@ -124,6 +124,151 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// A handful of queries over all rows: bound by reading the rows once (memory), so the loads are what the kernel is
+// built around.  Two lanes share a row -- 32 contiguous bytes per load and row, each lane with its four of the
+// reference's eight chains -- and request 8 pieces (64 dimensions) before the first is used; 16 rows per warp and step.
+// QT queries are worked on side by side, each with its L best keys in the warp's registers (KR * 32 places).  The
+// warps' lists are merged in the block, the blocks' lists by the last block of the query group to finish (tickets,
+// zero at launch and zero again afterwards), which writes keys or neighbours: one launch for the whole search.
+// A call for 1 query over 5,183 x 384: 50 us; over 1M x 128: 128 us (the rows at 4 TB/s, launch and wait included).
+static constexpr int FEW_WARPS = 8;
+static constexpr size_t FEW_QUERIES_MAX = 64;  // (a ticket per query group in fv_ctx::d_flags)
+template <int QT, int KR, bool IS_L2>
+__global__ void __launch_bounds__(FEW_WARPS * 32, 2)
+    few_scan_kernel(const float* __restrict__ rows, size_t n, int pd, const float* __restrict__ queries, size_t q_stride,
+                    const uint32_t* __restrict__ qids, int nq, int L, int prefilter_inf, uint32_t id_base,
+                    size_t rows_per_block, u64* __restrict__ parts, uint32_t* __restrict__ tickets, u64* __restrict__ out_keys,
+                    fv_neighbor* __restrict__ out, uint32_t* __restrict__ counts) {
+  float* sq = reinterpret_cast<float*>(dyn_smem());            // [QT][pd]
+  u64* lists = reinterpret_cast<u64*>(sq + size_t(QT) * pd);   // [FEW_WARPS][32 * KR], one query at a time
+  const int w = threadIdx.x >> 5, lane = lane_id(), half = lane & 1;
+  const int q0 = blockIdx.y * QT;
+  for (int i = threadIdx.x; i < QT * pd; i += blockDim.x) {
+    const int qi = min(q0 + i / pd, nq - 1);  // (a missing query repeats the last one)
+    sq[i] = queries[size_t(qids ? qids[qi] : uint32_t(qi)) * q_stride + i % pd];
+  }
+  __syncthreads();
+  TopList<KR> top[QT];
+  u64 bound[QT];
+#pragma unroll
+  for (int t = 0; t < QT; ++t) {
+    top[t].init(L);
+    bound[t] = FV_EMPTY_KEY;
+  }
+  const size_t r_begin = size_t(blockIdx.x) * rows_per_block, r_end = min(n, r_begin + rows_per_block);
+  for (size_t r0 = r_begin + size_t(w) * 16; r0 < r_end; r0 += FEW_WARPS * 16) {
+    const size_t row = r0 + (lane >> 1);
+    const bool valid = row < r_end;
+    const float4* src = reinterpret_cast<const float4*>(rows + (valid ? row : r_end - 1) * pd) + half;
+    float acc[QT][4];
+#pragma unroll
+    for (int t = 0; t < QT; ++t)
+#pragma unroll
+      for (int l = 0; l < 4; ++l) acc[t][l] = 0.f;
+    auto work = [&](const float4& b, int c) {  // elements 8 c + 4 half .. + 3 of the row
+#pragma unroll
+      for (int t = 0; t < QT; ++t) {
+        const float4 a = *reinterpret_cast<const float4*>(sq + t * pd + 8 * c + 4 * half);
+        if (IS_L2) {
+          float d;
+          d = __fsub_rn(a.x, b.x); acc[t][0] = __fmaf_rn(d, d, acc[t][0]);
+          d = __fsub_rn(a.y, b.y); acc[t][1] = __fmaf_rn(d, d, acc[t][1]);
+          d = __fsub_rn(a.z, b.z); acc[t][2] = __fmaf_rn(d, d, acc[t][2]);
+          d = __fsub_rn(a.w, b.w); acc[t][3] = __fmaf_rn(d, d, acc[t][3]);
+        } else {
+          acc[t][0] = __fmaf_rn(a.x, b.x, acc[t][0]);
+          acc[t][1] = __fmaf_rn(a.y, b.y, acc[t][1]);
+          acc[t][2] = __fmaf_rn(a.z, b.z, acc[t][2]);
+          acc[t][3] = __fmaf_rn(a.w, b.w, acc[t][3]);
+        }
+      }
+    };
+    int c = 0;
+    for (; c + 8 <= pd / 8; c += 8) {
+      float4 b[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) b[u] = __ldg(src + 2 * (c + u));
+#pragma unroll
+      for (int u = 0; u < 8; ++u) work(b[u], c + u);
+    }
+    for (; c < pd / 8; ++c) work(__ldg(src + 2 * c), c);
+#pragma unroll
+    for (int t = 0; t < QT; ++t) {
+      // lanes hold l0..l3 and l4..l7: ((l0 + l4) + (l2 + l6)) + ((l1 + l5) + (l3 + l7))
+      float s[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) s[l] = __fadd_rn(acc[t][l], __shfl_xor_sync(FV_FULL, acc[t][l], 1));
+      float d = __fadd_rn(__fadd_rn(s[0], s[2]), __fadd_rn(s[1], s[3]));
+      if (!IS_L2) d = -d;
+      const bool in = valid && half == 0 && (!prefilter_inf || d < INFINITY);
+      top[t].offer(in ? make_key(d, id_base + uint32_t(row)) : FV_EMPTY_KEY, bound[t]);
+    }
+  }
+  // the block's list of each query: warp 0 takes in the other warps' lists
+  u64* slot = parts + (size_t(blockIdx.y) * gridDim.x + blockIdx.x) * QT * L;
+  const int first = 32 * KR - L;  // places before it hold no entry
+#pragma unroll
+  for (int t = 0; t < QT; ++t) {
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < KR; ++r) lists[w * 32 * KR + r * 32 + lane] = top[t].e[r];
+    __syncthreads();
+    if (w == 0) {
+      for (int i = 1; i < FEW_WARPS; ++i)
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+          const int at = r * 32 + lane;
+          top[t].offer(at >= first ? lists[i * 32 * KR + at] : FV_EMPTY_KEY, bound[t]);
+        }
+#pragma unroll
+      for (int r = 0; r < KR; ++r)
+        if (r * 32 + lane >= first) slot[t * L + r * 32 + lane - first] = top[t].e[r];
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  __shared__ uint32_t arrived;
+  if (threadIdx.x == 0) arrived = atomicAdd(tickets + blockIdx.y, 1u);
+  __syncthreads();
+  if (arrived != gridDim.x - 1) return;
+  __threadfence();
+  if (threadIdx.x == 0) tickets[blockIdx.y] = 0;
+  // the last block: each warp takes a share of the blocks' lists, then warp 0 the warps' lists
+  const int total = int(gridDim.x) * L;
+  for (int t = 0; t < QT && q0 + t < nq; ++t) {
+    TopList<KR> all;
+    u64 b = FV_EMPTY_KEY;
+    all.init(L);
+    const u64* src = parts + (size_t(blockIdx.y) * gridDim.x * QT + t) * L;
+    for (int i0 = w * 32; i0 < total; i0 += FEW_WARPS * 32) {
+      const int i = i0 + lane;
+      all.offer(i < total ? __ldcg(src + size_t(i / L) * QT * L + i % L) : FV_EMPTY_KEY, b);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < KR; ++r) lists[w * 32 * KR + r * 32 + lane] = all.e[r];
+    __syncthreads();
+    if (w != 0) continue;
+    for (int i = 1; i < FEW_WARPS; ++i)
+#pragma unroll
+      for (int r = 0; r < KR; ++r) {
+        const int at = r * 32 + lane;
+        all.offer(at >= first ? lists[i * 32 * KR + at] : FV_EMPTY_KEY, b);
+      }
+    int found = 0;
+#pragma unroll
+    for (int r = 0; r < KR; ++r) {
+      const int e = r * 32 + lane - first;
+      const u64 key = all.e[r];
+      if (e >= 0 && out_keys) out_keys[size_t(q0 + t) * L + e] = key;
+      if (e >= 0 && out)
+        out[size_t(q0 + t) * L + e] = key == FV_EMPTY_KEY ? fv_neighbor{0xFFFFFFFFu, INFINITY} : fv_neighbor{key_id(key), key_distance(key)};
+      found += __popc(__ballot_sync(FV_FULL, e >= 0 && key != FV_EMPTY_KEY));
+    }
+    if (counts && lane == 0) counts[q0 + t] = uint32_t(found);
+  }
+}
+
 // One block per query: the L smallest of n keys (n <= npow2, a power of two), by sorting them in shared memory.
 __global__ void __launch_bounds__(256) block_select_kernel(const u64* __restrict__ dense, size_t stride, int n, int npow2,
                                                            int L, u64* __restrict__ out) {
@@ -294,11 +439,50 @@ static int launch_scan(fv_ctx* ctx, bool is_l2, dim3 grid, int threads, size_t s
   return FV_OK;
 }
 
+// The scan of a handful of queries in one launch (few_scan_kernel): keys and/or neighbours with counts.
+// scratch: `scratch_slot` holds the blocks' lists
+static size_t few_smem(int QT, int KR, int pd) { return size_t(QT) * pd * 4 + size_t(FEW_WARPS) * 32 * KR * 8; }
+
+bool few_scan_usable(fv_ctx* ctx, size_t n, int pd, size_t nq, int L) {
+  return n > 0 && n <= 0x7FFFFFFFull && nq <= FEW_QUERIES_MAX && L <= 128 && few_smem(4, 4, pd) <= 48 * 1024;
+}
+
+int few_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, const float* d_queries, size_t q_stride,
+             const uint32_t* d_query_ids, size_t nq, int L, bool prefilter_inf, uint32_t id_base, u64* d_out_keys,
+             fv_neighbor* d_out, uint32_t* d_counts, int scratch_slot) {
+  const int KR = L <= 32 ? 1 : 4;
+  const int QT = nq == 1 ? 1 : (KR == 1 ? 4 : 2);
+  const size_t groups = (nq + QT - 1) / QT;
+  // at least one step of 16 rows per warp, and no more blocks than are resident
+  const size_t step = FEW_WARPS * 16;
+  size_t blocks = std::max<size_t>(1, std::min((n + step - 1) / step, std::max<size_t>(1, size_t(ctx->sm_count) * 2 / groups)));
+  const size_t rpb = ((n + blocks - 1) / blocks + step - 1) / step * step;
+  blocks = (n + rpb - 1) / rpb;
+  FV_TRY(ctx->scratch[scratch_slot].reserve(groups * blocks * QT * L * sizeof(u64)));
+  uint32_t* tickets = reinterpret_cast<uint32_t*>(ctx->d_flags + 64);  // zero between launches
+  auto pick = [&](auto l2) {
+    constexpr bool IS_L2 = decltype(l2)::value;
+    return KR == 1 ? (QT == 1 ? few_scan_kernel<1, 1, IS_L2> : few_scan_kernel<4, 1, IS_L2>)
+                   : (QT == 1 ? few_scan_kernel<1, 4, IS_L2> : few_scan_kernel<2, 4, IS_L2>);
+  };
+  auto kern = metric == FV_L2 ? pick(std::true_type{}) : pick(std::false_type{});
+  kern<<<dim3(unsigned(blocks), unsigned(groups)), FEW_WARPS * 32, few_smem(QT, KR, pd), ctx->stream>>>(
+      d_rows, n, pd, d_queries, q_stride, d_query_ids, int(nq), L, prefilter_inf ? 1 : 0, id_base, rpb,
+      ctx->scratch[scratch_slot].as<u64>(), tickets, d_out_keys, d_out, d_counts);
+  ctx->stats.launches++;
+  FV_CUDA(cudaGetLastError());
+  return FV_OK;
+}
+
 int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, const float* d_queries, size_t q_stride,
                const uint32_t* d_query_ids, size_t nq, int L, bool prefilter_inf, uint32_t id_base, u64* d_out_keys,
                int scratch_slot) {
   if (nq == 0) return FV_OK;
   if (L < 1 || L > 4096) return fail(FV_ERR_UNSUPPORTED, "top-k list length must be in 1..4096");
+  // up to four passes over the rows: beyond, eight queries a warp and more blocks make up for the merge
+  if (nq <= 16 && few_scan_usable(ctx, n, pd, nq, L))
+    return few_scan(ctx, metric, d_rows, n, pd, d_queries, q_stride, d_query_ids, nq, L, prefilter_inf, id_base, d_out_keys,
+                    nullptr, nullptr, scratch_slot);
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
   // choose queries per warp (QT) and warps per block (W) so that queries + lists fit in shared memory
   int QT = 8, W = 4;
@@ -482,6 +666,21 @@ int fv_flat_set_mode(fv_flat* ix, int mode) {
   return FV_OK;
 }
 
+// The one-launch scan against the tensor-core path.  Fitted to calls timed at 5,183 x 384, 100,000 x 128 and 1M x 128
+// (1 to 64 queries, k = 10): the scan takes about 60 us and, for every four queries, the time to read the rows at
+// 5 TB/s; the tensor-core path 130 us and the time to read its 16-bit rows at 2 TB/s.  (100,000 rows: 16 queries 122
+// against 150 us, 64 queries 239 against 151; 1M rows: 4 queries 209 against 269, 8 queries 298 against 272.)  With more
+// than 32 results the scan takes two queries at a time and its merge costs more; so does the other path's re-rank
+// (1 query 287 against 410 us on 1M rows, 2 queries 488 against 409; 100,000 rows: 16 queries 367 against 400).
+static bool flat_prefers_few(size_t n, int pd, size_t nq, int L) {
+  const double mb = double(n) * pd * 4e-6;
+  const size_t qt = nq == 1 ? 1 : (L <= 32 ? 4 : 2);
+  const double passes = double((nq + qt - 1) / qt);
+  const double few = (L <= 32 ? 60.0 : (nq == 1 ? 160.0 : 280.0)) + passes * mb / 5.0;
+  const double tc = (L <= 32 ? 130.0 : 370.0) + mb / 4.0;
+  return few < tc;
+}
+
 // scratch slots: 0 padded queries, 1 final keys, 2 scan partials, 3.. tensor-core path
 int fv_flat_search_batch_dev(fv_flat* ix, const float* d_queries, size_t nq, size_t k, fv_neighbor* d_out,
                              uint32_t* d_counts) {
@@ -501,11 +700,20 @@ int fv_flat_search_batch_dev(fv_flat* ix, const float* d_queries, size_t nq, siz
     q = ctx->scratch[0].as<float>();
   }
   const int L = int(k);
+  if (ix->mode == 0 && fv::few_scan_usable(ctx, ix->n, pd, nq, L) &&
+      (!fv::tc_usable(ix->tc, ix->n, nq, L) || flat_prefers_few(ix->n, pd, nq, L))) {
+    FV_TRY(fv::few_scan(ctx, ix->metric, ix->data.as<float>(), ix->n, pd, q, size_t(pd), nullptr, nq, L, true, ix->id_base,
+                        nullptr, d_out, d_counts, 2));
+    fv::stage_mark(ctx);
+    FV_CUDA(cudaStreamSynchronize(ctx->stream));
+    fv::stage_end(ctx);
+    return FV_OK;
+  }
   FV_TRY(ctx->scratch[1].reserve(nq * size_t(L) * sizeof(u64)));
   u64* keys = ctx->scratch[1].as<u64>();
   const bool want_tc = ix->mode == 1 || (ix->mode == 0 && fv::tc_usable(ix->tc, ix->n, nq, L));
   if (want_tc) {
-    if (!fv::tc_usable(ix->tc, ix->n, nq, L))
+    if (!fv::tc_usable(ix->tc, ix->n, nq, L) || (ix->mode == 1 && L > 32))
       return fv::fail(FV_ERR_UNSUPPORTED, "tensor-core search needs k <= 32, at least 4096 rows and a padded dimension of at most 384");
     FV_TRY(fv::tc_search(ctx, ix->tc, ix->metric, ix->data.as<float>(), ix->n, pd, q, nq, L, ix->id_base, keys, true, true));
   } else {

@@ -318,6 +318,7 @@ __host__ __device__ __forceinline__ int list_of_row(int MH, int r, int li) {
 // search over 16384 rows failed their certificate and went to the full-precision scan).  E follows the base size
 // (about sqrt(n / 1000)): the sample pass costs ~ n / E, the re-rank ~ R * E.
 static constexpr int SAMPLE_R_MIN = 5, SAMPLE_R_MAX = 13;
+static constexpr int TC_MAX_K = 128;  // results per query: what a warp of the re-rank still keeps sorted cheaply
 
 static int pick_sample_every(size_t n) {
   int e = 8;
@@ -325,9 +326,10 @@ static int pick_sample_every(size_t n) {
   return e;
 }
 
+// SAMPLE_R_MAX + 1: no R up to SAMPLE_R_MAX will do at this rate
 static int pick_sample_r(int k, int every) {
   const double p = 1.0 / every;
-  for (int r = SAMPLE_R_MIN; r < SAMPLE_R_MAX; ++r) {
+  for (int r = SAMPLE_R_MIN; r <= SAMPLE_R_MAX; ++r) {
     // P(Binomial(k - 1, p) >= r) by summing the lower tail
     double tail = 1.0, term = std::pow(1.0 - p, k - 1);
     for (int i = 0; i < r; ++i) {
@@ -336,7 +338,7 @@ static int pick_sample_r(int k, int every) {
     }
     if (tail < 2e-5) return r;
   }
-  return SAMPLE_R_MAX;
+  return SAMPLE_R_MAX + 1;
 }
 
 // The R-th smallest score of every query over the lists the sample pass left (+inf when the sample holds fewer rows).
@@ -1096,13 +1098,24 @@ __global__ void rerank_kernel(RerankParams p) {
   }
 }
 
-// rows of the strided sample: sample row i is base row floor(i * n / ns)
+// Rows of the strided sample: sample row i is base row floor(i * n / ns).  They are stored with the multiples of 16
+// first, then the other multiples of 8, 4 and 2, then the odd ones: the first ceil(ns / 2^j) rows are the sample of
+// every 2^j-th of them (j <= 4), for searches that want a coarser one.
+static constexpr int SAMPLE_LEVELS = 4;
+__host__ __device__ __forceinline__ size_t sample_prefix(size_t ns, int j) { return (ns + (size_t(1) << j) - 1) >> j; }
+__device__ __forceinline__ size_t sample_row_at(size_t slot, size_t ns) {  // the sample row stored in `slot`
+  if (slot < sample_prefix(ns, SAMPLE_LEVELS)) return slot << SAMPLE_LEVELS;
+  int j = SAMPLE_LEVELS - 1;
+  while (slot >= sample_prefix(ns, j)) --j;
+  return ((slot - sample_prefix(ns, j + 1)) << (j + 1)) + (size_t(1) << j);
+}
+
 __global__ void gather_sample_kernel(const uint16_t* __restrict__ half, const float* __restrict__ norm2, size_t n, int Kp,
                                      size_t ns, uint16_t* __restrict__ samp, float* __restrict__ snorm) {
   const int lane = threadIdx.x & 31;
   const size_t i = blockIdx.x * size_t(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i >= ns) return;
-  const size_t src = size_t((unsigned long long)i * n / ns);
+  const size_t src = size_t((unsigned long long)sample_row_at(i, ns) * n / ns);
   const uint4* a = reinterpret_cast<const uint4*>(half + src * size_t(Kp));
   uint4* b = reinterpret_cast<uint4*>(samp + i * size_t(Kp));
   for (int c = lane; c < Kp / 8; c += 32) b[c] = a[c];
@@ -1299,7 +1312,7 @@ int tc_append(fv_ctx* ctx, TcSide** ptc, int metric, const float* d_rows_new, si
 
 bool tc_usable(const TcSide* tc, size_t n, size_t nq, int k) {
   (void)nq;
-  return tc && tc->n == n && k <= 32 && n >= 4096 && n <= 0x7FFFFF00ull;
+  return tc && tc->n == n && k <= TC_MAX_K && n >= 4096 && n <= 0x7FFFFF00ull;
 }
 
 // One launch of the GEMM kernel over `rows` operand rows.
@@ -1455,8 +1468,16 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
               size_t nq, int k, uint32_t id_base, u64* d_out_keys, bool mark_stages, bool prefilter_inf) {
   const int Kp = tc->Kp;
   const bool is_l2 = metric == FV_L2;
+  // The rank R of the sampled bound has to fit the epilogue's register lists: a long result takes a coarser sample (a
+  // prefix of the stored one), where fewer of its rows are sampled.  k = 100 over 50,000 rows: 1 row in 32 instead of
+  // 1 in 8, R = 13 (at 1 in 8 the bound would have to be about the 29th).
+  int level = 0;
+  int R = pick_sample_r(k, tc->every);
+  while (R > SAMPLE_R_MAX && level < SAMPLE_LEVELS) R = pick_sample_r(k, tc->every << ++level);
+  R = std::min(R, SAMPLE_R_MAX);
+  const size_t ns = sample_prefix(tc->ns, level);
   Tiling ts{}, tm{};
-  FV_TRY(make_tiling(ctx, Kp, nq, tc->ns, SCRATCH_BYTES, &ts));
+  FV_TRY(make_tiling(ctx, Kp, nq, ns, SCRATCH_BYTES, &ts));
   FV_TRY(make_tiling(ctx, Kp, nq, n, 0, &tm));
   const int rows_per_tile = 128 * tm.MH;
 
@@ -1484,7 +1505,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   int* err = reinterpret_cast<int*>(retry_count + 1);
   CUtensorMap tmA, tmS, tmB;
   FV_TRY(make_tmap(&tmA, tc->bf16, dA, nq_pad, Kp, 128));
-  FV_TRY(make_tmap(&tmS, tc->bf16, tc->samp.p, tc->ns, Kp, TILE_N));
+  FV_TRY(make_tmap(&tmS, tc->bf16, tc->samp.p, ns, Kp, TILE_N));
   FV_TRY(make_tmap(&tmB, tc->bf16, tc->half.p, n, Kp, TILE_N));
 
   init_stats_kernel<<<1, 1, 0, ctx->stream>>>(qst);
@@ -1496,10 +1517,9 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   // sample pass: per query the R (+1) best scores over the sampled rows
   // the epilogue keeps its lists in registers, so their length is a template parameter: R is rounded up to the next
   // instantiated length - 1 (a larger R only loosens the bound)
-  int R = pick_sample_r(k, tc->every);
   R = R <= 7 ? R : (R <= 9 ? 9 : 13);
   GemmParams gs{};
-  fill_params(&gs, ts, tc->ns, nq, SCRATCH_BYTES);
+  fill_params(&gs, ts, ns, nq, SCRATCH_BYTES);
   gs.has_ext = is_l2 ? 1 : 0;
   gs.aext_c = tc->bf16 ? 0x3F80u : uint32_t((tc->ext_e + 15) << 10);  // 1.0 (bf16) or 2^ext_e (fp16)
   gs.idesc = make_idesc(128, TILE_N, tc->bf16);

@@ -73,6 +73,8 @@ struct DevBuf {
 };
 
 enum { FV_NSCRATCH = 18, FV_NSTAGE = 8 };
+// words of fv_ctx::d_flags: 0..63 counters of the searches, then one ticket per query group of the few-query scan
+enum { FV_NFLAGS = 128 };
 
 struct fv_ctx {
   // Every entry point that uses the stream, the scratch arena, the events or the counters holds this lock for the
@@ -168,6 +170,12 @@ int merge_topk_impl(fv_ctx* ctx, const fv_neighbor* d_parts, const uint32_t* d_p
 int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, const float* d_queries,
                size_t q_stride, const uint32_t* d_query_ids, size_t nq, int L, bool prefilter_inf,
                uint32_t id_base, u64* d_out_keys, int scratch_slot);
+
+// ---- the same for a handful of queries, in one launch: keys and/or neighbours with counts (each may be null).
+bool few_scan_usable(fv_ctx* ctx, size_t n, int pd, size_t nq, int L);
+int few_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, const float* d_queries, size_t q_stride,
+             const uint32_t* d_query_ids, size_t nq, int L, bool prefilter_inf, uint32_t id_base, u64* d_out_keys,
+             fv_neighbor* d_out, uint32_t* d_counts, int scratch_slot);
 
 // keys -> fv_neighbor rows and counts.  in: nq * L keys (ascending), out: nq * k neighbours.
 int keys_to_neighbors(fv_ctx* ctx, const u64* d_keys, size_t nq, int L, int k, fv_neighbor* d_out,

@@ -1,0 +1,75 @@
+"""Exact search over the paths the library picks by itself: the one-launch scan of a handful of queries, the tensor-core
+front end with results longer than 32, and the selection over few rows; against the oracle, ties included."""
+import numpy as np
+import pytest
+
+from tests.parity import assert_same_neighbours
+
+pytestmark = pytest.mark.gpu
+
+L2, IP = 0, 1
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import ferrolm_b200 as fv
+
+    c = fv.Context(0)
+    yield c
+    c.close()
+
+
+def rows(oracle, metric, n, dim, seed):
+    x = oracle.testdata(n, dim, seed)
+    # coarse grid: many exactly equal distances, ordered by id on both sides
+    return np.round(x * 2).astype(np.float32) if metric == L2 else oracle.normalize(x)
+
+
+def check(oracle, ctx, metric, n, dim, nq, k, what):
+    import ferrolm_b200 as fv
+
+    base, q = rows(oracle, metric, n, dim, 1), rows(oracle, metric, nq, dim, 2)
+    ix = fv.FlatIndex(ctx, metric, dim)
+    ix.add(base)
+    o = oracle.FlatIndex(metric, dim)
+    o.add(base)
+    want, wc = o.search_batch(q, k)
+    for mode in (0, 2):
+        ix.set_mode(mode)
+        got, gc = ix.search_batch(q, k)
+        bits, total = assert_same_neighbours(got, gc, want, wc, f"{what}, mode {mode}")
+        assert bits == total
+    one, oc = ix.search_batch(q[:1], k)
+    assert_same_neighbours(one, oc, want[:1], wc[:1], f"{what}, one query")
+
+
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 127, 128, 129, 4095, 4096, 40_001])
+@pytest.mark.parametrize("nq,k", [(1, 1), (3, 10), (4, 32), (5, 33), (16, 100), (17, 128), (64, 10), (65, 40)])
+def test_few_queries(oracle, ctx, metric, n, nq, k):
+    check(oracle, ctx, metric, n, 20 if n % 2 else 72, nq, k, f"{nq} queries of {n} rows, k={k}")
+
+
+@pytest.mark.parametrize("metric,n,dim,nq,k", [
+    (L2, 4096, 24, 300, 33), (IP, 4100, 130, 257, 64), (L2, 20_000, 100, 300, 100), (IP, 20_000, 64, 129, 128),
+    (L2, 9000, 128, 300, 129),  # one beyond the tensor-core path
+])
+def test_long_results(oracle, ctx, metric, n, dim, nq, k):
+    check(oracle, ctx, metric, n, dim, nq, k, f"k={k}")
+    if k <= 128:
+        assert ctx.stats()["launches"] > 0
+
+
+@pytest.mark.parametrize("n,nq,k", [(1, 70, 2), (31, 70, 5), (33, 100, 31), (1025, 300, 2), (2049, 80, 300)])
+def test_few_rows(oracle, ctx, n, nq, k):
+    check(oracle, ctx, L2, n, 12, nq, k, f"{n} rows, k={k}")
+
+
+def test_a_long_result_is_refused_by_the_forced_tensor_core_mode(oracle, ctx):
+    import ferrolm_b200 as fv
+
+    ix = fv.FlatIndex(ctx, L2, 16)
+    ix.add(rows(oracle, L2, 5000, 16, 1))
+    ix.set_mode(1)
+    with pytest.raises(fv.FerrovecError):
+        ix.search_batch(rows(oracle, L2, 4, 16, 2), 33)
