@@ -317,9 +317,44 @@ __device__ __forceinline__ float quad_distances(const float* sq, const float* __
   return d;
 }
 
-// The L best keys in a warp's registers (32 * KR places, L <= 32 * KR).
+// Sorts one key per lane, ascending, and turns a bitonic sequence of 32 * R keys (place 32 r + lane in e[r]) into an
+// ascending one: compare-exchange networks over shuffles.
+__device__ __forceinline__ u64 cmp_exchange(u64 v, int stride, bool keep_min) {
+  const u64 o = __shfl_xor_sync(FV_FULL, v, stride);
+  return (v < o) == keep_min ? v : o;
+}
+__device__ __forceinline__ u64 warp_sort32(u64 v) {
+  const int lane = lane_id();
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) v = cmp_exchange(v, stride, ((lane & stride) == 0) == ((lane & size) == 0));
+  return v;
+}
+template <int R>
+__device__ __forceinline__ void bitonic_merge(u64* e) {
+#pragma unroll
+  for (int s = R >> 1; s > 0; s >>= 1)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (!(r & s)) {
+        const u64 x = e[r], y = e[r | s];
+        e[r] = x < y ? x : y;
+        e[r | s] = x < y ? y : x;
+      }
+#pragma unroll
+  for (int stride = 16; stride > 0; stride >>= 1)
+#pragma unroll
+    for (int r = 0; r < R; ++r) e[r] = cmp_exchange(e[r], stride, (lane_id() & stride) == 0);
+}
+
+// The L best keys in a warp's registers (32 * KR places, L <= 32 * KR), ascending; the last of the L entries sits in
+// the last place, the places before the first hold 0.  Both ascending lists of N places, one read backwards: the
+// smaller of each pair are the N smallest of both, as a bitonic sequence.  So 32 candidates at a time cost a sort and
+// a merge whatever their number, and a candidate alone one shuffle per 32 places; the line between the two is where
+// they take equally long.
 template <int KR>
-struct TopList {  // ascending; the last of the L entries sits in the last place, the places before the first hold 0
+struct TopList {
   u64 e[KR];
   __device__ __forceinline__ void init(int L) {
 #pragma unroll
@@ -328,6 +363,14 @@ struct TopList {  // ascending; the last of the L entries sits in the last place
   __device__ __forceinline__ u64 last() const { return __shfl_sync(FV_FULL, e[KR - 1], 31); }
   __device__ __forceinline__ void offer(u64 key, u64& bound) {  // a key per lane, FV_EMPTY_KEY for none
     unsigned pending = __ballot_sync(FV_FULL, key < bound);
+    if (__popc(pending) > 6) {
+      const u64 c = warp_sort32(key < bound ? key : FV_EMPTY_KEY);
+      const u64 back = __shfl_sync(FV_FULL, c, 31 - lane_id());
+      e[KR - 1] = min(e[KR - 1], back);
+      bitonic_merge<KR>(e);
+      bound = last();
+      return;
+    }
     while (pending) {
       const int src = __ffs(pending) - 1;
       const u64 k = __shfl_sync(FV_FULL, key, src);
@@ -340,6 +383,31 @@ struct TopList {  // ascending; the last of the L entries sits in the last place
       }
       bound = last();
       pending = __ballot_sync(FV_FULL, lane_id() > src && key < bound);
+    }
+  }
+  // takes in another list's entries: ascending from place 0 on, FV_EMPTY_KEY behind them
+  __device__ __forceinline__ void merge(const u64* c) {
+    u64 back[KR];
+#pragma unroll
+    for (int r = 0; r < KR; ++r) back[r] = __shfl_sync(FV_FULL, c[KR - 1 - r], 31 - lane_id());
+#pragma unroll
+    for (int r = 0; r < KR; ++r) e[r] = min(e[r], back[r]);
+    bitonic_merge<KR>(e);
+  }
+  // writes the L entries to dst[0 ..]
+  __device__ __forceinline__ void store(u64* dst, int L) const {
+#pragma unroll
+    for (int r = 0; r < KR; ++r) {
+      const int i = r * 32 + lane_id() - (32 * KR - L);
+      if (i >= 0) dst[i] = e[r];
+    }
+  }
+  // a list of L entries in memory, as merge takes it
+  __device__ __forceinline__ static void load(u64* c, const u64* src, int L) {
+#pragma unroll
+    for (int r = 0; r < KR; ++r) {
+      const int i = r * 32 + lane_id();
+      c[r] = i < L ? src[i] : FV_EMPTY_KEY;
     }
   }
 };

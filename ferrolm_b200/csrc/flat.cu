@@ -204,26 +204,24 @@ __global__ void __launch_bounds__(FEW_WARPS * 32, 2)
       top[t].offer(in ? make_key(d, id_base + uint32_t(row)) : FV_EMPTY_KEY, bound[t]);
     }
   }
-  // the block's list of each query: warp 0 takes in the other warps' lists
+  // The block's list of each query: the warps' lists are merged in pairs, then the pairs' lists in pairs ...
+  auto merge_warps = [&](TopList<KR>& mine) {
+    for (int step = 1; step < FEW_WARPS; step <<= 1) {
+      __syncthreads();
+      if ((w & (2 * step - 1)) == step) mine.store(lists + w * 32 * KR, L);
+      __syncthreads();
+      if ((w & (2 * step - 1)) == 0) {
+        u64 c[KR];
+        TopList<KR>::load(c, lists + (w + step) * 32 * KR, L);
+        mine.merge(c);
+      }
+    }
+  };
   u64* slot = parts + (size_t(blockIdx.y) * gridDim.x + blockIdx.x) * QT * L;
-  const int first = 32 * KR - L;  // places before it hold no entry
 #pragma unroll
   for (int t = 0; t < QT; ++t) {
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < KR; ++r) lists[w * 32 * KR + r * 32 + lane] = top[t].e[r];
-    __syncthreads();
-    if (w == 0) {
-      for (int i = 1; i < FEW_WARPS; ++i)
-#pragma unroll
-        for (int r = 0; r < KR; ++r) {
-          const int at = r * 32 + lane;
-          top[t].offer(at >= first ? lists[i * 32 * KR + at] : FV_EMPTY_KEY, bound[t]);
-        }
-#pragma unroll
-      for (int r = 0; r < KR; ++r)
-        if (r * 32 + lane >= first) slot[t * L + r * 32 + lane - first] = top[t].e[r];
-    }
+    merge_warps(top[t]);
+    if (w == 0) top[t].store(slot + t * L, L);
   }
   __threadfence();
   __syncthreads();
@@ -233,28 +231,20 @@ __global__ void __launch_bounds__(FEW_WARPS * 32, 2)
   if (arrived != gridDim.x - 1) return;
   __threadfence();
   if (threadIdx.x == 0) tickets[blockIdx.y] = 0;
-  // the last block: each warp takes a share of the blocks' lists, then warp 0 the warps' lists
-  const int total = int(gridDim.x) * L;
+  // the last block: each warp takes in a share of the blocks' lists
   for (int t = 0; t < QT && q0 + t < nq; ++t) {
     TopList<KR> all;
-    u64 b = FV_EMPTY_KEY;
     all.init(L);
     const u64* src = parts + (size_t(blockIdx.y) * gridDim.x * QT + t) * L;
-    for (int i0 = w * 32; i0 < total; i0 += FEW_WARPS * 32) {
-      const int i = i0 + lane;
-      all.offer(i < total ? __ldcg(src + size_t(i / L) * QT * L + i % L) : FV_EMPTY_KEY, b);
+    for (int i = w; i < int(gridDim.x); i += FEW_WARPS) {
+      u64 c[KR];
+#pragma unroll
+      for (int r = 0; r < KR; ++r) c[r] = r * 32 + lane < L ? __ldcg(src + size_t(i) * QT * L + r * 32 + lane) : FV_EMPTY_KEY;
+      all.merge(c);
     }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < KR; ++r) lists[w * 32 * KR + r * 32 + lane] = all.e[r];
-    __syncthreads();
+    merge_warps(all);
     if (w != 0) continue;
-    for (int i = 1; i < FEW_WARPS; ++i)
-#pragma unroll
-      for (int r = 0; r < KR; ++r) {
-        const int at = r * 32 + lane;
-        all.offer(at >= first ? lists[i * 32 * KR + at] : FV_EMPTY_KEY, b);
-      }
+    const int first = 32 * KR - L;  // places before it hold no entry
     int found = 0;
 #pragma unroll
     for (int r = 0; r < KR; ++r) {
