@@ -955,17 +955,19 @@ struct RerankParams {
   unsigned int* retry_count;
 };
 
-__global__ void rerank_kernel(RerankParams p) {
-  unsigned char* smem_raw = dyn_smem();
+// Bound by gathering the candidates' rows (about 160 per query at k = 10): eight rows at a time, four lanes to a row
+// (group_distance), the result list in registers (32 * KR places).  With four rows of eight lanes staged through shared
+// memory and the list there too, as it was: RR_FIGURES.
+template <bool IS_L2, int KR>
+__global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankParams p) {
   const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t q = size_t(blockIdx.x) * W + w;
   if (q >= size_t(p.nq)) return;
-  float* sq = reinterpret_cast<float*>(smem_raw) + size_t(w) * p.pd;
-  u64* list = reinterpret_cast<u64*>(smem_raw + size_t(W) * p.pd * sizeof(float)) + size_t(w) * p.k;
-  float* stage = reinterpret_cast<float*>(smem_raw + ((size_t(W) * (size_t(p.pd) * 4 + size_t(p.k) * 8) + 15) & ~size_t(15))) +
-                 size_t(w) * 8 * quad_stride(p.pd);  // two stage buffers
+  float* sq = reinterpret_cast<float*>(dyn_smem()) + size_t(w) * p.pd;
   for (int c = lane; c < p.pd; c += 32) sq[c] = p.queries[q * size_t(p.pd) + c];
-  warp_list_init(list, p.k);
+  TopList<KR> top;
+  top.init(p.k);
+  __syncwarp();
 
   // exact-arithmetic regime: integer-valued inputs small enough that every product, partial sum and
   // distance is an integer below 2^24 in both the tensor-core score and the reference's fp32 chain
@@ -1059,7 +1061,7 @@ __global__ void rerank_kernel(RerankParams p) {
       }
       const unsigned int pj = __shfl_sync(FV_FULL, pre, j), cj = __shfl_sync(FV_FULL, cnt, j);
       const unsigned long long sj = __shfl_sync(FV_FULL, slot, j);
-      u64 key = FV_EMPTY_KEY, ck = 0;
+      u64 ck = 0;
       uint32_t id = 0;
       bool have = false;
       if (x < total) {
@@ -1068,20 +1070,21 @@ __global__ void rerank_kernel(RerankParams p) {
         have = id < uint32_t(p.n);
         if (!have) mismatch = true;  // a padded row can only get here through a non-finite score
       }
-      // four candidates' rows at a time (asynchronous coalesced gathers, 4 rows x 8 chain lanes)
-      const float d = p.is_l2 ? quad_distances<true>(sq, p.rows, p.pd, id, have, stage)
-                              : quad_distances<false>(sq, p.rows, p.pd, id, have, stage);
-      if (have) {
-        if (exact_regime && d != key_distance(ck) + qn2) mismatch = true;
-        if (d < INFINITY) key = make_key(d, id + p.id_base);
+      for (int s = 0; s < 32 && t0 + s < total; s += 8) {
+        const int from = s + (lane >> 2);
+        const uint32_t rid = __shfl_sync(FV_FULL, id, from);
+        const bool rhave = __shfl_sync(FV_FULL, int(have), from) != 0;
+        const float score = __shfl_sync(FV_FULL, key_distance(ck), from);
+        const float d = group_distance<IS_L2, 4>(sq, p.rows + size_t(rhave ? rid : 0u) * p.pd, p.pd);
+        if (rhave && exact_regime && d != score + qn2) mismatch = true;
+        const bool in = rhave && (lane & 3) == 0 && d < INFINITY;
+        top.offer(in ? make_key(d, rid + p.id_base) : FV_EMPTY_KEY, bound);
       }
-      bound = warp_list_offer(list, p.k, key, bound);
     }
   }
-  __syncwarp();
   mismatch = __any_sync(FV_FULL, mismatch);
   overflow = __any_sync(FV_FULL, overflow);
-  const u64 kth = list[p.k - 1];
+  const u64 kth = top.last();
   bool certified;
   if (overflow || mismatch || !q_in_range || !(tau == tau)) {
     certified = false;
@@ -1091,7 +1094,11 @@ __global__ void rerank_kernel(RerankParams p) {
     // the k-th result must be provably nearer than anything that was not a candidate
     certified = kth != FV_EMPTY_KEY && (key_distance(kth) - qn2) + eps < tau;
   }
-  for (int e = lane; e < p.k; e += 32) p.out_keys[q * size_t(p.k) + e] = list[e];
+#pragma unroll
+  for (int r = 0; r < KR; ++r) {
+    const int e = r * 32 + lane - (32 * KR - p.k);
+    if (e >= 0) p.out_keys[q * size_t(p.k) + e] = top.e[r];
+  }
   if (!certified && lane == 0) {
     const unsigned int slot = atomicAdd(p.retry_count, 1u);
     p.retry_ids[slot] = uint32_t(q);
@@ -1575,12 +1582,12 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   rp.out_keys = d_out_keys;
   rp.retry_ids = ctx->scratch[7].as<uint32_t>();
   rp.retry_count = retry_count;
+  // few queries: a warp per block, so that they spread over the SMs
   int wpb = 8;
-  const size_t rwarp = size_t(pd) * 4 + size_t(k) * 8 + size_t(8 * quad_stride(pd)) * 4;  // query, list, two stages of four rows
-  while (wpb > 1 && size_t(wpb) * rwarp + 16 > 72 * 1024) wpb >>= 1;
-  const size_t rsmem = ((size_t(wpb) * (size_t(pd) * 4 + size_t(k) * 8) + 15) & ~size_t(15)) + size_t(wpb) * 8 * quad_stride(pd) * 4;
-  if (rsmem > 48 * 1024) FV_CUDA(cudaFuncSetAttribute(rerank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rsmem)));
-  rerank_kernel<<<unsigned((nq + wpb - 1) / wpb), wpb * 32, rsmem, ctx->stream>>>(rp);
+  while (wpb > 1 && nq < size_t(wpb) * ctx->sm_count) wpb >>= 1;
+  const size_t rsmem = size_t(wpb) * pd * sizeof(float);
+  auto rk = k <= 32 ? (is_l2 ? rerank_kernel<true, 1> : rerank_kernel<false, 1>) : (is_l2 ? rerank_kernel<true, 4> : rerank_kernel<false, 4>);
+  rk<<<unsigned((nq + wpb - 1) / wpb), wpb * 32, rsmem, ctx->stream>>>(rp);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   if (mark_stages) stage_mark(ctx);
