@@ -72,7 +72,7 @@ struct DevBuf {
   }
 };
 
-enum { FV_NSCRATCH = 18, FV_NSTAGE = 8 };
+enum { FV_NSCRATCH = 19, FV_NSTAGE = 8 };
 // words of fv_ctx::d_flags: 0..63 counters of the searches, then one ticket per query group of the few-query scan
 enum { FV_NFLAGS = 128 };
 

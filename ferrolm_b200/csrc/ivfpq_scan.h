@@ -49,7 +49,7 @@ struct ScanOut {
 // `cells`: nq x nprobe keys (distance, list), ascending.  `keep` = candidates kept by compressed distance;
 // `refine`: re-rank them exactly and cut to k.  Marks the context's stages and fills stats.rows_scanned.
 // `cand_slots`: candidate slots per query of the list-major scans (0 = default).
-// Scratch slots used: 5, 6, 7, 8, 9, 12, 13, 14, 15.
+// Scratch slots used: 5, 6, 7, 8, 9, 12, 13, 14, 15, 18.
 int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* d_queries, size_t nq, const u64* d_cells, int nprobe,
                int keep, int k, bool refine, bool candidates, int mode, int cand_slots, const ScanOut& out);
 
