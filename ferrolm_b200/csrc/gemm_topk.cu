@@ -949,20 +949,27 @@ struct RerankParams {
   const RangeStats* bst;  // base statistics
   const RangeStats* qst;  // query statistics
   int n, nq, pd, Kp, k, MH, is_l2, bf16;
+  int wpq;                // warps per query: 1, 2, 4 or 8
   uint32_t id_base;
   u64* out_keys;          // nq x k
   uint32_t* retry_ids;    // queries that did not certify
   unsigned int* retry_count;
 };
 
-// Bound by gathering the candidates' rows (about 160 per query at k = 10): eight rows at a time, four lanes to a row
-// (group_distance), the result list in registers (32 * KR places).  With four rows of eight lanes staged through shared
-// memory and the list there too, as it was: RR_FIGURES.
-template <bool IS_L2, int KR>
+// Bound by gathering the candidates' rows (about 160 per query at k = 10, 420 at k = 100): eight rows at a time, four
+// lanes to a row (group_distance), the result list in registers (32 * KR places).  With four rows of eight lanes staged
+// through shared memory and the list there too 10,000 queries at 1M x 128 took 274 us (201 now).  A batch that leaves
+// the SMs short of warps and has long results is given `wpq` warps per query, which share its candidates and merge
+// their lists: 501 queries with k = 100 over 50,001 x 100, the whole search 455 us in the old form, 315 with a warp per
+// query, 217 with eight.
+template <bool IS_L2, int KR, bool MULTI>  // MULTI: several warps per query
 __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankParams p) {
   const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t q = size_t(blockIdx.x) * W + w;
-  if (q >= size_t(p.nq)) return;
+  const int sub = MULTI ? w % p.wpq : 0;  // which share of the query's candidates this warp takes
+  const size_t q_own = MULTI ? size_t(blockIdx.x) * (W / p.wpq) + w / p.wpq : size_t(blockIdx.x) * W + w;
+  if (!MULTI && q_own >= size_t(p.nq)) return;
+  // (MULTI: a warp beyond the last query works on the last one and writes nothing: all warps meet at the barriers below)
+  const size_t q = MULTI ? min(q_own, size_t(p.nq) - 1) : q_own;
   float* sq = reinterpret_cast<float*>(dyn_smem()) + size_t(w) * p.pd;
   for (int c = lane; c < p.pd; c += 32) sq[c] = p.queries[q * size_t(p.pd) + c];
   TopList<KR> top;
@@ -1029,6 +1036,7 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
   // one list's count, a prefix sum lines the entries up, and the warp walks them 32 per step (a lane finds the
   // list of its entry by bisection over the prefix sums), so every step computes 32 exact distances.
   const int nlist = p.parts * lists_per_seg;
+  int taken = 0;  // runs of eight candidates seen so far, the same in all warps of the query
   for (int l0 = 0; l0 < nlist; l0 += 32) {
     const int l = l0 + lane;
     unsigned int cnt = 0;
@@ -1071,6 +1079,7 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
         if (!have) mismatch = true;  // a padded row can only get here through a non-finite score
       }
       for (int s = 0; s < 32 && t0 + s < total; s += 8) {
+        if (MULTI && ((taken++) & (p.wpq - 1)) != sub) continue;  // runs of eight are dealt in turn
         const int from = s + (lane >> 2);
         const uint32_t rid = __shfl_sync(FV_FULL, id, from);
         const bool rhave = __shfl_sync(FV_FULL, int(have), from) != 0;
@@ -1084,6 +1093,23 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
   }
   mismatch = __any_sync(FV_FULL, mismatch);
   overflow = __any_sync(FV_FULL, overflow);
+  if (MULTI) {
+    u64* lists = reinterpret_cast<u64*>(reinterpret_cast<float*>(dyn_smem()) + size_t(W) * p.pd) + size_t(w) * 32 * KR;  // 16-byte aligned: pd is a multiple of 8
+    __shared__ int bad[8];
+    if (lane == 0) bad[w] = mismatch ? 1 : 0;
+    for (int step = 1; step < p.wpq; step <<= 1) {
+      __syncthreads();
+      if ((sub & (2 * step - 1)) == step) top.store(lists, p.k);
+      __syncthreads();
+      if ((sub & (2 * step - 1)) == 0) {
+        u64 c[KR];
+        TopList<KR>::load(c, lists + size_t(step) * 32 * KR, p.k);
+        top.merge(c);
+      }
+    }
+    for (int i = 0; i < p.wpq; ++i) mismatch = mismatch || bad[w - sub + i];
+  }
+  if (sub != 0 || q_own >= size_t(p.nq)) return;
   const u64 kth = top.last();
   bool certified;
   if (overflow || mismatch || !q_in_range || !(tau == tau)) {
@@ -1582,12 +1608,18 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   rp.out_keys = d_out_keys;
   rp.retry_ids = ctx->scratch[7].as<uint32_t>();
   rp.retry_count = retry_count;
-  // few queries: a warp per block, so that they spread over the SMs
-  int wpb = 8;
-  while (wpb > 1 && nq < size_t(wpb) * ctx->sm_count) wpb >>= 1;
-  const size_t rsmem = size_t(wpb) * pd * sizeof(float);
-  auto rk = k <= 32 ? (is_l2 ? rerank_kernel<true, 1> : rerank_kernel<false, 1>) : (is_l2 ? rerank_kernel<true, 4> : rerank_kernel<false, 4>);
-  rk<<<unsigned((nq + wpb - 1) / wpb), wpb * 32, rsmem, ctx->stream>>>(rp);
+  // long results: several warps per query while the batch fills the resident warps (16 to 24 per SM) at most one and a
+  // half to two times (with 10 results, some 20 runs of eight rows, the merge takes what the shares save)
+  const int wpb = 8;
+  rp.wpq = 1;
+  while (k > 32 && rp.wpq < 8 && nq * size_t(rp.wpq) * 2 <= size_t(ctx->sm_count) * 36) rp.wpq <<= 1;
+  const size_t rsmem = size_t(wpb) * (pd * sizeof(float) + (rp.wpq > 1 ? 128 * sizeof(u64) : 0));
+  auto pick = [&](auto l2) {
+    constexpr bool IS_L2 = decltype(l2)::value;
+    return k <= 32 ? rerank_kernel<IS_L2, 1, false> : rp.wpq > 1 ? rerank_kernel<IS_L2, 4, true> : rerank_kernel<IS_L2, 4, false>;
+  };
+  auto rk = is_l2 ? pick(std::true_type{}) : pick(std::false_type{});
+  rk<<<unsigned((nq * size_t(rp.wpq) + wpb - 1) / wpb), wpb * 32, rsmem, ctx->stream>>>(rp);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   if (mark_stages) stage_mark(ctx);
