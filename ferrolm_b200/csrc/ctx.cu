@@ -84,6 +84,40 @@ int upload_padded(fv_ctx* ctx, const float* src, bool src_is_device, size_t n, s
   return FV_OK;
 }
 
+int pin_ready(fv_ctx* ctx) {
+  if (ctx->h_pin) return FV_OK;
+  void* p = nullptr;
+  if (cudaMallocHost(&p, FV_PIN_BYTES) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return fail(FV_ERR_NOMEM, "cudaMallocHost failed");
+  }
+  ctx->h_pin = static_cast<unsigned char*>(p);
+  return FV_OK;
+}
+
+static size_t results_bytes(size_t nq, size_t k) { return nq * k * sizeof(fv_neighbor) + nq * sizeof(uint32_t); }
+bool results_fit_pin(size_t nq, size_t k) { return results_bytes(nq, k) <= size_t(FV_PIN_BYTES - FV_PIN_RESULTS); }
+
+int fetch_results(fv_ctx* ctx, const fv_neighbor* d_out, size_t nq, size_t k, fv_neighbor* out, uint32_t* counts, bool fetched) {
+  const size_t obytes = nq * k * sizeof(fv_neighbor);
+  const uint32_t* d_counts = reinterpret_cast<const uint32_t*>(d_out + nq * k);
+  if (!results_fit_pin(nq, k)) {
+    FV_CUDA(cudaMemcpyAsync(out, d_out, obytes, cudaMemcpyDeviceToHost, ctx->stream));
+    if (counts) FV_CUDA(cudaMemcpyAsync(counts, d_counts, nq * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    FV_CUDA(cudaStreamSynchronize(ctx->stream));
+    return FV_OK;
+  }
+  FV_TRY(pin_ready(ctx));
+  unsigned char* pin = ctx->h_pin + FV_PIN_RESULTS;
+  if (!fetched) {
+    FV_CUDA(cudaMemcpyAsync(pin, d_out, results_bytes(nq, k), cudaMemcpyDeviceToHost, ctx->stream));
+    FV_CUDA(cudaStreamSynchronize(ctx->stream));
+  }
+  std::memcpy(out, pin, obytes);
+  if (counts) std::memcpy(counts, pin + obytes, nq * sizeof(uint32_t));
+  return FV_OK;
+}
+
 }  // namespace fv
 
 static void ctx_destroy_now(fv_ctx* ctx) {
@@ -94,6 +128,7 @@ static void ctx_destroy_now(fv_ctx* ctx) {
   for (auto& ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
   if (ctx->d_flags) cudaFree(ctx->d_flags);
+  if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -136,6 +171,7 @@ int fv_ctx_create(int device, fv_ctx** out) {
     return fv::fail(FV_ERR_NOMEM, "cudaMalloc failed");
   }
   cudaMemsetAsync(ctx->d_flags, 0, FV_NFLAGS * sizeof(int), ctx->stream);
+  (void)fv::pin_ready(ctx);  // (the first call that needs it reports a failure)
   *out = ctx;
   return FV_OK;
 }

@@ -672,8 +672,9 @@ static bool flat_prefers_few(size_t n, int pd, size_t nq, int L) {
 }
 
 // scratch slots: 0 padded queries, 1 final keys, 2 scan partials, 3.. tensor-core path
-int fv_flat_search_batch_dev(fv_flat* ix, const float* d_queries, size_t nq, size_t k, fv_neighbor* d_out,
-                             uint32_t* d_counts) {
+// `wait`: return when the results are there (a caller that queues their copy behind them waits for both itself)
+static int flat_search_impl(fv_flat* ix, const float* d_queries, size_t nq, size_t k, fv_neighbor* d_out, uint32_t* d_counts,
+                            bool wait) {
   if (!ix || (nq && (!d_queries || !d_out))) return fv::fail(FV_ERR_ARG, "fv_flat_search_batch: null argument");
   if (k == 0) return fv::fail(FV_ERR_ARG, "k must be at least 1");
   if (k > 4096) return fv::fail(FV_ERR_UNSUPPORTED, "k above 4096 is not supported");
@@ -690,32 +691,39 @@ int fv_flat_search_batch_dev(fv_flat* ix, const float* d_queries, size_t nq, siz
     q = ctx->scratch[0].as<float>();
   }
   const int L = int(k);
+  auto finish = [&]() -> int {
+    fv::stage_mark(ctx);
+    if (wait || ctx->timing) FV_CUDA(cudaStreamSynchronize(ctx->stream));
+    fv::stage_end(ctx);
+    return FV_OK;
+  };
   if (ix->mode == 0 && fv::few_scan_usable(ctx, ix->n, pd, nq, L) &&
       (!fv::tc_usable(ix->tc, ix->n, nq, L) || flat_prefers_few(ix->n, pd, nq, L))) {
     FV_TRY(fv::few_scan(ctx, ix->metric, ix->data.as<float>(), ix->n, pd, q, size_t(pd), nullptr, nq, L, true, ix->id_base,
                         nullptr, d_out, d_counts, 2));
-    fv::stage_mark(ctx);
-    FV_CUDA(cudaStreamSynchronize(ctx->stream));
-    fv::stage_end(ctx);
-    return FV_OK;
+    return finish();
   }
   FV_TRY(ctx->scratch[1].reserve(nq * size_t(L) * sizeof(u64)));
   u64* keys = ctx->scratch[1].as<u64>();
+  auto neighbours = [&]() { return fv::keys_to_neighbors(ctx, keys, nq, L, int(k), d_out, d_counts); };
   const bool want_tc = ix->mode == 1 || (ix->mode == 0 && fv::tc_usable(ix->tc, ix->n, nq, L));
   if (want_tc) {
     if (!fv::tc_usable(ix->tc, ix->n, nq, L) || (ix->mode == 1 && L > 32))
       return fv::fail(FV_ERR_UNSUPPORTED, "tensor-core search needs k <= 32, at least 4096 rows and a padded dimension of at most 384");
-    FV_TRY(fv::tc_search(ctx, ix->tc, ix->metric, ix->data.as<float>(), ix->n, pd, q, nq, L, ix->id_base, keys, true, true));
+    FV_TRY(fv::tc_search(ctx, ix->tc, ix->metric, ix->data.as<float>(), ix->n, pd, q, nq, L, ix->id_base, keys, true, true,
+                         neighbours));
   } else {
     FV_TRY(fv::exact_scan(ctx, ix->metric, ix->data.as<float>(), ix->n, pd, q, size_t(pd), nullptr, nq, L, true,
                           ix->id_base, keys, 2));
     fv::stage_mark(ctx);
+    FV_TRY(neighbours());
   }
-  FV_TRY(fv::keys_to_neighbors(ctx, keys, nq, L, int(k), d_out, d_counts));
-  fv::stage_mark(ctx);
-  FV_CUDA(cudaStreamSynchronize(ctx->stream));
-  fv::stage_end(ctx);
-  return FV_OK;
+  return finish();
+}
+
+int fv_flat_search_batch_dev(fv_flat* ix, const float* d_queries, size_t nq, size_t k, fv_neighbor* d_out,
+                             uint32_t* d_counts) {
+  return flat_search_impl(ix, d_queries, nq, k, d_out, d_counts, true);
 }
 
 int fv_flat_search_batch(fv_flat* ix, const float* queries, size_t nq, size_t k, fv_neighbor* out, uint32_t* counts) {
@@ -731,11 +739,8 @@ int fv_flat_search_batch(fv_flat* ix, const float* queries, size_t nq, size_t k,
   fv_neighbor* dout = ctx->scratch[11].as<fv_neighbor>();
   uint32_t* dc = reinterpret_cast<uint32_t*>(ctx->scratch[11].as<unsigned char>() + obytes);
   FV_CUDA(cudaMemcpyAsync(dq, queries, qbytes, cudaMemcpyHostToDevice, ctx->stream));
-  FV_TRY(fv_flat_search_batch_dev(ix, dq, nq, k, dout, dc));
-  FV_CUDA(cudaMemcpyAsync(out, dout, obytes, cudaMemcpyDeviceToHost, ctx->stream));
-  if (counts) FV_CUDA(cudaMemcpyAsync(counts, dc, nq * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-  FV_CUDA(cudaStreamSynchronize(ctx->stream));
-  return FV_OK;
+  FV_TRY(flat_search_impl(ix, dq, nq, k, dout, dc, false));
+  return fv::fetch_results(ctx, dout, nq, k, out, counts);
 }
 
 int fv_flat_search(fv_flat* ix, const float* query, size_t k, fv_neighbor* out, uint32_t* count) {

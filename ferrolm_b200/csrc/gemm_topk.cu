@@ -1498,7 +1498,9 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
 // scratch slots: 2 scan partials (fallback), 3 A operand, 5 query norms + bounds + candidate counters, 6 sample lists,
 // 7 retry ids, 8 fallback keys, 9 candidate buffers
 int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n, int pd, const float* d_queries,
-              size_t nq, int k, uint32_t id_base, u64* d_out_keys, bool mark_stages, bool prefilter_inf) {
+              size_t nq, int k, uint32_t id_base, u64* d_out_keys, bool mark_stages, bool prefilter_inf,
+              const std::function<int()>& then) {
+  FV_TRY(pin_ready(ctx));
   const int Kp = tc->Kp;
   const bool is_l2 = metric == FV_L2;
   // The rank R of the sampled bound has to fit the epilogue's register lists: a long result takes a coarser sample (a
@@ -1624,8 +1626,9 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   FV_CUDA(cudaGetLastError());
   if (mark_stages) stage_mark(ctx);
 
-  unsigned int h_words[2] = {0, 0};  // retry count, error word
-  FV_CUDA(cudaMemcpyAsync(h_words, retry_count, sizeof(h_words), cudaMemcpyDeviceToHost, ctx->stream));
+  if (then) FV_TRY(then());
+  const unsigned int* h_words = reinterpret_cast<const unsigned int*>(ctx->h_pin);  // retry count, error word
+  FV_CUDA(cudaMemcpyAsync(ctx->h_pin, retry_count, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream));
   FV_CUDA(cudaStreamSynchronize(ctx->stream));
   if (h_words[1]) return fail(FV_ERR_TIMEOUT, "a bounded wait inside the tensor-core kernel ran out");
   ctx->stats.uncertified = h_words[0];
@@ -1637,6 +1640,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
     scatter_keys_kernel<<<ctx->sm_count, 256, 0, ctx->stream>>>(sub, rp.retry_ids, nsub, k, d_out_keys);
     ctx->stats.launches++;
     FV_CUDA(cudaGetLastError());
+    if (then) FV_TRY(then());
   }
   if (mark_stages) stage_mark(ctx);
   return FV_OK;

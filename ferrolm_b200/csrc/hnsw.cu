@@ -418,9 +418,11 @@ static int search_shape(fv_ctx* ctx, bool is_l2, int pd, int ef, size_t active, 
 }
 
 // scratch slots: 0 padded queries, 1 keys, 5 overflow flags, 6 retry ids, 7 global tables
+// `h_out`, `h_counts` (may be null): bring the results out to the host as well (d_counts lies directly behind d_out then)
 static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t k, size_t ef_in, fv_neighbor* d_out,
-                           uint32_t* d_counts) {
+                           uint32_t* d_counts, fv_neighbor* h_out = nullptr, uint32_t* h_counts = nullptr) {
   fv_ctx* ctx = h->ctx;
+  FV_TRY(pin_ready(ctx));
   if (k == 0) return fail(FV_ERR_ARG, "k must be at least 1");
   if (nq == 0) return FV_OK;
   ctx->stats = fv_stats{};
@@ -430,6 +432,7 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
     u64* keys = ctx->scratch[1].as<u64>();
     FV_CUDA(cudaMemsetAsync(keys, 0xFF, nq * k * sizeof(u64), ctx->stream));
     FV_TRY(keys_to_neighbors(ctx, keys, nq, int(k), int(k), d_out, d_counts));
+    if (h_out) return fetch_results(ctx, d_out, nq, k, h_out, h_counts);
     FV_CUDA(cudaStreamSynchronize(ctx->stream));
     return FV_OK;
   }
@@ -467,7 +470,11 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   const uint32_t* d_qids = nullptr;
   size_t active = nq;
   std::vector<uint32_t> h_over, retry;
-  unsigned long long wk[4] = {0, 0, 0, 0}, total[3] = {0, 0, 0};
+  const unsigned long long* wk = reinterpret_cast<const unsigned long long*>(ctx->h_pin);
+  unsigned long long total[3] = {0, 0, 0};
+  // the results follow the counters out at once: nearly always the first attempt is the last
+  const bool early = h_out && results_fit_pin(nq, k);
+  bool fetched = false;
   for (int attempt = 0; attempt < 8 && active; ++attempt) {
     SearchShape sh{};
     FV_TRY(search_shape(ctx, h->metric == FV_L2, pd, int(ef), active, &sh));
@@ -479,11 +486,15 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
                                                                        d_work, d_next);
     ctx->stats.launches++;
     FV_CUDA(cudaGetLastError());
-    FV_CUDA(cudaMemcpyAsync(wk, d_work, sizeof(wk), cudaMemcpyDeviceToHost, ctx->stream));
+    FV_CUDA(cudaMemcpyAsync(ctx->h_pin, d_work, 4 * sizeof(*wk), cudaMemcpyDeviceToHost, ctx->stream));
+    if (early)
+      FV_CUDA(cudaMemcpyAsync(ctx->h_pin + FV_PIN_RESULTS, d_out, nq * k * sizeof(fv_neighbor) + nq * sizeof(uint32_t),
+                              cudaMemcpyDeviceToHost, ctx->stream));
     FV_CUDA(cudaStreamSynchronize(ctx->stream));
     for (int i = 0; i < 3; ++i) total[i] += wk[i];
     if (wk[3] == 0) {
       active = 0;
+      fetched = early;
       break;
     }
     h_over.resize(active);
@@ -506,7 +517,7 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   ctx->stats.dist_evals = total[0];
   ctx->stats.expansions = total[1];
   ctx->stats.uncertified = total[2];  // queries whose list of tied, pushed-out entries overflowed (see TIED_CAP)
-  FV_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (h_out) FV_TRY(fetch_results(ctx, d_out, nq, k, h_out, h_counts, fetched));
   stage_end(ctx);
   return bounds_report_hnsw();
 }
@@ -647,11 +658,7 @@ int fv_hnsw_search_batch(fv_hnsw* ix, const float* queries, size_t nq, size_t k,
   fv_neighbor* dout = ctx->scratch[11].as<fv_neighbor>();
   uint32_t* dc = reinterpret_cast<uint32_t*>(ctx->scratch[11].as<unsigned char>() + obytes);
   FV_CUDA(cudaMemcpyAsync(dq, queries, qbytes, cudaMemcpyHostToDevice, ctx->stream));
-  FV_TRY(fv::hnsw_search_dev(ix, dq, nq, k, ef, dout, dc));
-  FV_CUDA(cudaMemcpyAsync(out, dout, obytes, cudaMemcpyDeviceToHost, ctx->stream));
-  if (counts) FV_CUDA(cudaMemcpyAsync(counts, dc, nq * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-  FV_CUDA(cudaStreamSynchronize(ctx->stream));
-  return FV_OK;
+  return fv::hnsw_search_dev(ix, dq, nq, k, ef, dout, dc, out, counts);
 }
 
 int fv_hnsw_search(fv_hnsw* ix, const float* query, size_t k, size_t ef, fv_neighbor* out, uint32_t* count) {

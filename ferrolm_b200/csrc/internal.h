@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -91,6 +92,11 @@ struct fv_ctx {
   bool timing = false;
   cudaEvent_t ev[FV_NSTAGE + 1] = {};
   int ev_used = 0;
+  // Pinned host memory, allocated with the context and given back with it: read-backs of
+  // counters (the first FV_PIN_RESULTS bytes) and results of up to FV_PIN_BYTES - FV_PIN_RESULTS bytes.  A copy into
+  // the caller's pageable memory makes the host wait for each piece; into this one the pieces queue up behind the
+  // kernels and are waited for once.
+  unsigned char* h_pin = nullptr;
   int* d_flags = nullptr;  // small device word array for error / overflow flags
   bool stage_outer = false;  // an enclosing call owns the stage table: nested searches leave it alone
   // the group this context belongs to (fv_ctx_comm_init): one rank per GPU, NCCL over NVLink for the one exchange step
@@ -100,7 +106,16 @@ struct fv_ctx {
   bool closing = false;    // fv_ctx_destroy was called while indexes were alive
 };
 
+enum { FV_PIN_BYTES = 1 << 20, FV_PIN_RESULTS = 4096 };
+
 namespace fv {
+
+int pin_ready(fv_ctx* ctx);  // makes ctx->h_pin usable
+// Brings the results of a host call out: nq * k neighbours and, directly behind them on the device, nq counts (which
+// the caller may not want).  Queues the copies behind what runs on the stream and waits for it once.  `fetched`: the
+// block already sits in the pinned memory and has been waited for.
+int fetch_results(fv_ctx* ctx, const fv_neighbor* d_out, size_t nq, size_t k, fv_neighbor* out, uint32_t* counts, bool fetched = false);
+bool results_fit_pin(size_t nq, size_t k);
 
 // RAII: makes the context's device current for the duration of a call.
 struct DeviceGuard {
@@ -187,8 +202,11 @@ struct TcSide;
 void tc_free(TcSide* tc);
 int tc_append(fv_ctx* ctx, TcSide** tc, int metric, const float* d_rows_new, size_t n_old, size_t n_new, int pd);
 // `prefilter_inf`: what the full-precision scan that re-runs uncertified queries is told (see exact_scan).
+// `then` (may be empty): launches what follows on the keys.  It is called before the host waits for the certificates,
+// so that the GPU has no gap there, and once more if queries had to be re-run.
 int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n, int pd, const float* d_queries,
-              size_t nq, int k, uint32_t id_base, u64* d_out_keys, bool mark_stages, bool prefilter_inf);
+              size_t nq, int k, uint32_t id_base, u64* d_out_keys, bool mark_stages, bool prefilter_inf,
+              const std::function<int()>& then = {});
 bool tc_usable(const TcSide* tc, size_t n, size_t nq, int k);
 
 // ---- the same kernel in task mode, for callers that bring their own operand rows and work table (the IVF-PQ scan).

@@ -824,10 +824,12 @@ int fv_ivfpq_add_dev(fv_ivfpq* ix, const float* d_vectors, size_t n) { return iv
 
 // scratch slots: 0 padded queries, 1 final keys, 2 scan partials, 4 cells, 5 per-query tables (after the coarse search is done with it)
 // `cells_in`: the probed cells of every query if the caller already has them (nq x min(nprobe, nlist) keys from
-// fv_ivfpq_coarse_dev), else null.  `cells_only`: stop after the coarse search and leave the keys there.
+// fv_ivfpq_coarse_dev), else null.  `cells_only`: stop after the coarse search and leave the keys there.  `h_out`,
+// `h_counts`: bring the results out to the host as well (d_counts has to lie directly behind d_out then).
 static int ivfpq_search_impl(fv_ivfpq* ix, const float* d_queries, size_t nq, size_t k, size_t nprobe, size_t refine,
                              bool candidates, fv_neighbor* d_out, uint32_t* d_counts, fv_neighbor* d_adc, float* d_exact,
-                             const uint64_t* cells_in = nullptr, uint64_t* cells_only = nullptr) {
+                             const uint64_t* cells_in = nullptr, uint64_t* cells_only = nullptr, fv_neighbor* h_out = nullptr,
+                             uint32_t* h_counts = nullptr) {
   fv_ctx* ctx = ix->ctx;
   if (k == 0) return fv::fail(FV_ERR_ARG, "k must be at least 1");
   if (nprobe == 0) return fv::fail(FV_ERR_ARG, "nprobe must be at least 1");
@@ -912,10 +914,12 @@ static int ivfpq_search_impl(fv_ivfpq* ix, const float* d_queries, size_t nq, si
   so.adc = d_adc;
   so.exact = d_exact;
   so.counts = d_counts;
+  if (!candidates) so.then = [&]() { return fv::keys_to_neighbors(ctx, so.keys, nq, int(k), int(k), d_out, d_counts); };
   FV_TRY(fv::ivfpq_scan(ctx, si, q, nq, cells, np, int(keep), int(k), rerank, candidates, ix->scan_mode, ix->cand_slots, so));
-  if (!candidates) FV_TRY(fv::keys_to_neighbors(ctx, so.keys, nq, int(k), int(k), d_out, d_counts));
   fv::stage_mark(ctx);
+  if (h_out) FV_TRY(fv::fetch_results(ctx, d_out, nq, k, h_out, h_counts));
   FV_CUDA(cudaStreamSynchronize(ctx->stream));
+  fv::ivfpq_scan_stats(ctx);
   fv::stage_end(ctx);
   return fv::bounds_report_ivfpq_scan();
 }
@@ -993,11 +997,7 @@ int fv_ivfpq_search_batch(fv_ivfpq* ix, const float* queries, size_t nq, size_t 
   fv_neighbor* dout = ctx->scratch[11].as<fv_neighbor>();
   uint32_t* dc = reinterpret_cast<uint32_t*>(ctx->scratch[11].as<unsigned char>() + obytes);
   FV_CUDA(cudaMemcpyAsync(dq, queries, qbytes, cudaMemcpyHostToDevice, ctx->stream));
-  FV_TRY(ivfpq_search_impl(ix, dq, nq, k, nprobe, refine, false, dout, dc, nullptr, nullptr));
-  FV_CUDA(cudaMemcpyAsync(out, dout, obytes, cudaMemcpyDeviceToHost, ctx->stream));
-  if (counts) FV_CUDA(cudaMemcpyAsync(counts, dc, nq * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-  FV_CUDA(cudaStreamSynchronize(ctx->stream));
-  return FV_OK;
+  return ivfpq_search_impl(ix, dq, nq, k, nprobe, refine, false, dout, dc, nullptr, nullptr, nullptr, nullptr, out, counts);
 }
 
 int fv_ivfpq_search(fv_ivfpq* ix, const float* query, size_t k, size_t nprobe, size_t refine, fv_neighbor* out,

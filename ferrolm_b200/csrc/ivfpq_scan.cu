@@ -1677,6 +1677,7 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
   const bool use_pre = ix.metric == FV_L2 && ix.pre != nullptr;
   const bool separable = use_pre || ix.metric == FV_INNER_PRODUCT;
   const size_t tab = size_t(ix.m) * KSUB;
+  FV_TRY(pin_ready(ctx));
   unsigned long long* d_rows = reinterpret_cast<unsigned long long*>(ctx->d_flags + 16);  // [0] per-query kernel, [1] list-major
   FV_CUDA(cudaMemsetAsync(d_rows, 0, 2 * sizeof(unsigned long long), ctx->stream));
   const float* qtab = nullptr;
@@ -2058,41 +2059,46 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       ctx->stats.launches += 2;
       FV_CUDA(cudaGetLastError());
     }
-    // one read-back for the whole scan: counters, pool fill, the kernel's error word, rows scanned
-    uint32_t h_ctr[LS_NCOUNTERS] = {};
-    std::vector<unsigned int> h_pool(size_t(tc_grid) + 1, 0u);
-    unsigned long long rows2[2] = {0, 0};
-    FV_CUDA(cudaMemcpyAsync(h_ctr, pb_set.counters, sizeof(h_ctr), cudaMemcpyDeviceToHost, ctx->stream));
+    if (out.then) FV_TRY(out.then());
+    // one read-back for the whole scan: rows scanned, counters, pool fill, the kernel's error word
+    unsigned long long* h_rows = reinterpret_cast<unsigned long long*>(ctx->h_pin);
+    uint32_t* h_ctr = reinterpret_cast<uint32_t*>(h_rows + 2);
+    uint32_t* h_pool = h_ctr + LS_NCOUNTERS;  // tc_grid counts, the error word
+    static_assert(FV_PIN_RESULTS >= 16 + 4 * LS_NCOUNTERS + 4 * (512 + 1), "the read-back has to fit the pinned page");
+    if (tc_grid > 512) return fail(FV_ERR_UNSUPPORTED, "more than 512 multiprocessors");
+    FV_CUDA(cudaMemcpyAsync(h_ctr, pb_set.counters, LS_NCOUNTERS * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     if (tc_grid) {
-      FV_CUDA(cudaMemcpyAsync(h_pool.data(), pool_cnt, size_t(tc_grid) * sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream));
-      FV_CUDA(cudaMemcpyAsync(&h_pool[tc_grid], tc_error_word(ix.recon), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      FV_CUDA(cudaMemcpyAsync(h_pool, pool_cnt, size_t(tc_grid) * sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream));
+      FV_CUDA(cudaMemcpyAsync(h_pool + tc_grid, tc_error_word(ix.recon), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     }
-    FV_CUDA(cudaMemcpyAsync(rows2, d_rows, sizeof(rows2), cudaMemcpyDeviceToHost, ctx->stream));
+    FV_CUDA(cudaMemcpyAsync(h_rows, d_rows, 2 * sizeof(*h_rows), cudaMemcpyDeviceToHost, ctx->stream));
     FV_CUDA(cudaStreamSynchronize(ctx->stream));
     if (tc_grid && h_pool[tc_grid]) return fail(FV_ERR_TIMEOUT, "a bounded wait inside the tensor-core kernel ran out");
     // survivors of the tensor-core pass: pairs re-scored exactly (a pool that ran over dropped the rest, and the
     // finishing kernel has put the queries they belonged to on the re-run list)
     for (int c = 0; c < tc_grid; ++c) ctx->stats.dist_evals += std::min(h_pool[c], pool_cap);
     const uint32_t n_rerun = h_ctr[LS_C_RERUN];
+    ctx->stats.regrown = h_ctr[LS_C_OVER];
+    ctx->stats.uncertified = n_rerun;
     if (n_rerun) {  // whatever is left: those queries once more, by the per-query kernel (their rows are counted already)
       ScanArgs r = a;
       r.qids = fa.rerun_ids;
       r.rows_scanned = nullptr;
       FV_TRY(launch_block_scan(ctx, r, n_rerun, use_pre));
+      if (out.then) FV_TRY(out.then());
     }
-    ctx->stats.regrown = h_ctr[LS_C_OVER];
-    ctx->stats.uncertified = n_rerun;
     stage_mark(ctx);  // 5
-    ctx->stats.rows_scanned = rows2[0] + rows2[1];
-    ctx->stats.rows_list_scan = rows2[1];
     return FV_OK;
   }
-  unsigned long long rows[2] = {0, 0};
-  FV_CUDA(cudaMemcpyAsync(rows, d_rows, sizeof(rows), cudaMemcpyDeviceToHost, ctx->stream));
-  FV_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (out.then) FV_TRY(out.then());
+  FV_CUDA(cudaMemcpyAsync(ctx->h_pin, d_rows, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
+  return FV_OK;
+}
+
+void ivfpq_scan_stats(fv_ctx* ctx) {
+  const unsigned long long* rows = reinterpret_cast<const unsigned long long*>(ctx->h_pin);  // per-query kernel, list-major
   ctx->stats.rows_scanned = rows[0] + rows[1];
   ctx->stats.rows_list_scan = rows[1];
-  return FV_OK;
 }
 
 }  // namespace fv

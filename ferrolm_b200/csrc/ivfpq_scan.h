@@ -41,6 +41,9 @@ struct ScanOut {
   fv_neighbor* adc;      // nq x keep kept candidates          (candidates == true)
   float* exact;          // nq x keep their exact distances
   uint32_t* counts;      // nq                                 (candidates == true)
+  // What follows on the keys (may be empty): launched before the host waits for the scan's counters, and once more if
+  // queries had to be re-run.
+  std::function<int()> then;
 };
 
 // mode: 0 = pick by size, 1 = one block per query only, 2 = the list-major table scan whenever the index allows it,
@@ -49,7 +52,9 @@ struct ScanOut {
 // `cells`: nq x nprobe keys (distance, list), ascending.  `keep` = candidates kept by compressed distance;
 // `refine`: re-rank them exactly and cut to k.  Marks the context's stages and fills stats.rows_scanned.
 // `cand_slots`: candidate slots per query of the list-major scans (0 = default).
-// Scratch slots used: 5, 6, 7, 8, 9, 12, 13, 14, 15, 18.
+// Scratch slots used: 5, 6, 7, 8, 9, 12, 13, 14, 15, 18.  The rows scanned are on their way to the context's pinned
+// memory when it returns: ivfpq_scan_stats puts them into the statistics once the stream has been waited for.
+void ivfpq_scan_stats(fv_ctx* ctx);
 int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* d_queries, size_t nq, const u64* d_cells, int nprobe,
                int keep, int k, bool refine, bool candidates, int mode, int cand_slots, const ScanOut& out);
 
