@@ -35,6 +35,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "ivfpq_scan.h"
 
 FV_BOUNDS_TU(ivfpq_scan)
@@ -485,6 +487,181 @@ __global__ void __launch_bounds__(256, 4) ivfpq_scan_kernel(ScanArgs a) {
     block_sort(lists, n);
   }
   scan_tail(a, q, lists, rerank, sq);
+}
+
+
+// The same search for results short enough for a warp's registers (keep <= 32 * KR; at most 32 of them after a
+// re-rank) and tables that separate into a list's and a query's part.  Every warp keeps its own best `keep` rows in
+// registers and all share the smallest of their bounds, so nothing is appended, sorted or compacted and no barrier
+// stands between the steps of a list; the shared memory the candidate buffer took lets one more block live on an SM.
+// Bound by the table lookups (bank conflicts: about 3.4 cycles of the SM per 32 of them).  With the buffer, and
+// without it: 32 queries, 16 probes of 590 rows, m = 16, 10 kept, the call 91 -> 77 us; 1,000 queries, 16 probes of 390
+// rows, m = 48, 40 kept and re-ranked, 373 -> 278 us.
+template <bool M16, int CW, int KR, bool PRE>
+__global__ void __launch_bounds__(256, 4) probe_scan_kernel(ScanArgs a) {
+  constexpr int WARPS = 8, NP = PRE ? 2 : 0, WC = WARPS - NP, R = 2;  // PRE: two warps build the next list's table
+  const int w = threadIdx.x >> 5, lane = lane_id(), tid = threadIdx.x, cw = w - NP;
+  const int tab = a.m * int(KSUB);
+  float* lut0 = reinterpret_cast<float*>(dyn_smem());  // tab, at a multiple of 1024 as lut_entry wants it; the lists of the
+  u64* lists = reinterpret_cast<u64*>(lut0);           // merges go over it when the scan is done: [WARPS][32 * KR]
+  float* lut1 = lut0 + max(tab, WARPS * 32 * KR * 2);  // PRE: the other table
+  float* sq = lut1 + (PRE ? tab : 0);                  // pd
+  u64* cand = reinterpret_cast<u64*>(sq + a.pd);       // keep
+  __shared__ uint32_t shared_hi;                       // no row whose distance word is above it can be kept
+  const size_t q = a.qids ? size_t(a.qids[blockIdx.x]) : size_t(blockIdx.x);
+  const float* qtab = a.qtab + q * size_t(tab);
+  for (int c = tid; c < a.pd; c += 256) sq[c] = a.queries[q * size_t(a.pd) + c];
+  if (tid == 0) shared_hi = 0xFFFFFFFFu;
+  if (!PRE)  // inner product: the query's own table is the lookup table (ivfpq.rs:236-238, :307)
+    for (int i = tid; i < tab / 4; i += 256) reinterpret_cast<float4*>(lut0)[i] = __ldg(reinterpret_cast<const float4*>(qtab) + i);
+  unsigned long long scanned = 0;
+  auto next_probe = [&](int p) {
+    for (p += a.splits; p < a.nprobe; p += a.splits) {
+      const u64 c = a.cells[q * size_t(a.nprobe) + p];
+      if (c == FV_EMPTY_KEY) return -1;
+      if (!FV_IDX_OK(key_id(c), a.nlist, 1)) continue;
+      return p;
+    }
+    return -1;
+  };
+  // table of list l (ivfpq.rs:256-262), by `nthr` threads of which this is number `t`
+  auto build_pre = [&](float* dst, uint32_t l, int t, int nthr) {
+    const float4* pre = reinterpret_cast<const float4*>(a.pre + size_t(l) * tab);
+    const float4* qt = reinterpret_cast<const float4*>(qtab);
+#pragma unroll 8
+    for (int i = t; i < tab / 4; i += nthr) {
+      const float4 x = __ldg(pre + i), y = __ldg(qt + i);
+      reinterpret_cast<float4*>(dst)[i] =
+          make_float4(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y), __fadd_rn(x.z, y.z), __fadd_rn(x.w, y.w));
+    }
+  };
+  int p = next_probe(int(blockIdx.y) - a.splits);
+  if (PRE && p >= 0) build_pre(lut0, key_id(a.cells[q * size_t(a.nprobe) + p]), tid, 256);
+  __syncthreads();
+
+  TopList<KR> top;
+  top.init(a.keep);
+  u64 bound = FV_EMPTY_KEY;
+  int cur = 0, steps = 0;  // which table the scan reads; steps of the lists so far, dealt to the warps in turn
+  while (p >= 0) {
+    const u64 cell = a.cells[q * size_t(a.nprobe) + p];
+    const uint32_t l = key_id(cell);
+    const size_t off = a.list_off[l];
+    const int len = int(a.list_off[l + 1] - off);
+    const int pnext = next_probe(p);
+    const float base = key_distance(cell);  // ivfpq.rs:256 (L2 with tables), :270 (inner product)
+    const uint32_t lut_s = uint32_t(__cvta_generic_to_shared(cur ? lut1 : lut0));
+    if (PRE && cw < 0 && pnext >= 0)
+      build_pre(cur ? lut0 : lut1, key_id(a.cells[q * size_t(a.nprobe) + pnext]), tid, NP * 32);
+    scanned += len;
+    const int nsteps = (len + 32 * R - 1) / (32 * R);
+    if (cw >= 0) {
+      int s0 = (cw - steps) % WC;
+      if (s0 < 0) s0 += WC;
+      for (int st = s0; st < nsteps; st += WC) {
+        float d[R];
+        uint32_t cws[R][4];
+        int row[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          row[i] = st * (32 * R) + i * 32 + lane;
+          d[i] = base;  // ivfpq.rs:273-276: base first, then the m table entries in order
+        }
+        for (int j0 = 0; j0 < a.m; j0 += 4 * CW) {
+#pragma unroll
+          for (int i = 0; i < R; ++i)  // (a lane past the end repeats the last row)
+            load_code<CW>(a.codes + (off + min(row[i], len - 1)) * size_t(a.m) + j0, cws[i]);
+          const uint32_t base_s = lut_s + uint32_t(j0) * 1024u;
+#define FV_ADC_STEP(J)                                                              \
+  _Pragma("unroll") for (int i = 0; i < R; ++i) d[i] = __fadd_rn(d[i], lut_entry<J>(cws[i][(J) >> 2], base_s));
+          FV_ADC_STEP(0) FV_ADC_STEP(1) FV_ADC_STEP(2) FV_ADC_STEP(3)
+          if (CW > 1) { FV_ADC_STEP(4) FV_ADC_STEP(5) FV_ADC_STEP(6) FV_ADC_STEP(7) }
+          if (CW > 2) {
+            FV_ADC_STEP(8) FV_ADC_STEP(9) FV_ADC_STEP(10) FV_ADC_STEP(11)
+            FV_ADC_STEP(12) FV_ADC_STEP(13) FV_ADC_STEP(14) FV_ADC_STEP(15)
+          }
+#undef FV_ADC_STEP
+          if (M16) break;
+        }
+        const uint32_t lim = min(*reinterpret_cast<volatile uint32_t*>(&shared_hi), uint32_t(bound >> 32));
+        bool pass[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) pass[i] = row[i] < len && d[i] < INFINITY && order_bits(d[i]) <= lim;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          if (__any_sync(FV_FULL, pass[i])) {  // the id is fetched only when it can matter
+            u64 key = FV_EMPTY_KEY;
+            if (pass[i] && FV_IDX_OK(off + row[i], a.nrows, 2)) key = make_key(d[i], __ldg(a.ids + off + row[i]));
+            top.offer(key, bound);
+          }
+        }
+        if (lane == 0 && uint32_t(bound >> 32) < lim) atomicMin(&shared_hi, uint32_t(bound >> 32));
+      }
+    }
+    steps += nsteps;
+    if (PRE) {
+      __syncthreads();  // the next table is ready and nobody reads this one any more
+      cur ^= 1;
+    }
+    p = pnext;
+  }
+  if (tid == 0 && a.rows_scanned) atomicAdd(a.rows_scanned, scanned);
+
+  // the lists of all warps into warp 0's, in pairs
+  auto merge_warps = [&](auto& list, int L, u64* buf) {
+    constexpr int PLACES = 32 * (sizeof(list.e) / sizeof(u64));
+    for (int step = 1; step < WARPS; step <<= 1) {
+      __syncthreads();
+      if ((w & (2 * step - 1)) == step) list.store(buf + w * PLACES, L);
+      __syncthreads();
+      if ((w & (2 * step - 1)) == 0) {
+        u64 c[PLACES / 32];
+        list.load(c, buf + (w + step) * PLACES, L);
+        list.merge(c);
+      }
+    }
+  };
+  merge_warps(top, a.keep, lists);
+  if (a.splits > 1) {  // the last block of the query to arrive takes in the others' lists
+    u64* parts = a.parts + q * size_t(a.splits) * a.keep;
+    if (w == 0) top.store(parts + size_t(blockIdx.y) * a.keep, a.keep);
+    __threadfence();
+    __syncthreads();
+    __shared__ uint32_t arrived;
+    if (tid == 0) arrived = atomicAdd(a.tickets + q, 1u);
+    __syncthreads();
+    if (arrived != uint32_t(a.splits - 1)) return;
+    __threadfence();
+    top.init(a.keep);
+    for (int i = w; i < a.splits; i += WARPS) {
+      u64 c[KR];
+#pragma unroll
+      for (int r = 0; r < KR; ++r) c[r] = r * 32 + lane < a.keep ? __ldcg(parts + size_t(i) * a.keep + r * 32 + lane) : FV_EMPTY_KEY;
+      top.merge(c);
+    }
+    merge_warps(top, a.keep, lists);
+  }
+  if (!a.refine) {  // ivfpq.rs:285-288
+    if (w == 0) top.store(a.out_keys + q * size_t(a.k), a.k);  // k == keep
+    return;
+  }
+  if (w == 0) top.store(cand, a.keep);
+  __syncthreads();
+  TopList<1> fin;
+  fin.init(a.k);
+  bound = FV_EMPTY_KEY;
+  for (int i0 = w * 8; i0 < a.keep; i0 += WARPS * 8) {  // exact distances (ivfpq.rs:289-296), eight rows per warp at a time
+    const int i = i0 + (lane >> 2);
+    const u64 c = i < a.keep ? cand[i] : FV_EMPTY_KEY;
+    size_t slot = size_t(key_id(c) - a.id_base);
+    const bool ok = c != FV_EMPTY_KEY && FV_IDX_OK(slot, a.nvec, 3);
+    if (!ok) slot = 0;
+    const float* row = a.vectors + slot * a.pd;
+    const float d = a.metric == FV_L2 ? group_distance<true, 4>(sq, row, a.pd) : group_distance<false, 4>(sq, row, a.pd);
+    fin.offer(ok && (lane & 3) == 0 ? make_key(d, key_id(c)) : FV_EMPTY_KEY, bound);
+  }
+  merge_warps(fin, a.k, lists);
+  if (w == 0) fin.store(a.out_keys + q * size_t(a.k), a.k);
 }
 
 
@@ -1573,20 +1750,42 @@ __global__ void __launch_bounds__(128) rescore_kernel(RescoreArgs a) {
 // scratch slot 6 holds the parts of a split search
 static int launch_block_scan(fv_ctx* ctx, ScanArgs a, size_t nblocks, bool use_pre) {
   const size_t tab = size_t(a.m) * KSUB;
-  const size_t smem = (2 * size_t(a.pd) + tab * (use_pre ? 2 : 1)) * sizeof(float) +
-                      (size_t(a.cap) + size_t(a.keep) + size_t(a.k)) * sizeof(u64);
+  // results that fit a warp's registers (see probe_scan_kernel)
+  const bool separable = use_pre || a.metric == FV_INNER_PRODUCT;
+  const bool in_regs = separable && !a.candidates && !a.bound_out && !a.row_budget && a.shard_world <= 1 && !a.owned_ids &&
+                       a.keep <= 128 && (a.refine ? a.k <= 32 : a.k == a.keep) && a.m % 4 == 0;
+  const int KR = a.keep <= 32 ? 1 : 4;
+  size_t smem;
+  void (*kern)(ScanArgs);
+  if (in_regs) {
+    smem = (std::max<size_t>(tab, size_t(8) * 32 * KR * 2) + (use_pre ? tab : 0) + size_t(a.pd)) * sizeof(float) + size_t(a.keep) * sizeof(u64);
+    auto pick = [&](auto kr, auto pre) -> void (*)(ScanArgs) {
+      constexpr int K = decltype(kr)::value;
+      constexpr bool P = decltype(pre)::value;
+      return a.m == 16       ? probe_scan_kernel<true, 4, K, P>
+             : a.m % 16 == 0 ? probe_scan_kernel<false, 4, K, P>
+             : a.m % 8 == 0  ? probe_scan_kernel<false, 2, K, P>
+                             : probe_scan_kernel<false, 1, K, P>;
+    };
+    using one = std::integral_constant<int, 1>;
+    using four = std::integral_constant<int, 4>;
+    kern = KR == 1 ? (use_pre ? pick(one{}, std::true_type{}) : pick(one{}, std::false_type{}))
+                   : (use_pre ? pick(four{}, std::true_type{}) : pick(four{}, std::false_type{}));
+  } else {
+    smem = (2 * size_t(a.pd) + tab * (use_pre ? 2 : 1)) * sizeof(float) + (size_t(a.cap) + size_t(a.keep) + size_t(a.k)) * sizeof(u64);
+    kern = a.m == 16       ? ivfpq_scan_kernel<true, 4, 2>
+           : a.m % 16 == 0 ? ivfpq_scan_kernel<false, 4, 2>
+           : a.m % 8 == 0  ? ivfpq_scan_kernel<false, 2, 2>
+           : a.m % 4 == 0  ? ivfpq_scan_kernel<false, 1, 2>
+                           : ivfpq_scan_kernel<false, 0, 1>;
+  }
   if (smem + 256 > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "m, k * refine too large for shared memory");
-  auto kern = a.m == 16       ? ivfpq_scan_kernel<true, 4, 2>
-              : a.m % 16 == 0 ? ivfpq_scan_kernel<false, 4, 2>
-              : a.m % 8 == 0  ? ivfpq_scan_kernel<false, 2, 2>
-              : a.m % 4 == 0  ? ivfpq_scan_kernel<false, 1, 2>
-                              : ivfpq_scan_kernel<false, 0, 1>;
   // A batch that leaves SMs without a block: each query's lists are dealt to several blocks, as long as one block can
   // sort what they leave (32 queries, 16 probes of 590 rows, m = 16: 89 us with a block per query, 35 us with 16).
   a.splits = 1;
   if (!a.row_budget && !a.qids) {
     const size_t room = size_t(ctx->sm_count) * 4 / nblocks;
-    a.splits = int(std::max<size_t>(1, std::min({room, size_t(a.nprobe), size_t(a.cap / a.keep)})));
+    a.splits = int(std::max<size_t>(1, std::min({room, size_t(a.nprobe), in_regs ? size_t(64) : size_t(a.cap / a.keep)})));
   }
   if (a.splits > 1) {
     const size_t part_bytes = nblocks * size_t(a.splits) * a.keep * sizeof(u64);

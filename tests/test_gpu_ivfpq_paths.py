@@ -1,0 +1,60 @@
+"""The per-query IVF-PQ scan over its branches: code loads of 4, 2 and 1 words and of single bytes, results in registers
+(up to 32, up to 128 kept) and in the block's buffer, one and several blocks per query; against the oracle."""
+import numpy as np
+import pytest
+
+from tests.parity import assert_same_neighbours
+
+pytestmark = pytest.mark.gpu
+
+L2, IP = 0, 1
+
+
+@pytest.fixture(scope="module")
+def made(oracle):
+    import ferrolm_b200 as fv
+
+    ctx = fv.Context(0)
+    cache = {}
+
+    def get(metric, m):
+        if (metric, m) not in cache:
+            dim = 96
+            base = oracle.testdata(5000, dim, 3)
+            base[100:140] = base[99]  # rows that tie, at the cut of some queries' lists too
+            if metric == IP:
+                base = oracle.normalize(base)
+            ix = fv.IvfPq.train(ctx, metric, dim, base[:1500], fv.IvfPqParams(20, m, 3, True, 1))
+            ix.add(base)
+            ix.set_scan_mode(1)
+            q = np.concatenate([base[99:100], oracle.testdata(699, dim, 4)])
+            cache[metric, m] = ix, oracle.IvfPq.load(ix.save()), oracle.normalize(q) if metric == IP else q
+        return cache[metric, m]
+
+    yield get
+    cache.clear()
+    ctx.close()
+
+
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("m", [6, 4, 8, 16, 24, 48])
+@pytest.mark.parametrize("k,refine", [(1, 0), (32, 0), (33, 0), (128, 0), (129, 0), (8, 4), (32, 4), (33, 3), (10, 12), (10, 13)])
+def test_scan_equals_the_oracle(made, metric, m, k, refine):
+    ix, o, q = made(metric, m)
+    for nq, nprobe in ((1, 20), (3, 7), (40, 1), (700, 3)):
+        got, gc = ix.search_batch(q[:nq], k, nprobe, refine)
+        want, wc = o.search_batch(q[:nq], k, nprobe, refine)
+        bits, total = assert_same_neighbours(got, gc, want, wc, f"m={m} nq={nq} nprobe={nprobe}")
+        assert bits == total
+
+
+@pytest.mark.parametrize("k,refine", [(10, 0), (32, 8), (10, 10), (40, 4), (10, 40)])
+def test_tensor_pass_finish_equals_the_per_query_scan(made, k, refine):
+    ix, _, q = made(L2, 16)
+    ix.set_scan_mode(1)
+    want, wc = ix.search_batch(q, k, 12, refine)
+    for mode in (3, 4):
+        ix.set_scan_mode(mode)
+        got, gc = ix.search_batch(q, k, 12, refine)
+        assert np.array_equal(gc, wc) and np.array_equal(got, want), f"mode {mode}"
+    ix.set_scan_mode(1)
