@@ -193,6 +193,25 @@ struct Beam {
       if (!(e[r] < key)) e[r] = prev < key ? key : prev;
     }
   }
+  // All pending keys at once, by a sort and a merge (bitonic_merge): what the insertions one by one would leave, as long
+  // as no entry that falls off the end is as far as the last one kept -- everything up to that distance is then admitted
+  // whenever it comes and never pushed out again, and nothing pushed out can tie.  Otherwise nothing is done.
+  __device__ __forceinline__ void take(unsigned& pending, u64 key, u64& bound, int& ntied) {
+    const u64 c = warp_sort32((pending >> lane_id()) & 1u ? key : FV_EMPTY_KEY);
+    const u64 back = __shfl_sync(FV_FULL, c, 31 - lane_id());
+    const u64 x = e[R - 1];
+    const u64 low = x < back ? x : back;
+    const uint32_t drop = __reduce_min_sync(FV_FULL, uint32_t((x < back ? back : x) >> 32));
+    uint32_t keep = __reduce_max_sync(FV_FULL, uint32_t(low >> 32));
+    if (R > 1) keep = max(keep, uint32_t(__shfl_sync(FV_FULL, e[R > 1 ? R - 2 : 0], 31) >> 32));
+    if (drop == keep && keep != 0xFFFFFFFFu) return;
+    e[R - 1] = low;
+    bitonic_merge<R>(e);
+    const u64 now = last();
+    if (uint32_t(now >> 32) < uint32_t(bound >> 32)) ntied = 0;
+    bound = now;
+    pending = 0;
+  }
   // the first entry that is not expanded: its position (-1: none) and key
   __device__ __forceinline__ int first_open(u64& key) const {
     int pos = -1;
@@ -261,6 +280,7 @@ struct Beam<0> {
     if (n < ef) n++;
     if (below < cursor) cursor = below;
   }
+  __device__ __forceinline__ void take(unsigned&, u64, u64&, int&) {}
   __device__ __forceinline__ int first_open(u64& key) const {
     for (int e0 = cursor & ~31; e0 < n; e0 += 32) {
       const int i = e0 + lane_id();
@@ -478,6 +498,8 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
       __syncwarp();
       const uint32_t hi = uint32_t(key >> 32);
       unsigned pending = __ballot_sync(FV_FULL, lane < nfresh && hi < uint32_t(bound >> 32));
+      if (R > 0 && __popc(pending) > (R == 1 ? 8 : R == 2 ? 6 : R == 4 ? 5 : 4))
+        best.take(pending, key, bound, ntied);  // (leaves them pending if ties at the cut need the order they came in)
       while (pending) {
         const int src = __ffs(pending) - 1;
         const u64 pushed = bound;  // the entry that falls off the end, if the beam is full
