@@ -392,7 +392,7 @@ static int search_shape(fv_ctx* ctx, bool is_l2, int pd, int ef, size_t active, 
   const int R = ef <= 32 ? 1 : ef <= 64 ? 2 : ef <= 128 ? 4 : ef <= 256 ? 8 : 0;
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
   const bool team = active <= size_t(ctx->sm_count) * TEAM_SEARCHES_PER_SM;
-  s->sbits = visit_sbits(ef, team ? 13 : 11);
+  s->sbits = visit_sbits(ef, team);
   size_t per = R == 0 ? search_smem<0>(pd, ef, s->sbits) : search_smem<1>(pd, ef, s->sbits);
   int W = 8;
   if (team) {

@@ -443,7 +443,7 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
   const bool is_l2 = h->metric == FV_L2;
   const size_t link_warp = link_smem(pd, int(m0));
-  int sbits = visit_sbits(int(ef), 11), team_sbits = visit_sbits(int(ef), 13), W = 8, LW = 8;
+  int sbits = visit_sbits(int(ef), false), team_sbits = visit_sbits(int(ef), true), W = 8, LW = 8;
   auto ins_bytes = [&](int bits) { return insert_smem(pd, int(m0), int(ef), bits); };
   while (W > 1 && ins_bytes(sbits) * W > budget / BUILD_BLOCKS_PER_SM) W >>= 1;
   while (LW > 1 && link_warp * LW > budget / BUILD_BLOCKS_PER_SM) LW >>= 1;
