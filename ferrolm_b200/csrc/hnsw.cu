@@ -1,20 +1,13 @@
-// Hnsw (src/vector/hnsw.rs): batched search on the GPU, one warp per query.
+// Hnsw (src/vector/hnsw.rs): batched search on the GPU, a warp per query or, for small batches, a team of warps.
 //
 // Device layout: data n x pd f32; links0 n x (m0+1) u32 (count, then ids) exactly as the
 // reference stores layer 0 (hnsw.rs:50-51, :154-157); the upper layers as one flat u32 array in
 // the order of the FLHNSW01 file (per node, per layer: count, ids) with a per-node start offset.
 //
-// Search of one query (hnsw.rs:323-351): greedy descent on the upper layers, then the best-first
-// beam of search_layer (hnsw.rs:179-226) kept as ONE sorted list of ef entries with an "expanded"
-// bit per entry.  That is the reference's pair of heaps: a candidate that has been evicted from
-// `best` can only be popped after every entry of `best` has been expanded, and then it trips the
-// stop test (hnsw.rs:203-205) unless its distance ties the current worst exactly.  Neighbours of
-// the expanded node are evaluated one per lane and offered to the list in stored order, so the
-// admission test (hnsw.rs:214) sees the same evolving bound as the sequential loop.
-//
-// The visited set is an exact open-addressing hash table per warp (shared memory when it fits,
-// global memory otherwise).  A query that fills more than half of it stops with an overflow mark
-// and is re-run by the host with a table four times larger.
+// Search of one query (hnsw.rs:323-351): greedy descent on the upper layers, then the best-first beam of search_layer
+// (hnsw.rs:179-226), both in hnsw.cuh: the beam as ONE sorted list of ef entries with an "expanded" bit per entry, the
+// visited set exact, in shared memory first and in global memory for what does not fit.  A query that fills more than
+// half of the second part stops with an overflow mark and is re-run by the host with a table four times larger.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
