@@ -647,18 +647,21 @@ __global__ void __launch_bounds__(256, 4) probe_scan_kernel(ScanArgs a) {
   }
   if (w == 0) top.store(cand, a.keep);
   __syncthreads();
+  int used = 0;  // candidates found, at the front of `cand`; an index without rows has none, nor vectors to read
+  for (int e0 = 0; e0 < a.keep; e0 += 32)
+    used += __popc(__ballot_sync(FV_FULL, e0 + lane < a.keep && cand[e0 + lane] != FV_EMPTY_KEY));
   TopList<1> fin;
   fin.init(a.k);
   bound = FV_EMPTY_KEY;
-  for (int i0 = w * 8; i0 < a.keep; i0 += WARPS * 8) {  // exact distances (ivfpq.rs:289-296), eight rows per warp at a time
+  for (int i0 = w * 8; i0 < used; i0 += WARPS * 8) {  // exact distances (ivfpq.rs:289-296), eight rows per warp at a time
     const int i = i0 + (lane >> 2);
-    const u64 c = i < a.keep ? cand[i] : FV_EMPTY_KEY;
+    const u64 c = cand[min(i, used - 1)];  // (a group of lanes past the end repeats the last row)
     size_t slot = size_t(key_id(c) - a.id_base);
-    const bool ok = c != FV_EMPTY_KEY && FV_IDX_OK(slot, a.nvec, 3);
+    const bool ok = FV_IDX_OK(slot, a.nvec, 3);
     if (!ok) slot = 0;
     const float* row = a.vectors + slot * a.pd;
     const float d = a.metric == FV_L2 ? group_distance<true, 4>(sq, row, a.pd) : group_distance<false, 4>(sq, row, a.pd);
-    fin.offer(ok && (lane & 3) == 0 ? make_key(d, key_id(c)) : FV_EMPTY_KEY, bound);
+    fin.offer(ok && i < used && (lane & 3) == 0 ? make_key(d, key_id(c)) : FV_EMPTY_KEY, bound);
   }
   merge_warps(fin, a.k, lists);
   if (w == 0) fin.store(a.out_keys + q * size_t(a.k), a.k);
