@@ -511,6 +511,7 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   ctx->stats.expansions = total[1];
   ctx->stats.uncertified = total[2];  // queries whose list of tied, pushed-out entries overflowed (see TIED_CAP)
   if (h_out) FV_TRY(fetch_results(ctx, d_out, nq, k, h_out, h_counts, fetched));
+  if (ctx->timing) FV_CUDA(cudaStreamSynchronize(ctx->stream));  // the mark was recorded after the last wait
   stage_end(ctx);
   return bounds_report_hnsw();
 }
