@@ -2243,11 +2243,13 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
     if (fsmem + 256 > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "k * refine too large for shared memory");
     if (fsmem > 40 * 1024)
       FV_CUDA(cudaFuncSetAttribute(ivfpq_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(fsmem)));
-    if (!candidates && !ix.owned_ids && k <= 32 && keep <= 256) {
+    // eight queries' vectors and selected ids per block: up to about 7,200 dimensions
+    const size_t wsmem = size_t(8) * (ix.pd + ((keep + 7) & ~7)) * sizeof(float);
+    if (!candidates && !ix.owned_ids && k <= 32 && keep <= 256 && wsmem + 256 <= ctx->smem_optin) {
       FV_TRY(ctx->scratch[18].reserve(nq * sizeof(uint32_t)));
       uint32_t* large = ctx->scratch[18].as<uint32_t>();
-      const size_t wsmem = size_t(8) * (ix.pd + ((keep + 7) & ~7)) * sizeof(float);
       auto fw = ix.metric == FV_L2 ? finish_warp_kernel<true> : finish_warp_kernel<false>;
+      if (wsmem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(fw, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wsmem)));
       fw<<<unsigned((nq + 7) / 8), 256, wsmem, ctx->stream>>>(a, fa, nq, large);
       FinishArgs fl = fa;  // (a count only the device knows; nearly always none)
       fl.qids = large;

@@ -58,3 +58,23 @@ def test_tensor_pass_finish_equals_the_per_query_scan(made, k, refine):
         got, gc = ix.search_batch(q, k, 12, refine)
         assert np.array_equal(gc, wc) and np.array_equal(got, want), f"mode {mode}"
     ix.set_scan_mode(1)
+
+
+# the finishing step's queries and selected ids in shared memory: at and beyond the 48 KB a launch has unasked, and
+# beyond what an SM has
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("dim,k,refine", [(1520, 10, 0), (1536, 10, 0), (1536, 10, 4), (1400, 32, 8), (8000, 10, 4)])
+def test_table_scan_of_long_vectors(oracle, metric, dim, k, refine):
+    import ferrolm_b200 as fv
+
+    ctx = fv.Context(0)
+    base, q = oracle.testdata(1500, dim, 3), oracle.testdata(40, dim, 4)
+    ix = fv.IvfPq.train(ctx, metric, dim, base[:300], fv.IvfPqParams(8, 16, 1, True, 1))
+    ix.add(base)
+    want, wc = oracle.IvfPq.load(ix.save()).search_batch(q, k, 4, refine)
+    for mode in (1, 2):
+        ix.set_scan_mode(mode)
+        got, gc = ix.search_batch(q, k, 4, refine)
+        bits, total = assert_same_neighbours(got, gc, want, wc, f"mode {mode}")
+        assert bits == total
+    ctx.close()
