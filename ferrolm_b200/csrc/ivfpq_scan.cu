@@ -1243,8 +1243,9 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
     lo[j] = uint32_t(key);
   }
   for (int c = lane; c < a.pd; c += 32) sq[c] = a.queries[q * size_t(a.pd) + c];
-  // The best `keep`: the rows whose word is below T, and those at T with ids up to id_cut.
+  // The best `keep`: the rows whose word is below T, those at T with ids below id_cut, and `room` of those at both.
   uint32_t T = 0xFFFFFFFFu, id_cut = 0xFFFFFFFFu;
+  int room = 0;  // rows AT the cut that belong to the best `keep`: one, unless a file holds an id more than once
   if (have > a.keep) {
     auto count_le = [&](uint32_t x) {
       int c = 0;
@@ -1275,7 +1276,7 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
     }
     T = lo_w;
     if (at < 0) at = count_le(T);
-    if (at > a.keep) {  // rows tie at the cut: the smallest ids among them (ids are unique)
+    if (at > a.keep) {  // rows tie at the cut: the smallest ids among them
       const int want = a.keep - (T ? count_le(T - 1) : 0);
       uint32_t l = 0, h = 0xFFFFFFFFu;
       while (l < h) {
@@ -1287,6 +1288,10 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
         else l = mid + 1;
       }
       id_cut = l;
+      int below = 0;
+#pragma unroll
+      for (int j = 0; j < FW_NPL; ++j) below += (j * 32 + lane < have && hi[j] == T && lo[j] < id_cut) ? 1 : 0;
+      room = want - __reduce_add_sync(FV_FULL, below);
     }
   }
   TopList<1> top;
@@ -1295,7 +1300,11 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
   int nsel = 0;
 #pragma unroll
   for (int j = 0; j < FW_NPL; ++j) {
-    const bool take = j * 32 + lane < have && (hi[j] < T || (hi[j] == T && lo[j] <= id_cut));
+    const bool live = j * 32 + lane < have;
+    bool take = live && (hi[j] < T || (hi[j] == T && lo[j] < id_cut));
+    const unsigned at_cut = __ballot_sync(FV_FULL, live && hi[j] == T && lo[j] == id_cut);
+    if ((at_cut >> lane) & 1u) take = __popc(at_cut & ((1u << lane) - 1u)) < room;
+    room = max(0, room - __popc(at_cut));
     const unsigned m = __ballot_sync(FV_FULL, take);
     if (m == 0) continue;
     if (!a.refine) {  // the compressed distances are the result

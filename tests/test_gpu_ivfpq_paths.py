@@ -78,3 +78,29 @@ def test_table_scan_of_long_vectors(oracle, metric, dim, k, refine):
         bits, total = assert_same_neighbours(got, gc, want, wc, f"mode {mode}")
         assert bits == total
     ctx.close()
+
+
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("k,refine", [(10, 0), (32, 0), (10, 4), (8, 10)])
+def test_a_file_that_holds_ids_more_than_once(made, oracle, metric, k, refine):
+    import ferrolm_b200 as fv
+
+    ix, _, q = made(metric, 16)
+    data = bytearray(ix.save())
+    nlist, m, dim = 20, 16, 96
+    at = 8 + 5 * 4 + 8 + nlist * dim * 4 + 8 + m * 256 * (dim // m) * 4
+    for _ in range(nlist):  # per list: count, ids, bytes of codes, codes; the first 60 rows become copies of the first
+        n = int.from_bytes(data[at : at + 8], "little")
+        c, d = at + 8 + 4 * n + 8, min(n, 60)
+        data[at + 8 : at + 8 + 4 * d] = bytes(data[at + 8 : at + 12]) * d
+        data[c : c + m * d] = bytes(data[c : c + m]) * d
+        at = c + n * m
+    ctx = fv.Context(0)
+    dup, o = fv.IvfPq.load(ctx, bytes(data)), oracle.IvfPq.load(bytes(data))
+    want, wc = o.search_batch(q, k, 5, refine)
+    for mode in (1, 2, 3):
+        dup.set_scan_mode(mode)
+        got, gc = dup.search_batch(q, k, 5, refine)
+        bits, total = assert_same_neighbours(got, gc, want, wc, f"mode {mode}")
+        assert bits == total
+    ctx.close()
