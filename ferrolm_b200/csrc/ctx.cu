@@ -16,6 +16,9 @@ int fail(int status, const std::string& msg) {
   return status;
 }
 
+static thread_local size_t g_alloc_limit = 0;
+bool alloc_refused(size_t bytes) { return g_alloc_limit && bytes > g_alloc_limit; }
+
 static std::mutex g_ctx_mutex;
 }  // namespace fv
 static void ctx_destroy_now(fv_ctx* ctx);
@@ -134,6 +137,11 @@ static void ctx_destroy_now(fv_ctx* ctx) {
 }
 
 extern "C" {
+
+int fv_debug_alloc_limit(size_t bytes) {
+  fv::g_alloc_limit = bytes;
+  return FV_OK;
+}
 
 const char* fv_last_error(void) { return fv::g_error.c_str(); }
 const char* fv_version(void) { return "ferrovec 0.1 (sm_100a)"; }

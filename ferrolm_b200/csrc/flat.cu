@@ -464,6 +464,10 @@ int few_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, con
   return FV_OK;
 }
 
+// Keys written at a time by the scan that keeps them all: 256 MB.  The workspace stays with the context, and a batch of
+// that size fills the GPU many times over (8,192 queries of 4,096 rows).
+static constexpr size_t DENSE_KEYS = size_t(1) << 25;
+
 int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, const float* d_queries, size_t q_stride,
                const uint32_t* d_query_ids, size_t nq, int L, bool prefilter_inf, uint32_t id_base, u64* d_out_keys,
                int scratch_slot) {
@@ -488,43 +492,50 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
   // (both launches): 1,000 queries, 16 of 256 cells x 384: 67 us against 205; 32 queries, 16 of 512 cells x 128: 15 us
   // against 45; 10,000 queries, 64 of 1,024 cells x 128: 218 us, with the lists over 1,000.
   // (not where the keys of a very large batch would take more than 1 GB that the lists do without)
+  const size_t most = std::max<size_t>(64, DENSE_KEYS / std::max<size_t>(1, n)), runs = (nq + most - 1) / most;
+  const size_t chunk = (nq + runs - 1) / runs;  // queries at a time
   if (L >= 2 && n > 0 && n <= 4096 && !d_query_ids && size_t(8) * (size_t(pd) * 4 + 8) <= budget &&
-      (L >= 32 || nq * n * sizeof(u64) <= size_t(1) << 30)) {
+      (L >= 32 || nq * n * sizeof(u64) <= size_t(1) << 30) &&
+      ctx->scratch[scratch_slot].reserve(chunk * n * sizeof(u64)) == FV_OK) {  // (no room for the keys: the lists)
     int npow2 = 32;
     while (size_t(npow2) < n) npow2 <<= 1;
-    FV_TRY(ctx->scratch[scratch_slot].reserve(nq * n * sizeof(u64)));
     u64* dense = ctx->scratch[scratch_slot].as<u64>();
     const int w4 = 4;
     const size_t row_bytes = size_t(pd) * 4 + 8;
-    // two queries per warp where eight would leave SMs idle or pass the shared memory of a block
-    int DQ = 8;
-    const size_t most_splits = std::max<size_t>(1, n / 32);
-    if ((nq + 31) / 32 * most_splits < size_t(ctx->sm_count) * 4 || size_t(w4) * 8 * row_bytes > budget) DQ = 2;
-    const size_t groups = (nq + size_t(DQ) * w4 - 1) / (size_t(DQ) * w4);
-    size_t S = std::max<size_t>(1, std::min(most_splits, (size_t(ctx->sm_count) * 8 + groups - 1) / groups));
-    size_t rps = ((n + S - 1) / S + 31) / 32 * 32;
-    S = (n + rps - 1) / rps;
-    const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(S));
-    const size_t smem = size_t(w4) * DQ * row_bytes;
-    if (DQ == 8)
-      FV_TRY(launch_scan<8>(ctx, metric == FV_L2, grid, w4 * 32, smem, d_rows, n, pd, d_queries, q_stride, nullptr, nq, 1,
-                            prefilter_inf, id_base, rps, nullptr, dense, n));
-    else
-      FV_TRY(launch_scan<2>(ctx, metric == FV_L2, grid, w4 * 32, smem, d_rows, n, pd, d_queries, q_stride, nullptr, nq, 1,
-                            prefilter_inf, id_base, rps, nullptr, dense, n));
-    if (n <= 2048 && L <= 256) {
-      int lp = 32;
-      while (lp < L) lp <<= 1;
-      const unsigned blocks = unsigned((nq + 3) / 4);
-      if (n <= 1024)
-        warp_select_kernel<32><<<blocks, 128, size_t(4) * lp * 8, ctx->stream>>>(dense, n, int(n), L, lp, nq, d_out_keys);
+    for (size_t q0 = 0; q0 < nq; q0 += chunk) {
+      const size_t nc = std::min(chunk, nq - q0);
+      const float* queries = d_queries + q0 * q_stride;
+      u64* out = d_out_keys + q0 * size_t(L);
+      // two queries per warp where eight would leave SMs idle or pass the shared memory of a block
+      int DQ = 8;
+      const size_t most_splits = std::max<size_t>(1, n / 32);
+      if ((nc + 31) / 32 * most_splits < size_t(ctx->sm_count) * 4 || size_t(w4) * 8 * row_bytes > budget) DQ = 2;
+      const size_t groups = (nc + size_t(DQ) * w4 - 1) / (size_t(DQ) * w4);
+      size_t S = std::max<size_t>(1, std::min(most_splits, (size_t(ctx->sm_count) * 8 + groups - 1) / groups));
+      size_t rps = ((n + S - 1) / S + 31) / 32 * 32;
+      S = (n + rps - 1) / rps;
+      const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(S));
+      const size_t smem = size_t(w4) * DQ * row_bytes;
+      if (DQ == 8)
+        FV_TRY(launch_scan<8>(ctx, metric == FV_L2, grid, w4 * 32, smem, d_rows, n, pd, queries, q_stride, nullptr, nc, 1,
+                              prefilter_inf, id_base, rps, nullptr, dense, n));
       else
-        warp_select_kernel<64><<<blocks, 128, size_t(4) * lp * 8, ctx->stream>>>(dense, n, int(n), L, lp, nq, d_out_keys);
-    } else {
-      block_select_kernel<<<unsigned(nq), 256, size_t(npow2) * 8, ctx->stream>>>(dense, n, int(n), npow2, L, d_out_keys);
+        FV_TRY(launch_scan<2>(ctx, metric == FV_L2, grid, w4 * 32, smem, d_rows, n, pd, queries, q_stride, nullptr, nc, 1,
+                              prefilter_inf, id_base, rps, nullptr, dense, n));
+      if (n <= 2048 && L <= 256) {
+        int lp = 32;
+        while (lp < L) lp <<= 1;
+        const unsigned blocks = unsigned((nc + 3) / 4);
+        if (n <= 1024)
+          warp_select_kernel<32><<<blocks, 128, size_t(4) * lp * 8, ctx->stream>>>(dense, n, int(n), L, lp, nc, out);
+        else
+          warp_select_kernel<64><<<blocks, 128, size_t(4) * lp * 8, ctx->stream>>>(dense, n, int(n), L, lp, nc, out);
+      } else {
+        block_select_kernel<<<unsigned(nc), 256, size_t(npow2) * 8, ctx->stream>>>(dense, n, int(n), npow2, L, out);
+      }
+      ctx->stats.launches++;
+      FV_CUDA(cudaGetLastError());
     }
-    ctx->stats.launches++;
-    FV_CUDA(cudaGetLastError());
     return FV_OK;
   }
   const size_t qgroups = (nq + size_t(QT) * W - 1) / (size_t(QT) * W);

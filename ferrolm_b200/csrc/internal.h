@@ -12,6 +12,10 @@
 
 #include "common.cuh"
 
+namespace fv {
+bool alloc_refused(size_t bytes);  // the test hook fv_debug_alloc_limit
+}
+
 // A growable device allocation (raw bytes).
 struct DevBuf {
   void* p = nullptr;
@@ -30,7 +34,7 @@ struct DevBuf {
     if (bytes <= cap) return FV_OK;
     release();
     size_t want = bytes + bytes / 8 + 256;
-    cudaError_t e = cudaMalloc(&p, want);
+    cudaError_t e = fv::alloc_refused(want) ? cudaErrorMemoryAllocation : cudaMalloc(&p, want);
     if (e != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();

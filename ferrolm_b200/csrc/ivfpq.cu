@@ -650,13 +650,13 @@ int fv_ivfpq_train(fv_ctx* ctx, int metric, uint32_t dim, const float* sample, s
   const size_t dsub = ix->dsub, ksub = std::min(fv::KSUB, n);
   ix->h_codebooks.assign(p->m * fv::KSUB * dsub, 0.f);
   const size_t ps = fv::padded(dsub);  // sub-vectors are padded when dsub is not a multiple of 8 (ivfpq.rs:80-87)
-  // the sub-quantizers are independent: as many at once as 1 GB of sub-vectors holds
-  const size_t batch = std::min(p->m, std::max<size_t>(1, (size_t(1) << 30) / (n * ps * sizeof(float))));
-  FV_TRY(d_sub.reserve(batch * n * ps * sizeof(float)));
-  FV_TRY(d_cb.reserve(batch * ksub * ps * sizeof(float)));
+  // the sub-quantizers are independent: as many at once as 1 GB of sub-vectors holds, and fewer where the device has no
+  // room for them
+  size_t batch = std::min(p->m, std::max<size_t>(1, (size_t(1) << 30) / (n * ps * sizeof(float))));
   std::vector<float> cb(batch * ksub * ps);
-  for (size_t j0 = 0; j0 < p->m; j0 += batch) {
-    const size_t nz = std::min(batch, p->m - j0);
+  auto train_batch = [&](size_t j0, size_t nz) -> int {
+    FV_TRY(d_sub.reserve(nz * n * ps * sizeof(float)));
+    FV_TRY(d_cb.reserve(nz * ksub * ps * sizeof(float)));
     fv::split_residuals_kernel<<<dim3(unsigned(ctx->sm_count * 4), unsigned(nz)), 256, 0, ctx->stream>>>(
         d_x.as<float>(), d_assign.as<uint32_t>(), d_cen.as<float>(), n, int(pd), int(dsub), int(ps), int(j0), d_sub.as<float>());
     ctx->stats.launches++;
@@ -664,9 +664,21 @@ int fv_ivfpq_train(fv_ctx* ctx, int metric, uint32_t dim, const float* sample, s
     FV_TRY(fv::kmeans_train_dev(ctx, d_sub.as<float>(), n, nz, ps, ksub, p->iters, p->seed + 1 + j0, d_cb.as<float>()));
     FV_CUDA(cudaMemcpyAsync(cb.data(), d_cb.p, nz * ksub * ps * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     FV_CUDA(cudaStreamSynchronize(ctx->stream));
+    return FV_OK;
+  };
+  for (size_t j0 = 0; j0 < p->m;) {
+    const size_t nz = std::min(batch, p->m - j0);
+    const int status = train_batch(j0, nz);
+    if (status == FV_ERR_NOMEM && batch > 1) {
+      d_sub.release();
+      batch = (batch + 1) / 2;
+      continue;
+    }
+    FV_TRY(status);
     for (size_t z = 0; z < nz; z++)
       for (size_t r = 0; r < ksub; r++)
         std::memcpy(&ix->h_codebooks[((j0 + z) * fv::KSUB + r) * dsub], &cb[(z * ksub + r) * ps], dsub * sizeof(float));
+    j0 += nz;
   }
   ix->h_off.assign(ix->nlist + 1, 0);
   FV_TRY(fv::upload_quantizers(ix.get()));

@@ -1,0 +1,81 @@
+"""Searches and trainings on a device with little room: a workspace that cannot be had is done without."""
+import contextlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+L2, IP = 0, 1
+
+
+@contextlib.contextmanager
+def at_most(nbytes):
+    from ferrolm_b200._lib import check, lib
+
+    check(lib().fv_debug_alloc_limit(nbytes))
+    try:
+        yield
+    finally:
+        check(lib().fv_debug_alloc_limit(0))
+
+
+@pytest.fixture()
+def ctx():
+    import ferrolm_b200 as fv
+
+    c = fv.Context(0)  # one per test: workspaces stay with their context
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("metric,k", [(L2, 10), (IP, 2), (L2, 40)])
+def test_search_of_few_rows_without_room_for_every_key(oracle, ctx, metric, k):
+    import ferrolm_b200 as fv
+
+    base, q = oracle.testdata(4000, 48, 1), oracle.testdata(3000, 48, 2)
+    ix = fv.FlatIndex(ctx, metric, 48)
+    ix.add(base)
+    with at_most(16 << 20):  # the keys take 96 MB
+        got, gc = ix.search_batch(q, k)
+    want, wc = ix.search_batch(q, k)
+    assert got.tobytes() == want.tobytes() and (gc == wc).all()
+    o = oracle.FlatIndex(metric, 48)
+    o.add(base)
+    assert o.search_batch(q[:100], k)[0].tobytes() == want[:100].tobytes()
+
+
+def test_search_of_few_rows_in_several_runs(oracle, ctx):
+    import ferrolm_b200 as fv
+
+    # the keys of at most 8,388 queries of 4,000 rows are written at a time: two runs
+    base, q = oracle.testdata(4000, 24, 1), oracle.testdata(9001, 24, 2)
+    ix = fv.FlatIndex(ctx, L2, 24)
+    ix.add(base)
+    got, gc = ix.search_batch(q, 33)
+    o = oracle.FlatIndex(L2, 24)
+    o.add(base)
+    want, wc = o.search_batch(q, 33)
+    assert got.tobytes() == want.tobytes() and (gc == wc).all()
+
+
+@pytest.mark.parametrize("m,limit", [(16, 2 << 20), (16, 1_800_000), (12, 2_000_000)])
+def test_training_without_room_for_all_sub_quantizers(oracle, ctx, m, limit):
+    import ferrolm_b200 as fv
+
+    dim = m * 4  # sub-vectors of 4 are padded to 8: together twice the sample's size (3.5 MB at m = 16)
+    sample = oracle.testdata(6000, dim, 1)
+    p = fv.IvfPqParams(20, m, 2, True, 1)
+    with at_most(limit):
+        small = fv.IvfPq.train(ctx, L2, dim, sample, p)
+    assert small.save() == fv.IvfPq.train(ctx, L2, dim, sample, p).save()
+
+
+def test_what_cannot_be_done_without_is_an_error(oracle, ctx):
+    import ferrolm_b200 as fv
+    from ferrolm_b200._lib import FV_ERR_NOMEM
+
+    with at_most(1 << 20), pytest.raises(fv.FerrovecError) as e:
+        fv.IvfPq.train(ctx, L2, 64, oracle.testdata(6000, 64, 1), fv.IvfPqParams(20, 16, 2, True, 1))
+    assert e.value.status == FV_ERR_NOMEM
+    assert len(fv.IvfPq.train(ctx, L2, 64, oracle.testdata(6000, 64, 1), fv.IvfPqParams(20, 16, 2, True, 1))) == 0
