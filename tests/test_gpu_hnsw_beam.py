@@ -57,9 +57,31 @@ def test_search_equals_the_oracle(setup, oracle, metric, n, dim, m, efc, ef, nq)
     got, gc = g.search_batch(q, k, ef)
     stats = ctx.stats()
     want, wc, work = o.search_batch(q, k, ef, want_work=True)
-    if stats["uncertified"] == 0:  # (a tie list that overflowed may resolve later ties differently)
-        assert np.array_equal(gc, wc) and np.array_equal(got["id"], want["id"])
-        assert np.array_equal(got["distance"].view(np.uint32), want["distance"].view(np.uint32))
+    same = (gc == wc) & (got.view(np.uint64) == want.view(np.uint64)).all(axis=1)  # ids and distance bits
+    # a query whose tie list overflowed may resolve later ties differently; all others may not
+    assert (~same).sum() <= stats["uncertified"] <= 0.01 * nq, (int((~same).sum()), stats["uncertified"])
+    if stats["uncertified"] == 0:
         assert stats["dist_evals"] == work[0] and stats["expansions"] == work[1]
-    else:
-        assert stats["uncertified"] <= 0.01 * nq + 1
+
+
+def test_queries_that_overflow_the_visited_set_are_run_again(setup, oracle):
+    import torch
+
+    import ferrolm_b200 as fv
+
+    # 128 links a node and a beam of 32: half of the queries visit more nodes than both parts of the set take
+    _, ctx = setup
+    rng = np.random.default_rng(1)
+    n, dim, nq, k, ef = 20_000, 100, TEAM_MAX + 30, 5, 32
+    base, q = (rng.standard_normal((r, dim)).astype(np.float32) for r in (n, nq))
+    o = oracle.Hnsw.build_batched(L2, dim, base, m=64, ef_construction=64, seed=1, max_batch=4096, divisor=1)
+    g = fv.Hnsw.load(ctx, o.save())
+    want, wc, work = o.search_batch(q, k, ef, want_work=True)
+    got, gc = g.search_batch(q, k, ef)
+    st = ctx.stats()
+    assert got.tobytes() == want.tobytes() and (gc == wc).all()
+    assert st["regrown"] > nq // 10 and (st["dist_evals"], st["expansions"]) == tuple(work[:2])
+    out, dc = g.search_batch(torch.from_numpy(q).cuda(), k, ef)
+    st = ctx.stats()
+    assert fv.neighbors_from_tensor(out).tobytes() == want.tobytes() and (dc.cpu().numpy() == wc).all()
+    assert st["regrown"] > nq // 10 and (st["dist_evals"], st["expansions"]) == tuple(work[:2])

@@ -63,7 +63,7 @@ def test_tensor_pass_finish_equals_the_per_query_scan(made, k, refine):
 # the finishing step's queries and selected ids in shared memory: at and beyond the 48 KB a launch has unasked, and
 # beyond what an SM has
 @pytest.mark.parametrize("metric", [L2, IP])
-@pytest.mark.parametrize("dim,k,refine", [(1520, 10, 0), (1536, 10, 0), (1536, 10, 4), (1400, 32, 8), (8000, 10, 4)])
+@pytest.mark.parametrize("dim,k,refine", [(1520, 10, 0), (1536, 10, 0), (1536, 10, 4), (1408, 32, 8), (8000, 10, 4)])
 def test_table_scan_of_long_vectors(oracle, metric, dim, k, refine):
     import ferrolm_b200 as fv
 
@@ -103,4 +103,27 @@ def test_a_file_that_holds_ids_more_than_once(made, oracle, metric, k, refine):
         got, gc = dup.search_batch(q, k, 5, refine)
         bits, total = assert_same_neighbours(got, gc, want, wc, f"mode {mode}")
         assert bits == total
+    ctx.close()
+
+
+# 4,096 lists and more are looked for by the tensor-core front end: up to 32 probes, and from 33 with its long results
+@pytest.mark.parametrize("metric", [L2, IP])
+def test_many_probes_of_many_lists(oracle, metric):
+    import ferrolm_b200 as fv
+
+    ctx = fv.Context(0)
+    base, q = oracle.testdata(9000, 32, 3), oracle.testdata(300, 32, 4)
+    if metric == IP:
+        base, q = oracle.normalize(base), oracle.normalize(q)
+    ix = fv.IvfPq.train(ctx, metric, 32, base, fv.IvfPqParams(4100, 8, 1, True, 1))
+    ix.add(base)
+    o = oracle.IvfPq.load(ix.save())
+    for nprobe in (32, 33, 100, 128, 129):
+        got, gc = ix.search_batch(q, 10, nprobe, 4)
+        launches = ctx.stats()["launches"]
+        want, wc = o.search_batch(q, 10, nprobe, 4)
+        bits, total = assert_same_neighbours(got, gc, want, wc, f"{nprobe} probes")
+        assert bits == total
+        # tables, scan and conversion; the coarse step's passes besides
+        assert (launches >= 8) == (nprobe <= 128), launches
     ctx.close()
