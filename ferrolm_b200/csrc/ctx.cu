@@ -1,5 +1,6 @@
 // Context, error reporting and the small host-side helpers of src/vector/mod.rs.
 #include <cmath>
+#include <map>
 #include <mutex>
 #include <thread>
 #include <unordered_set>
@@ -84,6 +85,17 @@ int upload_padded(fv_ctx* ctx, const float* src, bool src_is_device, size_t n, s
   FV_CUDA(cudaMemsetAsync(d_dst, 0, n * pd * sizeof(float), ctx->stream));
   FV_CUDA(cudaMemcpy2DAsync(d_dst, pd * sizeof(float), src, dim * sizeof(float), dim * sizeof(float), n,
                             cudaMemcpyHostToDevice, ctx->stream));
+  return FV_OK;
+}
+
+int allow_smem_of(fv_ctx* ctx, const void* kern, size_t bytes) {
+  static std::mutex m;
+  static std::map<std::pair<const void*, int>, size_t> allowed;  // an entry per kernel and device
+  std::lock_guard<std::mutex> g(m);
+  size_t& have = allowed[{kern, ctx->device}];
+  if (bytes <= have) return FV_OK;
+  FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  have = bytes;
   return FV_OK;
 }
 

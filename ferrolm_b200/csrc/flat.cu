@@ -421,7 +421,7 @@ static int launch_scan(fv_ctx* ctx, bool is_l2, dim3 grid, int threads, size_t s
   auto k = is_l2 ? (tiled ? exact_scan_kernel<QT, true, true> : exact_scan_kernel<QT, true, false>)
                  : (tiled ? exact_scan_kernel<QT, false, true> : exact_scan_kernel<QT, false, false>);
   if (tiled) smem = with_tile;
-  if (smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FV_TRY(allow_smem(ctx, k, smem));
   k<<<grid, threads, smem, ctx->stream>>>(rows, n, pd, q, q_stride, qids, nq, L, prefilter ? 1 : 0, id_base, rps, parts,
                                           dense, dense_stride);
   ctx->stats.launches++;
@@ -571,8 +571,7 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
     int wpb = 4;
     while (wpb > 1 && size_t(wpb) * L * 8 > 96 * 1024) wpb >>= 1;
     const size_t msmem = size_t(wpb) * L * 8;
-    if (msmem > 40 * 1024)
-      FV_CUDA(cudaFuncSetAttribute(merge_keys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(msmem)));
+    FV_TRY(allow_smem(ctx, merge_keys_kernel, msmem));
     merge_keys_kernel<<<unsigned((nq + wpb - 1) / wpb), wpb * 32, msmem, ctx->stream>>>(parts, int(S), L, nq, L,
                                                                                          d_out_keys);
     ctx->stats.launches++;
@@ -797,8 +796,7 @@ int merge_topk_impl(fv_ctx* ctx, const fv_neighbor* d_parts, const uint32_t* d_p
   int wpb = 4;
   while (wpb > 1 && size_t(wpb) * k_out * 8 > 96 * 1024) wpb >>= 1;
   const size_t smem = size_t(wpb) * k_out * 8;
-  if (smem > 40 * 1024)
-    FV_CUDA(cudaFuncSetAttribute(merge_parts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FV_TRY(allow_smem(ctx, merge_parts_kernel, smem));
   merge_parts_kernel<<<unsigned((nq + wpb - 1) / wpb), wpb * 32, smem, ctx->stream>>>(d_parts, d_part_counts, int(nparts), nq,
                                                                                      int(k_in), int(k_out), part_stride, keys);
   ctx->stats.launches++;

@@ -1400,7 +1400,7 @@ static int launch_gemm(fv_ctx* ctx, const Tiling& t, const CUtensorMap& tmA, con
                        const GemmParams& gp) {
   void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams) =
       t.MH == 2 ? gemm_topk_kernel<2, KPT, THRESH> : gemm_topk_kernel<1, KPT, THRESH>;
-  FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(t.smem)));
+  FV_TRY(allow_smem(ctx, kern, t.smem));
   kern<<<t.grid, NTHREADS, t.smem, ctx->stream>>>(tmA, tmB, gp);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
@@ -1486,7 +1486,7 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
   FV_CUDA(cudaMemsetAsync(d_next_task, 0, sizeof(unsigned int), ctx->stream));
   void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams) =
       tile_rows == 128 ? gemm_topk_kernel<1, 2, true, true> : gemm_topk_kernel<2, 2, true, true>;
-  FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(t.smem)));
+  FV_TRY(allow_smem(ctx, kern, t.smem));
   kern<<<ctx->sm_count, NTHREADS, t.smem, ctx->stream>>>(tmA, tmB, gp);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());

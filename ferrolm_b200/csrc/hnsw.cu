@@ -406,7 +406,7 @@ static int search_shape(fv_ctx* ctx, bool is_l2, int pd, int ef, size_t active, 
   const size_t per_sm = std::max<size_t>(1, std::min(size_t(227 * 1024) / (s->smem + 1024), by_warps));
   s->blocks = std::min<size_t>((active + s->searchers - 1) / s->searchers, size_t(ctx->sm_count) * per_sm);
   s->kern = team ? pick_search<TEAM_WARPS>(is_l2, R) : pick_search<1>(is_l2, R);
-  if (s->smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(s->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s->smem)));
+  FV_TRY(allow_smem(ctx, s->kern, s->smem));
   return FV_OK;
 }
 

@@ -455,12 +455,9 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
   const size_t searchers_max = std::min(resident_blocks * W, std::max<size_t>(widest, 1));  // (a team is one searcher)
   InsertKernel ins = pick_insert<1>(is_l2, R), ins_team = pick_insert<TEAM_WARPS>(is_l2, R);
   auto lnk = is_l2 ? hnsw_link_kernel<true> : hnsw_link_kernel<false>;
-  auto allow = [&](auto kern, size_t bytes) {
-    return bytes > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) : cudaSuccess;
-  };
-  FV_CUDA(allow(ins, ins_bytes(sbits) * W));
-  FV_CUDA(allow(ins_team, ins_bytes(team_sbits)));
-  FV_CUDA(allow(lnk, link_warp * LW));
+  FV_TRY(allow_smem(ctx, ins, ins_bytes(sbits) * W));
+  FV_TRY(allow_smem(ctx, ins_team, ins_bytes(team_sbits)));
+  FV_TRY(allow_smem(ctx, lnk, link_warp * LW));
 
   int log2slots = 11;
   while ((size_t(1) << log2slots) < ef * 128 && log2slots < 24) log2slots++;

@@ -121,6 +121,15 @@ int pin_ready(fv_ctx* ctx);  // makes ctx->h_pin usable
 int fetch_results(fv_ctx* ctx, const fv_neighbor* d_out, size_t nq, size_t k, fv_neighbor* out, uint32_t* counts, bool fetched = false);
 bool results_fit_pin(size_t nq, size_t k);
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory.  The limit belongs to the kernel on a device, not to a
+// launch or a context, so it is only ever raised: a thread that needs less must not lower it between another thread's
+// call here and its launch.
+int allow_smem_of(fv_ctx* ctx, const void* kern, size_t bytes);
+template <class... Args>
+int allow_smem(fv_ctx* ctx, void (*kern)(Args...), size_t bytes) {
+  return bytes <= 40 * 1024 ? FV_OK : allow_smem_of(ctx, reinterpret_cast<const void*>(kern), bytes);
+}
+
 // RAII: makes the context's device current for the duration of a call.
 struct DeviceGuard {
   int prev = -1;

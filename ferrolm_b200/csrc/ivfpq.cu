@@ -114,7 +114,7 @@ static int assign_keys(fv_ctx* ctx, bool is_l2, bool prefilter, const float* d_d
                        size_t k, size_t pd, u64* d_keys) {
   const size_t smem = assign_smem(pd), blocks = (n + 127) / 128;
   auto kern = is_l2 ? assign_kernel<true> : assign_kernel<false>;
-  if (smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FV_TRY(allow_smem(ctx, kern, smem));
   const size_t tiles = (k + ASSIGN_TILE - 1) / ASSIGN_TILE, want = size_t(ctx->sm_count) * 8;
   size_t shares = std::max<size_t>(1, std::min(tiles, want / std::max<size_t>(1, blocks * nz)));
   const size_t per = (tiles + shares - 1) / shares * ASSIGN_TILE;
@@ -572,7 +572,7 @@ static int launch_encode(fv_ctx* ctx, const fv_ivfpq* ix, const float* d_x, cons
     smem = 0;
   }
   auto kern = dsub == 4 ? encode_kernel<4> : dsub == 8 ? encode_kernel<8> : dsub == 16 ? encode_kernel<16> : encode_kernel<0>;
-  if (smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FV_TRY(allow_smem(ctx, kern, smem));
   kern<<<dim3(unsigned((n + 127) / 128), unsigned(m)), 128, smem, ctx->stream>>>(d_x, d_assign, cen, cb, n, pd, m, dsub, tile,
                                                                           staged ? 1 : 0, d_codes);
   ctx->stats.launches++;
@@ -1302,8 +1302,7 @@ static int merge_refine_impl(fv_ctx* ctx, const fv_neighbor* d_adc_parts, const 
   FV_TRY(ctx->scratch[1].reserve(nq * k * sizeof(u64)));
   u64* keys = ctx->scratch[1].as<u64>();
   const size_t smem = (keep + k) * sizeof(u64);
-  if (smem > 40 * 1024)
-    FV_CUDA(cudaFuncSetAttribute(fv::merge_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FV_TRY(fv::allow_smem(ctx, fv::merge_refine_kernel, smem));
   if (nparts * keep <= 1024 && k <= 256) {
     const unsigned blocks = unsigned((nq + 3) / 4);
     const size_t sm = 4 * k * sizeof(u64);

@@ -1819,7 +1819,7 @@ static int launch_block_scan(fv_ctx* ctx, ScanArgs a, size_t nblocks, bool use_p
     a.tickets = reinterpret_cast<uint32_t*>(ctx->scratch[6].as<unsigned char>() + part_bytes);
     FV_CUDA(cudaMemsetAsync(a.tickets, 0, nblocks * sizeof(uint32_t), ctx->stream));
   }
-  if (smem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FV_TRY(allow_smem(ctx, kern, smem));
   kern<<<dim3(unsigned(nblocks), unsigned(a.splits)), 256, smem, ctx->stream>>>(a);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
@@ -2140,7 +2140,7 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       while (vcap < 16384 && size_t(vcap) < 2 * size_t(bound_rows_tc / 32) + 512) vcap <<= 1;
       const int wpb = vcap <= 4096 ? 4 : 1;  // warps (queries) per block, by the shared memory their bounds take
       const size_t ssmem = size_t(wpb) * vcap * sizeof(uint32_t);
-      FV_CUDA(cudaFuncSetAttribute(tc_bound_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssmem)));
+      FV_TRY(allow_smem(ctx, tc_bound_select_kernel, ssmem));
       tc_bound_select_kernel<<<unsigned((nq + wpb - 1) / wpb), wpb * 32, ssmem, ctx->stream>>>(
           ctx->scratch[6].as<float>(), tasks, tile_task0, task_moff, task_rows, thr, q_rows, q_cnt, q_slots, vcap, keep, nq, tau_bits,
           tr_a == 128u ? 7 : 8);
@@ -2158,13 +2158,12 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       FV_TRY(ctx->scratch[6].reserve(nq * mcap * sizeof(float)));
       la.minima = ctx->scratch[6].as<float>();
       auto bound_k = use_pre ? ivfpq_list_scan_kernel<true, true> : ivfpq_list_scan_kernel<false, true>;
-      FV_CUDA(cudaFuncSetAttribute(bound_k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LS_SMEM)));
+      FV_TRY(allow_smem(ctx, bound_k, LS_SMEM));
       bound_k<<<ctx->sm_count, LS_THREADS, LS_SMEM, ctx->stream>>>(la);
       {
         const int wpb = mcap <= 2048 ? 4 : 1;  // warps (queries) per block, by the shared memory their minima take
         const size_t ssmem = size_t(wpb) * mcap * sizeof(uint32_t);
-        if (ssmem > 40 * 1024)
-          FV_CUDA(cudaFuncSetAttribute(bound_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssmem)));
+        FV_TRY(allow_smem(ctx, bound_select_kernel, ssmem));
         bound_select_kernel<<<unsigned((nq + wpb - 1) / wpb), wpb * 32, ssmem, ctx->stream>>>(la.minima, la.minima_cnt, int(mcap),
                                                                                                keep, nq, tau_bits);
       }
@@ -2188,7 +2187,7 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       la.cand_cnt = cand_cnt;
       la.cap = cap;
       la.rows_scanned = d_rows + 1;
-      FV_CUDA(cudaFuncSetAttribute(main_k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LS_SMEM)));
+      FV_TRY(allow_smem(ctx, main_k, LS_SMEM));
       main_k<<<ctx->sm_count, LS_THREADS, LS_SMEM, ctx->stream>>>(la);
       ctx->stats.launches++;
       FV_CUDA(cudaGetLastError());
@@ -2250,15 +2249,14 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
     while (n2max < cap || n2max < keep) n2max <<= 1;
     const size_t fsmem = (size_t(n2max) + size_t(keep) + size_t(k)) * sizeof(u64) + size_t(ix.pd) * sizeof(float);
     if (fsmem + 256 > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "k * refine too large for shared memory");
-    if (fsmem > 40 * 1024)
-      FV_CUDA(cudaFuncSetAttribute(ivfpq_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(fsmem)));
+    FV_TRY(allow_smem(ctx, ivfpq_finish_kernel, fsmem));
     // eight queries' vectors and selected ids per block: up to about 7,200 dimensions
     const size_t wsmem = size_t(8) * (ix.pd + ((keep + 7) & ~7)) * sizeof(float);
     if (!candidates && !ix.owned_ids && k <= 32 && keep <= 256 && wsmem + 256 <= ctx->smem_optin) {
       FV_TRY(ctx->scratch[18].reserve(nq * sizeof(uint32_t)));
       uint32_t* large = ctx->scratch[18].as<uint32_t>();
       auto fw = ix.metric == FV_L2 ? finish_warp_kernel<true> : finish_warp_kernel<false>;
-      if (wsmem > 40 * 1024) FV_CUDA(cudaFuncSetAttribute(fw, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wsmem)));
+      FV_TRY(allow_smem(ctx, fw, wsmem));
       fw<<<unsigned((nq + 7) / 8), 256, wsmem, ctx->stream>>>(a, fa, nq, large);
       FinishArgs fl = fa;  // (a count only the device knows; nearly always none)
       fl.qids = large;
