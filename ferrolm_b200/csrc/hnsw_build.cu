@@ -3,10 +3,10 @@
 //
 // The reference hands nodes out in id order to the pool's threads; what each thread's search sees of the others'
 // half-made links depends on timing.  Here nodes go in in id order in BATCHES:
-//   1. hnsw_insert_kernel, one warp per node of the batch: the greedy descent and the per-layer search_layer of
-//      insert() against the graph as it stood when the batch began (no node of the batch is visible to another),
-//      then select() over what was found; the node's own lists are written and one edge (target, layer, source) per
-//      chosen neighbour is pushed on a chain headed at (target, layer);
+//   1. hnsw_insert_kernel, a warp per node of the batch (a team of eight in batches of up to 16 nodes per SM): the
+//      greedy descent and the per-layer search_layer of insert() against the graph as it stood when the batch began
+//      (no node of the batch is visible to another), then select() over what was found; the node's own lists are
+//      written and one edge (target, layer, source) per chosen neighbour is pushed on a chain headed at (target, layer);
 //   2. hnsw_link_kernel, one warp per (target, layer) chain: add_links(target, layer, [source]) for the chain's
 //      sources in ascending id, that is in the order a single thread would have reached them.
 // Between batches the entry point moves as in hnsw.rs:285-289; a node above the current top layer ends its batch

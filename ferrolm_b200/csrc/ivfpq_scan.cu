@@ -1,8 +1,9 @@
 // IvfPq::search (ivfpq.rs:225-297) on the GPU: lookup tables, ADC scan, top-k and the optional exact re-rank.
 //
-// Two scans produce the same result.
+// Two scans produce the same result (and a third, the tensor-core pass further down).
 //
-//  * ivfpq_scan_kernel: one block per query.  Per probed cell the block builds the cell's table in shared memory and
+//  * ivfpq_scan_kernel: one block per query, or several that share its lists while a batch leaves SMs idle;
+//    probe_scan_kernel is the same search for results that fit the warps' registers.  Per probed cell the block builds the cell's table in shared memory and
 //    its lanes walk the list's rows (codes differ per lane: the sixteen lookups of a row land in random banks).
 //    It serves every index (any m, with or without precomputed tables), small batches and the fallback of the
 //    list-major scan.
@@ -26,7 +27,7 @@
 //    thread, the minimum of every 8 rows; the keep-th smallest of a query's minima is a distance that at least
 //    `keep` of its rows reach (every minimum is a different row), hence an upper bound of its keep-th best.  The
 //    main pass appends every row at or below that bound to the query's buffer in global memory; a finishing kernel
-//    sorts the buffer, keeps the best `keep` and re-ranks.  A query whose buffer overflows is re-run by the
+//    selects the best `keep` of the buffer and re-ranks them.  A query whose buffer overflows is re-run by the
 //    per-query kernel.
 #include <algorithm>
 #include <cmath>
@@ -1894,8 +1895,9 @@ bool ivfpq_wants_tensor(int mode, size_t nq, size_t nprobe, size_t nlist, int sh
 // Stages (fv_stats.stage_ms) of an IVF-PQ search: 0 coarse cells (marked by the caller); 1 query tables and, on the
 // list-major paths, the bound pass; 2 bucketing the (query, probe) pairs by list (tensor-core pass: plus the task
 // table and the gathered operand rows); 3 the scan (the per-query kernel, the list-major table kernel, or the
-// tensor-core kernel); 4 re-scoring survivors (tensor-core pass); 5 sorting the candidates, re-ranking and any re-run
-// of queries by the per-query kernel; 6 keys -> neighbours (marked by the caller).
+// tensor-core kernel); 4 re-scoring survivors (tensor-core pass); 5 selecting the candidates, re-ranking, what follows on
+// the keys (ScanOut::then: keys -> neighbours), the read-back of the counters and any re-run of queries by the per-query
+// kernel; 6 (marked by the caller) what follows on the keys after the per-query kernel, empty on the list-major paths.
 int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, const u64* cells, int nprobe, int keep,
                int k, bool refine, bool candidates, int mode, int cand_slots, const ScanOut& out) {
   const bool use_pre = ix.metric == FV_L2 && ix.pre != nullptr;
