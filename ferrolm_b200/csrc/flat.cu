@@ -491,11 +491,14 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
   // every key, split by rows down to one tile, and let a warp or a block per query select.  Measured against the lists
   // (both launches): 1,000 queries, 16 of 256 cells x 384: 67 us against 205; 32 queries, 16 of 512 cells x 128: 15 us
   // against 45; 10,000 queries, 64 of 1,024 cells x 128: 218 us, with the lists over 1,000.
-  // (not where the keys of a very large batch would take more than 1 GB that the lists do without)
+  // Beyond 2,048 rows a block sorts the keys of a query, and for lists of up to 31 the lists win on large batches: 10 of
+  // 4,095 rows, 1,000 and 10,000 queries x 32 223 and 645 us with the lists against 296 and 2,368, x 128 315 and 1,078
+  // against 342 and 2,760, 2,000 and 10,000 queries x 384 1,029 and 3,992 against 1,100 and 5,010.
+  // (nor where the keys of a very large batch would take more than 1 GB that the lists do without)
   const size_t most = std::max<size_t>(64, DENSE_KEYS / std::max<size_t>(1, n)), runs = (nq + most - 1) / most;
   const size_t chunk = (nq + runs - 1) / runs;  // queries at a time
   if (L >= 2 && n > 0 && n <= 4096 && !d_query_ids && size_t(8) * (size_t(pd) * 4 + 8) <= budget &&
-      (L >= 32 || nq * n * sizeof(u64) <= size_t(1) << 30) &&
+      (L >= 32 || ((n <= 2048 || nq <= 512 + 3 * size_t(pd)) && nq * n * sizeof(u64) <= size_t(1) << 30)) &&
       ctx->scratch[scratch_slot].reserve(chunk * n * sizeof(u64)) == FV_OK) {  // (no room for the keys: the lists)
     int npow2 = 32;
     while (size_t(npow2) < n) npow2 <<= 1;
@@ -506,12 +509,21 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
       const size_t nc = std::min(chunk, nq - q0);
       const float* queries = d_queries + q0 * q_stride;
       u64* out = d_out_keys + q0 * size_t(L);
-      // two queries per warp where eight would leave SMs idle or pass the shared memory of a block
+      // Eight queries per warp and 128 rows per block, split down to 32 rows while that leaves SMs without a block, and two
+      // queries per warp where it still does (or where eight pass the shared memory of a block).  Long rows pay for
+      // every further split with another read of the queries: 1,000 queries, 512 rows x 1,024, 40 results 202 us in
+      // blocks of 64 rows, 436 with two queries per warp; 500 queries, 512 rows x 384 71 with 32 rows, 107 with 128.
       int DQ = 8;
-      const size_t most_splits = std::max<size_t>(1, n / 32);
-      if ((nc + 31) / 32 * most_splits < size_t(ctx->sm_count) * 4 || size_t(w4) * 8 * row_bytes > budget) DQ = 2;
-      const size_t groups = (nc + size_t(DQ) * w4 - 1) / (size_t(DQ) * w4);
-      size_t S = std::max<size_t>(1, std::min(most_splits, (size_t(ctx->sm_count) * 8 + groups - 1) / groups));
+      size_t S = 1, groups = (nc + 8 * w4 - 1) / (8 * w4);
+      auto split = [&](size_t rows) {
+        S = std::max<size_t>(1, std::min(n / rows, (size_t(ctx->sm_count) * 8 + groups - 1) / groups));
+        return groups * S >= size_t(ctx->sm_count);
+      };
+      if (size_t(w4) * 8 * row_bytes > budget || !(split(128) || split(64) || split(32))) {
+        DQ = 2;
+        groups = (nc + 2 * w4 - 1) / (2 * w4);
+        split(32);
+      }
       size_t rps = ((n + S - 1) / S + 31) / 32 * 32;
       S = (n + rps - 1) / rps;
       const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(S));
