@@ -1808,9 +1808,13 @@ static int launch_block_scan(fv_ctx* ctx, ScanArgs a, size_t nblocks, bool use_p
   if (smem + 256 > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "m, k * refine too large for shared memory");
   // A batch that leaves SMs without a block: each query's lists are dealt to several blocks, as long as one block can
   // sort what they leave (32 queries, 16 probes of 590 rows, m = 16: 89 us with a block per query, 35 us with 16).
+  // Long lists in the buffer (room for fewer than four) only up to a block per SM: what the blocks of a query sort and
+  // merge grows with them, and each of them finds its bound by itself (255 queries, 1,000 kept of 32 lists, m = 8: two
+  // blocks each 473 us, one 386).
   a.splits = 1;
   if (!a.row_budget && !a.qids) {
-    const size_t room = size_t(ctx->sm_count) * 4 / nblocks;
+    const bool long_list = !in_regs && a.keep > a.cap / 4;
+    const size_t room = size_t(ctx->sm_count) * (long_list ? 1 : 4) / nblocks;
     a.splits = int(std::max<size_t>(1, std::min({room, size_t(a.nprobe), in_regs ? size_t(64) : size_t(a.cap / a.keep)})));
   }
   if (a.splits > 1) {

@@ -38,7 +38,7 @@ def made(oracle):
 
 @pytest.mark.parametrize("metric", [L2, IP])
 @pytest.mark.parametrize("m", [6, 4, 8, 16, 24, 48])
-@pytest.mark.parametrize("k,refine", [(1, 0), (32, 0), (33, 0), (128, 0), (129, 0), (8, 4), (32, 4), (33, 3), (10, 12), (10, 13)])
+@pytest.mark.parametrize("k,refine", [(1, 0), (32, 0), (33, 0), (128, 0), (129, 0), (8, 4), (32, 4), (33, 3), (10, 12), (10, 13), (65, 8)])
 def test_scan_equals_the_oracle(made, metric, m, k, refine):
     ix, o, q = made(metric, m)
     for nq, nprobe in ((1, 20), (3, 7), (40, 1), (700, 3)):
