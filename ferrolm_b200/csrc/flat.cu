@@ -409,18 +409,22 @@ int keys_to_neighbors(fv_ctx* ctx, const u64* d_keys, size_t nq, int L, int k, f
   return FV_OK;
 }
 
+// Shared memory of a block of the scan: the row tile goes behind the queries and lists when an SM still holds four such
+// blocks (and only for full blocks: a single warp that scans a long run of rows for a few queries streams them faster).
+static size_t scan_smem(size_t smem, int pd, int threads) {
+  const size_t with_tile = ((smem + 15) & ~size_t(15)) + 2 * size_t(32) * (size_t(pd) + 4) * sizeof(float);  // two buffers
+  return with_tile <= 72 * 1024 && threads >= 128 ? with_tile : smem;
+}
+
 template <int QT>
 static int launch_scan(fv_ctx* ctx, bool is_l2, dim3 grid, int threads, size_t smem, const float* rows, size_t n, int pd,
                        const float* q, size_t q_stride, const uint32_t* qids, size_t nq, int L, bool prefilter,
                        uint32_t id_base, size_t rps, u64* parts, u64* dense = nullptr, size_t dense_stride = 0) {
-  // the row tile goes behind the queries and lists when the shared memory of an SM still holds four such blocks
-  const size_t tile_bytes = 2 * size_t(32) * (size_t(pd) + 4) * sizeof(float);  // two buffers
-  const size_t with_tile = ((smem + 15) & ~size_t(15)) + tile_bytes;
-  // (only for full blocks: a single warp that scans a long run of rows for a few queries streams them faster itself)
-  const bool tiled = with_tile <= 72 * 1024 && threads >= 128;
+  const size_t whole = scan_smem(smem, pd, threads);
+  const bool tiled = whole > smem;
   auto k = is_l2 ? (tiled ? exact_scan_kernel<QT, true, true> : exact_scan_kernel<QT, true, false>)
                  : (tiled ? exact_scan_kernel<QT, false, true> : exact_scan_kernel<QT, false, false>);
-  if (tiled) smem = with_tile;
+  smem = whole;
   FV_TRY(allow_smem(ctx, k, smem));
   k<<<grid, threads, smem, ctx->stream>>>(rows, n, pd, q, q_stride, qids, nq, L, prefilter ? 1 : 0, id_base, rps, parts,
                                           dense, dense_stride);
@@ -513,23 +517,37 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
       const size_t nc = std::min(chunk, nq - q0);
       const float* queries = d_queries + q0 * q_stride;
       u64* out = d_out_keys + q0 * size_t(L);
-      // Eight queries per warp and 128 rows per block, split down to 32 rows while that leaves SMs without a block, and two
-      // queries per warp where it still does (or where eight pass the shared memory of a block).  Long rows pay for
-      // every further split with another read of the queries: 1,000 queries, 512 rows x 1,024, 40 results 202 us in
-      // blocks of 64 rows, 436 with two queries per warp; 500 queries, 512 rows x 384 71 with 32 rows, 107 with 128.
+      // Eight queries per warp and blocks of 128, 64 or 32 rows, whichever has the fewest rows in a row: waves of resident
+      // blocks (three per SM by registers, fewer by shared memory) times rows.  Two queries per warp where even 32 rows
+      // leave SMs without a block (or where eight pass the shared memory of one).  40 results, 128 / 64 / 32 rows / two
+      // queries per warp: 500 queries, 512 rows x 384 107 / 78 / 70 / 98 us; 1,000 of 2,048 x 384 276 / 239 / 238; 500 of
+      // 2,048 x 384 138 / 181 / 159; 300 of 2,048 x 1,024 345 / 281 / 258; 1,000 of 512 x 1,024 198 / 202 / 214 / 436.
       int DQ = 8;
-      size_t S = 1, groups = (nc + 8 * w4 - 1) / (8 * w4);
+      size_t S = 1, rps = 0, groups = (nc + 8 * w4 - 1) / (8 * w4);
       auto split = [&](size_t rows) {
         S = std::max<size_t>(1, std::min(n / rows, (size_t(ctx->sm_count) * 8 + groups - 1) / groups));
-        return groups * S >= size_t(ctx->sm_count);
+        rps = ((n + S - 1) / S + 31) / 32 * 32;
+        S = (n + rps - 1) / rps;
       };
-      if (size_t(w4) * 8 * row_bytes > budget || !(split(128) || split(64) || split(32))) {
+      split(32);
+      if (size_t(w4) * 8 * row_bytes > budget || groups * S < size_t(ctx->sm_count)) {
         DQ = 2;
         groups = (nc + 2 * w4 - 1) / (2 * w4);
         split(32);
+      } else {
+        const size_t block = scan_smem(size_t(w4) * 8 * row_bytes, pd, w4 * 32) + 1024;
+        const size_t resident = size_t(ctx->sm_count) * std::max<size_t>(1, std::min<size_t>(3, 227 * 1024 / block));
+        size_t best = ~size_t(0), best_rows = 32;
+        for (size_t rows : {128, 64, 32}) {
+          split(rows);
+          const size_t in_a_row = (groups * S + resident - 1) / resident * rps;
+          if (in_a_row < best) {
+            best = in_a_row;
+            best_rows = rows;
+          }
+        }
+        split(best_rows);
       }
-      size_t rps = ((n + S - 1) / S + 31) / 32 * 32;
-      S = (n + rps - 1) / rps;
       const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(S));
       const size_t smem = size_t(w4) * DQ * row_bytes;
       if (DQ == 8)

@@ -82,7 +82,7 @@ def test_long_results(oracle, ctx, metric, n, dim, nq, k):
     (1, 70, 2), (31, 70, 5), (33, 100, 31), (1025, 300, 2), (2049, 80, 300),
     # eight queries per warp with 128, 64 and 32 rows per block, two per warp; and on either side of the line beyond which
     # short results are kept in lists (512 + 3 padded dimensions)
-    (600, 1184, 33), (300, 1184, 33), (160, 1184, 33), (127, 1184, 33), (2049, 560, 10), (2049, 561, 10), (2048, 561, 10),
+    (600, 1184, 33), (300, 1184, 33), (160, 1184, 33), (127, 1184, 33), (4095, 400, 33), (2049, 560, 10), (2049, 561, 10), (2048, 561, 10),
 ])
 def test_few_rows(oracle, ctx, n, nq, k):
     check(oracle, ctx, L2, n, 12, nq, k, f"{n} rows, k={k}")
