@@ -1347,7 +1347,7 @@ int tc_append(fv_ctx* ctx, TcSide** ptc, int metric, const float* d_rows_new, si
 // fitted to calls at 32, 128 and 384 dimensions.  Here / there: 33 results of 65 queries x 128 136 / 112, of 300 152 / 166,
 // of 2,000 207 / 607; 128 results 177 / 112, 202 / 166, 420 / 607; 33 of 300 x 384 147 / 240; 128 of 256 x 32 150 / 112.
 static bool tc_beats_dense(size_t nq, int k, int Kp) {
-  const double here = 115.0 + 0.45 * k + double(nq) * k * (0.0005 + 3e-6 * Kp), there = 65.0 + double(nq) * (0.2 + 0.00086 * Kp);
+  const double here = 115.0 + 0.45 * k + double(nq) * k * (0.0004 + 3e-6 * Kp), there = 65.0 + double(nq) * (0.2 + 0.001 * Kp);
   return here < there;
 }
 
