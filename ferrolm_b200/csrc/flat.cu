@@ -518,9 +518,9 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
       const float* queries = d_queries + q0 * q_stride;
       u64* out = d_out_keys + q0 * size_t(L);
       // Eight queries per warp and blocks of 128, 64 or 32 rows, whichever has the fewest rows in a row: waves of resident
-      // blocks (three per SM by registers, fewer by shared memory) times rows.  Two queries per warp where even 32 rows
-      // leave SMs without a block (or where eight pass the shared memory of one).  40 results, 128 / 64 / 32 rows / two
-      // queries per warp: 500 queries, 512 rows x 384 107 / 78 / 70 / 98 us; 1,000 of 2,048 x 384 276 / 239 / 238; 500 of
+      // blocks (three per SM by registers, fewer by shared memory) times rows, a block's start counted as 16.  Two queries
+      // per warp where even 32 rows leave SMs without a block (or where eight pass the shared memory of one).  40 results,
+      // 128 / 64 / 32 rows / two queries per warp: 500 queries, 512 rows x 384 107 / 78 / 70 / 98 us; 1,000 of 2,048 x 384 276 / 239 / 238; 500 of
       // 2,048 x 384 138 / 181 / 159; 300 of 2,048 x 1,024 345 / 281 / 258; 1,000 of 512 x 1,024 198 / 202 / 214 / 436.
       int DQ = 8;
       size_t S = 1, rps = 0, groups = (nc + 8 * w4 - 1) / (8 * w4);
@@ -535,12 +535,12 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
         groups = (nc + 2 * w4 - 1) / (2 * w4);
         split(32);
       } else {
-        const size_t block = scan_smem(size_t(w4) * 8 * row_bytes, pd, w4 * 32) + 1024;
+        const size_t start = 16, block = scan_smem(size_t(w4) * 8 * row_bytes, pd, w4 * 32) + 1024;
         const size_t resident = size_t(ctx->sm_count) * std::max<size_t>(1, std::min<size_t>(3, 227 * 1024 / block));
         size_t best = ~size_t(0), best_rows = 32;
         for (size_t rows : {128, 64, 32}) {
           split(rows);
-          const size_t in_a_row = (groups * S + resident - 1) / resident * rps;
+          const size_t in_a_row = (groups * S + resident - 1) / resident * (rps + start);
           if (in_a_row < best) {
             best = in_a_row;
             best_rows = rows;
