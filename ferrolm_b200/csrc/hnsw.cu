@@ -6,8 +6,8 @@
 //
 // Search of one query (hnsw.rs:323-351): greedy descent on the upper layers, then the best-first beam of search_layer
 // (hnsw.rs:179-226), both in hnsw.cuh: the beam as ONE sorted list of ef entries with an "expanded" bit per entry, the
-// visited set exact, in shared memory first and in global memory for what does not fit.  A query that fills more than
-// half of the second part stops with an overflow mark and is re-run by the host with a table four times larger.
+// visited set exact, in global memory (a team's, and a small graph's, in shared memory first).  A query that fills more than
+// half of the latter stops with an overflow mark and is re-run by the host with a table four times larger.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -37,7 +37,7 @@ struct HnswDev {
 static constexpr int SEARCH_BLOCKS_PER_SM = 3;  // of 256 threads
 template <int R>
 __host__ __device__ __forceinline__ size_t search_smem(int pd, int ef, int sbits) {
-  return size_t(pd) * 4 + (size_t(4) << sbits) + (TIED_CAP + 32 + 32) * 4 + sizeof(TeamJob) +
+  return size_t(pd) * 4 + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + sizeof(TeamJob) +
          (R == 0 ? ((size_t(ef) * 8 + 15) & ~size_t(15)) : 0);
 }
 
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256, SEARCH_BLOCKS_PER_SM)
   unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, ef, sbits);
   float* sq = reinterpret_cast<float*>(mine);
   uint32_t* small = reinterpret_cast<uint32_t*>(sq + g.pd);
-  uint32_t* tied = small + (size_t(1) << sbits);
+  uint32_t* tied = small + visit_smem(sbits) / 4;
   Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + 32),
                 reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64)};
   u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + sizeof(TeamJob));
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256, SEARCH_BLOCKS_PER_SM)
     const size_t qsrc = qids ? size_t(qids[qi]) : qi;
     const unsigned long long n_dist0 = n_dist, n_exp0 = n_exp;  // a query that overflows its table is re-run: its work counts once
     for (int c = lane; c < g.pd; c += 32) sq[c] = queries[qsrc * size_t(g.pd) + c];
-    visit_clear(seen, lane, 32);
+    visit_clear(seen);
 
     // entry point and greedy descent (hnsw.rs:329-347)
     uint32_t cur = g.ep;
@@ -358,10 +358,10 @@ struct Builder {
 };
 
 // ---- launch shape of a search
-// A team of TEAM_WARPS warps per query while the batch is small, a warp per query beyond.  Measured (us a batch, team /
-// warp): 200k x 128, ef 64: 1 query 193 / 279, 592 queries 516 / 1,300, 2,368 queries 1,070 / 1,500, 10,000 queries
-// 3,850 / 2,020; 5,183 x 384, ef 64: 1 query 267 / 680, 2,368 queries 1,240 / 1,700, 5,000 queries 2,350 / 2,370; the
-// lines meet near 16 queries per SM at ef 16 and 200 too.
+// A team of TEAM_WARPS warps per query while the batch is small, a warp per query beyond (team_searches_per_sm).  Measured
+// (us a batch, team / warp): 100,000 x 128, ef 64: 1 query 186 / 345, 592 queries 372 / 668, 2,368 queries 926 / 967; ef
+// 256: 592 queries 1,274 / 1,829, 2,368 queries 3,342 / 2,382; 50,000 x 32, ef 64: 592 queries 320 / 369, 2,368 queries
+// 766 / 390.
 typedef void (*SearchKernel)(HnswDev, const float*, const uint32_t*, size_t, int, int, int, int, uint32_t*, fv_neighbor*,
                              uint32_t*, uint32_t*, unsigned long long*, unsigned int*);
 struct SearchShape {
@@ -381,24 +381,24 @@ static SearchKernel pick_search(bool is_l2, int R) {
   }
 }
 
-static int search_shape(fv_ctx* ctx, bool is_l2, int pd, int ef, size_t active, SearchShape* s) {
+static int search_shape(fv_ctx* ctx, bool is_l2, size_t n, int pd, int m0, int ef, size_t active, SearchShape* s) {
   const int R = ef <= 32 ? 1 : ef <= 64 ? 2 : ef <= 128 ? 4 : ef <= 256 ? 8 : 0;
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
-  const bool team = active <= size_t(ctx->sm_count) * TEAM_SEARCHES_PER_SM;
-  s->sbits = visit_sbits(ef, team);
+  const bool team = active <= size_t(ctx->sm_count) * team_searches_per_sm(pd, m0, ef);
+  s->sbits = team ? visit_sbits(ef) : visit_sbits_single(n, ef);
   size_t per = R == 0 ? search_smem<0>(pd, ef, s->sbits) : search_smem<1>(pd, ef, s->sbits);
   int W = 8;
   if (team) {
     s->searchers = 1;
     s->threads = TEAM_WARPS * 32;
+    while (s->sbits > 7 && per > budget) {
+      per -= size_t(2) << s->sbits;
+      s->sbits--;
+    }
   } else {
     while (W > 1 && per * W > budget / 2) W >>= 1;
     s->searchers = size_t(W);
     s->threads = W * 32;
-  }
-  while (s->sbits > 7 && per * s->searchers > budget) {
-    per -= size_t(2) << s->sbits;
-    s->sbits--;
   }
   s->smem = per * s->searchers;
   if (s->smem > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "dimension and ef too large for shared memory");
@@ -456,10 +456,14 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   g.top = int(h->top);
   g.ep = h->ep;
   g.n = n;
-  // second part of the visited set: 48 * ef slots to begin with (it may fill to one half); the overflow path
-  // quadruples it for the queries that need more
+  // The visited set's part in global memory: 48 slots per entry of the beam to begin with, one per link of a node where
+  // that is more and they stay within 8,192, and twice as many (four times with more than 48 links) within 4,096; it may
+  // fill to one half.  The overflow path quadruples it for the queries that need more.  A second launch, for however few,
+  // takes as long as the search of one query: 1,776 queries of 50,000 x 96, m = 48, ef 10 285 us, 568 with one of them run
+  // again.
   int log2slots = 11;
-  while ((size_t(1) << log2slots) < ef * 48 && log2slots < 26) log2slots++;
+  const size_t want = ef * (h->m0 > 48 && ef * h->m0 <= 8192 ? h->m0 : 48), roomy = want * (h->m0 > 48 ? 4 : 2);
+  while ((size_t(1) << log2slots) < (roomy <= 4096 ? roomy : want) && log2slots < 26) log2slots++;
   const uint32_t* d_qids = nullptr;
   size_t active = nq;
   std::vector<uint32_t> h_over, retry;
@@ -470,7 +474,7 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   bool fetched = false;
   for (int attempt = 0; attempt < 8 && active; ++attempt) {
     SearchShape sh{};
-    FV_TRY(search_shape(ctx, h->metric == FV_L2, pd, int(ef), active, &sh));
+    FV_TRY(search_shape(ctx, h->metric == FV_L2, n, pd, int(h->m0), int(ef), active, &sh));
     const size_t tables = sh.blocks * sh.searchers;
     FV_TRY(ctx->scratch[7].reserve((tables << log2slots) * 4));
     FV_CUDA(cudaMemsetAsync(d_work, 0, 4 * sizeof(unsigned long long) + sizeof(unsigned int), ctx->stream));

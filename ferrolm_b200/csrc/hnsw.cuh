@@ -43,10 +43,18 @@ int upload_graph(fv_hnsw* h, bool with_data = true);
 // distance) and take their turn in (distance, id) order; the list is dropped as soon as the worst distance goes down.
 static constexpr int TIED_CAP = 64;
 
-// Searches of one launch are run by teams of TEAM_WARPS warps up to this many per SM, by single warps beyond (the
-// figures are at search_shape in hnsw.cu).
+// Searches of one launch are run by teams of TEAM_WARPS warps up to a number per SM, by single warps beyond.  A team
+// shortens the distances of an expansion and leaves the rest of it to one warp, so it pays the longer the longer the rows
+// and the shorter the beam.  Where the two cross, in queries per SM (m = 16, 30,000 to 100,000 nodes): rows of 32
+// dimensions 6 at ef 10 and 64, 4 to 7 at 100 to 160, 3 at 200 and 256; of 64 and 96 dimensions 12 and 15 at ef 10, 7 to
+// 11 at 32 and 64, 6 to 10, 4 to 8; of 128 and more 10 to 20, 11 to 15, 7 to 9 (with m = 24 and 200 dimensions 7 and 5 from
+// ef 100 on); with the beam in shared memory (ef 400 and 1,000) 2 to 4 at any dimension.
 static constexpr int TEAM_WARPS = 8;
-static constexpr int TEAM_SEARCHES_PER_SM = 16;
+static inline size_t team_searches_per_sm(int pd, int m0, int ef) {
+  static constexpr size_t most[5][3] = {{6, 14, 16}, {6, 10, 16}, {6, 8, 14}, {3, 6, 8}, {2, 2, 2}};
+  const size_t line = most[ef <= 16 ? 0 : ef <= 64 ? 1 : ef <= 160 ? 2 : ef <= 256 ? 3 : 4][pd < 64 ? 0 : pd < 128 ? 1 : 2];
+  return ef > 64 && ef <= 256 && m0 > 32 && m0 <= 64 ? line * 3 / 4 : line;
+}
 
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t hash_slot(uint32_t x, int log2slots) { return (x * 2654435761u) >> (32 - log2slots); }
@@ -69,55 +77,83 @@ __device__ __forceinline__ u64 beam_key(float d, uint32_t id) { return (u64(orde
 __device__ __forceinline__ uint32_t beam_id(u64 key) { return uint32_t(key >> 1) & 0x7FFFFFFFu; }
 __device__ __forceinline__ float beam_distance(u64 key) { return order_bits_to_float(uint32_t(key >> 32)); }
 
-// ---- visited set: exact, in two parts.
-// The first part is a small table in shared memory with two 16-bit entries per word.  x -> x * odd (mod 2^b, b bits
+// ---- visited set: exact.
+// It is an open-addressing table of whole ids in global memory, cleared by the first id it gets.  A team, which has a
+// block's shared memory to itself, puts a first part there, and so does a single warp with a beam beyond 64 where that
+// part holds every node of the graph (4,096): a small table in shared memory with two 16-bit entries per word.  x -> x * odd (mod 2^b, b bits
 // holding every id) is a bijection; the high bits of the image name the home bucket, so an entry needs only the low
 // `rb` bits and how many buckets it sits behind its home.  An id that finds all of its `probes` buckets full goes to
 // the second part, an open-addressing table of whole ids in global memory that is cleared by the first id it gets.
 // Nothing is ever removed, so a bucket that was full when an id passed it is full whenever the id comes back.
-// With the whole set in global memory, as it was, an expansion spent 2,100 of 10,600 cycles in atomics on L2.
+// Measured with and without the first part (us): 592 queries by teams, 100,000 x 128, ef 64 372 and 571, ef 256 1,274 and
+// 1,731.  Single warps, with the 32 * ef places that 24 of them have room for, so that more and more ids find their
+// buckets full: 10,000 queries, ef 64 2,346 and 1,816, ef 128 3,697 and 3,046, ef 256 8,837 and 5,166; on a graph of 3,000
+// nodes, which fit, 10,000 x 48 at ef 100 1,028 and 1,138, at ef 256 2,585 and 3,046.
 struct VisitSet {
   uint32_t* small;    // shared memory: 2^sbits words
   uint32_t* big;      // global memory: 2^log2slots words
-  int sbits, rb, probes, log2slots;
+  int sbits, rb, probes, log2slots;  // sbits < 0: no part in shared memory
   uint32_t idmask;
   int in_big;         // ids in `big`, the same in every lane; -1: not cleared yet
 };
 
-// Words of the shared part for a beam of ef entries: about 12 ids are visited per entry of the beam on the benchmark's
-// graphs (22 on a graph of 5,183 text-like rows), and 32 * ef places keep the table below half full where 24 warps share
-// an SM's memory.  A team has four times the room: at 70 % full a look-up took 1,900 cycles of the 6,400 of an expansion.
-__host__ __device__ __forceinline__ int visit_sbits(int ef, bool team) {
-  const int words = ef * (team ? 64 : 16), most = team ? 13 : 11;
+// Words of a team's shared part for a beam of ef entries: 128 * ef places (rounded up to a power of two, up to 16,384).
+// About 12 ids are visited per entry of the beam on the benchmark's graphs, 22 on a graph of 5,183 text-like rows; at 70 %
+// full a look-up takes 1,900 cycles of the 6,400 of an expansion.
+__host__ __device__ __forceinline__ int visit_sbits(int ef) {
   int s = 7;
-  while (s < most && (1 << s) < words) ++s;
+  while (s < 13 && (1 << s) < ef * 64) ++s;
   return s;
+}
+
+// bytes of the shared part
+__host__ __device__ __forceinline__ size_t visit_smem(int sbits) { return sbits < 0 ? 0 : size_t(4) << sbits; }
+// a single warp's: one place per node, if those are at most 4,096 and the beam is long enough to visit many of them
+static inline int visit_sbits_single(size_t n, int ef) {
+  int s = 7;
+  while (s < 11 && (size_t(2) << s) < n) ++s;
+  return ef <= 64 || (size_t(2) << s) < n ? -1 : s;
 }
 
 __device__ __forceinline__ void visit_setup(VisitSet& v, uint32_t* small, int sbits, uint32_t* big, int log2slots,
                                             size_t n) {
+  v.big = big;
+  v.log2slots = log2slots;
+  v.in_big = -1;
+  v.sbits = sbits;
+  if (sbits < 0) return;
   int b = 1;
   while (b < 32 && (size_t(1) << b) < n) ++b;
   v.small = small;
-  v.big = big;
-  v.sbits = sbits;
   v.rb = b > sbits ? b - sbits : 0;
   v.probes = min(32, int(0xFFFFu >> min(v.rb, 16)));  // (the largest displacement must leave 0xFFFF, "empty", unused)
   v.idmask = b == 32 ? 0xFFFFFFFFu : (1u << b) - 1u;
-  v.log2slots = log2slots;
+}
+
+// empties the set; called by a whole warp, which the caller lines up afterwards
+__device__ __forceinline__ void visit_clear(VisitSet& v) {
+  if (v.sbits >= 0)
+    for (int i = lane_id() * 4; i < (1 << v.sbits); i += 128) *reinterpret_cast<uint4*>(v.small + i) = make_uint4(~0u, ~0u, ~0u, ~0u);
   v.in_big = -1;
 }
 
-// empties the set; `nthreads` threads (of which this is `tid`) share the work, and the caller lines them up afterwards
-__device__ __forceinline__ void visit_clear(VisitSet& v, int tid, int nthreads) {
-  for (int i = tid * 4; i < (1 << v.sbits); i += nthreads * 4) *reinterpret_cast<uint4*>(v.small + i) = make_uint4(~0u, ~0u, ~0u, ~0u);
-  v.in_big = -1;
+// an id into the part in global memory: true in the lanes whose x (on) was not there and is now; called by a whole warp
+__device__ __forceinline__ bool visit_big(VisitSet& v, bool on, uint32_t x) {
+  if (v.in_big < 0) {
+    for (int s = lane_id() * 4; s < (1 << v.log2slots); s += 128) *reinterpret_cast<uint4*>(v.big + s) = make_uint4(~0u, ~0u, ~0u, ~0u);
+    v.in_big = 0;
+    __syncwarp();
+  }
+  const bool fresh = on && visit(v.big, v.log2slots, x);
+  v.in_big += __popc(__ballot_sync(FV_FULL, fresh));
+  return fresh;
 }
 
 // called by a whole warp: true in the lanes whose x (on && x < n) was not in the set and is now.
 // The usual case -- the home bucket holds x, or has room and no other lane wants it -- is straight-line code: a branch
 // costs a warp here about as much as a trip to shared memory.
 __device__ __forceinline__ bool visit_warp(VisitSet& v, bool on, uint32_t x) {
+  if (v.sbits < 0) return visit_big(v, on, x);
   const uint32_t h = (x * 0x9E3779B1u) & v.idmask;
   const uint32_t bucket = h >> v.rb, rem = h & ((1u << v.rb) - 1u);
   uint32_t* p = v.small + bucket;
@@ -157,14 +193,8 @@ __device__ __forceinline__ bool visit_warp(VisitSet& v, bool on, uint32_t x) {
     }
   }
   if (__any_sync(FV_FULL, full)) {
-    const int lane = lane_id();
-    if (v.in_big < 0) {
-      for (int s = lane * 4; s < (1 << v.log2slots); s += 128) *reinterpret_cast<uint4*>(v.big + s) = make_uint4(~0u, ~0u, ~0u, ~0u);
-      v.in_big = 0;
-      __syncwarp();
-    }
-    if (full) fresh = visit(v.big, v.log2slots, x);
-    v.in_big += __popc(__ballot_sync(FV_FULL, full && fresh));
+    const bool big_fresh = visit_big(v, full, x);
+    fresh = full ? big_fresh : fresh;
   }
   return fresh;
 }
@@ -434,7 +464,7 @@ __device__ __forceinline__ void greedy_descent(const Team<NW>& t, size_t n, Rows
 // trips the stop test (hnsw.rs:203-205) unless its distance ties the current worst exactly -- see TIED_CAP.
 // The unvisited neighbours of the expanded node are offered to the list in stored order, so the admission test
 // (hnsw.rs:214) sees the same evolving bound as the sequential loop.  A search that fills more than half of the
-// visited set's second part stops with `over`.  n_dist and n_exp grow by the distances evaluated and the nodes
+// visited set's part in global memory stops with `over`.  n_dist and n_exp grow by the distances evaluated and the nodes
 // expanded.
 template <bool IS_L2, int R, int NW, class Rows>
 __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows rows, int width, const float* sq, Beam<R>& best,
@@ -476,8 +506,9 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
     const uint32_t x_first = lane < width ? __ldg(row + 1 + lane) : 0u;
     const int cnt = min(int(__ldg(row)), width);
     n_exp += 1;
-    {
+    if (R > 0) {
       // the entry that is next in line now is expanded next unless a nearer one is found: its links are on their way
+      // (with the beam in shared memory finding it costs what this saves, and 1 to 3 % more)
       u64 nk = 0;
       if (best.first_open(nk) >= 0) {
         const uint32_t* nrow = rows(beam_id(nk));

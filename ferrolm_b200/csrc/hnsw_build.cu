@@ -26,6 +26,7 @@ namespace fv {
 
 static constexpr uint32_t NIL = 0xFFFFFFFFu;
 static constexpr int BUILD_BLOCKS_PER_SM = 3;  // of 256 threads: 24 warps per SM at up to 80 registers
+static constexpr int TEAM_INSERTS_PER_SM = 16;  // batches up to this many nodes per SM are inserted by teams
 static constexpr int SRC_CAP = 128;  // sources of one chain sorted in shared memory; longer chains are walked again per source
 
 struct Edge {
@@ -119,13 +120,11 @@ __device__ __forceinline__ int select_links(const BuildDev& g, const Team<NW>& t
   return nsel;
 }
 
-// Shared memory of one insertion: the node's row and a kept candidate's, the visited set's first part, the tie list,
-// a run of rows and
-// their distances, the chosen links, the bits of select_links, the team's job, the
-// found list.
+// Shared memory of one insertion: the node's row and a kept candidate's, the visited set's first part (a team's), the tie
+// list, a run of rows and their distances, the chosen links, the bits of select_links, the team's job, the found list.
 __host__ __device__ __forceinline__ size_t insert_smem(int pd, int m0, int ef, int sbits) {
   const size_t run = size_t(run_rows(ef));
-  return size_t(pd) * 8 + (size_t(4) << sbits) + (TIED_CAP + 2 * run + ((m0 + 3) & ~3) + 128) * 4 + sizeof(TeamJob) +
+  return size_t(pd) * 8 + visit_smem(sbits) + (TIED_CAP + 2 * run + ((m0 + 3) & ~3) + 128) * 4 + sizeof(TeamJob) +
          ((size_t(ef) * 8 + 15) & ~size_t(15));
 }
 
@@ -143,7 +142,7 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
   float* sq = reinterpret_cast<float*>(mine);
   float* sc = sq + g.pd;
   uint32_t* small = reinterpret_cast<uint32_t*>(sc + g.pd);
-  uint32_t* tied = small + (size_t(1) << sbits);
+  uint32_t* tied = small + visit_smem(sbits) / 4;
   uint32_t* sel = tied + TIED_CAP + 2 * run;
   uint32_t* gone = sel + ((g.m0 + 3) & ~3);
   Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + run),
@@ -183,7 +182,7 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
     bool tie_lost = false;
     for (int layer = min(level, top); layer >= 0; --layer) {
       // search_layer starts from everything the layer above found (hnsw.rs:181-193), none of it expanded
-      visit_clear(seen, lane, 32);
+      visit_clear(seen);
       __syncwarp();
       best.reopen([&](bool on, uint32_t x) { visit_warp(seen, on, x); });
       bool over = false;
@@ -443,20 +442,20 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
   const bool is_l2 = h->metric == FV_L2;
   const size_t link_warp = link_smem(pd, int(m0));
-  int sbits = visit_sbits(int(ef), false), team_sbits = visit_sbits(int(ef), true), W = 8, LW = 8;
-  auto ins_bytes = [&](int bits) { return insert_smem(pd, int(m0), int(ef), bits); };
-  while (W > 1 && ins_bytes(sbits) * W > budget / BUILD_BLOCKS_PER_SM) W >>= 1;
+  int sbits = visit_sbits(int(ef)), W = 8, LW = 8;
+  const size_t ins_warp = insert_smem(pd, int(m0), int(ef), -1);  // a single warp's visited set is in global memory
+  auto team_bytes = [&](int bits) { return insert_smem(pd, int(m0), int(ef), bits); };
+  while (W > 1 && ins_warp * W > budget / BUILD_BLOCKS_PER_SM) W >>= 1;
   while (LW > 1 && link_warp * LW > budget / BUILD_BLOCKS_PER_SM) LW >>= 1;
-  while (sbits > 7 && ins_bytes(sbits) * W > ctx->smem_optin) sbits--;
-  while (team_sbits > 7 && ins_bytes(team_sbits) > ctx->smem_optin) team_sbits--;
-  if (std::max(ins_bytes(sbits) * W, link_warp * LW) > ctx->smem_optin)
+  while (sbits > 7 && team_bytes(sbits) > ctx->smem_optin) sbits--;
+  if (std::max({ins_warp * W, team_bytes(sbits), link_warp * LW}) > ctx->smem_optin)
     return fail(FV_ERR_UNSUPPORTED, "dimension and ef_construction too large for shared memory");
   const size_t resident_blocks = size_t(ctx->sm_count) * BUILD_BLOCKS_PER_SM;
   const size_t searchers_max = std::min(resident_blocks * W, std::max<size_t>(widest, 1));  // (a team is one searcher)
   InsertKernel ins = pick_insert<1>(is_l2, R), ins_team = pick_insert<TEAM_WARPS>(is_l2, R);
   auto lnk = is_l2 ? hnsw_link_kernel<true> : hnsw_link_kernel<false>;
-  FV_TRY(allow_smem(ctx, ins, ins_bytes(sbits) * W));
-  FV_TRY(allow_smem(ctx, ins_team, ins_bytes(team_sbits)));
+  FV_TRY(allow_smem(ctx, ins, ins_warp * W));
+  FV_TRY(allow_smem(ctx, ins_team, team_bytes(sbits)));
   FV_TRY(allow_smem(ctx, lnk, link_warp * LW));
 
   int log2slots = 11;
@@ -474,13 +473,13 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
     while (inserted < n) {
       const size_t b = next_batch(h->levels, inserted, top, max_batch, divisor);
       FV_CUDA(cudaMemsetAsync(d_edge_cnt, 0, 8, st));  // and the node counter
-      if (b <= size_t(ctx->sm_count) * TEAM_SEARCHES_PER_SM)
-        ins_team<<<unsigned(std::min(b, resident_blocks)), TEAM_WARPS * 32, ins_bytes(team_sbits), st>>>(
-            g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), team_sbits, log2slots, d_tables.as<uint32_t>(),
+      if (b <= size_t(ctx->sm_count) * TEAM_INSERTS_PER_SM)
+        ins_team<<<unsigned(std::min(b, resident_blocks)), TEAM_WARPS * 32, team_bytes(sbits), st>>>(
+            g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), sbits, log2slots, d_tables.as<uint32_t>(),
             d_edges.as<Edge>(), d_edge_cnt, d_next_node, uint32_t(edge_cap), d_head.as<uint32_t>(), d_flags);
       else
-        ins<<<unsigned(std::min(resident_blocks, (b + W - 1) / W)), W * 32, ins_bytes(sbits) * W, st>>>(
-            g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), sbits, log2slots, d_tables.as<uint32_t>(),
+        ins<<<unsigned(std::min(resident_blocks, (b + W - 1) / W)), W * 32, ins_warp * W, st>>>(
+            g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), -1, log2slots, d_tables.as<uint32_t>(),
             d_edges.as<Edge>(), d_edge_cnt, d_next_node, uint32_t(edge_cap), d_head.as<uint32_t>(), d_flags);
       FV_CUDA(cudaGetLastError());
       size_t e_max = 0;

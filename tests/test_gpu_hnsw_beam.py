@@ -6,7 +6,13 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 L2, IP = 0, 1
-TEAM_MAX = 16 * 148  # a launch of up to 16 searches per SM is run by teams
+
+
+def team_max(dim, m, ef):
+    """The largest batch of searches that is run by teams."""
+    line = ((6, 14, 16) if ef <= 16 else (6, 10, 16) if ef <= 64 else (6, 8, 14) if ef <= 160 else (3, 6, 8) if ef <= 256 else (2, 2, 2))
+    line = line[0 if dim <= 56 else 1 if dim <= 120 else 2]
+    return 148 * (line * 3 // 4 if 64 < ef <= 256 and 16 < m <= 32 else line)
 
 
 @pytest.fixture(scope="module")
@@ -33,7 +39,7 @@ def setup(oracle):
 
 
 @pytest.mark.parametrize("metric,n,dim,m,efc", [
-    (L2, 9000, 17, 8, 33),    # the widest batch (4,500 nodes) is inserted by single warps, the others by teams
+    (L2, 9000, 17, 8, 33),    # the widest batch (4,500 nodes) is inserted by single warps, those of up to 16 nodes per SM by teams
     (IP, 3000, 104, 40, 100),  # 80 links per node: three runs per expansion
     (L2, 700, 392, 4, 300),   # the found list in shared memory
 ])
@@ -43,12 +49,12 @@ def test_graph_equals_the_oracles(setup, metric, n, dim, m, efc):
     assert g.save() == o.save()
 
 
-@pytest.mark.parametrize("nq", [1, 37, TEAM_MAX, TEAM_MAX + 1])
+@pytest.mark.parametrize("nq", [1, 37, "at", "beyond"])  # one query more than teams take
 @pytest.mark.parametrize("ef", [1, 31, 32, 33, 64, 65, 128, 129, 256, 257])
 @pytest.mark.parametrize("metric,n,dim,m,efc", [(L2, 9000, 17, 8, 33), (IP, 3000, 104, 40, 100)])
 def test_search_equals_the_oracle(setup, oracle, metric, n, dim, m, efc, ef, nq):
-    if nq > TEAM_MAX and ef > 129 and metric == IP:
-        nq = TEAM_MAX + 1 if ef == 257 else 40  # (the oracle's time)
+    if isinstance(nq, str):
+        nq = team_max(dim, m, ef) + (nq == "beyond")
     graph, ctx = setup
     g, o = graph(metric, n, dim, m, efc)
     q = oracle.testdata(nq, dim, 6)
@@ -69,10 +75,10 @@ def test_queries_that_overflow_the_visited_set_are_run_again(setup, oracle):
 
     import ferrolm_b200 as fv
 
-    # 128 links a node and a beam of 32: half of the queries visit more nodes than both parts of the set take
+    # 128 links a node and a beam of 32: most queries visit more than half as many nodes as the set has room for at first
     _, ctx = setup
     rng = np.random.default_rng(1)
-    n, dim, nq, k, ef = 20_000, 100, TEAM_MAX + 30, 5, 32
+    n, dim, nq, k, ef = 20_000, 100, 2400, 5, 32
     base, q = (rng.standard_normal((r, dim)).astype(np.float32) for r in (n, nq))
     o = oracle.Hnsw.build_batched(L2, dim, base, m=64, ef_construction=64, seed=1, max_batch=4096, divisor=1)
     g = fv.Hnsw.load(ctx, o.save())
