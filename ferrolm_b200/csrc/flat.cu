@@ -130,7 +130,8 @@ __global__ void __launch_bounds__(128)
 // QT queries are worked on side by side, each with its L best keys in the warp's registers (KR * 32 places).  The
 // warps' lists are merged in the block, the blocks' lists by the last block of the query group to finish (tickets,
 // zero at launch and zero again afterwards), which writes keys or neighbours: one launch for the whole search.
-// A call for 1 query over 5,183 x 384: 50 us; over 1M x 128: 128 us (the rows at 4 TB/s, launch and wait included).
+// A call for 1 query over 5,183 x 384, host vectors in and out: 36 us, the kernel 10 of them; over 1M x 128, on the
+// device: 128 us (the rows at 4 TB/s, launch and wait included).
 static constexpr int FEW_WARPS = 8;
 static constexpr size_t FEW_QUERIES_MAX = 64;  // (a ticket per query group in fv_ctx::d_flags)
 template <int QT, int KR, bool IS_L2>
