@@ -1328,10 +1328,13 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
   if (lane >= 32 - a.k) a.out_keys[q * size_t(a.k) + lane - (32 - a.k)] = top.e[0];
 }
 
+// keys for the re-rank: an even number, so that the query behind them is read 16 bytes at a time
+__host__ __device__ __forceinline__ int rerank_keys(int keep, int k) { return (keep + k + 1) & ~1; }
+
 __global__ void __launch_bounds__(256) ivfpq_finish_kernel(ScanArgs a, FinishArgs f, int n2max) {
-  u64* lists = reinterpret_cast<u64*>(dyn_smem());  // n2max keys
+  u64* lists = reinterpret_cast<u64*>(dyn_smem());  // n2max keys, a power of two from 32 on
   u64* rerank = lists + n2max;                      // keep + k
-  float* sq = reinterpret_cast<float*>(rerank + a.keep + a.k);
+  float* sq = reinterpret_cast<float*>(rerank + rerank_keys(a.keep, a.k));
   if (!f.qids) {
     finish_block_query(a, f, blockIdx.x, lists, rerank, sq);
     return;
@@ -2253,7 +2256,7 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
     fa.dropped = dropped;
     int n2max = 32;
     while (n2max < cap || n2max < keep) n2max <<= 1;
-    const size_t fsmem = (size_t(n2max) + size_t(keep) + size_t(k)) * sizeof(u64) + size_t(ix.pd) * sizeof(float);
+    const size_t fsmem = (size_t(n2max) + size_t(rerank_keys(keep, k))) * sizeof(u64) + size_t(ix.pd) * sizeof(float);
     if (fsmem + 256 > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "k * refine too large for shared memory");
     FV_TRY(allow_smem(ctx, ivfpq_finish_kernel, fsmem));
     // eight queries' vectors and selected ids per block: up to about 7,200 dimensions

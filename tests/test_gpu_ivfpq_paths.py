@@ -60,6 +60,22 @@ def test_tensor_pass_finish_equals_the_per_query_scan(made, k, refine):
     ix.set_scan_mode(1)
 
 
+# the block finishing kernel: k (refine + 1) keys lie before the query it reads 16 bytes at a time, an odd number here
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("k,refine,slots", [(33, 4, 0), (35, 2, 0), (31, 10, 0), (7, 10, 80), (1, 4, 8)])
+def test_block_finish_of_odd_results(made, metric, k, refine, slots):
+    ix, o, q = made(metric, 16)
+    want, wc = o.search_batch(q, k, 12, refine)
+    ix.set_candidate_slots(slots)  # (few slots: the buffers run over and go to the block kernel too)
+    for mode in (2, 3):
+        ix.set_scan_mode(mode)
+        got, gc = ix.search_batch(q, k, 12, refine)
+        bits, total = assert_same_neighbours(got, gc, want, wc, f"mode {mode}")
+        assert bits == total
+    ix.set_candidate_slots(0)
+    ix.set_scan_mode(1)
+
+
 # the finishing step's queries and selected ids in shared memory: at and beyond the 48 KB a launch has unasked, and
 # beyond what an SM has
 @pytest.mark.parametrize("metric", [L2, IP])
