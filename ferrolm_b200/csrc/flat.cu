@@ -519,10 +519,14 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
       const float* queries = d_queries + q0 * q_stride;
       u64* out = d_out_keys + q0 * size_t(L);
       // Eight queries per warp and blocks of 128, 64 or 32 rows, whichever has the fewest rows in a row: waves of resident
-      // blocks (three per SM by registers, fewer by shared memory) times rows, a block's start counted as 16.  Two queries
-      // per warp where even 32 rows leave SMs without a block (or where eight pass the shared memory of one).  40 results,
-      // 128 / 64 / 32 rows / two queries per warp: 500 queries, 512 rows x 384 107 / 78 / 70 / 98 us; 1,000 of 2,048 x 384 276 / 239 / 238; 500 of
-      // 2,048 x 384 138 / 181 / 159; 300 of 2,048 x 1,024 345 / 281 / 258; 1,000 of 512 x 1,024 198 / 202 / 214 / 436.
+      // blocks (three per SM by registers, fewer by shared memory) times rows, a block's start counted as 16.  Measured
+      // with 40 results, 128 / 64 / 32 rows / two queries per warp: 500 queries, 512 rows x 384 107 / 78 / 70 / 98 us;
+      // 1,000 of 2,048 x 384 276 / 239 / 238; 500 of 2,048 x 384 138 / 181 / 159; 300 of 2,048 x 1,024 345 / 281 / 258;
+      // 1,000 of 512 x 1,024 198 / 202 / 214 / 436.
+      // Two queries per warp where eight pass the shared memory of a block, or have too few blocks: less than one per SM,
+      // or less than four runs of 32 rows per SM where two queries leave room for the row tile (below 256 dimensions).
+      // Coarse calls for 4 cells, two / eight queries per warp: 1,000 queries, 300 cells x 64 44 / 49 us, x 192 56 / 64,
+      // x 384 (no tile) 112 / 81; 1,413 of 200 x 192 54 / 61, x 384 104 / 76; 632 of 574 x 192 59 / 67, x 384 118 / 84.
       int DQ = 8;
       size_t S = 1, rps = 0, groups = (nc + 8 * w4 - 1) / (8 * w4);
       auto split = [&](size_t rows) {
@@ -531,7 +535,10 @@ int exact_scan(fv_ctx* ctx, int metric, const float* d_rows, size_t n, int pd, c
         S = (n + rps - 1) / rps;
       };
       split(32);
-      if (size_t(w4) * 8 * row_bytes > budget || groups * S < size_t(ctx->sm_count)) {
+      const size_t two = size_t(w4) * 2 * row_bytes, sms = size_t(ctx->sm_count);
+      const bool tile_of_two = scan_smem(two, pd, w4 * 32) > two;
+      if (size_t(w4) * 8 * row_bytes > budget || groups * S < sms ||
+          (tile_of_two && groups * std::max<size_t>(1, n / 32) < 4 * sms)) {
         DQ = 2;
         groups = (nc + 2 * w4 - 1) / (2 * w4);
         split(32);

@@ -78,14 +78,17 @@ def test_long_results(oracle, ctx, metric, n, dim, nq, k):
     assert got.tobytes() == want.tobytes() and (gc == wc).all()
 
 
-@pytest.mark.parametrize("n,nq,k", [
-    (1, 70, 2), (31, 70, 5), (33, 100, 31), (1025, 300, 2), (2049, 80, 300),
-    # eight queries per warp with 128, 64 and 32 rows per block, two per warp; and on either side of the line beyond which
-    # short results are kept in lists (512 + 3 padded dimensions)
-    (600, 1184, 33), (300, 1184, 33), (160, 1184, 33), (127, 1184, 33), (4095, 400, 33), (2049, 560, 10), (2049, 561, 10), (2048, 561, 10),
+@pytest.mark.parametrize("n,dim,nq,k", [
+    (1, 12, 70, 2), (31, 12, 70, 5), (33, 12, 100, 31), (1025, 12, 300, 2), (2049, 12, 80, 300),
+    # eight queries per warp with 128, 64 and 32 rows per block; on either side of four runs of 32 rows per SM, below which
+    # two per warp take the rows of short vectors; of long ones, on either side of one block per SM
+    (100, 12, 10_000, 33), (576, 12, 1184, 33), (600, 12, 1184, 33), (511, 12, 1184, 33), (512, 12, 1184, 33),
+    (160, 260, 1184, 33), (127, 260, 1184, 33), (300, 252, 1000, 10), (300, 256, 1000, 10),
+    # on either side of the line beyond which short results are kept in lists (512 + 3 padded dimensions)
+    (4095, 12, 400, 33), (2049, 12, 560, 10), (2049, 12, 561, 10), (2048, 12, 561, 10),
 ])
-def test_few_rows(oracle, ctx, n, nq, k):
-    check(oracle, ctx, L2, n, 12, nq, k, f"{n} rows, k={k}")
+def test_few_rows(oracle, ctx, n, dim, nq, k):
+    check(oracle, ctx, L2, n, dim, nq, k, f"{n} rows x {dim}, k={k}")
 
 
 def test_a_long_result_is_refused_by_the_forced_tensor_core_mode(oracle, ctx):
