@@ -16,7 +16,8 @@
 // chain (src/kernels.rs:200-231) for those candidates, picks the k best by (distance, id) and
 // CERTIFIES the result: a query passes only if every row that was not a candidate is provably
 // farther than its k-th result.  Queries that do not pass are re-run by the full-precision scan,
-// so the tensor cores never decide a result on their own.
+// so 16-bit scores never decide a result on their own.  L2 over whole numbers within 255 of each other is scored in 8-bit
+// integers instead, exactly (convert8_rows_kernel): there the scores are the distances, and the re-rank reads no row.
 //
 // Work split: a unit is (query tile, 256 base rows); see make_tiling for how units become chunks
 // and chunks are dealt to the persistent CTAs (one per SM) so that base tiles are shared in L2.
@@ -138,6 +139,19 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
       : "memory");
 }
 
+// 8-bit signed operands, 32-bit integer accumulators: exact, and K = 32 in the time and bytes of a 16-bit K = 16.
+__device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // 32 lanes x 32 columns of 32-bit accumulators: thread l of the warp gets lane (base + l), columns c..c+31.
 // The load is asynchronous: the registers are valid only after tc_ld_wait on the same array, which takes
 // them as in/out operands so that no use can be scheduled ahead of the wait.
@@ -201,33 +215,37 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
   return r;
 }
 
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128 bytes, groups of
-// 8 rows 1024 bytes apart; bits 46-47 carry the descriptor version of this architecture.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= uint64_t((saddr & 0x3FFFF) >> 4);  // start address
-  d |= uint64_t(1) << 16;                 // leading byte offset (unused with swizzle): 1
-  d |= uint64_t(1024 >> 4) << 32;         // stride byte offset
-  d |= uint64_t(1) << 46;                 // version
-  d |= uint64_t(2) << 61;                 // SWIZZLE_128B
-  return d;
-}
+// Shared-memory matrix descriptors of K-major operands.  Low word: start address and leading byte offset (unused with
+// swizzle: 1), both in 16-byte units; high word: stride byte offset, the descriptor version of this architecture (bit 46)
+// and the swizzle (bits 61-63).  SW128: rows of 128 bytes, groups of 8 rows 1024 bytes apart; SW32 (a K of 32 bytes): rows
+// of 32 bytes, groups 256 bytes apart.  Shared memory ends below 2^18, so an offset is added to the low word.
+static constexpr uint32_t DESC_HI_SW128 = (1024u >> 4) | (1u << 14) | (2u << 29);
+static constexpr uint32_t DESC_HI_SW32 = (256u >> 4) | (1u << 14) | (6u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
+__device__ __forceinline__ uint64_t make_desc(uint32_t lo, uint32_t hi) { return (uint64_t(hi) << 32) | lo; }
 
-// The same for a K = 16 operand: rows of 32 bytes with the 32-byte swizzle, groups of 8 rows 256 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= uint64_t((saddr & 0x3FFFF) >> 4);
-  d |= uint64_t(1) << 16;
-  d |= uint64_t(256 >> 4) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(6) << 61;                 // SWIZZLE_32B
-  return d;
+// true in one lane of the (converged) warp, always the same one
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xFFFFFFFF;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(on));
+  return on != 0;
 }
 
 // Instruction descriptor of kind::f16: fp32 accumulate, A and B both K-major, M x N tile.
 __host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool bf16) {
   return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | (uint32_t(n >> 3) << 17) |
          (uint32_t(m >> 4) << 24);
+}
+
+// Instruction descriptor of kind::i8: 32-bit integer accumulate, A and B signed and K-major.
+__host__ __device__ constexpr uint32_t make_idesc_i8(int m, int n) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
 }
 
 // Ring position (stage index and phase bit), advanced without divisions: each role loop is a single thread on
@@ -247,7 +265,9 @@ struct StageCursor {
 // ------------------------------------------------------------------------------------------------
 struct GemmParams {
   int n, nq;
-  int KB;          // 64-wide k blocks
+  int grid;        // CTAs that take work (task mode: all)
+  int KB;          // k blocks of 128 bytes per row (64 16-bit or 128 8-bit elements)
+  int last_steps;  // MMAs (32 bytes per row) of the last k block: 4 less the ones that would only meet padding
   int NT;          // base tiles of 256 rows
   int MT;          // query tiles of 128 * MH rows
   int cpn;         // base tiles per chunk
@@ -257,7 +277,7 @@ struct GemmParams {
   int scratch_bytes;  // SCRATCH_BYTES in list mode, 0 in threshold mode
   int has_ext;        // L2: one more k step of 16 adds the row norms inside the MMA
   int ext_ring;       // norm-step tiles (8 KB each) kept in shared memory
-  uint32_t aext_c;    // 16-bit pattern of the constant the query side of the norm step holds
+  uint4 aext;         // the query side of the norm step: both 16-byte halves of every row
   const uint16_t* ext;  // base side of the norm step: 32 bytes per row, padded to whole tiles
   uint32_t idesc;
   u64* cand;           // [grid * segmax][LISTS][KP]  (list mode: output)
@@ -341,15 +361,29 @@ static int pick_sample_r(int k, int every) {
   return SAMPLE_R_MAX + 1;
 }
 
+// How a pass dealt out its work, for the kernels that read what it left; where a search may take the 8-bit operands, the
+// device word q8_bad says which of the two passes ran.
+struct PassShape {
+  int MT, parts, grid, segmax, MH;
+};
+struct PassShapes {
+  PassShape s16, s8;
+  const unsigned int* q8_bad;  // null: the base has no 8-bit operands
+  __device__ __forceinline__ bool is8() const { return q8_bad && *q8_bad == 0u; }
+  __device__ __forceinline__ const PassShape& taken() const { return is8() ? s8 : s16; }
+};
+
 // The R-th smallest score of every query over the lists the sample pass left (+inf when the sample holds fewer rows).
 // Bound by latency: the lists of a query are a few dozen short runs of memory.  One warp per query, a list per lane
 // (the next 32 lists after that), each lane with its R smallest in registers; then R rounds take the smallest head
 // over the lanes.  One thread per query, as it was, put 1,000 queries on 4 SMs and read their lists one after
 // another: 94 us for 1,000 queries at 100k x 128 (the whole search 281 -> 203 us), 26 us for 10,000 at 1M x 128.
-__global__ void __launch_bounds__(256) sample_tau_kernel(const u64* __restrict__ lists, int MT, int parts, int grid,
-                                                         int segmax, int MH, int nq_pad, int R, float* __restrict__ tau) {
+__global__ void __launch_bounds__(256) sample_tau_kernel(const u64* __restrict__ lists, PassShapes shapes, int nq_pad, int R,
+                                                         float* __restrict__ tau) {
   const int q = blockIdx.x * int(blockDim.x >> 5) + int(threadIdx.x >> 5), lane = lane_id();
-  if (q >= nq_pad) return;
+  const PassShape& sh = shapes.taken();
+  const int MT = sh.MT, parts = sh.parts, grid = sh.grid, segmax = sh.segmax, MH = sh.MH;
+  if (q >= nq_pad || q >= MT * 128 * MH) return;
   const int rows_per_tile = 128 * MH;
   const int mt = q / rows_per_tile, r = q - mt * rows_per_tile;
   float best[SAMPLE_R_MAX];
@@ -396,9 +430,31 @@ __global__ void __launch_bounds__(256) sample_tau_kernel(const u64* __restrict__
   if (lane == 0) tau[q] = order_bits_to_float(w);
 }
 
-template <int MH, int KPT, bool THRESH, bool TASKS = false>
-__global__ void __launch_bounds__(NTHREADS, 1)
-    gemm_topk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
+// Accumulators as the epilogue compares them: scores in fp32, or whole numbers (I8), whose order is the same.
+template <bool I8>
+struct Score {
+  typedef float T;
+  __device__ static __forceinline__ T of(uint32_t r) { return __uint_as_float(r); }
+  __device__ static __forceinline__ T bound(float f) { return f; }
+  __device__ static __forceinline__ T min2(T a, T b) { return fminf(a, b); }
+  __device__ static __forceinline__ T min3(T a, T b, T c) { return fv::min3(a, b, c); }
+};
+template <>
+struct Score<true> {
+  typedef int T;
+  __device__ static __forceinline__ T of(uint32_t r) { return int(r); }
+  // bounds are scores that this kernel wrote as floats (exact: below 2^24), or +inf
+  __device__ static __forceinline__ T bound(float f) { return f < 2.0e9f ? int(f) : 0x7FFFFFFF; }
+  __device__ static __forceinline__ T min2(T a, T b) { return min(a, b); }
+  __device__ static __forceinline__ T min3(T a, T b, T c) { return min(min(a, b), c); }
+};
+
+template <int MH, int KPT, bool THRESH, bool TASKS, bool I8>
+__device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p) {
+  typedef Score<I8> S;
+  typedef typename S::T T;
+  constexpr int KE = I8 ? 2 * KBLK : KBLK;  // elements of a k block
+  if (!TASKS && int(blockIdx.x) >= p.grid) return;
   unsigned char* raw = dyn_smem();
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sA = base;                                            // [MH][KB] blocks of 16 KB
@@ -427,10 +483,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     bars->pool_pos = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // Query side of the norm step: every row is {c, c, c, 0, 0, 0, 0, 0} twice.  Both 16-byte halves of a row are
-  // equal, so the 32-byte swizzle (which only exchanges the halves of some rows) leaves the tile as written.
-  if (threadIdx.x < A_EXT_BYTES / 16)
-    reinterpret_cast<uint4*>(sAext)[threadIdx.x] = make_uint4(p.aext_c | (p.aext_c << 16), p.aext_c, 0u, 0u);
+  // Query side of the norm step.  Both 16-byte halves of a row are equal, so the 32-byte swizzle (which only exchanges
+  // the halves of some rows) leaves the tile as written.
+  if (threadIdx.x < A_EXT_BYTES / 16) reinterpret_cast<uint4*>(sAext)[threadIdx.x] = p.aext;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 1) {  // the MMA warp owns the tensor memory: all 512 columns (one CTA per SM)
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&bars->tmem_base))
@@ -450,12 +505,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // the latest (two accumulator slots).  The caller sorts the tasks by decreasing length: longest first.
   const int nwork = TASKS ? int(*p.ntasks) : p.nchunks;
   auto work_of = [&](int seg) -> int {  // consumer side
-    if (!TASKS) return int(blockIdx.x) + seg * int(gridDim.x);
+    if (!TASKS) return int(blockIdx.x) + seg * p.grid;
     if (!mbar_wait(&bars->tq_full[seg & 7], uint32_t(seg >> 3) & 1, abort_flag)) return 0x7FFFFFFF;
     return int(*reinterpret_cast<volatile unsigned int*>(&bars->tq[seg & 7]));
   };
   auto draw = [&](int seg) -> int {  // producer side
-    if (!TASKS) return int(blockIdx.x) + seg * int(gridDim.x);
+    if (!TASKS) return int(blockIdx.x) + seg * p.grid;
     const unsigned int g = min(atomicAdd(p.next_task, 1u), 0x7FFFFFFEu);
     bars->tq[seg & 7] = g;
     mbar_arrive(&bars->tq_full[seg & 7]);  // release: the entry is visible to whoever sees this phase complete
@@ -487,7 +542,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         mbar_expect_tx(&bars->a_full, uint32_t(MH * p.KB * A_BLOCK_BYTES));
         for (int mh = 0; mh < MH; ++mh)
           for (int kb = 0; kb < p.KB; ++kb)
-            tma_load_2d(sA + size_t(mh * p.KB + kb) * A_BLOCK_BYTES, &tmA, &bars->a_full, kb * KBLK, a_row0 + mh * 128);
+            tma_load_2d(sA + size_t(mh * p.KB + kb) * A_BLOCK_BYTES, &tmA, &bars->a_full, kb * KE, a_row0 + mh * 128);
         for (int nt = nt0; nt < nt1 && ok; ++nt) {
           for (int kb = 0; kb < p.KB; ++kb, st.next()) {
             const int s = st.s;
@@ -504,7 +559,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const size_t brow = size_t(b_row0) + size_t(nt) * TILE_N;
             if (with_ext)  // stored as the swizzled shared-memory image: one contiguous 8 KB copy
               bulk_load_1d(sE + size_t(ring) * B_EXT_BYTES, p.ext + brow * EXT_K, B_EXT_BYTES, &bars->full[s]);
-            tma_load_2d(sB + size_t(s) * B_STAGE_BYTES, &tmB, &bars->full[s], kb * KBLK, int(brow));
+            tma_load_2d(sB + size_t(s) * B_STAGE_BYTES, &tmB, &bars->full[s], kb * KE, int(brow));
           }
           if (++ring == p.ext_ring) ring = 0;
         }
@@ -519,62 +574,76 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      int job = 0, ring = 0;
-      bool ok = true;
-      StageCursor st(p.nstage);
-      const uint32_t a_base = smem_u32(sA), b_base = smem_u32(sB), e_base = smem_u32(sE);
-      const uint64_t aext_desc = smem_desc_sw32(smem_u32(sAext));
-      for (int seg = 0, g = work_of(0); g < nwork && ok; g = work_of(++seg)) {
-        int nt0, nt1;
-        if (TASKS) {
-          nt0 = 0;
-          nt1 = int(p.tasks[g].z & 0xFFFFu);
-        } else {
-          const int part = g / p.MT;
-          nt0 = part * p.cpn;
-          nt1 = min(p.NT, nt0 + p.cpn);
-        }
-        ok = mbar_wait(&bars->a_full, seg & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        for (int nt = nt0; nt < nt1 && ok; ++nt) {
-          for (int mh = 0; mh < MH && ok; ++mh, ++job) {
-            const int slot = job & 1;
-            ok = mbar_wait(&bars->tempty[slot], (uint32_t(job >> 1) & 1) ^ 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t d_tmem = tmem_base + uint32_t(slot * TILE_N);
-            StageCursor sk = st;  // both halves walk the same stages of this unit
-            uint32_t acc = 0;     // the first MMA of a job overwrites the accumulator
-            for (int kb = 0; kb < p.KB; ++kb, sk.next()) {
-              const int s = sk.s;
-              if (mh == 0) {
-                ok = mbar_wait(&bars->full[s], sk.phase, abort_flag);
-                if (!ok) break;
-                tc_fence_after();
-              }
-              if (kb == 0 && p.has_ext) {  // + ||b||^2: always the first step of a job
-                tc_mma_f16(d_tmem, aext_desc, smem_desc_sw32(e_base + uint32_t(ring * B_EXT_BYTES)), p.idesc, 0u);
+    // The whole warp walks the loop, so that everything an MMA is issued with is uniform, and one elected lane issues.
+    // Descriptors advance by adding to their low words.
+    const bool leader = elect_one();
+    int job = 0, ring = 0;
+    bool ok = true;
+    StageCursor st(p.nstage);
+    const uint32_t a_lo0 = desc_lo(smem_u32(sA)), b_lo0 = desc_lo(smem_u32(sB)), e_lo0 = desc_lo(smem_u32(sE));
+    const uint32_t aext_lo = desc_lo(smem_u32(sAext));
+    auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
+      if (I8) tc_mma_i8(d, a, b, p.idesc, accumulate);
+      else tc_mma_f16(d, a, b, p.idesc, accumulate);
+    };
+    for (int seg = 0, g = work_of(0); g < nwork && ok; g = work_of(++seg)) {
+      int nt0, nt1;
+      if (TASKS) {
+        nt0 = 0;
+        nt1 = int(p.tasks[g].z & 0xFFFFu);
+      } else {
+        const int part = g / p.MT;
+        nt0 = part * p.cpn;
+        nt1 = min(p.NT, nt0 + p.cpn);
+      }
+      ok = __all_sync(FV_FULL, mbar_wait(&bars->a_full, seg & 1, abort_flag, 0));
+      if (!ok) break;
+      tc_fence_after();
+      for (int nt = nt0; nt < nt1 && ok; ++nt) {
+#pragma unroll
+        for (int mh = 0; mh < MH; ++mh, ++job) {
+          const int slot = job & 1;
+          ok = ok && __all_sync(FV_FULL, mbar_wait(&bars->tempty[slot], (uint32_t(job >> 1) & 1) ^ 1, abort_flag, 0));
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + uint32_t(slot * TILE_N);
+          StageCursor sk = st;  // both halves walk the same stages of this unit
+          for (int kb = 0; kb < p.KB; ++kb, sk.next()) {
+            const int s = sk.s;
+            if (mh == 0) {
+              ok = __all_sync(FV_FULL, mbar_wait(&bars->full[s], sk.phase, abort_flag, 0));
+              if (!ok) break;
+              tc_fence_after();
+            }
+            if (leader) {
+              uint32_t acc = kb != 0 ? 1u : 0u;  // the first MMA of a job overwrites the accumulator
+              if (kb == 0 && p.has_ext) {        // + ||b||^2: always the first step of a job
+                mma(d_tmem, make_desc(aext_lo, DESC_HI_SW32), make_desc(e_lo0 + uint32_t(ring * (B_EXT_BYTES >> 4)), DESC_HI_SW32), 0u);
                 acc = 1;
               }
-              const uint32_t a_addr = a_base + uint32_t((mh * p.KB + kb) * A_BLOCK_BYTES);
-              const uint32_t b_addr = b_base + uint32_t(s * B_STAGE_BYTES);
+              const uint32_t a_lo = a_lo0 + uint32_t((mh * p.KB + kb) * (A_BLOCK_BYTES >> 4));
+              const uint32_t b_lo = b_lo0 + uint32_t(s * (B_STAGE_BYTES >> 4));
+              mma(d_tmem, make_desc(a_lo, DESC_HI_SW128), make_desc(b_lo, DESC_HI_SW128), acc);
+              if (kb + 1 < p.KB || p.last_steps == 4) {
 #pragma unroll
-              for (int k4 = 0; k4 < KBLK / 16; ++k4)
-                tc_mma_f16(d_tmem, smem_desc_sw128(a_addr + k4 * 32), smem_desc_sw128(b_addr + k4 * 32), p.idesc,
-                           k4 != 0 ? 1u : acc);
-              acc = 1;
+                for (int k4 = 1; k4 < 4; ++k4)
+                  mma(d_tmem, make_desc(a_lo + 2 * k4, DESC_HI_SW128), make_desc(b_lo + 2 * k4, DESC_HI_SW128), 1u);
+              } else {
+                for (int k4 = 1; k4 < p.last_steps; ++k4)
+                  mma(d_tmem, make_desc(a_lo + 2 * k4, DESC_HI_SW128), make_desc(b_lo + 2 * k4, DESC_HI_SW128), 1u);
+              }
               if (mh == MH - 1) tc_commit(&bars->empty[s]);  // the stage is free once these MMAs have read it
+              if (kb + 1 == p.KB) tc_commit(&bars->tfull[slot]);
             }
-            if (!ok) break;
-            tc_commit(&bars->tfull[slot]);
+            __syncwarp();
           }
-          for (int kb = 0; kb < p.KB; ++kb) st.next();
-          if (++ring == p.ext_ring) ring = 0;
+          if (!ok) break;
         }
-        if (ok) tc_commit(&bars->a_empty);  // the query tile may be replaced once every MMA above has read it
+        for (int kb = 0; kb < p.KB; ++kb) st.next();
+        if (++ring == p.ext_ring) ring = 0;
       }
+      if (ok && leader) tc_commit(&bars->a_empty);  // the query tile may be replaced once every MMA above has read it
+      __syncwarp();
     }
   } else {
     // ---------------------------------------------------------------- epilogue: 16 warps, one query row per thread
@@ -588,7 +657,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // rows arrive in ascending id order, so a strict score compare keeps the (score, id) order
     float sc[KPT];
     uint32_t idv[KPT];
-    float thr = INFINITY;
+    T thr = S::bound(INFINITY);
     size_t cslot = 0;        // this thread's list of the current segment
     unsigned int ncand = 0;
     float* sv = reinterpret_cast<float*>(scratch) + size_t(ew) * 512;  // list mode: 16 columns x 32 rows of scores
@@ -623,9 +692,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       cslot = (size_t(blockIdx.x) * p.segmax + seg) * LISTS + e;
       ncand = 0;
       if (THRESH) {  // the bound is fixed: the sample pass's estimate for this query
-        thr = TASKS ? (p.minima ? 0.f : p.tau[a_row]) : p.tau[mt * (128 * MH) + (MH == 2 ? grp * 128 : 0) + quad * 32 + lane];
+        thr = S::bound(TASKS ? (p.minima ? 0.f : p.tau[a_row]) : p.tau[mt * (128 * MH) + (MH == 2 ? grp * 128 : 0) + quad * 32 + lane]);
       } else {
-        thr = INFINITY;
+        thr = S::bound(INFINITY);
 #pragma unroll
         for (int j = 0; j < KPT; ++j) {
           sc[j] = INFINITY;
@@ -646,30 +715,32 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           // below the bound is appended to this thread's private list: a plain store and a register counter.
           // (Issuing the next load before working on this one was tried and ran slower than this plain loop.)
           auto chunk = [&](const uint32_t* r, int c) {
-            float g8[8];
+            T g8[8];
 #pragma unroll
             for (int gi = 0; gi < 8; ++gi) {
               const uint32_t* q = r + gi * 8;
-              const float t0 = min3(__uint_as_float(q[0]), __uint_as_float(q[1]), __uint_as_float(q[2]));
-              const float t1 = min3(__uint_as_float(q[3]), __uint_as_float(q[4]), __uint_as_float(q[5]));
-              g8[gi] = fminf(min3(t0, t1, __uint_as_float(q[6])), __uint_as_float(q[7]));
+              const T t0 = S::min3(S::of(q[0]), S::of(q[1]), S::of(q[2]));
+              const T t1 = S::min3(S::of(q[3]), S::of(q[4]), S::of(q[5]));
+              g8[gi] = S::min2(S::min3(t0, t1, S::of(q[6])), S::of(q[7]));
             }
-            const float m = fminf(min3(g8[0], g8[1], g8[2]), min3(min3(g8[3], g8[4], g8[5]), g8[6], g8[7]));
-            if (__any_sync(FV_FULL, m < thr)) {
-              u64* cl = p.cbuf + cslot * size_t(p.ccap);
+            const T m = S::min2(S::min3(g8[0], g8[1], g8[2]), S::min3(S::min3(g8[3], g8[4], g8[5]), g8[6], g8[7]));
+            if (!__any_sync(FV_FULL, m < thr)) return;
+            uint32_t groups = 0;  // the runs of eight columns in which some row of the warp has a hit
 #pragma unroll
-              for (int gi = 0; gi < 8; ++gi) {
-                if (__any_sync(FV_FULL, g8[gi] < thr)) {
+            for (int gi = 0; gi < 8; ++gi) groups |= g8[gi] < thr ? 1u << gi : 0u;
+            groups = __reduce_or_sync(FV_FULL, groups);
+            u64* cl = p.cbuf + cslot * size_t(p.ccap);
 #pragma unroll
-                  for (int i = gi * 8; i < gi * 8 + 8; ++i) {
-                    const float v = __uint_as_float(r[i]);
-                    const uint32_t row = row_base + uint32_t(c + i);
-                    if (v < thr && row < n_rows) {
-                      if (ncand < unsigned(p.ccap)) cl[ncand] = make_key(v, row);
-                      ncand++;
-                    }
-                  }
-                }
+            for (int gi = 0; gi < 8; ++gi) {
+              if (!(groups & (1u << gi))) continue;
+#pragma unroll
+              for (int i = gi * 8; i < gi * 8 + 8; ++i) {
+                const T v = S::of(r[i]);
+                const uint32_t row = row_base + uint32_t(c + i);
+                const u64 key = make_key(float(v), row);
+                const bool hit = v < thr && row < n_rows;
+                if (hit) cl[min(ncand, unsigned(p.ccap) - 1u)] = key;  // (a list that ran over is thrown away: its count tells)
+                ncand += hit ? 1u : 0u;
               }
             }
           };
@@ -678,14 +749,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           // as two bit masks, the warp reserves room for all of them with ONE atomic on the CTA's counter, and each
           // thread stores its own.
           auto chunk_tasks = [&](const uint32_t* r, int c) {
-            float m = __uint_as_float(r[0]);
+            T m = S::of(r[0]);
 #pragma unroll
-            for (int i = 1; i < 64; ++i) m = fminf(m, __uint_as_float(r[i]));
+            for (int i = 1; i < 64; ++i) m = S::min2(m, S::of(r[i]));
             if (!__any_sync(FV_FULL, m < thr)) return;
             uint32_t mk[2] = {0u, 0u};
 #pragma unroll
             for (int i = 0; i < 64; ++i)
-              if (__uint_as_float(r[i]) < thr && row_base + uint32_t(c + i) < n_rows) mk[i >> 5] |= 1u << (i & 31);
+              if (S::of(r[i]) < thr && row_base + uint32_t(c + i) < n_rows) mk[i >> 5] |= 1u << (i & 31);
             const int mine = __popc(mk[0]) + __popc(mk[1]);
             int incl = mine;  // inclusive prefix sum over the warp
 #pragma unroll
@@ -757,17 +828,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           for (int c = 0; c < NCOL; c += 32) {
             tc_ld32_issue(t_addr + uint32_t(c), rbuf);
             tc_ld_wait(rbuf);
-            float m = INFINITY;
+            T m = S::of(rbuf[0]);
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) m = min3(m, __uint_as_float(rbuf[i]), __uint_as_float(rbuf[i + 1]));
+            for (int i = 1; i < 31; i += 2) m = S::min3(m, S::of(rbuf[i]), S::of(rbuf[i + 1]));
+            m = S::min2(m, S::of(rbuf[31]));
             if (__any_sync(FV_FULL, m < thr)) {
 #pragma unroll
               for (int h = 0; h < 2; ++h) {  // two halves of 16 columns, in id order; the scratch holds one half
                 unsigned mask = 0;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                  const float v = __uint_as_float(rbuf[h * 16 + i]);
-                  sv[i * 32 + lane] = v;
+                  const T v = S::of(rbuf[h * 16 + i]);
+                  sv[i * 32 + lane] = float(v);
                   mask |= (v < thr && row_base + uint32_t(c + h * 16 + i) < n_rows) ? (1u << i) : 0u;
                 }
                 while (__any_sync(FV_FULL, mask != 0)) {
@@ -775,7 +847,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     const int i = __ffs(mask) - 1;
                     mask &= mask - 1;
                     const float val = sv[i * 32 + lane];
-                    if (val < thr) {
+                    if (val < sc[KPT - 1]) {
                       float cs = val;
                       uint32_t ci = row_base + uint32_t(c + h * 16 + i);
 #pragma unroll
@@ -788,7 +860,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         cs = lt ? ts : cs;
                         ci = lt ? ti : ci;
                       }
-                      thr = sc[KPT - 1];
+                      thr = S::bound(sc[KPT - 1]);
                     }
                   }
                 }
@@ -827,6 +899,26 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
 }
 
+template <int MH, int KPT, bool THRESH, bool TASKS = false>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    gemm_topk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ GemmParams p) {
+  gemm_topk_body<MH, KPT, THRESH, TASKS, false>(tmA, tmB, p);
+}
+
+// The pass over the 8-bit operands or, where a query of the batch does not fit them (q8_bad, known on the device only), over
+// the 16-bit ones: one launch, since one that leaves at once costs a pass over 100,000 rows 3 us of 40.
+struct GemmWay {
+  CUtensorMap tmA, tmB;
+  GemmParams p;
+};
+template <int MH16, int KPT, bool THRESH>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    gemm_topk_either_kernel(const __grid_constant__ GemmWay w16, const __grid_constant__ GemmWay w8, const unsigned int* q8_bad) {
+  if (*q8_bad) gemm_topk_body<MH16, KPT, THRESH, false, false>(w16.tmA, w16.tmB, w16.p);
+  else gemm_topk_body<2, KPT, THRESH, false, true>(w8.tmA, w8.tmB, w8.p);
+}
+
 // ------------------------------------------------------------------------------------------------
 // fp32 rows -> 16-bit operand rows (zero padded to Kp), squared norms and range statistics
 struct RangeStats {
@@ -845,10 +937,57 @@ __device__ __forceinline__ void atomic_max_f(float* a, float v) {
   else atomicMin(reinterpret_cast<unsigned*>(a), __float_as_uint(v));
 }
 
-// one warp per row
+// ---- 8-bit operands, for L2 over whole numbers that lie within 255 of each other (bytes, as SIFT's components are).
+// With b' = b - lo - 128 and a = 127 - (q - lo), both in [-128, 127], and t = sum (b' + 1)^2,
+//   ||q - b||^2 = 2 (a . b' + floor(t / 2)) + (t & 1) + sum (q - lo - 128)^2 - pd
+// in whole numbers, so the tensor cores' integer score a . b' + floor(t / 2) and the parity of t give the distance
+// itself.  floor(t / 2) enters in one MMA of K = 32 like the norm of the 16-bit form: it is 127 times a number that 30
+// bytes of at most 255 add up to (stored less 128, which takes I8_SHIFT off every score), plus a remainder that the
+// query side multiplies by 1.  Scores stay below 2^22, distances and doubled scores below 2^24: exact as floats too.
+// Half the MMAs per score, and the re-rank has no row left to read: 10,000 queries at 1M x 128, main pass 2,400 -> 1,837 us,
+// re-rank 196 -> 57, the search 2,964 -> 2,181; 501 queries, 100 results of 50,001 x 100 211 -> 176.
+static constexpr int I8_MAX_PD = 224;
+static constexpr int I8_MAX_HALF = 30 * 255 * 127 + 126;  // the largest floor(t / 2) that fits
+static constexpr int I8_SHIFT = 30 * 127 * 128;
+
+// one warp per row: the operand row, the image of its 32 bytes of the norm step (rows from n on: a large one), the parity
+// of t; `too_large` is set when a row's floor(t / 2) does not fit
+__global__ void convert8_rows_kernel(const float* __restrict__ src, size_t first, size_t n, size_t n_pad, int pd, int Kp8, float lo,
+                                     uint8_t* __restrict__ dst, uint8_t* __restrict__ ext, uint8_t* __restrict__ parity,
+                                     unsigned int* __restrict__ too_large) {
+  const int lane = threadIdx.x & 31;
+  const size_t row = first + blockIdx.x * size_t(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= n_pad) return;
+  int t = 2 * I8_MAX_HALF;
+  if (row < n) {
+    t = 0;
+    for (int c = lane; c < Kp8; c += 32) {
+      int v = 0;
+      if (c < pd) {
+        v = int(src[row * size_t(pd) + c] - lo) - 128;
+        t += (v + 1) * (v + 1);
+      }
+      dst[row * size_t(Kp8) + c] = uint8_t(int8_t(v));
+    }
+    t = __reduce_add_sync(FV_FULL, t);
+    if (lane == 0) {
+      parity[row] = uint8_t(t & 1);
+      if (t / 2 > I8_MAX_HALF) *too_large = 1u;
+    }
+  }
+  const int h = min(t / 2, I8_MAX_HALF);
+  const int left = h / 127, j = lane < 16 ? lane - 1 : lane - 2;  // the lane's place among the 30
+  const int x = lane == 0 ? h % 127 : lane == 16 ? 0 : min(255, max(0, left - 255 * j)) - 128;
+  ext[row * 32 + (lane ^ ((int(row >> 2) & 1) << 4))] = uint8_t(int8_t(x));
+}
+
+// one warp per row.  dst8 (queries over a base with 8-bit operands): the 8-bit query row and the query's constant of the
+// formula above as well; q8_bad is set when a component is not one of the base's 256 numbers.
 template <bool BF16>
 __global__ void convert_rows_kernel(const float* __restrict__ src, size_t n, int pd, int Kp, uint16_t* __restrict__ dst,
-                                    float* __restrict__ norm2, int is_l2, float mul, RangeStats* __restrict__ st) {
+                                    float* __restrict__ norm2, int is_l2, float mul, RangeStats* __restrict__ st,
+                                    uint8_t* __restrict__ dst8, int Kp8, float lo8, float* __restrict__ const8,
+                                    unsigned int* __restrict__ q8_bad) {
   const int lane = threadIdx.x & 31;
   const size_t row = blockIdx.x * size_t(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n) return;
@@ -874,6 +1013,23 @@ __global__ void convert_rows_kernel(const float* __restrict__ src, size_t n, int
     mx = fmaxf(mx, __shfl_xor_sync(FV_FULL, mx, o));
     bad_int |= __shfl_xor_sync(FV_FULL, bad_int, o);
     bad_fin |= __shfl_xor_sync(FV_FULL, bad_fin, o);
+  }
+  if (dst8) {
+    int t = 0;
+    bool bad = bad_int || bad_fin;
+    for (int c = lane; c < Kp8; c += 32) {
+      const float v = c < pd ? src[row * size_t(pd) + c] - lo8 : 127.f;
+      bad = bad || !(v >= 0.f && v <= 255.f);
+      const int w = bad ? 127 : int(v);
+      if (c < pd) t += (w - 128) * (w - 128);
+      dst8[row * size_t(Kp8) + c] = uint8_t(int8_t(127 - w));
+    }
+    t = __reduce_add_sync(FV_FULL, t);
+    bad = __any_sync(FV_FULL, bad);
+    if (lane == 0) {
+      const8[row] = float(t - pd + 2 * I8_SHIFT);
+      if (bad) *q8_bad = 1u;
+    }
   }
   if (lane == 0) {
     if (norm2) norm2[row] = is_l2 ? s : 0.f;
@@ -936,19 +1092,32 @@ __global__ void init_stats_kernel(RangeStats* st) {
   st->not_finite = 0;
 }
 
+// what a search begins with: the queries' statistics, no query to re-run, no error, no query known to miss the 8-bit form
+__global__ void init_search_kernel(RangeStats* qst, unsigned int* words) {
+  qst->min_v = INFINITY;
+  qst->max_v = -INFINITY;
+  qst->max_norm2 = 0.f;
+  qst->not_integer = 0;
+  qst->not_finite = 0;
+  for (int i = 0; i < 3; ++i) words[i] = 0u;
+}
+
 // ------------------------------------------------------------------------------------------------
 // Exact re-rank and certification: one warp per query.
 struct RerankParams {
   const float* tau;       // the bound every candidate was tested against
   const u64* cbuf;        // candidates of the main pass: [grid * segmax][LISTS][ccap]
   const unsigned int* ccnt;
-  int ccap, MT, parts, grid, segmax;  // main-pass tiling
+  int ccap;
+  PassShapes shapes;      // main pass
+  const float* const8;    // 8-bit operands: the queries' constants, the parity of every row's t
+  const uint8_t* parity8;
   const float* rows;      // n x pd fp32
   const float* queries;   // nq x pd fp32
   const float* qnorm2;    // nq (0 for inner product)
   const RangeStats* bst;  // base statistics
   const RangeStats* qst;  // query statistics
-  int n, nq, pd, Kp, k, MH, is_l2, bf16;
+  int n, nq, pd, Kp, k, is_l2, bf16;
   int wpq;                // warps per query: 1, 2, 4 or 8
   uint32_t id_base;
   u64* out_keys;          // nq x k
@@ -1024,18 +1193,21 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
     eps = exact_regime ? 0.f : eps * 1.01f + 1e-30f;
   }
 
-  const int rows_per_tile = 128 * p.MH;
+  const bool is8 = IS_L2 && p.shapes.is8();
+  const PassShape& sh = p.shapes.taken();
+  const int rows_per_tile = 128 * sh.MH;
   const int mt = int(q / rows_per_tile), r = int(q % rows_per_tile);
+  const float const8 = is8 ? p.const8[q] : 0.f;
   // every row whose score is below tau is in the buffer; every other row scores >= tau
   const float tau = p.tau[q];
   bool overflow = false;
   bool mismatch = false;  // exact regime only: a score that is not the exact distance
   u64 bound = FV_EMPTY_KEY;
-  const int lists_per_seg = p.MH == 2 ? 2 : 4;
+  const int lists_per_seg = sh.MH == 2 ? 2 : 4;
   // The candidates of this query sit in parts * lists_per_seg short lists.  32 lists at a time: each lane looks up
   // one list's count, a prefix sum lines the entries up, and the warp walks them 32 per step (a lane finds the
   // list of its entry by bisection over the prefix sums), so every step computes 32 exact distances.
-  const int nlist = p.parts * lists_per_seg;
+  const int nlist = sh.parts * lists_per_seg;
   int taken = 0;  // runs of eight candidates seen so far, the same in all warps of the query
   for (int l0 = 0; l0 < nlist; l0 += 32) {
     const int l = l0 + lane;
@@ -1043,9 +1215,9 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
     unsigned long long slot = 0;
     if (l < nlist) {
       const int part = l / lists_per_seg, li = l - part * lists_per_seg;
-      const int g = part * p.MT + mt;
-      const int c = g % p.grid, seg_local = g / p.grid;
-      slot = (size_t(c) * p.segmax + seg_local) * LISTS + list_of_row(p.MH, r, li);
+      const int g = part * sh.MT + mt;
+      const int c = g % sh.grid, seg_local = g / sh.grid;
+      slot = (size_t(c) * sh.segmax + seg_local) * LISTS + list_of_row(sh.MH, r, li);
       cnt = p.ccnt[slot];
       if (cnt > unsigned(p.ccap)) {
         overflow = true;
@@ -1077,6 +1249,12 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
         id = key_id(ck);
         have = id < uint32_t(p.n);
         if (!have) mismatch = true;  // a padded row can only get here through a non-finite score
+      }
+      if (is8) {  // the score is the distance but for the query's constant and one bit
+        if (MULTI && ((taken++) & (p.wpq - 1)) != sub) continue;
+        const float d = have ? 2.f * key_distance(ck) + float(p.parity8[id]) + const8 : INFINITY;
+        top.offer(have ? make_key(d, id + p.id_base) : FV_EMPTY_KEY, bound);
+        continue;
       }
       for (int s = 0; s < 32 && t0 + s < total; s += 8) {
         if (MULTI && ((taken++) & (p.wpq - 1)) != sub) continue;  // runs of eight are dealt in turn
@@ -1112,10 +1290,12 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
   if (sub != 0 || q_own >= size_t(p.nq)) return;
   const u64 kth = top.last();
   bool certified;
-  if (overflow || mismatch || !q_in_range || !(tau == tau)) {
+  if (overflow || mismatch || !(is8 || q_in_range) || !(tau == tau)) {
     certified = false;
   } else if (tau == INFINITY) {
     certified = true;  // every row with a finite score was a candidate
+  } else if (is8) {
+    certified = kth != FV_EMPTY_KEY && key_distance(kth) < 2.f * tau + const8;  // every other row's distance is at least that
   } else {
     // the k-th result must be provably nearer than anything that was not a candidate
     certified = kth != FV_EMPTY_KEY && (key_distance(kth) - qn2) + eps < tau;
@@ -1143,16 +1323,29 @@ __device__ __forceinline__ size_t sample_row_at(size_t slot, size_t ns) {  // th
   return ((slot - sample_prefix(ns, j + 1)) << (j + 1)) + (size_t(1) << j);
 }
 
+// base8 (bases with 8-bit operands): those and their norm bytes too, up to row nspad of the latter
 __global__ void gather_sample_kernel(const uint16_t* __restrict__ half, const float* __restrict__ norm2, size_t n, int Kp,
-                                     size_t ns, uint16_t* __restrict__ samp, float* __restrict__ snorm) {
+                                     size_t ns, uint16_t* __restrict__ samp, float* __restrict__ snorm,
+                                     const uint8_t* __restrict__ base8, const uint8_t* __restrict__ ext8, int Kp8, size_t nspad,
+                                     uint8_t* __restrict__ samp8, uint8_t* __restrict__ samp_ext8) {
   const int lane = threadIdx.x & 31;
   const size_t i = blockIdx.x * size_t(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= ns) return;
+  const auto swap8 = [](size_t row) { return (int(row >> 2) & 1) << 4; };  // the image's halves trade places in rows 4..7 of 8
+  if (i >= ns) {
+    if (base8 && i < nspad) samp_ext8[i * 32 + lane] = uint8_t((lane & 15) == 0 ? 0 : 127);  // beyond the sample: a large score
+    return;
+  }
   const size_t src = size_t((unsigned long long)sample_row_at(i, ns) * n / ns);
   const uint4* a = reinterpret_cast<const uint4*>(half + src * size_t(Kp));
   uint4* b = reinterpret_cast<uint4*>(samp + i * size_t(Kp));
   for (int c = lane; c < Kp / 8; c += 32) b[c] = a[c];
   if (lane == 0) snorm[i] = norm2[src];
+  if (base8) {
+    const uint4* a8 = reinterpret_cast<const uint4*>(base8 + src * size_t(Kp8));
+    uint4* b8 = reinterpret_cast<uint4*>(samp8 + i * size_t(Kp8));
+    for (int c = lane; c < Kp8 / 16; c += 32) b8[c] = a8[c];
+    samp_ext8[i * 32 + (lane ^ swap8(i))] = ext8[src * 32 + (lane ^ swap8(src))];
+  }
 }
 
 __global__ void scatter_keys_kernel(const u64* __restrict__ src, const uint32_t* __restrict__ qids, size_t nsub, int L,
@@ -1181,17 +1374,18 @@ static EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// rows x Kp 16-bit matrix, boxes of `box_rows` rows x 64 elements, 128-byte swizzle
-static int make_tmap(CUtensorMap* map, bool bf16, void* ptr, size_t rows, int Kp, int box_rows) {
+// rows x K matrix of operands, boxes of `box_rows` rows x 128 bytes, 128-byte swizzle
+static CUtensorMapDataType type16(bool bf16) { return bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16; }
+static int make_tmap(CUtensorMap* map, CUtensorMapDataType type, void* ptr, size_t rows, int K, int box_rows) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(FV_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  cuuint64_t gdim[2] = {cuuint64_t(Kp), cuuint64_t(rows)};
-  cuuint64_t gstride[1] = {cuuint64_t(Kp) * 2};
-  cuuint32_t box[2] = {cuuint32_t(KBLK), cuuint32_t(box_rows)};
+  const int size = type == CU_TENSOR_MAP_DATA_TYPE_UINT8 ? 1 : 2;
+  cuuint64_t gdim[2] = {cuuint64_t(K), cuuint64_t(rows)};
+  cuuint64_t gstride[1] = {cuuint64_t(K) * size};
+  cuuint32_t box[2] = {cuuint32_t(128 / size), cuuint32_t(box_rows)};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, ptr, gdim, gstride,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = fn(map, type, 2, ptr, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(FV_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
   return FV_OK;
 }
@@ -1207,6 +1401,10 @@ struct TcSide {
   int every = 32;          // 1 row in `every` is sampled
   DevBuf samp, samp_norm2; // the sample's operand rows and norms (+inf padded)
   DevBuf ext, samp_ext;    // norm pieces of the base rows and of the sample (padded like the norms), 32 B per row
+  bool i8 = false;         // the base has 8-bit operands too
+  int Kp8 = 0;             // their row length: pd rounded up to 128
+  float lo8 = 0.f;         // the value they store as -128
+  DevBuf rows8, ext8, parity8, samp8, samp_ext8;
   int ext_e = 0;           // the pieces hold ||b||^2 / 2^ext_e
   bool ext_valid = false;
   RangeStats h_stats{};
@@ -1214,17 +1412,31 @@ struct TcSide {
 
 void tc_free(TcSide* tc) { delete tc; }
 
+// the words behind the two RangeStats in `stats`
+enum { W_RETRY = 0, W_ERR = 1, W_Q8_BAD = 2, W_TOO_LARGE = 3 };
+static unsigned int* side_words(TcSide* tc) { return reinterpret_cast<unsigned int*>(tc->stats.as<RangeStats>() + 2); }
+
 static inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
+struct Queries8 {  // where convert puts the 8-bit form of queries
+  uint8_t* dst = nullptr;
+  int Kp8 = 0;
+  float lo8 = 0.f;
+  float* const8 = nullptr;
+  unsigned int* bad = nullptr;
+};
+
 static int convert(fv_ctx* ctx, bool bf16, const float* d_src, size_t n, int pd, int Kp, uint16_t* dst, float* norm2,
-                   bool is_l2, float mul, RangeStats* st) {
+                   bool is_l2, float mul, RangeStats* st, const Queries8& q8 = {}) {
   if (n == 0) return FV_OK;
   const int wpb = 8;
   const unsigned blocks = unsigned((n + wpb - 1) / wpb);
   if (bf16)
-    convert_rows_kernel<true><<<blocks, wpb * 32, 0, ctx->stream>>>(d_src, n, pd, Kp, dst, norm2, is_l2 ? 1 : 0, mul, st);
+    convert_rows_kernel<true><<<blocks, wpb * 32, 0, ctx->stream>>>(d_src, n, pd, Kp, dst, norm2, is_l2 ? 1 : 0, mul, st, q8.dst,
+                                            q8.Kp8, q8.lo8, q8.const8, q8.bad);
   else
-    convert_rows_kernel<false><<<blocks, wpb * 32, 0, ctx->stream>>>(d_src, n, pd, Kp, dst, norm2, is_l2 ? 1 : 0, mul, st);
+    convert_rows_kernel<false><<<blocks, wpb * 32, 0, ctx->stream>>>(d_src, n, pd, Kp, dst, norm2, is_l2 ? 1 : 0, mul, st, q8.dst,
+                                             q8.Kp8, q8.lo8, q8.const8, q8.bad);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   return FV_OK;
@@ -1238,6 +1450,37 @@ static int split_norms(fv_ctx* ctx, bool bf16, const float* norm2, size_t first,
   else split_norms_kernel<false><<<blocks, 256, 0, ctx->stream>>>(norm2, first, count, inv, ext);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
+  return FV_OK;
+}
+
+// The 8-bit form of rows n_old .. total, or of all of them where the rows before have none or another `lo`; none for a base
+// that does not qualify.  Costs 160 bytes per row and, beside the 16-bit form, a quarter more time in add.
+static int append8(fv_ctx* ctx, TcSide* tc, const float* all_rows, size_t n_old, size_t total, size_t npad) {
+  const RangeStats& st = tc->h_stats;
+  const float lo = st.min_v >= 0.f && st.max_v <= 255.f ? 0.f : st.min_v >= -128.f && st.max_v <= 127.f ? -128.f : st.min_v;
+  bool fits = !st.not_integer && !st.not_finite && tc->pd <= I8_MAX_PD && std::fabs(lo) <= 65536.f && st.max_v - lo <= 255.f;
+  if (fits) {
+    tc->Kp8 = round_up(tc->pd, 2 * KBLK);
+    const size_t first = tc->i8 && tc->lo8 == lo ? n_old : 0;
+    unsigned int* too_large = side_words(tc) + W_TOO_LARGE;
+    FV_TRY(tc->rows8.grow(total * size_t(tc->Kp8), first * size_t(tc->Kp8), ctx->stream));
+    FV_TRY(tc->ext8.grow(npad * 32, first * 32, ctx->stream));
+    FV_TRY(tc->parity8.grow(npad, first, ctx->stream));
+    FV_CUDA(cudaMemsetAsync(too_large, 0, sizeof(unsigned int), ctx->stream));
+    convert8_rows_kernel<<<unsigned((npad - first + 7) / 8), 256, 0, ctx->stream>>>(
+        all_rows, first, total, npad, tc->pd, tc->Kp8, lo, tc->rows8.as<uint8_t>(), tc->ext8.as<uint8_t>(),
+        tc->parity8.as<uint8_t>(), too_large);
+    ctx->stats.launches++;
+    FV_CUDA(cudaGetLastError());
+    unsigned int h_large = 0;
+    FV_CUDA(cudaMemcpyAsync(&h_large, too_large, sizeof(h_large), cudaMemcpyDeviceToHost, ctx->stream));
+    FV_CUDA(cudaStreamSynchronize(ctx->stream));
+    fits = h_large == 0;
+  }
+  tc->i8 = fits;
+  tc->lo8 = lo;
+  if (!fits)
+    for (DevBuf* b : {&tc->rows8, &tc->ext8, &tc->parity8, &tc->samp8, &tc->samp_ext8}) b->release();
   return FV_OK;
 }
 
@@ -1324,15 +1567,21 @@ int tc_append(fv_ctx* ctx, TcSide** ptc, int metric, const float* d_rows_new, si
     const size_t first = resplit ? 0 : n_old;
     FV_TRY(split_norms(ctx, tc->bf16, tc->norm2.as<float>(), first, npad - first, e, tc->ext.as<uint16_t>()));
   }
+  if (metric == FV_L2) FV_TRY(append8(ctx, tc, d_rows_new - n_old * size_t(pd), n_old, total, npad));
   // the strided sample the threshold of the main pass is estimated from
   tc->every = pick_sample_every(total);
   tc->ns = std::max<size_t>(SAMPLE_R_MAX, total / size_t(tc->every));
   const size_t nspad = (tc->ns + TILE_N - 1) / TILE_N * TILE_N + TILE_N;
   FV_TRY(tc->samp.reserve(tc->ns * size_t(Kp) * 2 + 1024));
   FV_TRY(tc->samp_norm2.reserve(nspad * sizeof(float)));
-  gather_sample_kernel<<<unsigned((tc->ns + 7) / 8), 256, 0, ctx->stream>>>(
-      tc->half.as<uint16_t>(), tc->norm2.as<float>(), total, Kp, tc->ns, tc->samp.as<uint16_t>(),
-      tc->samp_norm2.as<float>());
+  if (tc->i8) {
+    FV_TRY(tc->samp8.reserve(tc->ns * size_t(tc->Kp8)));
+    FV_TRY(tc->samp_ext8.reserve(nspad * 32));
+  }
+  gather_sample_kernel<<<unsigned((nspad + 7) / 8), 256, 0, ctx->stream>>>(
+      tc->half.as<uint16_t>(), tc->norm2.as<float>(), total, Kp, tc->ns, tc->samp.as<uint16_t>(), tc->samp_norm2.as<float>(),
+      tc->i8 ? tc->rows8.as<uint8_t>() : nullptr, tc->ext8.as<uint8_t>(), tc->Kp8, nspad, tc->samp8.as<uint8_t>(),
+      tc->samp_ext8.as<uint8_t>());
   fill_f32_kernel<<<8, 256, 0, ctx->stream>>>(tc->samp_norm2.as<float>() + tc->ns, nspad - tc->ns, INFINITY);
   ctx->stats.launches += 2;
   FV_CUDA(cudaGetLastError());
@@ -1365,12 +1614,14 @@ bool tc_usable(const TcSide* tc, size_t n, size_t nq, int k) {
 // units the 16-bit copy of the base was streamed from HBM once per query tile).  `parts` is the value that minimises
 // waves x (chunk length + a fixed cost per chunk).
 struct Tiling {
-  int KB, MH, MT, NT, grid, segmax, nstage, cpn, parts, nchunks, ext_ring;
+  int KB, last_steps, MH, MT, NT, grid, segmax, nstage, cpn, parts, nchunks, ext_ring;
   size_t smem;
 };
 
-static int make_tiling(fv_ctx* ctx, int Kp, size_t nq, size_t rows, int scratch_bytes, Tiling* t, int force_mh = 0) {
-  t->KB = Kp / KBLK;
+// `row_bytes`: bytes of an operand row that hold data
+static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, int scratch_bytes, Tiling* t, int force_mh = 0) {
+  t->KB = (row_bytes + 127) / 128;
+  t->last_steps = (row_bytes - (t->KB - 1) * 128 + 31) / 32;
   t->MH = force_mh ? force_mh : (t->KB <= 2 ? 2 : 1);
   const int rows_per_tile = 128 * t->MH;
   t->MT = int((nq + rows_per_tile - 1) / rows_per_tile);
@@ -1403,13 +1654,22 @@ static int make_tiling(fv_ctx* ctx, int Kp, size_t nq, size_t rows, int scratch_
   return fail(FV_ERR_UNSUPPORTED, "not enough shared memory for the tensor-core tiling");
 }
 
+static PassShape pass_shape(const Tiling& t) { return PassShape{t.MT, t.parts, t.grid, t.segmax, t.MH}; }
+
+// One launch over one way's operands, or over whichever of two the queries allow (`w8` and its word).
 template <int KPT, bool THRESH>
-static int launch_gemm(fv_ctx* ctx, const Tiling& t, const CUtensorMap& tmA, const CUtensorMap& tmB,
-                       const GemmParams& gp) {
-  void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams) =
-      t.MH == 2 ? gemm_topk_kernel<2, KPT, THRESH> : gemm_topk_kernel<1, KPT, THRESH>;
-  FV_TRY(allow_smem(ctx, kern, t.smem));
-  kern<<<t.grid, NTHREADS, t.smem, ctx->stream>>>(tmA, tmB, gp);
+static int launch_gemm(fv_ctx* ctx, const Tiling& t16, const GemmWay& w16, const Tiling& t8, const GemmWay* w8,
+                       const unsigned int* q8_bad) {
+  if (!w8) {
+    auto kern = t16.MH == 2 ? gemm_topk_kernel<2, KPT, THRESH> : gemm_topk_kernel<1, KPT, THRESH>;
+    FV_TRY(allow_smem(ctx, kern, t16.smem));
+    kern<<<t16.grid, NTHREADS, t16.smem, ctx->stream>>>(w16.tmA, w16.tmB, w16.p);
+  } else {
+    auto kern = t16.MH == 2 ? gemm_topk_either_kernel<2, KPT, THRESH> : gemm_topk_either_kernel<1, KPT, THRESH>;
+    const size_t smem = std::max(t16.smem, t8.smem);
+    FV_TRY(allow_smem(ctx, kern, smem));
+    kern<<<std::max(t16.grid, t8.grid), NTHREADS, smem, ctx->stream>>>(w16, *w8, q8_bad);
+  }
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   return FV_OK;
@@ -1420,17 +1680,33 @@ static int launch_gemm(fv_ctx* ctx, const Tiling& t, const CUtensorMap& tmA, con
 static std::atomic<long long> g_test_wait_limit{0};
 static std::atomic<int> g_test_skip_unit{-1};
 
-static void fill_params(GemmParams* g, const Tiling& t, size_t rows, size_t nq, int scratch_bytes) {
-  g->wait_limit = WAIT_LIMIT_CYCLES;
-  g->fault_skip_unit = -1;
+// The query side of the norm step, 16 bytes that a row holds twice: 2^ext_e for each of the three pieces of a norm (bf16:
+// 1.0); in the 8-bit form 1 for the remainder and 127 for the rest.
+static uint4 norm_step_queries(const TcSide* tc) {
+  const uint32_t c = tc->bf16 ? 0x3F80u : uint32_t((tc->ext_e + 15) << 10);
+  return make_uint4(c | (c << 16), c, 0u, 0u);
+}
+static uint4 norm_step_queries8() { return make_uint4(0x7F7F7F01u, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu); }
+
+struct WaitLimit {
+  long long cycles = WAIT_LIMIT_CYCLES;
+  int skip_unit = -1;
+};
+static WaitLimit next_wait_limit() {  // of one launch
+  WaitLimit l;
   const long long test_limit = g_test_wait_limit.exchange(0);
-  if (test_limit > 0) {
-    g->wait_limit = test_limit;
-    g->fault_skip_unit = g_test_skip_unit.exchange(-1);
-  }
+  if (test_limit > 0) l = WaitLimit{test_limit, g_test_skip_unit.exchange(-1)};
+  return l;
+}
+
+static void fill_params(GemmParams* g, const Tiling& t, size_t rows, size_t nq, int scratch_bytes, const WaitLimit& limit) {
+  g->wait_limit = limit.cycles;
+  g->fault_skip_unit = limit.skip_unit;
+  g->grid = t.grid;
   g->n = int(rows);
   g->nq = int(nq);
   g->KB = t.KB;
+  g->last_steps = t.last_steps;
   g->NT = t.NT;
   g->MT = t.MT;
   g->cpn = t.cpn;
@@ -1454,8 +1730,7 @@ void tc_info(const TcSide* tc, TcInfo* out) {
 }
 
 int* tc_error_word(TcSide* tc) {
-  RangeStats* qst = tc->stats.as<RangeStats>() + 1;
-  return reinterpret_cast<int*>(reinterpret_cast<unsigned int*>(qst + 1) + 1);
+  return reinterpret_cast<int*>(side_words(tc) + W_ERR);
 }
 
 int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_t a_rows, const float* d_thr,
@@ -1467,12 +1742,12 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
   if (tile_rows != 128 && tile_rows != 256) return fail(FV_ERR_ARG, "operand tiles have 128 or 256 rows");
   Tiling t{};
   // stages and shared memory for operand tiles of that height; the tiling itself is unused
-  FV_TRY(make_tiling(ctx, Kp, 256, size_t(TILE_N) * 1024, 0, &t, tile_rows == 128 ? 1 : 2));
+  FV_TRY(make_tiling(ctx, tc->pd * 2, 256, size_t(TILE_N) * 1024, 0, &t, tile_rows == 128 ? 1 : 2));
   GemmParams gp{};
-  fill_params(&gp, t, tc->n, a_rows, 0);
+  fill_params(&gp, t, tc->n, a_rows, 0, next_wait_limit());
   gp.nchunks = 0;
   gp.has_ext = metric == FV_L2 ? 1 : 0;
-  gp.aext_c = tc->bf16 ? 0x3F80u : uint32_t((tc->ext_e + 15) << 10);
+  gp.aext = norm_step_queries(tc);
   gp.idesc = make_idesc(128, TILE_N, tc->bf16);
   gp.err = tc_error_word(tc);
   gp.ext = tc->ext.as<uint16_t>();
@@ -1489,8 +1764,8 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
   gp.task_moff = d_task_moff;
   gp.task_rows = d_task_rows;
   CUtensorMap tmA, tmB;
-  FV_TRY(make_tmap(&tmA, tc->bf16, const_cast<uint16_t*>(d_A), a_rows, Kp, 128));
-  FV_TRY(make_tmap(&tmB, tc->bf16, tc->half.p, tc->n, Kp, TILE_N));
+  FV_TRY(make_tmap(&tmA, type16(tc->bf16), const_cast<uint16_t*>(d_A), a_rows, Kp, 128));
+  FV_TRY(make_tmap(&tmB, type16(tc->bf16), tc->half.p, tc->n, Kp, TILE_N));
   FV_CUDA(cudaMemsetAsync(d_next_task, 0, sizeof(unsigned int), ctx->stream));
   void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams) =
       tile_rows == 128 ? gemm_topk_kernel<1, 2, true, true> : gemm_topk_kernel<2, 2, true, true>;
@@ -1521,88 +1796,115 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   while (k > 32 && R > SAMPLE_R_MAX && level < SAMPLE_LEVELS) R = pick_sample_r(k, tc->every << ++level);
   R = std::min(R, SAMPLE_R_MAX);
   const size_t ns = sample_prefix(tc->ns, level);
-  Tiling ts{}, tm{};
-  FV_TRY(make_tiling(ctx, Kp, nq, ns, SCRATCH_BYTES, &ts));
-  FV_TRY(make_tiling(ctx, Kp, nq, n, 0, &tm));
-  const int rows_per_tile = 128 * tm.MH;
+  // R is rounded up to the next instantiated list length - 1 of the sample pass (a larger R only loosens the bound)
+  R = R <= 7 ? R : (R <= 9 ? 9 : 13);
 
-  // queries -> 16-bit operand rows scaled by -2 (L2) or -1 (inner product), padded to whole tiles with zeros;
-  // norms; statistics
-  const size_t nq_pad = size_t(tm.MT) * rows_per_tile;
-  FV_TRY(ctx->scratch[3].reserve(nq_pad * size_t(Kp) * 2));
-  const size_t nlists = size_t(tm.grid) * tm.segmax * LISTS;
+  // One way through both passes, or two: over the 8-bit operands where the base has them and, should a query of the batch
+  // not fit them (known on the device only), over the 16-bit ones.  The kernels of the way that is not taken leave at once.
+  const int ways = tc->i8 ? 2 : 1;
+  struct Way {
+    Tiling ts, tm;           // sample pass, main pass
+    CUtensorMap tmA, tmS, tmB;
+    size_t nq_pad = 0;
+  } way[2] = {};             // 0: 16-bit, 1: 8-bit
+  size_t nq_pad = 0, nlists = 0, sample_lists = 0;
+  for (int i = 0; i < ways; ++i) {
+    const int row_bytes = i ? pd : pd * 2;
+    FV_TRY(make_tiling(ctx, row_bytes, nq, ns, SCRATCH_BYTES, &way[i].ts));
+    FV_TRY(make_tiling(ctx, row_bytes, nq, n, 0, &way[i].tm));
+    way[i].nq_pad = size_t(way[i].tm.MT) * 128 * way[i].tm.MH;
+    nq_pad = std::max(nq_pad, way[i].nq_pad);
+    nlists = std::max(nlists, size_t(way[i].tm.grid) * way[i].tm.segmax * LISTS);
+    sample_lists = std::max(sample_lists, size_t(way[i].ts.grid) * way[i].ts.segmax * LISTS);
+  }
+
+  // queries -> operand rows (16 bits: scaled by -2 for L2, -1 for inner product), padded to whole tiles with zeros; norms;
+  // statistics
+  const size_t a16_bytes = (nq_pad * size_t(Kp) * 2 + 255) & ~size_t(255);
+  FV_TRY(ctx->scratch[3].reserve(a16_bytes + (tc->i8 ? nq_pad * size_t(tc->Kp8) : 0)));
   // Candidate slots per epilogue thread and segment: 256 unless the buffers would pass 2 GB (they are written
   // sparsely: about 160 entries per query in all).  A base stored cluster by cluster puts most of a query's
   // candidates into one or two chunks, so the slots must hold more than the average.
   int ccap = 256;
   while (ccap > 16 && nlists * size_t(ccap) * sizeof(u64) > (size_t(2) << 30)) ccap >>= 1;
-  FV_TRY(ctx->scratch[5].reserve(2 * nq_pad * sizeof(float) + nlists * sizeof(unsigned int)));
-  FV_TRY(ctx->scratch[6].reserve(size_t(ts.grid) * ts.segmax * LISTS * KP * sizeof(u64)));
+  FV_TRY(ctx->scratch[5].reserve(3 * nq_pad * sizeof(float) + nlists * sizeof(unsigned int)));
+  FV_TRY(ctx->scratch[6].reserve(sample_lists * KP * sizeof(u64)));
   FV_TRY(ctx->scratch[7].reserve(nq * sizeof(uint32_t)));
   FV_TRY(ctx->scratch[9].reserve(nlists * size_t(ccap) * sizeof(u64)));
   uint16_t* dA = ctx->scratch[3].as<uint16_t>();
+  uint8_t* dA8 = ctx->scratch[3].as<uint8_t>() + a16_bytes;
   float* qn2 = ctx->scratch[5].as<float>();
   float* tau = qn2 + nq_pad;
-  unsigned int* ccnt = reinterpret_cast<unsigned int*>(tau + nq_pad);
+  float* const8 = tau + nq_pad;
+  unsigned int* ccnt = reinterpret_cast<unsigned int*>(const8 + nq_pad);
   RangeStats* bst = tc->stats.as<RangeStats>();
   RangeStats* qst = bst + 1;
-  unsigned int* retry_count = reinterpret_cast<unsigned int*>(qst + 1);
-  int* err = reinterpret_cast<int*>(retry_count + 1);
-  CUtensorMap tmA, tmS, tmB;
-  FV_TRY(make_tmap(&tmA, tc->bf16, dA, nq_pad, Kp, 128));
-  FV_TRY(make_tmap(&tmS, tc->bf16, tc->samp.p, ns, Kp, TILE_N));
-  FV_TRY(make_tmap(&tmB, tc->bf16, tc->half.p, n, Kp, TILE_N));
+  unsigned int* words = side_words(tc);
+  unsigned int* retry_count = words + W_RETRY;
+  unsigned int* q8_bad = tc->i8 ? words + W_Q8_BAD : nullptr;
+  FV_TRY(make_tmap(&way[0].tmA, type16(tc->bf16), dA, nq_pad, Kp, 128));
+  FV_TRY(make_tmap(&way[0].tmS, type16(tc->bf16), tc->samp.p, ns, Kp, TILE_N));
+  FV_TRY(make_tmap(&way[0].tmB, type16(tc->bf16), tc->half.p, n, Kp, TILE_N));
+  if (tc->i8) {
+    const CUtensorMapDataType type8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    FV_TRY(make_tmap(&way[1].tmA, type8, dA8, nq_pad, tc->Kp8, 128));
+    FV_TRY(make_tmap(&way[1].tmS, type8, tc->samp8.p, ns, tc->Kp8, TILE_N));
+    FV_TRY(make_tmap(&way[1].tmB, type8, tc->rows8.p, n, tc->Kp8, TILE_N));
+  }
 
-  init_stats_kernel<<<1, 1, 0, ctx->stream>>>(qst);
-  FV_CUDA(cudaMemsetAsync(retry_count, 0, 8, ctx->stream));
-  if (nq_pad > nq) FV_CUDA(cudaMemsetAsync(dA + nq * size_t(Kp), 0, (nq_pad - nq) * size_t(Kp) * 2, ctx->stream));
-  FV_TRY(convert(ctx, tc->bf16, d_queries, nq, pd, Kp, dA, qn2, is_l2, is_l2 ? -2.f : -1.f, qst));
+  init_search_kernel<<<1, 1, 0, ctx->stream>>>(qst, words);
+  if (nq_pad > nq) {
+    FV_CUDA(cudaMemsetAsync(dA + nq * size_t(Kp), 0, (nq_pad - nq) * size_t(Kp) * 2, ctx->stream));
+    if (tc->i8) FV_CUDA(cudaMemsetAsync(dA8 + nq * size_t(tc->Kp8), 0, (nq_pad - nq) * size_t(tc->Kp8), ctx->stream));
+  }
+  Queries8 q8;
+  if (tc->i8) q8 = Queries8{dA8, tc->Kp8, tc->lo8, const8, q8_bad};
+  FV_TRY(convert(ctx, tc->bf16, d_queries, nq, pd, Kp, dA, qn2, is_l2, is_l2 ? -2.f : -1.f, qst, q8));
   if (mark_stages) stage_mark(ctx);
 
-  // sample pass: per query the R (+1) best scores over the sampled rows
-  // the epilogue keeps its lists in registers, so their length is a template parameter: R is rounded up to the next
-  // instantiated length - 1 (a larger R only loosens the bound)
-  R = R <= 7 ? R : (R <= 9 ? 9 : 13);
-  GemmParams gs{};
-  fill_params(&gs, ts, ns, nq, SCRATCH_BYTES);
-  gs.has_ext = is_l2 ? 1 : 0;
-  gs.aext_c = tc->bf16 ? 0x3F80u : uint32_t((tc->ext_e + 15) << 10);  // 1.0 (bf16) or 2^ext_e (fp16)
-  gs.idesc = make_idesc(128, TILE_N, tc->bf16);
-  gs.cand = ctx->scratch[6].as<u64>();
-  gs.err = err;
-  gs.ext = tc->samp_ext.as<uint16_t>();
-  if (R == 5) FV_TRY((launch_gemm<6, false>(ctx, ts, tmA, tmS, gs)));
-  else if (R == 6) FV_TRY((launch_gemm<7, false>(ctx, ts, tmA, tmS, gs)));
-  else if (R == 7) FV_TRY((launch_gemm<8, false>(ctx, ts, tmA, tmS, gs)));
-  else if (R == 9) FV_TRY((launch_gemm<10, false>(ctx, ts, tmA, tmS, gs)));
-  else FV_TRY((launch_gemm<14, false>(ctx, ts, tmA, tmS, gs)));
-  sample_tau_kernel<<<unsigned((nq_pad + 7) / 8), 256, 0, ctx->stream>>>(gs.cand, ts.MT, ts.parts, ts.grid, ts.segmax,
-                                                                         ts.MH, int(nq_pad), R, tau);
+  GemmWay ws[2], wm[2];  // sample pass, main pass
+  const WaitLimit limit_s = next_wait_limit(), limit_m = next_wait_limit();
+  for (int i = 0; i < ways; ++i) {
+    GemmParams g{};
+    g.has_ext = is_l2 ? 1 : 0;
+    g.aext = i ? norm_step_queries8() : norm_step_queries(tc);
+    g.idesc = i ? make_idesc_i8(128, TILE_N) : make_idesc(128, TILE_N, tc->bf16);
+    g.err = tc_error_word(tc);
+    ws[i] = GemmWay{way[i].tmA, way[i].tmS, g};
+    fill_params(&ws[i].p, way[i].ts, ns, nq, SCRATCH_BYTES, limit_s);
+    ws[i].p.cand = ctx->scratch[6].as<u64>();
+    ws[i].p.ext = (i ? tc->samp_ext8 : tc->samp_ext).as<uint16_t>();
+    wm[i] = GemmWay{way[i].tmA, way[i].tmB, g};
+    fill_params(&wm[i].p, way[i].tm, n, nq, 0, limit_m);
+    wm[i].p.tau = tau;
+    wm[i].p.cbuf = ctx->scratch[9].as<u64>();
+    wm[i].p.ccnt = ccnt;
+    wm[i].p.ccap = ccap;
+    wm[i].p.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
+  }
+
+  // sample pass: per query the R (+1) best scores over the sampled rows, in the epilogue's registers
+  auto sample = R == 5 ? launch_gemm<6, false> : R == 6 ? launch_gemm<7, false> : R == 7 ? launch_gemm<8, false>
+              : R == 9 ? launch_gemm<10, false> : launch_gemm<14, false>;
+  FV_TRY(sample(ctx, way[0].ts, ws[0], way[1].ts, tc->i8 ? &ws[1] : nullptr, q8_bad));
+  sample_tau_kernel<<<unsigned((nq_pad + 7) / 8), 256, 0, ctx->stream>>>(
+      ctx->scratch[6].as<u64>(), PassShapes{pass_shape(way[0].ts), pass_shape(way[1].ts), q8_bad}, int(nq_pad), R, tau);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   if (mark_stages) stage_mark(ctx);
 
   // main pass: every row scoring below the query's sampled bound becomes a candidate
-  GemmParams gp = gs;
-  fill_params(&gp, tm, n, nq, 0);
-  gp.cand = nullptr;
-  gp.tau = tau;
-  gp.cbuf = ctx->scratch[9].as<u64>();
-  gp.ccnt = ccnt;
-  gp.ccap = ccap;
-  gp.ext = tc->ext.as<uint16_t>();
-  FV_TRY((launch_gemm<2, true>(ctx, tm, tmA, tmB, gp)));
+  FV_TRY((launch_gemm<2, true>(ctx, way[0].tm, wm[0], way[1].tm, tc->i8 ? &wm[1] : nullptr, q8_bad)));
   if (mark_stages) stage_mark(ctx);
 
   RerankParams rp{};
   rp.tau = tau;
-  rp.cbuf = gp.cbuf;
-  rp.ccnt = gp.ccnt;
-  rp.ccap = gp.ccap;
-  rp.MT = tm.MT;
-  rp.parts = tm.parts;
-  rp.grid = tm.grid;
-  rp.segmax = tm.segmax;
+  rp.cbuf = ctx->scratch[9].as<u64>();
+  rp.ccnt = ccnt;
+  rp.ccap = ccap;
+  rp.shapes = PassShapes{pass_shape(way[0].tm), pass_shape(way[1].tm), q8_bad};
+  rp.const8 = const8;
+  rp.parity8 = tc->parity8.as<uint8_t>();
   rp.rows = d_rows;
   rp.queries = d_queries;
   rp.qnorm2 = qn2;
@@ -1613,7 +1915,6 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   rp.pd = pd;
   rp.Kp = Kp;
   rp.k = k;
-  rp.MH = tm.MH;
   rp.is_l2 = metric == FV_L2 ? 1 : 0;
   rp.bf16 = tc->bf16 ? 1 : 0;
   rp.id_base = id_base;
