@@ -10,8 +10,8 @@
 // into three 16-bit pieces, inside the MMA.  The epilogue reads the accumulators back with
 // tcgen05.ld (one query row per thread) and only compares.
 //
-// Two passes.  A sample pass over 1 base row in 32 keeps, per query, its best few scores in
-// registers; the fifth best is that query's bound.  The main pass appends every row scoring below
+// Two passes.  A sample pass over 1 base row in 32 leaves, per query, the smallest score of every few
+// rows; about the fifth smallest of those is that query's bound.  The main pass appends every row scoring below
 // the bound to a candidate list.  A third kernel recomputes the reference's exact fp32 distance
 // chain (src/kernels.rs:200-231) for those candidates, picks the k best by (distance, id) and
 // CERTIFIES the result: a query passes only if every row that was not a candidate is provably
@@ -34,12 +34,12 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <numeric>
 
 #include "internal.h"
 
 namespace fv {
 
-static constexpr int KP = 16;          // candidate slots per query and segment in the candidate buffer
 static constexpr int TILE_N = 256;     // base rows per unit
 static constexpr int KBLK = 64;        // k elements per shared-memory block (128 bytes)
 static constexpr int A_BLOCK_BYTES = 128 * 128;   // 128 rows x 128 B
@@ -49,7 +49,6 @@ static constexpr int A_EXT_BYTES = 128 * EXT_K * 2;     // query side of the nor
 static constexpr int B_EXT_BYTES = TILE_N * EXT_K * 2;  // base side: one 8 KB tile per unit
 static constexpr int NEPI = 16;        // epilogue warps: four per tensor-memory lane quadrant
 static constexpr int LISTS = NEPI * 32; // per-thread lists of one segment
-static constexpr int SCRATCH_BYTES = NEPI * 16 * 32 * 4;  // list mode only; per epilogue warp: 16 columns x 32 rows of scores
 static constexpr int NTHREADS = 64 + NEPI * 32;   // warp 0 TMA, warp 1 MMA, warps 2..17 epilogue
 static constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;  // about 2 s; then the kernel gives up
 
@@ -265,6 +264,7 @@ struct StageCursor {
 // ------------------------------------------------------------------------------------------------
 struct GemmParams {
   int n, nq;
+  int a_row0;      // operand row of the first query
   int grid;        // CTAs that take work (task mode: all)
   int KB;          // k blocks of 128 bytes per row (64 16-bit or 128 8-bit elements)
   int last_steps;  // MMAs (32 bytes per row) of the last k block: 4 less the ones that would only meet padding
@@ -274,13 +274,14 @@ struct GemmParams {
   int nchunks;     // MT * parts; chunk g = part * MT + query tile, taken by CTA g % grid as its (g / grid)-th segment
   int segmax;      // segments per CTA
   int nstage;
-  int scratch_bytes;  // SCRATCH_BYTES in list mode, 0 in threshold mode
   int has_ext;        // L2: one more k step of 16 adds the row norms inside the MMA
   int ext_ring;       // norm-step tiles (8 KB each) kept in shared memory
   uint4 aext;         // the query side of the norm step: both 16-byte halves of every row
   const uint16_t* ext;  // base side of the norm step: 32 bytes per row, padded to whole tiles
   uint32_t idesc;
-  u64* cand;           // [grid * segmax][LISTS][KP]  (list mode: output)
+  // sample mode: the smallest score of every `group` (1, 8, 32 or 64) base rows, +inf beyond the last row
+  float* smin;         // [MT * 128 * MH][smin_ld]
+  int smin_ld, group;
   int* err;            // set to 1 when a bounded wait ran out
   long long wait_limit;  // cycles a thread waits on one barrier before the kernel gives up (WAIT_LIMIT_CYCLES)
   int fault_skip_unit;   // test hook, -1 = off: the producer of work item 0 leaves out the loads of this unit of it
@@ -373,47 +374,25 @@ struct PassShapes {
   __device__ __forceinline__ const PassShape& taken() const { return is8() ? s8 : s16; }
 };
 
-// The R-th smallest score of every query over the lists the sample pass left (+inf when the sample holds fewer rows).
-// Bound by latency: the lists of a query are a few dozen short runs of memory.  One warp per query, a list per lane
-// (the next 32 lists after that), each lane with its R smallest in registers; then R rounds take the smallest head
-// over the lanes.  One thread per query, as it was, put 1,000 queries on 4 SMs and read their lists one after
-// another: 94 us for 1,000 queries at 100k x 128 (the whole search 281 -> 203 us), 26 us for 10,000 at 1M x 128.
-__global__ void __launch_bounds__(256) sample_tau_kernel(const u64* __restrict__ lists, PassShapes shapes, int nq_pad, int R,
+// A query's bound: the R-th smallest of the group minima the sample pass left (+inf where there are fewer), which that many
+// sampled rows do not exceed.  A warp per query, each lane with the four smallest of its share: where a lane holds more than
+// four of the R smallest the bound is a little looser.  Bound by reading the minima from L2.
+// With the R best scores of the sample kept in registers by the epilogue, as it was, every chunk of 32 columns had an
+// insertion in some row: 251 us for 31,250 rows x 10,000 queries, 52 and 16 now; 1,000 queries at 100k x 128 38, 12 and 10.
+__global__ void __launch_bounds__(256) sample_tau_kernel(const float* __restrict__ smin, int ld, int groups, int nq, int R,
                                                          float* __restrict__ tau) {
   const int q = blockIdx.x * int(blockDim.x >> 5) + int(threadIdx.x >> 5), lane = lane_id();
-  const PassShape& sh = shapes.taken();
-  const int MT = sh.MT, parts = sh.parts, grid = sh.grid, segmax = sh.segmax, MH = sh.MH;
-  if (q >= nq_pad || q >= MT * 128 * MH) return;
-  const int rows_per_tile = 128 * MH;
-  const int mt = q / rows_per_tile, r = q - mt * rows_per_tile;
-  float best[SAMPLE_R_MAX];
+  if (q >= nq) return;
+  const float* src = smin + size_t(q) * ld;
+  float best[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+#pragma unroll 4
+  for (int i = lane; i < groups; i += 32) {
+    float v = src[i];
 #pragma unroll
-  for (int j = 0; j < SAMPLE_R_MAX; ++j) best[j] = INFINITY;
-  const int nl = MH == 2 ? 2 : 4;
-  for (int l = lane; l < parts * nl; l += 32) {
-    const int part = l / nl, li = l - part * nl;
-    const int g = part * MT + mt;
-    const int c = g % grid, seg = g / grid;
-    const u64* src = lists + ((size_t(c) * segmax + seg) * LISTS + list_of_row(MH, r, li)) * KP;
-    u64 key[SAMPLE_R_MAX];
-#pragma unroll
-    for (int j = 0; j < SAMPLE_R_MAX; ++j) key[j] = j < R ? src[j] : FV_EMPTY_KEY;  // a list holds R + 1 entries; the slots behind are stale
-    if (l < 32) {  // the lane's first list: it is sorted
-#pragma unroll
-      for (int j = 0; j < SAMPLE_R_MAX; ++j) best[j] = key[j] != FV_EMPTY_KEY ? key_distance(key[j]) : INFINITY;
-    } else {
-#pragma unroll
-      for (int j = 0; j < SAMPLE_R_MAX; ++j) {
-        float sc = key[j] != FV_EMPTY_KEY ? key_distance(key[j]) : INFINITY;
-        if (!(sc < best[SAMPLE_R_MAX - 1])) break;  // ascending: nothing behind it enters either
-#pragma unroll
-        for (int t = 0; t < SAMPLE_R_MAX; ++t) {
-          const bool lt = sc < best[t];
-          const float tmp = best[t];
-          best[t] = lt ? sc : tmp;
-          sc = lt ? tmp : sc;
-        }
-      }
+    for (int t = 0; t < 4; ++t) {
+      const float lo = fminf(best[t], v);
+      v = fmaxf(best[t], v);
+      best[t] = lo;
     }
   }
   uint32_t w = 0;
@@ -423,8 +402,8 @@ __global__ void __launch_bounds__(256) sample_tau_kernel(const u64* __restrict__
     const int owner = __ffs(__ballot_sync(FV_FULL, head == w)) - 1;
     if (lane == owner) {
 #pragma unroll
-      for (int t = 0; t + 1 < SAMPLE_R_MAX; ++t) best[t] = best[t + 1];
-      best[SAMPLE_R_MAX - 1] = INFINITY;
+      for (int t = 0; t < 3; ++t) best[t] = best[t + 1];
+      best[3] = INFINITY;
     }
   }
   if (lane == 0) tau[q] = order_bits_to_float(w);
@@ -449,7 +428,7 @@ struct Score<true> {
   __device__ static __forceinline__ T min3(T a, T b, T c) { return min(min(a, b), c); }
 };
 
-template <int MH, int KPT, bool THRESH, bool TASKS, bool I8>
+template <int MH, bool SAMPLE, bool TASKS, bool I8>
 __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p) {
   typedef Score<I8> S;
   typedef typename S::T T;
@@ -461,8 +440,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
   unsigned char* sAext = sA + size_t(MH) * p.KB * A_BLOCK_BYTES;       // 4 KB: the constant rows of the norm step
   unsigned char* sB = sAext + A_EXT_BYTES;                             // [nstage] stages of 32 KB
   unsigned char* sE = sB + size_t(p.nstage) * B_STAGE_BYTES;           // [ext_ring] norm-step tiles of 8 KB
-  unsigned char* scratch = sE + size_t(p.ext_ring) * B_EXT_BYTES;      // list mode: 16 epilogue warps x 2 KB
-  Barriers* bars = reinterpret_cast<Barriers*>(scratch + p.scratch_bytes);
+  Barriers* bars = reinterpret_cast<Barriers*>(sE + size_t(p.ext_ring) * B_EXT_BYTES);
   const AbortCtl abort_flag{&bars->abort_flag, p.wait_limit};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -535,7 +513,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
           const int part = g / p.MT, mt = g - part * p.MT;
           nt0 = part * p.cpn;
           nt1 = min(p.NT, nt0 + p.cpn);
-          a_row0 = mt * MH * 128;
+          a_row0 = p.a_row0 + mt * MH * 128;
         }
         ok = mbar_wait(&bars->a_empty, (seg & 1) ^ 1, abort_flag);
         if (!ok) break;
@@ -653,14 +631,9 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
     const int grp = MH == 2 ? (sub & 1) : 0;  // MH = 2: which 128-row half (= accumulator slot)
     const int e = sub * 128 + quad * 32 + lane;  // list index inside a segment
     const uint32_t lane_addr = uint32_t(quad * 32) << 16;
-    // list mode: the KPT best (score, id) of this thread's query row in the current segment, ascending by score;
-    // rows arrive in ascending id order, so a strict score compare keeps the (score, id) order
-    float sc[KPT];
-    uint32_t idv[KPT];
     T thr = S::bound(INFINITY);
     size_t cslot = 0;        // this thread's list of the current segment
     unsigned int ncand = 0;
-    float* sv = reinterpret_cast<float*>(scratch) + size_t(ew) * 512;  // list mode: 16 columns x 32 rows of scores
     int tile_idx = 0;
     bool ok = true;
     constexpr int NCOL = MH == 2 ? TILE_N / 2 : TILE_N / 4;
@@ -668,6 +641,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
     uint32_t n_rows = uint32_t(p.n);
     uint32_t a_row = 0;  // task mode: this thread's operand row
     uint32_t unit0 = 0;  // task mode: number of the task's first unit within its B run
+    float* sdst = nullptr;  // sample mode: this thread's row of smin
     float* mdst = nullptr;  // task mode, minima variant: where this thread's minima of the current task go
     for (int seg = 0, g = work_of(0); g < nwork && ok; g = work_of(++seg)) {
       int nt0, nt1, mt = 0;
@@ -691,16 +665,9 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
       }
       cslot = (size_t(blockIdx.x) * p.segmax + seg) * LISTS + e;
       ncand = 0;
-      if (THRESH) {  // the bound is fixed: the sample pass's estimate for this query
-        thr = S::bound(TASKS ? (p.minima ? 0.f : p.tau[a_row]) : p.tau[mt * (128 * MH) + (MH == 2 ? grp * 128 : 0) + quad * 32 + lane]);
-      } else {
-        thr = S::bound(INFINITY);
-#pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-          sc[j] = INFINITY;
-          idv[j] = 0xFFFFFFFFu;
-        }
-      }
+      const int q = mt * (128 * MH) + (MH == 2 ? grp * 128 : 0) + quad * 32 + lane;
+      if (SAMPLE) sdst = p.smin + size_t(q) * p.smin_ld;
+      else thr = S::bound(TASKS ? (p.minima ? 0.f : p.tau[a_row]) : p.tau[q]);  // the bound is fixed: the sample pass's estimate for this query
       for (int nt = nt0; nt < nt1 && ok; ++nt, ++tile_idx) {
         const int job = MH == 2 ? tile_idx * 2 + grp : tile_idx;
         const int slot = job & 1;
@@ -709,7 +676,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
         tc_fence_after();
         const uint32_t row_base = (unit0 + uint32_t(nt)) * TILE_N + col0;
         const uint32_t t_addr = tmem_base + lane_addr + uint32_t(slot * TILE_N + col0);
-        if (THRESH) {
+        {
           // Threshold mode.  The accumulator IS the score (the norm step and the scaled query side put
           // ||b||^2 - 2<q,b> there), so a chunk of 64 columns costs a minimum tree and one vote.  Every column
           // below the bound is appended to this thread's private list: a plain store and a register counter.
@@ -783,6 +750,38 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
             }
             if (mine && pos > p.pool_cap) p.owner_dropped[p.row_owner[a_row]] = 1u;  // some of this row's did not fit
           };
+          // Sample mode.  Minima of 8 columns, of 32 or of 64, or every score: 4 to 256 bytes of the query's own row.
+          auto sample = [&](uint32_t* r, int c) {
+            const uint32_t row0 = row_base + uint32_t(c);
+            const T inf = S::bound(INFINITY);
+            if (row0 + 64 > n_rows) {
+#pragma unroll
+              for (int i = 0; i < 64; ++i)
+                if (row0 + uint32_t(i) >= n_rows) r[i] = I8 ? 0x7FFFFFFFu : 0x7F800000u;
+            }
+            const auto f = [&](T v) { return I8 && v == inf ? INFINITY : float(v); };
+            float4* d4 = reinterpret_cast<float4*>(sdst + row0 / uint32_t(p.group));
+            if (p.group == 1) {
+#pragma unroll
+              for (int i = 0; i < 64; i += 4) d4[i / 4] = make_float4(f(S::of(r[i])), f(S::of(r[i + 1])), f(S::of(r[i + 2])), f(S::of(r[i + 3])));
+              return;
+            }
+            T g8[8];
+#pragma unroll
+            for (int gi = 0; gi < 8; ++gi) {
+              const uint32_t* q = r + gi * 8;
+              g8[gi] = S::min2(S::min3(S::min3(S::of(q[0]), S::of(q[1]), S::of(q[2])), S::of(q[3]), S::of(q[4])),
+                               S::min3(S::of(q[5]), S::of(q[6]), S::of(q[7])));
+            }
+            if (p.group == 8) {
+              d4[0] = make_float4(f(g8[0]), f(g8[1]), f(g8[2]), f(g8[3]));
+              d4[1] = make_float4(f(g8[4]), f(g8[5]), f(g8[6]), f(g8[7]));
+              return;
+            }
+            const T a = S::min2(S::min3(g8[0], g8[1], g8[2]), g8[3]), b = S::min2(S::min3(g8[4], g8[5], g8[6]), g8[7]);
+            if (p.group == 32) *reinterpret_cast<float2*>(d4) = make_float2(f(a), f(b));
+            else *reinterpret_cast<float*>(d4) = f(S::min2(a, b));
+          };
           uint32_t rbuf[64];
 #pragma unroll 1
           for (int c = 0; c < NCOL; c += 64) {
@@ -793,7 +792,9 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
               __syncwarp();
               if (lane == 0) mbar_arrive(&bars->tempty[slot]);
             }
-            if (TASKS) {
+            if (SAMPLE) {
+              sample(rbuf, c);
+            } else if (TASKS) {
               if (p.minima) {
                 // minima variant: the smallest score of every 32 columns of this chunk, rows beyond the task's as +inf
                 if (mdst) {
@@ -818,73 +819,10 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
               chunk(rbuf, c);
             }
           }
-        } else {
-          // List mode.  Common path: the minimum of a chunk against the bound.  Rare path (entered by the whole
-          // warp when any of its 32 rows has a column below its bound): the scores are parked in this warp's
-          // shared-memory scratch so that they can be indexed, and each row inserts its passing columns, in
-          // ascending id order, into its sorted register list.
-          uint32_t rbuf[32];
-#pragma unroll 1
-          for (int c = 0; c < NCOL; c += 32) {
-            tc_ld32_issue(t_addr + uint32_t(c), rbuf);
-            tc_ld_wait(rbuf);
-            T m = S::of(rbuf[0]);
-#pragma unroll
-            for (int i = 1; i < 31; i += 2) m = S::min3(m, S::of(rbuf[i]), S::of(rbuf[i + 1]));
-            m = S::min2(m, S::of(rbuf[31]));
-            if (__any_sync(FV_FULL, m < thr)) {
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {  // two halves of 16 columns, in id order; the scratch holds one half
-                unsigned mask = 0;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                  const T v = S::of(rbuf[h * 16 + i]);
-                  sv[i * 32 + lane] = float(v);
-                  mask |= (v < thr && row_base + uint32_t(c + h * 16 + i) < n_rows) ? (1u << i) : 0u;
-                }
-                while (__any_sync(FV_FULL, mask != 0)) {
-                  if (mask) {
-                    const int i = __ffs(mask) - 1;
-                    mask &= mask - 1;
-                    const float val = sv[i * 32 + lane];
-                    if (val < sc[KPT - 1]) {
-                      float cs = val;
-                      uint32_t ci = row_base + uint32_t(c + h * 16 + i);
-#pragma unroll
-                      for (int j = 0; j < KPT; ++j) {
-                        const bool lt = cs < sc[j];
-                        const float ts = sc[j];
-                        const uint32_t ti = idv[j];
-                        sc[j] = lt ? cs : ts;
-                        idv[j] = lt ? ci : ti;
-                        cs = lt ? ts : cs;
-                        ci = lt ? ti : ci;
-                      }
-                      thr = S::bound(sc[KPT - 1]);
-                    }
-                  }
-                }
-              }
-            }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->tempty[slot]);
         }
       }
       if (!ok) break;
-      if (THRESH) {
-        if (!TASKS) p.ccnt[cslot] = ncand;
-      } else {
-        u64* dst = p.cand + cslot * KP;
-#pragma unroll
-        for (int j = 0; j + 1 < KPT; j += 2) {
-          const u64 k0 = idv[j] == 0xFFFFFFFFu ? FV_EMPTY_KEY : make_key(sc[j], idv[j]);
-          const u64 k1 = idv[j + 1] == 0xFFFFFFFFu ? FV_EMPTY_KEY : make_key(sc[j + 1], idv[j + 1]);
-          *reinterpret_cast<ulonglong2*>(dst + j) = make_ulonglong2(k0, k1);
-        }
-        if (KPT & 1) dst[KPT - 1] = idv[KPT - 1] == 0xFFFFFFFFu ? FV_EMPTY_KEY : make_key(sc[KPT - 1], idv[KPT - 1]);
-      }
+      if (!SAMPLE && !TASKS) p.ccnt[cslot] = ncand;
     }
   }
 
@@ -899,11 +837,11 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
   }
 }
 
-template <int MH, int KPT, bool THRESH, bool TASKS = false>
+template <int MH, bool SAMPLE, bool TASKS = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
     gemm_topk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ GemmParams p) {
-  gemm_topk_body<MH, KPT, THRESH, TASKS, false>(tmA, tmB, p);
+  gemm_topk_body<MH, SAMPLE, TASKS, false>(tmA, tmB, p);
 }
 
 // The pass over the 8-bit operands or, where a query of the batch does not fit them (q8_bad, known on the device only), over
@@ -912,11 +850,11 @@ struct GemmWay {
   CUtensorMap tmA, tmB;
   GemmParams p;
 };
-template <int MH16, int KPT, bool THRESH>
+template <int MH16, bool SAMPLE>
 __global__ void __launch_bounds__(NTHREADS, 1)
     gemm_topk_either_kernel(const __grid_constant__ GemmWay w16, const __grid_constant__ GemmWay w8, const unsigned int* q8_bad) {
-  if (*q8_bad) gemm_topk_body<MH16, KPT, THRESH, false, false>(w16.tmA, w16.tmB, w16.p);
-  else gemm_topk_body<2, KPT, THRESH, false, true>(w8.tmA, w8.tmB, w8.p);
+  if (*q8_bad) gemm_topk_body<MH16, SAMPLE, false, false>(w16.tmA, w16.tmB, w16.p);
+  else gemm_topk_body<2, SAMPLE, false, true>(w8.tmA, w8.tmB, w8.p);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1313,29 +1251,48 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
 
 // Rows of the strided sample: sample row i is base row floor(i * n / ns).  They are stored with the multiples of 16
 // first, then the other multiples of 8, 4 and 2, then the odd ones: the first ceil(ns / 2^j) rows are the sample of
-// every 2^j-th of them (j <= 4), for searches that want a coarser one.
+// every 2^j-th of them (j <= 4), for searches that want a coarser one.  Within each of these runs the order goes round by
+// steps of about 0.618 of its length, so that rows side by side, whose minimum stands for them all, come from all over the
+// base: in a base stored cluster by cluster neighbours in the base are neighbours in space.
 static constexpr int SAMPLE_LEVELS = 4;
 __host__ __device__ __forceinline__ size_t sample_prefix(size_t ns, int j) { return (ns + (size_t(1) << j) - 1) >> j; }
-__device__ __forceinline__ size_t sample_row_at(size_t slot, size_t ns) {  // the sample row stored in `slot`
-  if (slot < sample_prefix(ns, SAMPLE_LEVELS)) return slot << SAMPLE_LEVELS;
+struct SampleOrder {
+  size_t ns;
+  size_t step[SAMPLE_LEVELS + 1];  // of the run of the multiples of 2^j that no coarser run holds
+};
+static SampleOrder sample_order(size_t ns) {
+  SampleOrder o{ns, {}};
+  for (int j = 0; j <= SAMPLE_LEVELS; ++j) {
+    const size_t len = sample_prefix(ns, j) - (j < SAMPLE_LEVELS ? sample_prefix(ns, j + 1) : 0);
+    size_t s = std::max<size_t>(1, size_t(double(len) * 0.6180339887));
+    while (std::gcd(s, len) > 1) ++s;  // (len 0 has no rows; len 1: any step)
+    o.step[j] = s;
+  }
+  return o;
+}
+__device__ __forceinline__ size_t sample_row_at(size_t slot, const SampleOrder& o) {  // the sample row stored in `slot`
+  const size_t coarse = sample_prefix(o.ns, SAMPLE_LEVELS);
+  if (slot < coarse) return (slot * o.step[SAMPLE_LEVELS] % coarse) << SAMPLE_LEVELS;
   int j = SAMPLE_LEVELS - 1;
-  while (slot >= sample_prefix(ns, j)) --j;
-  return ((slot - sample_prefix(ns, j + 1)) << (j + 1)) + (size_t(1) << j);
+  while (slot >= sample_prefix(o.ns, j)) --j;
+  const size_t first = sample_prefix(o.ns, j + 1), len = sample_prefix(o.ns, j) - first;
+  return (((slot - first) * o.step[j] % len) << (j + 1)) + (size_t(1) << j);
 }
 
 // base8 (bases with 8-bit operands): those and their norm bytes too, up to row nspad of the latter
 __global__ void gather_sample_kernel(const uint16_t* __restrict__ half, const float* __restrict__ norm2, size_t n, int Kp,
-                                     size_t ns, uint16_t* __restrict__ samp, float* __restrict__ snorm,
+                                     SampleOrder order, uint16_t* __restrict__ samp, float* __restrict__ snorm,
                                      const uint8_t* __restrict__ base8, const uint8_t* __restrict__ ext8, int Kp8, size_t nspad,
                                      uint8_t* __restrict__ samp8, uint8_t* __restrict__ samp_ext8) {
   const int lane = threadIdx.x & 31;
   const size_t i = blockIdx.x * size_t(blockDim.x >> 5) + (threadIdx.x >> 5);
   const auto swap8 = [](size_t row) { return (int(row >> 2) & 1) << 4; };  // the image's halves trade places in rows 4..7 of 8
+  const size_t ns = order.ns;
   if (i >= ns) {
     if (base8 && i < nspad) samp_ext8[i * 32 + lane] = uint8_t((lane & 15) == 0 ? 0 : 127);  // beyond the sample: a large score
     return;
   }
-  const size_t src = size_t((unsigned long long)sample_row_at(i, ns) * n / ns);
+  const size_t src = size_t((unsigned long long)sample_row_at(i, order) * n / ns);
   const uint4* a = reinterpret_cast<const uint4*>(half + src * size_t(Kp));
   uint4* b = reinterpret_cast<uint4*>(samp + i * size_t(Kp));
   for (int c = lane; c < Kp / 8; c += 32) b[c] = a[c];
@@ -1579,7 +1536,7 @@ int tc_append(fv_ctx* ctx, TcSide** ptc, int metric, const float* d_rows_new, si
     FV_TRY(tc->samp_ext8.reserve(nspad * 32));
   }
   gather_sample_kernel<<<unsigned((nspad + 7) / 8), 256, 0, ctx->stream>>>(
-      tc->half.as<uint16_t>(), tc->norm2.as<float>(), total, Kp, tc->ns, tc->samp.as<uint16_t>(), tc->samp_norm2.as<float>(),
+      tc->half.as<uint16_t>(), tc->norm2.as<float>(), total, Kp, sample_order(tc->ns), tc->samp.as<uint16_t>(), tc->samp_norm2.as<float>(),
       tc->i8 ? tc->rows8.as<uint8_t>() : nullptr, tc->ext8.as<uint8_t>(), tc->Kp8, nspad, tc->samp8.as<uint8_t>(),
       tc->samp_ext8.as<uint8_t>());
   fill_f32_kernel<<<8, 256, 0, ctx->stream>>>(tc->samp_norm2.as<float>() + tc->ns, nspad - tc->ns, INFINITY);
@@ -1619,7 +1576,7 @@ struct Tiling {
 };
 
 // `row_bytes`: bytes of an operand row that hold data
-static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, int scratch_bytes, Tiling* t, int force_mh = 0) {
+static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, Tiling* t, int force_mh = 0) {
   t->KB = (row_bytes + 127) / 128;
   t->last_steps = (row_bytes - (t->KB - 1) * 128 + 31) / 32;
   t->MH = force_mh ? force_mh : (t->KB <= 2 ? 2 : 1);
@@ -1645,7 +1602,7 @@ static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, int s
   t->nchunks = int(chunks);
   t->segmax = int((chunks + t->grid - 1) / t->grid);
   const size_t a_bytes = size_t(t->MH) * t->KB * A_BLOCK_BYTES + A_EXT_BYTES;
-  const size_t tail = size_t(scratch_bytes) + sizeof(Barriers) + 64;
+  const size_t tail = sizeof(Barriers) + 64;
   for (t->nstage = 6; t->nstage >= 2; --t->nstage) {
     t->ext_ring = (t->nstage + t->KB - 1) / t->KB + 1;
     t->smem = 1024 + a_bytes + size_t(t->nstage) * B_STAGE_BYTES + size_t(t->ext_ring) * B_EXT_BYTES + tail;
@@ -1657,15 +1614,15 @@ static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, int s
 static PassShape pass_shape(const Tiling& t) { return PassShape{t.MT, t.parts, t.grid, t.segmax, t.MH}; }
 
 // One launch over one way's operands, or over whichever of two the queries allow (`w8` and its word).
-template <int KPT, bool THRESH>
+template <bool SAMPLE>
 static int launch_gemm(fv_ctx* ctx, const Tiling& t16, const GemmWay& w16, const Tiling& t8, const GemmWay* w8,
                        const unsigned int* q8_bad) {
   if (!w8) {
-    auto kern = t16.MH == 2 ? gemm_topk_kernel<2, KPT, THRESH> : gemm_topk_kernel<1, KPT, THRESH>;
+    auto kern = t16.MH == 2 ? gemm_topk_kernel<2, SAMPLE> : gemm_topk_kernel<1, SAMPLE>;
     FV_TRY(allow_smem(ctx, kern, t16.smem));
     kern<<<t16.grid, NTHREADS, t16.smem, ctx->stream>>>(w16.tmA, w16.tmB, w16.p);
   } else {
-    auto kern = t16.MH == 2 ? gemm_topk_either_kernel<2, KPT, THRESH> : gemm_topk_either_kernel<1, KPT, THRESH>;
+    auto kern = t16.MH == 2 ? gemm_topk_either_kernel<2, SAMPLE> : gemm_topk_either_kernel<1, SAMPLE>;
     const size_t smem = std::max(t16.smem, t8.smem);
     FV_TRY(allow_smem(ctx, kern, smem));
     kern<<<std::max(t16.grid, t8.grid), NTHREADS, smem, ctx->stream>>>(w16, *w8, q8_bad);
@@ -1699,7 +1656,7 @@ static WaitLimit next_wait_limit() {  // of one launch
   return l;
 }
 
-static void fill_params(GemmParams* g, const Tiling& t, size_t rows, size_t nq, int scratch_bytes, const WaitLimit& limit) {
+static void fill_params(GemmParams* g, const Tiling& t, size_t rows, size_t nq, const WaitLimit& limit) {
   g->wait_limit = limit.cycles;
   g->fault_skip_unit = limit.skip_unit;
   g->grid = t.grid;
@@ -1713,7 +1670,6 @@ static void fill_params(GemmParams* g, const Tiling& t, size_t rows, size_t nq, 
   g->nchunks = t.nchunks;
   g->segmax = t.segmax;
   g->nstage = t.nstage;
-  g->scratch_bytes = scratch_bytes;
   g->ext_ring = t.ext_ring;
 }
 
@@ -1742,9 +1698,9 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
   if (tile_rows != 128 && tile_rows != 256) return fail(FV_ERR_ARG, "operand tiles have 128 or 256 rows");
   Tiling t{};
   // stages and shared memory for operand tiles of that height; the tiling itself is unused
-  FV_TRY(make_tiling(ctx, tc->pd * 2, 256, size_t(TILE_N) * 1024, 0, &t, tile_rows == 128 ? 1 : 2));
+  FV_TRY(make_tiling(ctx, tc->pd * 2, 256, size_t(TILE_N) * 1024, &t, tile_rows == 128 ? 1 : 2));
   GemmParams gp{};
-  fill_params(&gp, t, tc->n, a_rows, 0, next_wait_limit());
+  fill_params(&gp, t, tc->n, a_rows, next_wait_limit());
   gp.nchunks = 0;
   gp.has_ext = metric == FV_L2 ? 1 : 0;
   gp.aext = norm_step_queries(tc);
@@ -1768,7 +1724,7 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
   FV_TRY(make_tmap(&tmB, type16(tc->bf16), tc->half.p, tc->n, Kp, TILE_N));
   FV_CUDA(cudaMemsetAsync(d_next_task, 0, sizeof(unsigned int), ctx->stream));
   void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams) =
-      tile_rows == 128 ? gemm_topk_kernel<1, 2, true, true> : gemm_topk_kernel<2, 2, true, true>;
+      tile_rows == 128 ? gemm_topk_kernel<1, false, true> : gemm_topk_kernel<2, false, true>;
   FV_TRY(allow_smem(ctx, kern, t.smem));
   kern<<<ctx->sm_count, NTHREADS, t.smem, ctx->stream>>>(tmA, tmB, gp);
   ctx->stats.launches++;
@@ -1796,26 +1752,21 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   while (k > 32 && R > SAMPLE_R_MAX && level < SAMPLE_LEVELS) R = pick_sample_r(k, tc->every << ++level);
   R = std::min(R, SAMPLE_R_MAX);
   const size_t ns = sample_prefix(tc->ns, level);
-  // R is rounded up to the next instantiated list length - 1 of the sample pass (a larger R only loosens the bound)
-  R = R <= 7 ? R : (R <= 9 ? 9 : 13);
-
   // One way through both passes, or two: over the 8-bit operands where the base has them and, should a query of the batch
   // not fit them (known on the device only), over the 16-bit ones.  The kernels of the way that is not taken leave at once.
   const int ways = tc->i8 ? 2 : 1;
   struct Way {
-    Tiling ts, tm;           // sample pass, main pass
+    Tiling tm;               // main pass
     CUtensorMap tmA, tmS, tmB;
     size_t nq_pad = 0;
   } way[2] = {};             // 0: 16-bit, 1: 8-bit
-  size_t nq_pad = 0, nlists = 0, sample_lists = 0;
+  size_t nq_pad = 0, nlists = 0;
   for (int i = 0; i < ways; ++i) {
     const int row_bytes = i ? pd : pd * 2;
-    FV_TRY(make_tiling(ctx, row_bytes, nq, ns, SCRATCH_BYTES, &way[i].ts));
-    FV_TRY(make_tiling(ctx, row_bytes, nq, n, 0, &way[i].tm));
+    FV_TRY(make_tiling(ctx, row_bytes, nq, n, &way[i].tm));
     way[i].nq_pad = size_t(way[i].tm.MT) * 128 * way[i].tm.MH;
     nq_pad = std::max(nq_pad, way[i].nq_pad);
     nlists = std::max(nlists, size_t(way[i].tm.grid) * way[i].tm.segmax * LISTS);
-    sample_lists = std::max(sample_lists, size_t(way[i].ts.grid) * way[i].ts.segmax * LISTS);
   }
 
   // queries -> operand rows (16 bits: scaled by -2 for L2, -1 for inner product), padded to whole tiles with zeros; norms;
@@ -1828,7 +1779,12 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   int ccap = 256;
   while (ccap > 16 && nlists * size_t(ccap) * sizeof(u64) > (size_t(2) << 30)) ccap >>= 1;
   FV_TRY(ctx->scratch[5].reserve(3 * nq_pad * sizeof(float) + nlists * sizeof(unsigned int)));
-  FV_TRY(ctx->scratch[6].reserve(sample_lists * KP * sizeof(u64)));
+  // Sample pass: the minima of 1, 8, 32 or 64 sampled rows, so that there are hundreds of groups and two of a query's R best
+  // seldom share one (their number times R (R - 1) / 2 is what the rank slips by), for at most 512 MB of queries at a time.
+  const int group = ns <= 1024 ? 1 : ns <= 16384 ? 8 : ns <= 65536 ? 32 : 64;
+  const size_t smin_ld = (ns + TILE_N - 1) / TILE_N * TILE_N / group;
+  const size_t slice = std::min(nq_pad, std::max<size_t>(256, ((size_t(512) << 20) / (smin_ld * sizeof(float))) & ~size_t(255)));
+  FV_TRY(ctx->scratch[6].reserve(slice * smin_ld * sizeof(float)));
   FV_TRY(ctx->scratch[7].reserve(nq * sizeof(uint32_t)));
   FV_TRY(ctx->scratch[9].reserve(nlists * size_t(ccap) * sizeof(u64)));
   uint16_t* dA = ctx->scratch[3].as<uint16_t>();
@@ -1862,39 +1818,55 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   FV_TRY(convert(ctx, tc->bf16, d_queries, nq, pd, Kp, dA, qn2, is_l2, is_l2 ? -2.f : -1.f, qst, q8));
   if (mark_stages) stage_mark(ctx);
 
-  GemmWay ws[2], wm[2];  // sample pass, main pass
-  const WaitLimit limit_s = next_wait_limit(), limit_m = next_wait_limit();
+  GemmParams gp[2];
   for (int i = 0; i < ways; ++i) {
-    GemmParams g{};
-    g.has_ext = is_l2 ? 1 : 0;
-    g.aext = i ? norm_step_queries8() : norm_step_queries(tc);
-    g.idesc = i ? make_idesc_i8(128, TILE_N) : make_idesc(128, TILE_N, tc->bf16);
-    g.err = tc_error_word(tc);
-    ws[i] = GemmWay{way[i].tmA, way[i].tmS, g};
-    fill_params(&ws[i].p, way[i].ts, ns, nq, SCRATCH_BYTES, limit_s);
-    ws[i].p.cand = ctx->scratch[6].as<u64>();
-    ws[i].p.ext = (i ? tc->samp_ext8 : tc->samp_ext).as<uint16_t>();
-    wm[i] = GemmWay{way[i].tmA, way[i].tmB, g};
-    fill_params(&wm[i].p, way[i].tm, n, nq, 0, limit_m);
-    wm[i].p.tau = tau;
-    wm[i].p.cbuf = ctx->scratch[9].as<u64>();
-    wm[i].p.ccnt = ccnt;
-    wm[i].p.ccap = ccap;
-    wm[i].p.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
+    gp[i] = GemmParams{};
+    gp[i].has_ext = is_l2 ? 1 : 0;
+    gp[i].aext = i ? norm_step_queries8() : norm_step_queries(tc);
+    gp[i].idesc = i ? make_idesc_i8(128, TILE_N) : make_idesc(128, TILE_N, tc->bf16);
+    gp[i].err = tc_error_word(tc);
   }
 
-  // sample pass: per query the R (+1) best scores over the sampled rows, in the epilogue's registers
-  auto sample = R == 5 ? launch_gemm<6, false> : R == 6 ? launch_gemm<7, false> : R == 7 ? launch_gemm<8, false>
-              : R == 9 ? launch_gemm<10, false> : launch_gemm<14, false>;
-  FV_TRY(sample(ctx, way[0].ts, ws[0], way[1].ts, tc->i8 ? &ws[1] : nullptr, q8_bad));
-  sample_tau_kernel<<<unsigned((nq_pad + 7) / 8), 256, 0, ctx->stream>>>(
-      ctx->scratch[6].as<u64>(), PassShapes{pass_shape(way[0].ts), pass_shape(way[1].ts), q8_bad}, int(nq_pad), R, tau);
-  ctx->stats.launches++;
-  FV_CUDA(cudaGetLastError());
+  // sample pass: group minima of the sampled rows' scores, and from them the queries' bounds
+  for (size_t q0 = 0; q0 < nq; q0 += slice) {
+    const size_t nqs = std::min(slice, nq - q0);
+    Tiling ts[2] = {};
+    GemmWay ws[2];
+    const WaitLimit limit = next_wait_limit();
+    for (int i = 0; i < ways; ++i) {
+      FV_TRY(make_tiling(ctx, i ? pd : pd * 2, nqs, ns, &ts[i]));
+      ws[i] = GemmWay{way[i].tmA, way[i].tmS, gp[i]};
+      GemmParams& g = ws[i].p;
+      fill_params(&g, ts[i], ns, nqs, limit);
+      g.a_row0 = int(q0);
+      g.smin = ctx->scratch[6].as<float>();
+      g.smin_ld = int(smin_ld);
+      g.group = group;
+      g.ext = (i ? tc->samp_ext8 : tc->samp_ext).as<uint16_t>();
+    }
+    FV_TRY((launch_gemm<true>(ctx, ts[0], ws[0], ts[1], tc->i8 ? &ws[1] : nullptr, q8_bad)));
+    const size_t with_bound = std::min(slice, nq_pad - q0);
+    sample_tau_kernel<<<unsigned((with_bound + 7) / 8), 256, 0, ctx->stream>>>(
+        ctx->scratch[6].as<float>(), int(smin_ld), int((ns + group - 1) / group), int(with_bound), R, tau + q0);
+    ctx->stats.launches++;
+    FV_CUDA(cudaGetLastError());
+  }
   if (mark_stages) stage_mark(ctx);
 
   // main pass: every row scoring below the query's sampled bound becomes a candidate
-  FV_TRY((launch_gemm<2, true>(ctx, way[0].tm, wm[0], way[1].tm, tc->i8 ? &wm[1] : nullptr, q8_bad)));
+  GemmWay wm[2];
+  const WaitLimit limit = next_wait_limit();
+  for (int i = 0; i < ways; ++i) {
+    wm[i] = GemmWay{way[i].tmA, way[i].tmB, gp[i]};
+    GemmParams& g = wm[i].p;
+    fill_params(&g, way[i].tm, n, nq, limit);
+    g.tau = tau;
+    g.cbuf = ctx->scratch[9].as<u64>();
+    g.ccnt = ccnt;
+    g.ccap = ccap;
+    g.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
+  }
+  FV_TRY((launch_gemm<false>(ctx, way[0].tm, wm[0], way[1].tm, tc->i8 ? &wm[1] : nullptr, q8_bad)));
   if (mark_stages) stage_mark(ctx);
 
   RerankParams rp{};
