@@ -48,7 +48,6 @@ static constexpr int EXT_K = 16;                  // k elements of the norm step
 static constexpr int A_EXT_BYTES = 128 * EXT_K * 2;     // query side of the norm step
 static constexpr int B_EXT_BYTES = TILE_N * EXT_K * 2;  // base side: one 8 KB tile per unit
 static constexpr int NEPI = 16;        // epilogue warps: four per tensor-memory lane quadrant
-static constexpr int LISTS = NEPI * 32; // per-thread lists of one segment
 static constexpr int NTHREADS = 64 + NEPI * 32;   // warp 0 TMA, warp 1 MMA, warps 2..17 epilogue
 static constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;  // about 2 s; then the kernel gives up
 
@@ -287,8 +286,8 @@ struct GemmParams {
   int fault_skip_unit;   // test hook, -1 = off: the producer of work item 0 leaves out the loads of this unit of it
   // threshold mode: per-query bounds from the sample pass, and the candidate buffers they fill
   const float* tau;      // [MT * 128 * MH]
-  u64* cbuf;             // [grid * segmax][LISTS][ccap] (score, row) keys: one private list per epilogue thread and segment
-  unsigned int* ccnt;    // [grid * segmax][LISTS] entries appended (may exceed ccap: overflow)
+  u64* cbuf;             // [grid * segmax][128 * MH][4][ccap] (score, row) keys: a list per query row, column quarter and segment
+  unsigned int* ccnt;    // [grid * segmax][128 * MH][4] entries appended (may exceed ccap: overflow)
   int ccap;
   // task mode (TASKS): the work is a table of (A tile, run of B units) pairs instead of the tiling above
   // x: first operand row of the 256-row A tile; y: first B row of the task; z: its B units of 256 rows (low 16 bits)
@@ -325,13 +324,6 @@ struct __align__(8) Barriers {
   unsigned int tq[8];
 };
 
-// Epilogue thread -> list index: warp group `sub` (0..3) * 128 + lane quadrant * 32 + lane.  MH = 2: sub & 1 is the
-// 128-row half of the query tile, sub >> 1 the half of the 256 columns; MH = 1: sub is the column quarter.
-// The li-th list that holds candidates of query row r of its tile:
-__host__ __device__ __forceinline__ int list_of_row(int MH, int r, int li) {
-  return MH == 2 ? ((r >> 7) + 2 * li) * 128 + (r & 127) : li * 128 + r;
-}
-
 // Sampling.  The sample pass scores 1 base row in E; a query's bound is its R-th best sampled score, so about R * E
 // rows of the full set score below it (negative binomial) and the k nearest are among them unless R or more of the
 // k - 1 nearest rows happen to be sampled: probability P(Binomial(k - 1, 1/E) >= R), kept below 2e-5 by the choice
@@ -366,6 +358,7 @@ static int pick_sample_r(int k, int every) {
 // device word q8_bad says which of the two passes ran.
 struct PassShape {
   int MT, parts, grid, segmax, MH;
+  int ccap;  // slots of a candidate list
 };
 struct PassShapes {
   PassShape s16, s8;
@@ -377,8 +370,6 @@ struct PassShapes {
 // A query's bound: the R-th smallest of the group minima the sample pass left (+inf where there are fewer), which that many
 // sampled rows do not exceed.  A warp per query, each lane with the four smallest of its share: where a lane holds more than
 // four of the R smallest the bound is a little looser.  Bound by reading the minima from L2.
-// With the R best scores of the sample kept in registers by the epilogue, as it was, every chunk of 32 columns had an
-// insertion in some row: 251 us for 31,250 rows x 10,000 queries, 52 and 16 now; 1,000 queries at 100k x 128 38, 12 and 10.
 __global__ void __launch_bounds__(256) sample_tau_kernel(const float* __restrict__ smin, int ld, int groups, int nq, int R,
                                                          float* __restrict__ tau) {
   const int q = blockIdx.x * int(blockDim.x >> 5) + int(threadIdx.x >> 5), lane = lane_id();
@@ -455,7 +446,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
     for (int i = 0; i < 8; ++i) mbar_init(&bars->tq_full[i], 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->tfull[i], 1);
-      mbar_init(&bars->tempty[i], MH == 2 ? NEPI / 2 : NEPI);
+      mbar_init(&bars->tempty[i], NEPI);
     }
     bars->abort_flag = 0;
     bars->pool_pos = 0;
@@ -625,63 +616,78 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
     }
   } else {
     // ---------------------------------------------------------------- epilogue: 16 warps, one query row per thread
+    // Every warp reads its 64 columns of every accumulator in one load and hands the slot back at once: what it then does
+    // with them delays no MMA as long as it keeps up on average.  (With MH = 2 each half's accumulators used to belong to
+    // half of the warps, 128 columns each in two loads: the slot then waited for the slowest warp's hits.  10,000 queries at
+    // 1M x 128, main pass over bytes: 1,785 us, now 1,449.)
     const int ew = warp - 2;
     const int quad = warp & 3;   // tensor-memory lanes this warp may read: 32 * quad .. +31
-    const int sub = ew >> 2;     // warp group 0..3
-    const int grp = MH == 2 ? (sub & 1) : 0;  // MH = 2: which 128-row half (= accumulator slot)
-    const int e = sub * 128 + quad * 32 + lane;  // list index inside a segment
+    const int sub = ew >> 2;     // warp group 0..3: which quarter of the columns
+    const int r0 = quad * 32 + lane;  // row within 128
     const uint32_t lane_addr = uint32_t(quad * 32) << 16;
-    T thr = S::bound(INFINITY);
-    size_t cslot = 0;        // this thread's list of the current segment
-    unsigned int ncand = 0;
-    int tile_idx = 0;
+    int job = 0;
     bool ok = true;
-    constexpr int NCOL = MH == 2 ? TILE_N / 2 : TILE_N / 4;
-    const int col0 = MH == 2 ? (sub >> 1) * NCOL : sub * NCOL;
+    constexpr int NCOL = TILE_N / 4;
+    const int col0 = sub * NCOL;
     uint32_t n_rows = uint32_t(p.n);
-    uint32_t a_row = 0;  // task mode: this thread's operand row
     uint32_t unit0 = 0;  // task mode: number of the task's first unit within its B run
-    float* sdst = nullptr;  // sample mode: this thread's row of smin
-    float* mdst = nullptr;  // task mode, minima variant: where this thread's minima of the current task go
+    struct Row {         // this thread's row of each 128-row half
+      T thr;
+      unsigned int ncand;
+      u64* list;         // threshold mode: its candidates of the current segment
+      float* sdst;       // sample mode: its row of smin
+      uint32_t a_row;    // task mode: the operand row
+      float* mdst;       // task mode, minima variant: where its minima of the current task go
+    } rows[MH];
     for (int seg = 0, g = work_of(0); g < nwork && ok; g = work_of(++seg)) {
       int nt0, nt1, mt = 0;
+      uint4 t = make_uint4(0, 0, 0, 0);
       if (TASKS) {
-        const uint4 t = p.tasks[g];
+        t = p.tasks[g];
         nt0 = 0;
         nt1 = int(t.z & 0xFFFFu);
         unit0 = t.z >> 16;
         n_rows = t.w;  // rows of this task's B run; the rest of its last unit belongs to someone else
-        a_row = t.x + uint32_t((MH == 2 ? grp * 128 : 0) + quad * 32 + lane);
-        if (p.minima) {
-          const uint32_t moff = p.task_moff[g];
-          const uint32_t rt = a_row - t.x;
-          mdst = (moff != 0xFFFFFFFFu && rt < p.task_rows[g]) ? p.minima + size_t(moff) + size_t(rt) * (t.z & 0xFFFFu) * 8 : nullptr;
-        }
       } else {
         const int part = g / p.MT;
         mt = g - part * p.MT;
         nt0 = part * p.cpn;
         nt1 = min(p.NT, nt0 + p.cpn);
       }
-      cslot = (size_t(blockIdx.x) * p.segmax + seg) * LISTS + e;
-      ncand = 0;
-      const int q = mt * (128 * MH) + (MH == 2 ? grp * 128 : 0) + quad * 32 + lane;
-      if (SAMPLE) sdst = p.smin + size_t(q) * p.smin_ld;
-      else thr = S::bound(TASKS ? (p.minima ? 0.f : p.tau[a_row]) : p.tau[q]);  // the bound is fixed: the sample pass's estimate for this query
-      for (int nt = nt0; nt < nt1 && ok; ++nt, ++tile_idx) {
-        const int job = MH == 2 ? tile_idx * 2 + grp : tile_idx;
-        const int slot = job & 1;
-        ok = mbar_wait(&bars->tfull[slot], uint32_t(job >> 1) & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
+      const size_t lists0 = (size_t(blockIdx.x) * p.segmax + seg) * (128 * MH * 4) + sub;
+#pragma unroll
+      for (int mh = 0; mh < MH; ++mh) {
+        Row& w = rows[mh];
+        const int r = mh * 128 + r0, q = mt * (128 * MH) + r;
+        w.ncand = 0;
+        if (SAMPLE) {
+          w.sdst = p.smin + size_t(q) * p.smin_ld;
+        } else if (TASKS) {
+          w.a_row = t.x + uint32_t(r);
+          w.thr = S::bound(p.minima ? 0.f : p.tau[w.a_row]);
+          w.mdst = nullptr;
+          if (p.minima) {
+            const uint32_t moff = p.task_moff[g];
+            if (moff != 0xFFFFFFFFu && uint32_t(r) < p.task_rows[g]) w.mdst = p.minima + size_t(moff) + size_t(r) * (t.z & 0xFFFFu) * 8;
+          }
+        } else {  // the bound is fixed: the sample pass's estimate for this query
+          w.thr = S::bound(p.tau[q]);
+          w.list = p.cbuf + (lists0 + size_t(r) * 4) * size_t(p.ccap);
+        }
+      }
+      for (int nt = nt0; nt < nt1 && ok; ++nt) {
         const uint32_t row_base = (unit0 + uint32_t(nt)) * TILE_N + col0;
-        const uint32_t t_addr = tmem_base + lane_addr + uint32_t(slot * TILE_N + col0);
-        {
+#pragma unroll
+        for (int mh = 0; mh < MH; ++mh, ++job) {
+          const int slot = job & 1;
+          ok = ok && __all_sync(FV_FULL, mbar_wait(&bars->tfull[slot], uint32_t(job >> 1) & 1, abort_flag));
+          if (!ok) break;
+          tc_fence_after();
+          Row& w = rows[mh];
           // Threshold mode.  The accumulator IS the score (the norm step and the scaled query side put
           // ||b||^2 - 2<q,b> there), so a chunk of 64 columns costs a minimum tree and one vote.  Every column
           // below the bound is appended to this thread's private list: a plain store and a register counter.
-          // (Issuing the next load before working on this one was tried and ran slower than this plain loop.)
-          auto chunk = [&](const uint32_t* r, int c) {
+          auto chunk = [&](const uint32_t* r) {
             T g8[8];
 #pragma unroll
             for (int gi = 0; gi < 8; ++gi) {
@@ -691,39 +697,60 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
               g8[gi] = S::min2(S::min3(t0, t1, S::of(q[6])), S::of(q[7]));
             }
             const T m = S::min2(S::min3(g8[0], g8[1], g8[2]), S::min3(S::min3(g8[3], g8[4], g8[5]), g8[6], g8[7]));
-            if (!__any_sync(FV_FULL, m < thr)) return;
+            if (!__any_sync(FV_FULL, m < w.thr)) return;
             uint32_t groups = 0;  // the runs of eight columns in which some row of the warp has a hit
 #pragma unroll
-            for (int gi = 0; gi < 8; ++gi) groups |= g8[gi] < thr ? 1u << gi : 0u;
+            for (int gi = 0; gi < 8; ++gi) groups |= g8[gi] < w.thr ? 1u << gi : 0u;
             groups = __reduce_or_sync(FV_FULL, groups);
-            u64* cl = p.cbuf + cslot * size_t(p.ccap);
+            // One run at a time: its eight scores are moved to the same registers, so that there is one copy of the code
+            // that looks at them (with eight the loop outgrew the instruction cache: 3 times the time at MH = 2).
+            while (groups) {
+              const int gi = __ffs(groups) - 1;
+              groups &= groups - 1;
+              T v[8];
+              auto run = [&](int k) {
 #pragma unroll
-            for (int gi = 0; gi < 8; ++gi) {
-              if (!(groups & (1u << gi))) continue;
-#pragma unroll
-              for (int i = gi * 8; i < gi * 8 + 8; ++i) {
-                const T v = S::of(r[i]);
-                const uint32_t row = row_base + uint32_t(c + i);
-                const u64 key = make_key(float(v), row);
-                const bool hit = v < thr && row < n_rows;
-                if (hit) cl[min(ncand, unsigned(p.ccap) - 1u)] = key;  // (a list that ran over is thrown away: its count tells)
-                ncand += hit ? 1u : 0u;
+                for (int i = 0; i < 8; ++i) v[i] = S::of(r[k * 8 + i]);
+              };
+              switch (gi) {
+                case 0: run(0); break;
+                case 1: run(1); break;
+                case 2: run(2); break;
+                case 3: run(3); break;
+                case 4: run(4); break;
+                case 5: run(5); break;
+                case 6: run(6); break;
+                default: run(7); break;
               }
+              const uint32_t row0 = row_base + uint32_t(gi * 8);
+              uint32_t hits = 0;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) hits |= v[i] < w.thr ? 1u << i : 0u;
+              if (row0 + 8 > n_rows) hits &= row0 < n_rows ? (1u << (n_rows - row0)) - 1u : 0u;
+              while (hits) {
+                const int i = __ffs(hits) - 1;
+                hits &= hits - 1;
+                const T a = i & 1 ? v[1] : v[0], b = i & 1 ? v[3] : v[2], c = i & 1 ? v[5] : v[4], d = i & 1 ? v[7] : v[6];
+                const T x = i & 4 ? (i & 2 ? d : c) : (i & 2 ? b : a);
+                if (w.ncand < unsigned(p.ccap)) w.list[w.ncand] = make_key(float(x), row0 + uint32_t(i));
+                w.ncand++;
+              }
+              __syncwarp();
             }
           };
           // Task mode.  Survivors are dense where a query meets its own neighbourhood (one row in ten of a near list),
           // so the append must not cost a shared-memory atomic per hit: every thread collects its hits of the chunk
           // as two bit masks, the warp reserves room for all of them with ONE atomic on the CTA's counter, and each
           // thread stores its own.
-          auto chunk_tasks = [&](const uint32_t* r, int c) {
+          auto chunk_tasks = [&](const uint32_t* r) {
             T m = S::of(r[0]);
 #pragma unroll
             for (int i = 1; i < 64; ++i) m = S::min2(m, S::of(r[i]));
-            if (!__any_sync(FV_FULL, m < thr)) return;
+            if (!__any_sync(FV_FULL, m < w.thr)) return;
             uint32_t mk[2] = {0u, 0u};
 #pragma unroll
             for (int i = 0; i < 64; ++i)
-              if (S::of(r[i]) < thr && row_base + uint32_t(c + i) < n_rows) mk[i >> 5] |= 1u << (i & 31);
+              if (S::of(r[i]) < w.thr && row_base + uint32_t(i) < n_rows) mk[i >> 5] |= 1u << (i & 31);
             const int mine = __popc(mk[0]) + __popc(mk[1]);
             int incl = mine;  // inclusive prefix sum over the warp
 #pragma unroll
@@ -744,15 +771,15 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
               while (mm) {
                 const int i = __ffs(mm) - 1;
                 mm &= mm - 1;
-                if (pos < p.pool_cap) dst[pos] = (u64(a_row) << 32) | u64(row_base + uint32_t(c + h * 32 + i));
+                if (pos < p.pool_cap) dst[pos] = (u64(w.a_row) << 32) | u64(row_base + uint32_t(h * 32 + i));
                 ++pos;
               }
             }
-            if (mine && pos > p.pool_cap) p.owner_dropped[p.row_owner[a_row]] = 1u;  // some of this row's did not fit
+            if (mine && pos > p.pool_cap) p.owner_dropped[p.row_owner[w.a_row]] = 1u;  // some of this row's did not fit
           };
           // Sample mode.  Minima of 8 columns, of 32 or of 64, or every score: 4 to 256 bytes of the query's own row.
-          auto sample = [&](uint32_t* r, int c) {
-            const uint32_t row0 = row_base + uint32_t(c);
+          auto sample = [&](uint32_t* r) {
+            const uint32_t row0 = row_base;
             const T inf = S::bound(INFINITY);
             if (row0 + 64 > n_rows) {
 #pragma unroll
@@ -760,7 +787,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
                 if (row0 + uint32_t(i) >= n_rows) r[i] = I8 ? 0x7FFFFFFFu : 0x7F800000u;
             }
             const auto f = [&](T v) { return I8 && v == inf ? INFINITY : float(v); };
-            float4* d4 = reinterpret_cast<float4*>(sdst + row0 / uint32_t(p.group));
+            float4* d4 = reinterpret_cast<float4*>(w.sdst + row0 / uint32_t(p.group));
             if (p.group == 1) {
 #pragma unroll
               for (int i = 0; i < 64; i += 4) d4[i / 4] = make_float4(f(S::of(r[i])), f(S::of(r[i + 1])), f(S::of(r[i + 2])), f(S::of(r[i + 3])));
@@ -783,46 +810,40 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
             else *reinterpret_cast<float*>(d4) = f(S::min2(a, b));
           };
           uint32_t rbuf[64];
-#pragma unroll 1
-          for (int c = 0; c < NCOL; c += 64) {
-            tc_ld64_issue(t_addr + uint32_t(c), rbuf);
-            tc_ld64_wait(rbuf);
-            if (c + 64 == NCOL) {  // the last load has landed: the MMA may overwrite this accumulator slot
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&bars->tempty[slot]);
-            }
-            if (SAMPLE) {
-              sample(rbuf, c);
-            } else if (TASKS) {
-              if (p.minima) {
-                // minima variant: the smallest score of every 32 columns of this chunk, rows beyond the task's as +inf
-                if (mdst) {
-                  float g2[2];
-                  const bool tail = row_base + uint32_t(c + 63) >= n_rows;
+          tc_ld64_issue(tmem_base + lane_addr + uint32_t(slot * TILE_N + col0), rbuf);
+          tc_ld64_wait(rbuf);
+          tc_fence_before();  // the load has landed: the MMA may overwrite this accumulator slot
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->tempty[slot]);
+          if (SAMPLE) {
+            sample(rbuf);
+          } else if (!TASKS) {
+            chunk(rbuf);
+          } else if (!p.minima) {
+            chunk_tasks(rbuf);
+          } else if (w.mdst) {
+            // minima variant: the smallest score of every 32 columns, rows beyond the task's as +inf
+            float g2[2];
+            const bool tail = row_base + 63u >= n_rows;
 #pragma unroll
-                  for (int gi = 0; gi < 2; ++gi) {
-                    float m = INFINITY;
+            for (int gi = 0; gi < 2; ++gi) {
+              float m = INFINITY;
 #pragma unroll
-                    for (int i = gi * 32; i < gi * 32 + 32; ++i) {
-                      const float v = __uint_as_float(rbuf[i]);
-                      m = fminf(m, (!tail || row_base + uint32_t(c + i) < n_rows) ? v : INFINITY);
-                    }
-                    g2[gi] = m;
-                  }
-                  *reinterpret_cast<float2*>(mdst + size_t(nt) * 8 + (col0 + c) / 32) = make_float2(g2[0], g2[1]);
-                }
-              } else {
-                chunk_tasks(rbuf, c);
+              for (int i = gi * 32; i < gi * 32 + 32; ++i) {
+                const float v = __uint_as_float(rbuf[i]);
+                m = fminf(m, (!tail || row_base + uint32_t(i) < n_rows) ? v : INFINITY);
               }
-            } else {
-              chunk(rbuf, c);
+              g2[gi] = m;
             }
+            *reinterpret_cast<float2*>(w.mdst + size_t(nt) * 8 + col0 / 32) = make_float2(g2[0], g2[1]);
           }
         }
       }
       if (!ok) break;
-      if (!SAMPLE && !TASKS) p.ccnt[cslot] = ncand;
+      if (!SAMPLE && !TASKS) {
+#pragma unroll
+        for (int mh = 0; mh < MH; ++mh) p.ccnt[lists0 + size_t(mh * 128 + r0) * 4] = rows[mh].ncand;
+      }
     }
   }
 
@@ -1044,9 +1065,8 @@ __global__ void init_search_kernel(RangeStats* qst, unsigned int* words) {
 // Exact re-rank and certification: one warp per query.
 struct RerankParams {
   const float* tau;       // the bound every candidate was tested against
-  const u64* cbuf;        // candidates of the main pass: [grid * segmax][LISTS][ccap]
+  const u64* cbuf;        // candidates of the main pass: [grid * segmax][128 * MH][4][ccap]
   const unsigned int* ccnt;
-  int ccap;
   PassShapes shapes;      // main pass
   const float* const8;    // 8-bit operands: the queries' constants, the parity of every row's t
   const uint8_t* parity8;
@@ -1141,26 +1161,25 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
   bool overflow = false;
   bool mismatch = false;  // exact regime only: a score that is not the exact distance
   u64 bound = FV_EMPTY_KEY;
-  const int lists_per_seg = sh.MH == 2 ? 2 : 4;
-  // The candidates of this query sit in parts * lists_per_seg short lists.  32 lists at a time: each lane looks up
-  // one list's count, a prefix sum lines the entries up, and the warp walks them 32 per step (a lane finds the
-  // list of its entry by bisection over the prefix sums), so every step computes 32 exact distances.
-  const int nlist = sh.parts * lists_per_seg;
+  const int ccap = sh.ccap;
+  // The candidates of this query sit in four short lists per chunk.  32 chunks at a time: each lane looks up the four
+  // counts of one, a prefix sum lines the entries up, and the warp walks them 32 per step (a lane finds the chunk of its
+  // entry by bisection over the prefix sums), so every step computes 32 exact distances.
   int taken = 0;  // runs of eight candidates seen so far, the same in all warps of the query
-  for (int l0 = 0; l0 < nlist; l0 += 32) {
+  for (int l0 = 0; l0 < sh.parts; l0 += 32) {
     const int l = l0 + lane;
     unsigned int cnt = 0;
+    u64 ends = 0;  // where the first three lists end, 16 bits each
     unsigned long long slot = 0;
-    if (l < nlist) {
-      const int part = l / lists_per_seg, li = l - part * lists_per_seg;
-      const int g = part * sh.MT + mt;
+    if (l < sh.parts) {
+      const int g = l * sh.MT + mt;
       const int c = g % sh.grid, seg_local = g / sh.grid;
-      slot = (size_t(c) * sh.segmax + seg_local) * LISTS + list_of_row(sh.MH, r, li);
-      cnt = p.ccnt[slot];
-      if (cnt > unsigned(p.ccap)) {
-        overflow = true;
-        cnt = unsigned(p.ccap);
-      }
+      slot = (size_t(c) * sh.segmax + seg_local) * rows_per_tile + r;
+      const uint4 c4 = reinterpret_cast<const uint4*>(p.ccnt)[slot];
+      if (max(max(c4.x, c4.y), max(c4.z, c4.w)) > unsigned(ccap)) overflow = true;
+      const unsigned int e0 = min(c4.x, unsigned(ccap)), e1 = e0 + min(c4.y, unsigned(ccap)), e2 = e1 + min(c4.z, unsigned(ccap));
+      cnt = e2 + min(c4.w, unsigned(ccap));
+      ends = u64(e0) | (u64(e1) << 16) | (u64(e2) << 32);
     }
     unsigned int pre = cnt;  // inclusive prefix sum
 #pragma unroll
@@ -1171,7 +1190,7 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
     const unsigned int total = __shfl_sync(FV_FULL, pre, 31);
     for (unsigned int t0 = 0; t0 < total; t0 += 32) {
       const unsigned int x = t0 + lane;
-      int j = 0;  // lists whose entries all come before entry x
+      int j = 0;  // chunks whose entries all come before entry x
 #pragma unroll
       for (int step = 16; step > 0; step >>= 1) {
         const unsigned int pv = __shfl_sync(FV_FULL, pre, j + step - 1);
@@ -1179,11 +1198,14 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
       }
       const unsigned int pj = __shfl_sync(FV_FULL, pre, j), cj = __shfl_sync(FV_FULL, cnt, j);
       const unsigned long long sj = __shfl_sync(FV_FULL, slot, j);
+      const u64 ej = __shfl_sync(FV_FULL, ends, j);
       u64 ck = 0;
       uint32_t id = 0;
       bool have = false;
       if (x < total) {
-        ck = p.cbuf[sj * size_t(p.ccap) + (x - (pj - cj))];
+        const unsigned int at = x - (pj - cj), e0 = unsigned(ej) & 0xFFFFu, e1 = unsigned(ej >> 16) & 0xFFFFu, e2 = unsigned(ej >> 32);
+        const int li = (at >= e0) + (at >= e1) + (at >= e2);
+        ck = p.cbuf[(sj * 4 + li) * size_t(ccap) + (at - (li == 0 ? 0u : li == 1 ? e0 : li == 2 ? e1 : e2))];
         id = key_id(ck);
         have = id < uint32_t(p.n);
         if (!have) mismatch = true;  // a padded row can only get here through a non-finite score
@@ -1573,6 +1595,8 @@ bool tc_usable(const TcSide* tc, size_t n, size_t nq, int k) {
 struct Tiling {
   int KB, last_steps, MH, MT, NT, grid, segmax, nstage, cpn, parts, nchunks, ext_ring;
   size_t smem;
+  size_t nlists;  // candidate lists of the pass, `ccap` slots each
+  int ccap;
 };
 
 // `row_bytes`: bytes of an operand row that hold data
@@ -1611,7 +1635,7 @@ static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, Tilin
   return fail(FV_ERR_UNSUPPORTED, "not enough shared memory for the tensor-core tiling");
 }
 
-static PassShape pass_shape(const Tiling& t) { return PassShape{t.MT, t.parts, t.grid, t.segmax, t.MH}; }
+static PassShape pass_shape(const Tiling& t) { return PassShape{t.MT, t.parts, t.grid, t.segmax, t.MH, t.ccap}; }
 
 // One launch over one way's operands, or over whichever of two the queries allow (`w8` and its word).
 template <bool SAMPLE>
@@ -1760,25 +1784,28 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
     CUtensorMap tmA, tmS, tmB;
     size_t nq_pad = 0;
   } way[2] = {};             // 0: 16-bit, 1: 8-bit
-  size_t nq_pad = 0, nlists = 0;
+  size_t nq_pad = 0, nlists = 0, cand_slots = 0;
   for (int i = 0; i < ways; ++i) {
     const int row_bytes = i ? pd : pd * 2;
     FV_TRY(make_tiling(ctx, row_bytes, nq, n, &way[i].tm));
     way[i].nq_pad = size_t(way[i].tm.MT) * 128 * way[i].tm.MH;
     nq_pad = std::max(nq_pad, way[i].nq_pad);
-    nlists = std::max(nlists, size_t(way[i].tm.grid) * way[i].tm.segmax * LISTS);
+    Tiling& t = way[i].tm;
+    // Candidate slots per list, 4 lists per query and chunk: 256 (128 with the twice as many lists of MH = 2) unless the
+    // buffers would pass 2 GB (they are written sparsely: about 160 entries per query in all).  A base stored cluster by
+    // cluster puts most of a query's candidates into one or two chunks, so the slots must hold more than the average.
+    t.nlists = size_t(t.grid) * t.segmax * (128 * t.MH * 4);
+    t.ccap = t.MH == 2 ? 128 : 256;
+    while (t.ccap > 16 && t.nlists * size_t(t.ccap) * sizeof(u64) > (size_t(2) << 30)) t.ccap >>= 1;
+    nlists = std::max(nlists, t.nlists);
+    cand_slots = std::max(cand_slots, t.nlists * size_t(t.ccap));
   }
 
   // queries -> operand rows (16 bits: scaled by -2 for L2, -1 for inner product), padded to whole tiles with zeros; norms;
   // statistics
   const size_t a16_bytes = (nq_pad * size_t(Kp) * 2 + 255) & ~size_t(255);
   FV_TRY(ctx->scratch[3].reserve(a16_bytes + (tc->i8 ? nq_pad * size_t(tc->Kp8) : 0)));
-  // Candidate slots per epilogue thread and segment: 256 unless the buffers would pass 2 GB (they are written
-  // sparsely: about 160 entries per query in all).  A base stored cluster by cluster puts most of a query's
-  // candidates into one or two chunks, so the slots must hold more than the average.
-  int ccap = 256;
-  while (ccap > 16 && nlists * size_t(ccap) * sizeof(u64) > (size_t(2) << 30)) ccap >>= 1;
-  FV_TRY(ctx->scratch[5].reserve(3 * nq_pad * sizeof(float) + nlists * sizeof(unsigned int)));
+  FV_TRY(ctx->scratch[5].reserve(3 * nq_pad * sizeof(float) + nlists * sizeof(unsigned int)));  // (nq_pad is a multiple of 128: the counts are aligned)
   // Sample pass: the minima of 1, 8, 32 or 64 sampled rows, so that there are hundreds of groups and two of a query's R best
   // seldom share one (their number times R (R - 1) / 2 is what the rank slips by), for at most 512 MB of queries at a time.
   const int group = ns <= 1024 ? 1 : ns <= 16384 ? 8 : ns <= 65536 ? 32 : 64;
@@ -1786,7 +1813,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   const size_t slice = std::min(nq_pad, std::max<size_t>(256, ((size_t(512) << 20) / (smin_ld * sizeof(float))) & ~size_t(255)));
   FV_TRY(ctx->scratch[6].reserve(slice * smin_ld * sizeof(float)));
   FV_TRY(ctx->scratch[7].reserve(nq * sizeof(uint32_t)));
-  FV_TRY(ctx->scratch[9].reserve(nlists * size_t(ccap) * sizeof(u64)));
+  FV_TRY(ctx->scratch[9].reserve(cand_slots * sizeof(u64)));
   uint16_t* dA = ctx->scratch[3].as<uint16_t>();
   uint8_t* dA8 = ctx->scratch[3].as<uint8_t>() + a16_bytes;
   float* qn2 = ctx->scratch[5].as<float>();
@@ -1863,7 +1890,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
     g.tau = tau;
     g.cbuf = ctx->scratch[9].as<u64>();
     g.ccnt = ccnt;
-    g.ccap = ccap;
+    g.ccap = way[i].tm.ccap;
     g.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
   }
   FV_TRY((launch_gemm<false>(ctx, way[0].tm, wm[0], way[1].tm, tc->i8 ? &wm[1] : nullptr, q8_bad)));
@@ -1873,7 +1900,6 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   rp.tau = tau;
   rp.cbuf = ctx->scratch[9].as<u64>();
   rp.ccnt = ccnt;
-  rp.ccap = ccap;
   rp.shapes = PassShapes{pass_shape(way[0].tm), pass_shape(way[1].tm), q8_bad};
   rp.const8 = const8;
   rp.parity8 = tc->parity8.as<uint8_t>();
