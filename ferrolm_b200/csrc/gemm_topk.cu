@@ -27,6 +27,7 @@
 //           the two 128-row halves use the two accumulator slots, so each B tile is read once
 //           from L2 for 256 queries.
 //   MH = 1: 128 queries per tile (K <= 384); the two accumulator slots alternate between units.
+// Batches with queries for more than one such tile are dealt to pairs of CTAs, two tiles at a time (gemm_topk_body, PAIR).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -43,7 +44,7 @@ namespace fv {
 static constexpr int TILE_N = 256;     // base rows per unit
 static constexpr int KBLK = 64;        // k elements per shared-memory block (128 bytes)
 static constexpr int A_BLOCK_BYTES = 128 * 128;   // 128 rows x 128 B
-static constexpr int B_STAGE_BYTES = TILE_N * 128;
+static constexpr int B_STAGE_BYTES = TILE_N * 128;  // (of a pair of CTAs: half in each)
 static constexpr int EXT_K = 16;                  // k elements of the norm step: one MMA
 static constexpr int A_EXT_BYTES = 128 * EXT_K * 2;     // query side of the norm step
 static constexpr int B_EXT_BYTES = TILE_N * EXT_K * 2;  // base side: one 8 KB tile per unit
@@ -110,6 +111,35 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// ---- two CTAs of a cluster working as a pair (cta_group::2): the first one's barriers are known to both by their
+// cluster-wide addresses, a commit arrives on the barriers of both
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t in_first_cta(const void* p) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+  return a;
+}
+// (at the scope of the CTA: what it hands over is tensor memory, not memory; a release at that of the cluster waits for the
+// thread's stores: 2,376 us for 10,000 queries at 1M x 128, 1,478 without)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+
 __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    smem_u32(dst)),
@@ -120,13 +150,33 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+template <bool PAIR>
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
+  if (PAIR) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                     smem_u32(bar)),
+                 "h"(uint16_t(3))
+                 : "memory");
+    return;
+  }
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
 
+template <bool PAIR>
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                            uint32_t accumulate) {
+  if (PAIR) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+    return;
+  }
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
@@ -138,8 +188,20 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
 }
 
 // 8-bit signed operands, 32-bit integer accumulators: exact, and K = 32 in the time and bytes of a 16-bit K = 16.
+template <bool PAIR>
 __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                           uint32_t accumulate) {
+  if (PAIR) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+    return;
+  }
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
@@ -264,7 +326,7 @@ struct StageCursor {
 struct GemmParams {
   int n, nq;
   int a_row0;      // operand row of the first query
-  int grid;        // CTAs that take work (task mode: all)
+  int grid;        // CTAs, or pairs of CTAs, that take work (task mode: all)
   int KB;          // k blocks of 128 bytes per row (64 16-bit or 128 8-bit elements)
   int last_steps;  // MMAs (32 bytes per row) of the last k block: 4 less the ones that would only meet padding
   int NT;          // base tiles of 256 rows
@@ -358,6 +420,7 @@ static int pick_sample_r(int k, int every) {
 // device word q8_bad says which of the two passes ran.
 struct PassShape {
   int MT, parts, grid, segmax, MH;
+  int ctas;  // 2: pairs of CTAs
   int ccap;  // slots of a candidate list
 };
 struct PassShapes {
@@ -419,19 +482,32 @@ struct Score<true> {
   __device__ static __forceinline__ T min3(T a, T b, T c) { return min(min(a, b), c); }
 };
 
-template <int MH, bool SAMPLE, bool TASKS, bool I8>
-__device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p) {
+// PAIR: the CTAs of a cluster of two work as one on tiles of twice as many queries (cta_group::2).  Each has its half of the
+// queries and, of every 256 base rows, 128 in its shared memory; the first one issues the MMAs, which read both halves, so a
+// base row is fetched into and read from shared memory once for twice the scores.  Each CTA's accumulators are its own
+// queries' scores.
+// 384 dimensions are bound by that traffic (209 cycles per 128 x 256 MMA with one CTA, 165 with pairs; 128 nominal): main
+// pass of 2,049 queries over 200,003 x 384 274 -> 230 us; 5,000 over 500,000 x 128 in 16 bits 578 -> 499, in bytes, where the
+// epilogue's hits bound it, 0.98 to 1.02 times.
+template <int MH, bool SAMPLE, bool TASKS, bool I8, bool PAIR>
+__device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmE,
+                                               const GemmParams& p) {
+  static_assert(!(TASKS && PAIR), "tasks are drawn by single CTAs");
   typedef Score<I8> S;
   typedef typename S::T T;
   constexpr int KE = I8 ? 2 * KBLK : KBLK;  // elements of a k block
-  if (!TASKS && int(blockIdx.x) >= p.grid) return;
+  constexpr int CTAS = PAIR ? 2 : 1;
+  constexpr int B_ROWS = TILE_N / CTAS;  // base rows of a unit in this CTA's shared memory
+  constexpr int STAGE_BYTES = B_ROWS * 128, EXT_BYTES = B_ROWS * EXT_K * 2;
+  const int rank = PAIR ? int(cluster_rank()) : 0, worker = int(blockIdx.x) / CTAS;
+  if (!TASKS && worker >= p.grid) return;
   unsigned char* raw = dyn_smem();
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sA = base;                                            // [MH][KB] blocks of 16 KB
   unsigned char* sAext = sA + size_t(MH) * p.KB * A_BLOCK_BYTES;       // 4 KB: the constant rows of the norm step
-  unsigned char* sB = sAext + A_EXT_BYTES;                             // [nstage] stages of 32 KB
-  unsigned char* sE = sB + size_t(p.nstage) * B_STAGE_BYTES;           // [ext_ring] norm-step tiles of 8 KB
-  Barriers* bars = reinterpret_cast<Barriers*>(sE + size_t(p.ext_ring) * B_EXT_BYTES);
+  unsigned char* sB = sAext + A_EXT_BYTES;                             // [nstage] stages of 32 KB (PAIR: 16)
+  unsigned char* sE = sB + size_t(p.nstage) * STAGE_BYTES;             // [ext_ring] norm-step tiles of 8 KB (4)
+  Barriers* bars = reinterpret_cast<Barriers*>(sE + size_t(p.ext_ring) * EXT_BYTES);
   const AbortCtl abort_flag{&bars->abort_flag, p.wait_limit};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -446,7 +522,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
     for (int i = 0; i < 8; ++i) mbar_init(&bars->tq_full[i], 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->tfull[i], 1);
-      mbar_init(&bars->tempty[i], NEPI);
+      mbar_init(&bars->tempty[i], NEPI * CTAS);
     }
     bars->abort_flag = 0;
     bars->pool_pos = 0;
@@ -457,12 +533,19 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
   if (threadIdx.x < A_EXT_BYTES / 16) reinterpret_cast<uint4*>(sAext)[threadIdx.x] = p.aext;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 1) {  // the MMA warp owns the tensor memory: all 512 columns (one CTA per SM)
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&bars->tmem_base))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&bars->tmem_base))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&bars->tmem_base))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // the other CTA's barriers are set up
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   // Work items.  Plain and threshold mode: chunk g of the tiling, CTA b taking g = b, b + grid, ...
@@ -474,12 +557,12 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
   // the latest (two accumulator slots).  The caller sorts the tasks by decreasing length: longest first.
   const int nwork = TASKS ? int(*p.ntasks) : p.nchunks;
   auto work_of = [&](int seg) -> int {  // consumer side
-    if (!TASKS) return int(blockIdx.x) + seg * p.grid;
+    if (!TASKS) return worker + seg * p.grid;
     if (!mbar_wait(&bars->tq_full[seg & 7], uint32_t(seg >> 3) & 1, abort_flag)) return 0x7FFFFFFF;
     return int(*reinterpret_cast<volatile unsigned int*>(&bars->tq[seg & 7]));
   };
   auto draw = [&](int seg) -> int {  // producer side
-    if (!TASKS) return int(blockIdx.x) + seg * p.grid;
+    if (!TASKS) return worker + seg * p.grid;
     const unsigned int g = min(atomicAdd(p.next_task, 1u), 0x7FFFFFFEu);
     bars->tq[seg & 7] = g;
     mbar_arrive(&bars->tq_full[seg & 7]);  // release: the entry is visible to whoever sees this phase complete
@@ -491,8 +574,13 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
     if (lane == 0) {
       bool ok = true;
       StageCursor st(p.nstage);
-      int ring = 0;
-      for (int seg = 0, g = draw(0); g < nwork && ok; g = draw(++seg)) {
+      int ring = 0, seg = 0;
+      // (both CTAs of a pair fill their halves of a stage and count on the first one's barrier)
+      auto load = [&](void* dst, const CUtensorMap& map, uint64_t* bar, int x, int y) {
+        if (PAIR) tma_load_2d_pair(dst, &map, in_first_cta(bar), x, y);
+        else tma_load_2d(dst, &map, bar, x, y);
+      };
+      for (int g = draw(0); g < nwork && ok; g = draw(++seg)) {
         int nt0, nt1, a_row0, b_row0 = 0;
         if (TASKS) {
           const uint4 t = p.tasks[g];
@@ -504,14 +592,14 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
           const int part = g / p.MT, mt = g - part * p.MT;
           nt0 = part * p.cpn;
           nt1 = min(p.NT, nt0 + p.cpn);
-          a_row0 = p.a_row0 + mt * MH * 128;
+          a_row0 = p.a_row0 + (mt * CTAS + rank) * MH * 128;
         }
         ok = mbar_wait(&bars->a_empty, (seg & 1) ^ 1, abort_flag);
         if (!ok) break;
-        mbar_expect_tx(&bars->a_full, uint32_t(MH * p.KB * A_BLOCK_BYTES));
+        if (rank == 0) mbar_expect_tx(&bars->a_full, uint32_t(CTAS * MH * p.KB * A_BLOCK_BYTES));
         for (int mh = 0; mh < MH; ++mh)
           for (int kb = 0; kb < p.KB; ++kb)
-            tma_load_2d(sA + size_t(mh * p.KB + kb) * A_BLOCK_BYTES, &tmA, &bars->a_full, kb * KE, a_row0 + mh * 128);
+            load(sA + size_t(mh * p.KB + kb) * A_BLOCK_BYTES, tmA, &bars->a_full, kb * KE, a_row0 + mh * 128);
         for (int nt = nt0; nt < nt1 && ok; ++nt) {
           for (int kb = 0; kb < p.KB; ++kb, st.next()) {
             const int s = st.s;
@@ -523,15 +611,21 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
             const bool with_ext = kb == 0 && p.has_ext;
             // (test hook: the stage is never posted, its consumer waits until the limit and the kernel gives up)
             if (p.fault_skip_unit >= 0 && g == 0 && nt == nt0 + p.fault_skip_unit) continue;
-            mbar_expect_tx(&bars->full[s], uint32_t(B_STAGE_BYTES + (with_ext ? B_EXT_BYTES : 0)));
+            if (rank == 0) mbar_expect_tx(&bars->full[s], uint32_t(CTAS * (STAGE_BYTES + (with_ext ? EXT_BYTES : 0))));
             // first B row of the unit (task mode: a multiple of 8, which keeps the norm tile's swizzle image in step)
-            const size_t brow = size_t(b_row0) + size_t(nt) * TILE_N;
-            if (with_ext)  // stored as the swizzled shared-memory image: one contiguous 8 KB copy
-              bulk_load_1d(sE + size_t(ring) * B_EXT_BYTES, p.ext + brow * EXT_K, B_EXT_BYTES, &bars->full[s]);
-            tma_load_2d(sB + size_t(s) * B_STAGE_BYTES, &tmB, &bars->full[s], kb * KE, int(brow));
+            const size_t brow = size_t(b_row0) + size_t(nt) * TILE_N + rank * B_ROWS;
+            if (with_ext) {  // stored as the swizzled shared-memory image: one contiguous copy (PAIR: as rows of 128 bytes)
+              if (PAIR) load(sE + size_t(ring) * EXT_BYTES, tmE, &bars->full[s], 0, int(brow / 4));
+              else bulk_load_1d(sE + size_t(ring) * EXT_BYTES, p.ext + brow * EXT_K, EXT_BYTES, &bars->full[s]);
+            }
+            load(sB + size_t(s) * STAGE_BYTES, tmB, &bars->full[s], kb * KE, int(brow));
           }
           if (++ring == p.ext_ring) ring = 0;
         }
+      }
+      if (PAIR && ok && seg > 0) {  // nor while the first CTA's commits may still arrive here: the last ones of all stages and tiles
+        for (int i = 0; i < p.nstage && ok; ++i, st.next()) ok = mbar_wait(&bars->empty[st.s], st.phase ^ 1, abort_flag);
+        ok = ok && mbar_wait(&bars->a_empty, (seg & 1) ^ 1, abort_flag);
       }
       // Do not leave while copies may still land in this CTA's shared memory: wait (bounded) until the
       // MMA side has consumed everything that was issued, or until the abort flag says nobody will.
@@ -541,7 +635,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 && rank == 0) {
     // ---------------------------------------------------------------- MMA issuer
     // The whole warp walks the loop, so that everything an MMA is issued with is uniform, and one elected lane issues.
     // Descriptors advance by adding to their low words.
@@ -552,8 +646,8 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
     const uint32_t a_lo0 = desc_lo(smem_u32(sA)), b_lo0 = desc_lo(smem_u32(sB)), e_lo0 = desc_lo(smem_u32(sE));
     const uint32_t aext_lo = desc_lo(smem_u32(sAext));
     auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
-      if (I8) tc_mma_i8(d, a, b, p.idesc, accumulate);
-      else tc_mma_f16(d, a, b, p.idesc, accumulate);
+      if (I8) tc_mma_i8<PAIR>(d, a, b, p.idesc, accumulate);
+      else tc_mma_f16<PAIR>(d, a, b, p.idesc, accumulate);
     };
     for (int seg = 0, g = work_of(0); g < nwork && ok; g = work_of(++seg)) {
       int nt0, nt1;
@@ -587,11 +681,11 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
             if (leader) {
               uint32_t acc = kb != 0 ? 1u : 0u;  // the first MMA of a job overwrites the accumulator
               if (kb == 0 && p.has_ext) {        // + ||b||^2: always the first step of a job
-                mma(d_tmem, make_desc(aext_lo, DESC_HI_SW32), make_desc(e_lo0 + uint32_t(ring * (B_EXT_BYTES >> 4)), DESC_HI_SW32), 0u);
+                mma(d_tmem, make_desc(aext_lo, DESC_HI_SW32), make_desc(e_lo0 + uint32_t(ring * (EXT_BYTES >> 4)), DESC_HI_SW32), 0u);
                 acc = 1;
               }
               const uint32_t a_lo = a_lo0 + uint32_t((mh * p.KB + kb) * (A_BLOCK_BYTES >> 4));
-              const uint32_t b_lo = b_lo0 + uint32_t(s * (B_STAGE_BYTES >> 4));
+              const uint32_t b_lo = b_lo0 + uint32_t(s * (STAGE_BYTES >> 4));
               mma(d_tmem, make_desc(a_lo, DESC_HI_SW128), make_desc(b_lo, DESC_HI_SW128), acc);
               if (kb + 1 < p.KB || p.last_steps == 4) {
 #pragma unroll
@@ -601,8 +695,8 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
                 for (int k4 = 1; k4 < p.last_steps; ++k4)
                   mma(d_tmem, make_desc(a_lo + 2 * k4, DESC_HI_SW128), make_desc(b_lo + 2 * k4, DESC_HI_SW128), 1u);
               }
-              if (mh == MH - 1) tc_commit(&bars->empty[s]);  // the stage is free once these MMAs have read it
-              if (kb + 1 == p.KB) tc_commit(&bars->tfull[slot]);
+              if (mh == MH - 1) tc_commit<PAIR>(&bars->empty[s]);  // the stage is free once these MMAs have read it
+              if (kb + 1 == p.KB) tc_commit<PAIR>(&bars->tfull[slot]);
             }
             __syncwarp();
           }
@@ -611,10 +705,10 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
         for (int kb = 0; kb < p.KB; ++kb) st.next();
         if (++ring == p.ext_ring) ring = 0;
       }
-      if (ok && leader) tc_commit(&bars->a_empty);  // the query tile may be replaced once every MMA above has read it
+      if (ok && leader) tc_commit<PAIR>(&bars->a_empty);  // the query tile may be replaced once every MMA above has read it
       __syncwarp();
     }
-  } else {
+  } else if (warp > 1) {
     // ---------------------------------------------------------------- epilogue: 16 warps, one query row per thread
     // Every warp reads its 64 columns of every accumulator in one load and hands the slot back at once: what it then does
     // with them delays no MMA as long as it keeps up on average.  (With MH = 2 each half's accumulators used to belong to
@@ -658,7 +752,7 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
 #pragma unroll
       for (int mh = 0; mh < MH; ++mh) {
         Row& w = rows[mh];
-        const int r = mh * 128 + r0, q = mt * (128 * MH) + r;
+        const int r = mh * 128 + r0, q = (mt * CTAS + rank) * (128 * MH) + r;
         w.ncand = 0;
         if (SAMPLE) {
           w.sdst = p.smin + size_t(q) * p.smin_ld;
@@ -814,7 +908,10 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
           tc_ld64_wait(rbuf);
           tc_fence_before();  // the load has landed: the MMA may overwrite this accumulator slot
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->tempty[slot]);
+          if (lane == 0) {
+            if (PAIR) mbar_arrive_cluster(in_first_cta(&bars->tempty[slot]));
+            else mbar_arrive(&bars->tempty[slot]);
+          }
           if (SAMPLE) {
             sample(rbuf);
           } else if (!TASKS) {
@@ -850,32 +947,33 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // nothing of the other CTA's is on its way here
   if (threadIdx.x == 0 && *abort_flag.flag) atomicExch(p.err, 1);
   if (TASKS && threadIdx.x == 0) p.pool_cnt[blockIdx.x] = bars->pool_pos;
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
   }
 }
 
-template <int MH, bool SAMPLE, bool TASKS = false>
-__global__ void __launch_bounds__(NTHREADS, 1)
-    gemm_topk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ GemmParams p) {
-  gemm_topk_body<MH, SAMPLE, TASKS, false>(tmA, tmB, p);
+// What a pass is launched with; the maps of the operands and, for pairs, of the norm step's tiles
+struct GemmWay {
+  CUtensorMap tmA, tmB, tmE;
+  GemmParams p;
+};
+template <int MH, bool SAMPLE, bool TASKS, bool PAIR>
+__global__ void __launch_bounds__(NTHREADS, 1) gemm_topk_kernel(const __grid_constant__ GemmWay w) {
+  gemm_topk_body<MH, SAMPLE, TASKS, false, PAIR>(w.tmA, w.tmB, w.tmE, w.p);
 }
 
 // The pass over the 8-bit operands or, where a query of the batch does not fit them (q8_bad, known on the device only), over
 // the 16-bit ones: one launch, since one that leaves at once costs a pass over 100,000 rows 3 us of 40.
-struct GemmWay {
-  CUtensorMap tmA, tmB;
-  GemmParams p;
-};
-template <int MH16, bool SAMPLE>
+template <int MH16, bool SAMPLE, bool PAIR>
 __global__ void __launch_bounds__(NTHREADS, 1)
     gemm_topk_either_kernel(const __grid_constant__ GemmWay w16, const __grid_constant__ GemmWay w8, const unsigned int* q8_bad) {
-  if (*q8_bad) gemm_topk_body<MH16, SAMPLE, false, false>(w16.tmA, w16.tmB, w16.p);
-  else gemm_topk_body<2, SAMPLE, false, true>(w8.tmA, w8.tmB, w8.p);
+  if (*q8_bad) gemm_topk_body<MH16, SAMPLE, false, false, PAIR>(w16.tmA, w16.tmB, w16.tmE, w16.p);
+  else gemm_topk_body<2, SAMPLE, false, true, PAIR>(w8.tmA, w8.tmB, w8.tmE, w8.p);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1154,7 +1252,8 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
   const bool is8 = IS_L2 && p.shapes.is8();
   const PassShape& sh = p.shapes.taken();
   const int rows_per_tile = 128 * sh.MH;
-  const int mt = int(q / rows_per_tile), r = int(q % rows_per_tile);
+  const int cta_tile = int(q / rows_per_tile), r = int(q % rows_per_tile);  // a CTA's share of a query tile
+  const int mt = cta_tile / sh.ctas, rank = cta_tile % sh.ctas;
   const float const8 = is8 ? p.const8[q] : 0.f;
   // every row whose score is below tau is in the buffer; every other row scores >= tau
   const float tau = p.tau[q];
@@ -1173,7 +1272,7 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
     unsigned long long slot = 0;
     if (l < sh.parts) {
       const int g = l * sh.MT + mt;
-      const int c = g % sh.grid, seg_local = g / sh.grid;
+      const int c = g % sh.grid * sh.ctas + rank, seg_local = g / sh.grid;
       slot = (size_t(c) * sh.segmax + seg_local) * rows_per_tile + r;
       const uint4 c4 = reinterpret_cast<const uint4*>(p.ccnt)[slot];
       if (max(max(c4.x, c4.y), max(c4.z, c4.w)) > unsigned(ccap)) overflow = true;
@@ -1365,6 +1464,20 @@ static int make_tmap(CUtensorMap* map, CUtensorMapDataType type, void* ptr, size
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, type, 2, ptr, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(FV_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
+  return FV_OK;
+}
+
+// the norm step's bytes as rows of 128, boxes of 32 rows: 128 rows' worth, as they lie in memory
+static int make_norm_tmap(CUtensorMap* map, void* ptr, size_t rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return fail(FV_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t gdim[2] = {128, cuuint64_t(rows / 4)};
+  cuuint64_t gstride[1] = {128};
+  cuuint32_t box[2] = {128, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, ptr, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(FV_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
   return FV_OK;
 }
@@ -1593,21 +1706,22 @@ bool tc_usable(const TcSide* tc, size_t n, size_t nq, int k) {
 // units the 16-bit copy of the base was streamed from HBM once per query tile).  `parts` is the value that minimises
 // waves x (chunk length + a fixed cost per chunk).
 struct Tiling {
-  int KB, last_steps, MH, MT, NT, grid, segmax, nstage, cpn, parts, nchunks, ext_ring;
+  int KB, last_steps, MH, ctas, MT, NT, grid, segmax, nstage, cpn, parts, nchunks, ext_ring;
   size_t smem;
   size_t nlists;  // candidate lists of the pass, `ccap` slots each
   int ccap;
 };
 
 // `row_bytes`: bytes of an operand row that hold data
-static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, Tiling* t, int force_mh = 0) {
+static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, Tiling* t, int force_mh = 0, bool pairs = false) {
   t->KB = (row_bytes + 127) / 128;
   t->last_steps = (row_bytes - (t->KB - 1) * 128 + 31) / 32;
   t->MH = force_mh ? force_mh : (t->KB <= 2 ? 2 : 1);
-  const int rows_per_tile = 128 * t->MH;
+  t->ctas = pairs ? 2 : 1;
+  const int rows_per_tile = 128 * t->MH * t->ctas;
   t->MT = int((nq + rows_per_tile - 1) / rows_per_tile);
   t->NT = int((rows + TILE_N - 1) / TILE_N);
-  t->grid = int(std::min<long long>(ctx->sm_count, (long long)t->MT * t->NT));
+  t->grid = int(std::min<long long>(ctx->sm_count / t->ctas, (long long)t->MT * t->NT));
   long long best = -1;
   for (int P = 1; P <= t->NT && P <= 4096; ++P) {
     const int cpn = (t->NT + P - 1) / P;
@@ -1627,29 +1741,42 @@ static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, Tilin
   t->segmax = int((chunks + t->grid - 1) / t->grid);
   const size_t a_bytes = size_t(t->MH) * t->KB * A_BLOCK_BYTES + A_EXT_BYTES;
   const size_t tail = sizeof(Barriers) + 64;
-  for (t->nstage = 6; t->nstage >= 2; --t->nstage) {
+  for (t->nstage = 6 + t->ctas; t->nstage >= 2; --t->nstage) {
     t->ext_ring = (t->nstage + t->KB - 1) / t->KB + 1;
-    t->smem = 1024 + a_bytes + size_t(t->nstage) * B_STAGE_BYTES + size_t(t->ext_ring) * B_EXT_BYTES + tail;
+    t->smem = 1024 + a_bytes + (size_t(t->nstage) * B_STAGE_BYTES + size_t(t->ext_ring) * B_EXT_BYTES) / t->ctas + tail;
     if (t->smem <= ctx->smem_optin) return FV_OK;
   }
   return fail(FV_ERR_UNSUPPORTED, "not enough shared memory for the tensor-core tiling");
 }
 
-static PassShape pass_shape(const Tiling& t) { return PassShape{t.MT, t.parts, t.grid, t.segmax, t.MH, t.ccap}; }
+static PassShape pass_shape(const Tiling& t) { return PassShape{t.MT, t.parts, t.grid, t.segmax, t.MH, t.ctas, t.ccap}; }
 
 // One launch over one way's operands, or over whichever of two the queries allow (`w8` and its word).
 template <bool SAMPLE>
 static int launch_gemm(fv_ctx* ctx, const Tiling& t16, const GemmWay& w16, const Tiling& t8, const GemmWay* w8,
                        const unsigned int* q8_bad) {
+  const bool pair = t16.ctas == 2;
+  const size_t smem = w8 ? std::max(t16.smem, t8.smem) : t16.smem;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim = {2, 1, 1};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = unsigned((w8 ? std::max(t16.grid, t8.grid) : t16.grid) * t16.ctas);
+  cfg.blockDim = NTHREADS;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = pair ? 1 : 0;
   if (!w8) {
-    auto kern = t16.MH == 2 ? gemm_topk_kernel<2, SAMPLE> : gemm_topk_kernel<1, SAMPLE>;
-    FV_TRY(allow_smem(ctx, kern, t16.smem));
-    kern<<<t16.grid, NTHREADS, t16.smem, ctx->stream>>>(w16.tmA, w16.tmB, w16.p);
-  } else {
-    auto kern = t16.MH == 2 ? gemm_topk_either_kernel<2, SAMPLE> : gemm_topk_either_kernel<1, SAMPLE>;
-    const size_t smem = std::max(t16.smem, t8.smem);
+    auto kern = t16.MH == 2 ? (pair ? gemm_topk_kernel<2, SAMPLE, false, true> : gemm_topk_kernel<2, SAMPLE, false, false>)
+                            : (pair ? gemm_topk_kernel<1, SAMPLE, false, true> : gemm_topk_kernel<1, SAMPLE, false, false>);
     FV_TRY(allow_smem(ctx, kern, smem));
-    kern<<<std::max(t16.grid, t8.grid), NTHREADS, smem, ctx->stream>>>(w16, *w8, q8_bad);
+    FV_CUDA(cudaLaunchKernelEx(&cfg, kern, w16));
+  } else {
+    auto kern = t16.MH == 2 ? (pair ? gemm_topk_either_kernel<2, SAMPLE, true> : gemm_topk_either_kernel<2, SAMPLE, false>)
+                            : (pair ? gemm_topk_either_kernel<1, SAMPLE, true> : gemm_topk_either_kernel<1, SAMPLE, false>);
+    FV_TRY(allow_smem(ctx, kern, smem));
+    FV_CUDA(cudaLaunchKernelEx(&cfg, kern, w16, *w8, q8_bad));
   }
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
@@ -1743,14 +1870,14 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
   gp.minima = d_minima;
   gp.task_moff = d_task_moff;
   gp.task_rows = d_task_rows;
-  CUtensorMap tmA, tmB;
-  FV_TRY(make_tmap(&tmA, type16(tc->bf16), const_cast<uint16_t*>(d_A), a_rows, Kp, 128));
-  FV_TRY(make_tmap(&tmB, type16(tc->bf16), tc->half.p, tc->n, Kp, TILE_N));
+  GemmWay w{};
+  w.p = gp;
+  FV_TRY(make_tmap(&w.tmA, type16(tc->bf16), const_cast<uint16_t*>(d_A), a_rows, Kp, 128));
+  FV_TRY(make_tmap(&w.tmB, type16(tc->bf16), tc->half.p, tc->n, Kp, TILE_N));
   FV_CUDA(cudaMemsetAsync(d_next_task, 0, sizeof(unsigned int), ctx->stream));
-  void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams) =
-      tile_rows == 128 ? gemm_topk_kernel<1, false, true> : gemm_topk_kernel<2, false, true>;
+  auto kern = tile_rows == 128 ? gemm_topk_kernel<1, false, true, false> : gemm_topk_kernel<2, false, true, false>;
   FV_TRY(allow_smem(ctx, kern, t.smem));
-  kern<<<ctx->sm_count, NTHREADS, t.smem, ctx->stream>>>(tmA, tmB, gp);
+  kern<<<ctx->sm_count, NTHREADS, t.smem, ctx->stream>>>(w);
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   *grid_out = ctx->sm_count;
@@ -1779,22 +1906,24 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   // One way through both passes, or two: over the 8-bit operands where the base has them and, should a query of the batch
   // not fit them (known on the device only), over the 16-bit ones.  The kernels of the way that is not taken leave at once.
   const int ways = tc->i8 ? 2 : 1;
+  // Pairs of CTAs where the batch has queries for both: more than one CTA's tile of the taller of the two ways.
+  const bool pairs = nq > (Kp <= 2 * KBLK || tc->i8 ? 256u : 128u);
   struct Way {
     Tiling tm;               // main pass
-    CUtensorMap tmA, tmS, tmB;
+    GemmWay main, sample;
     size_t nq_pad = 0;
   } way[2] = {};             // 0: 16-bit, 1: 8-bit
   size_t nq_pad = 0, nlists = 0, cand_slots = 0;
   for (int i = 0; i < ways; ++i) {
     const int row_bytes = i ? pd : pd * 2;
-    FV_TRY(make_tiling(ctx, row_bytes, nq, n, &way[i].tm));
-    way[i].nq_pad = size_t(way[i].tm.MT) * 128 * way[i].tm.MH;
+    FV_TRY(make_tiling(ctx, row_bytes, nq, n, &way[i].tm, 0, pairs));
+    way[i].nq_pad = size_t(way[i].tm.MT) * 128 * way[i].tm.MH * way[i].tm.ctas;
     nq_pad = std::max(nq_pad, way[i].nq_pad);
     Tiling& t = way[i].tm;
     // Candidate slots per list, 4 lists per query and chunk: 256 (128 with the twice as many lists of MH = 2) unless the
     // buffers would pass 2 GB (they are written sparsely: about 160 entries per query in all).  A base stored cluster by
     // cluster puts most of a query's candidates into one or two chunks, so the slots must hold more than the average.
-    t.nlists = size_t(t.grid) * t.segmax * (128 * t.MH * 4);
+    t.nlists = size_t(t.grid) * t.ctas * t.segmax * (128 * t.MH * 4);
     t.ccap = t.MH == 2 ? 128 : 256;
     while (t.ccap > 16 && t.nlists * size_t(t.ccap) * sizeof(u64) > (size_t(2) << 30)) t.ccap >>= 1;
     nlists = std::max(nlists, t.nlists);
@@ -1810,7 +1939,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   // seldom share one (their number times R (R - 1) / 2 is what the rank slips by), for at most 512 MB of queries at a time.
   const int group = ns <= 1024 ? 1 : ns <= 16384 ? 8 : ns <= 65536 ? 32 : 64;
   const size_t smin_ld = (ns + TILE_N - 1) / TILE_N * TILE_N / group;
-  const size_t slice = std::min(nq_pad, std::max<size_t>(256, ((size_t(512) << 20) / (smin_ld * sizeof(float))) & ~size_t(255)));
+  const size_t slice = std::min(nq_pad, std::max<size_t>(512, ((size_t(512) << 20) / (smin_ld * sizeof(float))) & ~size_t(511)));
   FV_TRY(ctx->scratch[6].reserve(slice * smin_ld * sizeof(float)));
   FV_TRY(ctx->scratch[7].reserve(nq * sizeof(uint32_t)));
   FV_TRY(ctx->scratch[9].reserve(cand_slots * sizeof(u64)));
@@ -1825,14 +1954,27 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   unsigned int* words = side_words(tc);
   unsigned int* retry_count = words + W_RETRY;
   unsigned int* q8_bad = tc->i8 ? words + W_Q8_BAD : nullptr;
-  FV_TRY(make_tmap(&way[0].tmA, type16(tc->bf16), dA, nq_pad, Kp, 128));
-  FV_TRY(make_tmap(&way[0].tmS, type16(tc->bf16), tc->samp.p, ns, Kp, TILE_N));
-  FV_TRY(make_tmap(&way[0].tmB, type16(tc->bf16), tc->half.p, n, Kp, TILE_N));
-  if (tc->i8) {
-    const CUtensorMapDataType type8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
-    FV_TRY(make_tmap(&way[1].tmA, type8, dA8, nq_pad, tc->Kp8, 128));
-    FV_TRY(make_tmap(&way[1].tmS, type8, tc->samp8.p, ns, tc->Kp8, TILE_N));
-    FV_TRY(make_tmap(&way[1].tmB, type8, tc->rows8.p, n, tc->Kp8, TILE_N));
+  const size_t n_pad = (n + TILE_N - 1) / TILE_N * TILE_N, ns_pad = (ns + TILE_N - 1) / TILE_N * TILE_N;
+  for (int i = 0; i < ways; ++i) {
+    Way& w = way[i];
+    const CUtensorMapDataType type = i ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : type16(tc->bf16);
+    const int K = i ? tc->Kp8 : Kp, box = TILE_N / w.tm.ctas;
+    FV_TRY(make_tmap(&w.main.tmA, type, i ? static_cast<void*>(dA8) : dA, nq_pad, K, 128));
+    FV_TRY(make_tmap(&w.main.tmB, type, (i ? tc->rows8 : tc->half).p, n, K, box));
+    GemmParams& g = w.main.p;
+    g = GemmParams{};
+    g.has_ext = is_l2 ? 1 : 0;
+    g.aext = i ? norm_step_queries8() : norm_step_queries(tc);
+    g.idesc = i ? make_idesc_i8(128 * w.tm.ctas, TILE_N) : make_idesc(128 * w.tm.ctas, TILE_N, tc->bf16);
+    g.err = tc_error_word(tc);
+    w.sample = w.main;
+    FV_TRY(make_tmap(&w.sample.tmB, type, (i ? tc->samp8 : tc->samp).p, ns, K, box));
+    if (is_l2) {
+      g.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
+      w.sample.p.ext = (i ? tc->samp_ext8 : tc->samp_ext).as<uint16_t>();
+      FV_TRY(make_norm_tmap(&w.main.tmE, (i ? tc->ext8 : tc->ext).p, n_pad));
+      FV_TRY(make_norm_tmap(&w.sample.tmE, (i ? tc->samp_ext8 : tc->samp_ext).p, ns_pad));
+    }
   }
 
   init_search_kernel<<<1, 1, 0, ctx->stream>>>(qst, words);
@@ -1845,33 +1987,21 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   FV_TRY(convert(ctx, tc->bf16, d_queries, nq, pd, Kp, dA, qn2, is_l2, is_l2 ? -2.f : -1.f, qst, q8));
   if (mark_stages) stage_mark(ctx);
 
-  GemmParams gp[2];
-  for (int i = 0; i < ways; ++i) {
-    gp[i] = GemmParams{};
-    gp[i].has_ext = is_l2 ? 1 : 0;
-    gp[i].aext = i ? norm_step_queries8() : norm_step_queries(tc);
-    gp[i].idesc = i ? make_idesc_i8(128, TILE_N) : make_idesc(128, TILE_N, tc->bf16);
-    gp[i].err = tc_error_word(tc);
-  }
-
   // sample pass: group minima of the sampled rows' scores, and from them the queries' bounds
   for (size_t q0 = 0; q0 < nq; q0 += slice) {
     const size_t nqs = std::min(slice, nq - q0);
     Tiling ts[2] = {};
-    GemmWay ws[2];
     const WaitLimit limit = next_wait_limit();
     for (int i = 0; i < ways; ++i) {
-      FV_TRY(make_tiling(ctx, i ? pd : pd * 2, nqs, ns, &ts[i]));
-      ws[i] = GemmWay{way[i].tmA, way[i].tmS, gp[i]};
-      GemmParams& g = ws[i].p;
+      FV_TRY(make_tiling(ctx, i ? pd : pd * 2, nqs, ns, &ts[i], 0, pairs));
+      GemmParams& g = way[i].sample.p;
       fill_params(&g, ts[i], ns, nqs, limit);
       g.a_row0 = int(q0);
       g.smin = ctx->scratch[6].as<float>();
       g.smin_ld = int(smin_ld);
       g.group = group;
-      g.ext = (i ? tc->samp_ext8 : tc->samp_ext).as<uint16_t>();
     }
-    FV_TRY((launch_gemm<true>(ctx, ts[0], ws[0], ts[1], tc->i8 ? &ws[1] : nullptr, q8_bad)));
+    FV_TRY(launch_gemm<true>(ctx, ts[0], way[0].sample, ts[1], tc->i8 ? &way[1].sample : nullptr, q8_bad));
     const size_t with_bound = std::min(slice, nq_pad - q0);
     sample_tau_kernel<<<unsigned((with_bound + 7) / 8), 256, 0, ctx->stream>>>(
         ctx->scratch[6].as<float>(), int(smin_ld), int((ns + group - 1) / group), int(with_bound), R, tau + q0);
@@ -1881,19 +2011,16 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   if (mark_stages) stage_mark(ctx);
 
   // main pass: every row scoring below the query's sampled bound becomes a candidate
-  GemmWay wm[2];
   const WaitLimit limit = next_wait_limit();
   for (int i = 0; i < ways; ++i) {
-    wm[i] = GemmWay{way[i].tmA, way[i].tmB, gp[i]};
-    GemmParams& g = wm[i].p;
+    GemmParams& g = way[i].main.p;
     fill_params(&g, way[i].tm, n, nq, limit);
     g.tau = tau;
     g.cbuf = ctx->scratch[9].as<u64>();
     g.ccnt = ccnt;
     g.ccap = way[i].tm.ccap;
-    g.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
   }
-  FV_TRY((launch_gemm<false>(ctx, way[0].tm, wm[0], way[1].tm, tc->i8 ? &wm[1] : nullptr, q8_bad)));
+  FV_TRY(launch_gemm<false>(ctx, way[0].tm, way[0].main, way[1].tm, tc->i8 ? &way[1].main : nullptr, q8_bad));
   if (mark_stages) stage_mark(ctx);
 
   RerankParams rp{};
