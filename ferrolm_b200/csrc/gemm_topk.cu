@@ -391,13 +391,15 @@ struct __align__(8) Barriers {
 // k - 1 nearest rows happen to be sampled: probability P(Binomial(k - 1, 1/E) >= R), kept below 2e-5 by the choice
 // of R (5..13: k = 10 takes 5 to 7, k = 32 up to 13 -- with R capped at 7 a quarter of the queries of a k = 32
 // search over 16384 rows failed their certificate and went to the full-precision scan).  E follows the base size
-// (about sqrt(n / 1000)): the sample pass costs ~ n / E, the re-rank ~ R * E.
+// (sqrt(n / 8000), up to twice that): the sample pass costs ~ n / E, hits and re-rank ~ R * E.  1M x 128, 10,000 queries over
+// bytes, E 32 -> 16: sample and bound 66 -> 110 us, main pass and re-rank 1,539 -> 1,400; 200,003 x 384, 2,049 queries,
+// E 16 -> 8: 34 -> 45 and 330 -> 301.
 static constexpr int SAMPLE_R_MIN = 5, SAMPLE_R_MAX = 13;
 static constexpr int TC_MAX_K = 128;  // results per query: what a warp of the re-rank still keeps sorted cheaply
 
 static int pick_sample_every(size_t n) {
   int e = 8;
-  while (e < 128 && double(e) * double(e) * 2000.0 < double(n)) e <<= 1;  // 1M -> 32, 125k -> 8, 6M -> 64
+  while (e < 128 && double(e) * double(e) * 8000.0 < double(n)) e <<= 1;  // 512k -> 8, 2M -> 16, 8M -> 32
   return e;
 }
 
@@ -429,39 +431,6 @@ struct PassShapes {
   __device__ __forceinline__ bool is8() const { return q8_bad && *q8_bad == 0u; }
   __device__ __forceinline__ const PassShape& taken() const { return is8() ? s8 : s16; }
 };
-
-// A query's bound: the R-th smallest of the group minima the sample pass left (+inf where there are fewer), which that many
-// sampled rows do not exceed.  A warp per query, each lane with the four smallest of its share: where a lane holds more than
-// four of the R smallest the bound is a little looser.  Bound by reading the minima from L2.
-__global__ void __launch_bounds__(256) sample_tau_kernel(const float* __restrict__ smin, int ld, int groups, int nq, int R,
-                                                         float* __restrict__ tau) {
-  const int q = blockIdx.x * int(blockDim.x >> 5) + int(threadIdx.x >> 5), lane = lane_id();
-  if (q >= nq) return;
-  const float* src = smin + size_t(q) * ld;
-  float best[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-#pragma unroll 4
-  for (int i = lane; i < groups; i += 32) {
-    float v = src[i];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float lo = fminf(best[t], v);
-      v = fmaxf(best[t], v);
-      best[t] = lo;
-    }
-  }
-  uint32_t w = 0;
-  for (int i = 0; i < R; ++i) {
-    const uint32_t head = order_bits(best[0]);
-    w = __reduce_min_sync(FV_FULL, head);
-    const int owner = __ffs(__ballot_sync(FV_FULL, head == w)) - 1;
-    if (lane == owner) {
-#pragma unroll
-      for (int t = 0; t < 3; ++t) best[t] = best[t + 1];
-      best[3] = INFINITY;
-    }
-  }
-  if (lane == 0) tau[q] = order_bits_to_float(w);
-}
 
 // Accumulators as the epilogue compares them: scores in fp32, or whole numbers (I8), whose order is the same.
 template <bool I8>
@@ -1160,6 +1129,105 @@ __global__ void init_search_kernel(RangeStats* qst, unsigned int* words) {
 }
 
 // ------------------------------------------------------------------------------------------------
+// A query's bound and the error bound of its scores, by a warp per query.
+//
+// The bound is the R-th smallest of the group minima the sample pass left (+inf where there are fewer), which that many
+// sampled rows do not exceed, plus the error bound: the re-rank's certificate asks for the k-th distance to lie below the
+// bound by that much, and a query that misses it costs a scan of the base (2,049 queries of 200,003 x 384: without it one
+// query in 2,000 did at a sample of 1 in 16, and several at 1 in 8).  Each lane keeps the four smallest of its share: where
+// a lane holds more than four of the R smallest the bound is a little looser.  Bound by reading the minima from L2.
+// With the R best scores of the sample kept in registers by the epilogue, as it was, every chunk of 32 columns had an
+// insertion in some row: 251 us for 31,250 rows x 10,000 queries, 52 and 16 now; 1,000 queries at 100k x 128 38, 12 and 10.
+struct TauParams {
+  const float* smin;
+  int ld, groups, nq, R;
+  const float* queries;    // nq x pd; rows from `real` on are padding
+  int real, pd, Kp, is_l2, bf16;
+  const float* qnorm2;
+  const RangeStats* bst;   // base statistics
+  const RangeStats* qst;   // query statistics
+  const unsigned int* q8_bad;
+  float* tau;
+  float* eps;
+};
+__global__ void __launch_bounds__(256) sample_tau_kernel(TauParams p) {
+  const int q = blockIdx.x * int(blockDim.x >> 5) + int(threadIdx.x >> 5), lane = lane_id();
+  if (q >= p.nq) return;
+  const float* src = p.smin + size_t(q) * p.ld;
+  float best[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+#pragma unroll 4
+  for (int i = lane; i < p.groups; i += 32) {
+    float v = src[i];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float lo = fminf(best[t], v);
+      v = fmaxf(best[t], v);
+      best[t] = lo;
+    }
+  }
+  float eps = 0.f;
+  if (q < p.real && !(p.q8_bad && *p.q8_bad == 0u)) {  // (8-bit scores are exact)
+    const float* query = p.queries + size_t(q) * p.pd;
+    float s = 0.f, qmax = 0.f;
+    bool fin = true;
+    for (int c = lane; c < p.pd; c += 32) {
+      const float x = query[c];
+      s = __fmaf_rn(x, x, s);
+      qmax = fmaxf(qmax, fabsf(x));
+      fin = fin && fabsf(x) <= 3.0e38f;  // false for inf and NaN
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(FV_FULL, s, o);
+      qmax = fmaxf(qmax, __shfl_xor_sync(FV_FULL, qmax, o));
+    }
+    fin = __all_sync(FV_FULL, fin);
+    // exact-arithmetic regime: integer-valued inputs small enough that every product, partial sum and
+    // distance is an integer below 2^24 in both the tensor-core score and the reference's fp32 chain
+    const float lo = fminf(p.bst->min_v, p.qst->min_v), hi = fmaxf(p.bst->max_v, p.qst->max_v);
+    const float mabs = fmaxf(fabsf(lo), fabsf(hi)), range = hi - lo;
+    // the accumulator starts at ||b||^2 <= Kp mabs^2 and then takes the terms -2 q_i b_i: it stays within
+    // [-2 Kp mabs^2, Kp mabs^2 + 2 Kp |lo hi|], the upper end only when the values take both signs
+    const float negprod = (lo < 0.f && hi > 0.f) ? -lo * hi : 0.f;
+    const float kf = float(p.Kp);
+    const bool exact_regime = !p.bst->not_integer && !p.qst->not_integer && !p.bst->not_finite && !p.qst->not_finite &&
+                              mabs <= (p.bf16 ? 256.f : 2048.f) && kf * mabs * mabs <= 8388608.f &&
+                              kf * (mabs * mabs + 2.f * negprod) <= 16777216.f && kf * range * range < 16777216.f;
+    // error bound of a score against the reference distance (minus ||q||^2 for L2) outside that regime
+    const float u16 = p.bf16 ? 0.00390625f : 0.00048828125f;
+    const float qnorm = sqrtf(p.is_l2 ? p.qnorm2[q] : s), bn = sqrtf(p.bst->max_norm2);
+    const float e_dot = (2.f * u16 * (1.f + u16) + kf * 4.7683716e-7f + kf * 1.1920929e-7f) * qnorm * bn +
+                        5.9604645e-8f * sqrtf(kf) * (qnorm + bn);
+    // L2: the norm is added inside the MMA (its split loses < 2^-24 of the largest norm, the accumulation
+    // about 2^-21 per step of a partial sum that now includes it), then the reference chain's own rounding
+    const float e_norm = (kf + 16.f) * 4.7683716e-7f * bn * bn + 1.1920929e-7f * bn * bn;
+    eps = p.is_l2 ? 2.f * e_dot + e_norm + kf * 2.3841858e-7f * (qnorm * qnorm + bn * bn) * 2.f : e_dot;
+    eps = exact_regime ? 0.f : eps * 1.01f + 1e-30f;
+    // The query operand of the GEMM is this row times -2 (L2) or -1 in the 16-bit type.  A component that leaves that
+    // type's range (fp16: 65504) turns every score of the query into +-inf or NaN, so no row is a candidate and the
+    // reasoning of the certificate ("a row that is not a candidate scores above the bound") says nothing: such a query is
+    // never certified and goes to the full-precision scan, which returns the reference's k finite neighbours.
+    const bool in_range = fin && (p.bf16 ? qmax <= 1.0e38f : qmax * (p.is_l2 ? 2.f : 1.f) <= 65504.f);
+    if (!in_range) eps = INFINITY;
+  }
+  uint32_t w = 0;
+  for (int i = 0; i < p.R; ++i) {
+    const uint32_t head = order_bits(best[0]);
+    w = __reduce_min_sync(FV_FULL, head);
+    const int owner = __ffs(__ballot_sync(FV_FULL, head == w)) - 1;
+    if (lane == owner) {
+#pragma unroll
+      for (int t = 0; t < 3; ++t) best[t] = best[t + 1];
+      best[3] = INFINITY;
+    }
+  }
+  if (lane == 0) {
+    const float t = order_bits_to_float(w);
+    p.tau[q] = eps < INFINITY ? __fadd_ru(t, eps) : t;
+    p.eps[q] = eps;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
 // Exact re-rank and certification: one warp per query.
 struct RerankParams {
   const float* tau;       // the bound every candidate was tested against
@@ -1171,9 +1239,8 @@ struct RerankParams {
   const float* rows;      // n x pd fp32
   const float* queries;   // nq x pd fp32
   const float* qnorm2;    // nq (0 for inner product)
-  const RangeStats* bst;  // base statistics
-  const RangeStats* qst;  // query statistics
-  int n, nq, pd, Kp, k, is_l2, bf16;
+  const float* eps;       // nq: error bound of a score
+  int n, nq, pd, k;
   int wpq;                // warps per query: 1, 2, 4 or 8
   uint32_t id_base;
   u64* out_keys;          // nq x k
@@ -1201,53 +1268,11 @@ __global__ void __launch_bounds__(256, KR == 1 ? 3 : 2) rerank_kernel(RerankPara
   top.init(p.k);
   __syncwarp();
 
-  // exact-arithmetic regime: integer-valued inputs small enough that every product, partial sum and
-  // distance is an integer below 2^24 in both the tensor-core score and the reference's fp32 chain
-  const float lo = fminf(p.bst->min_v, p.qst->min_v), hi = fmaxf(p.bst->max_v, p.qst->max_v);
-  const float mabs = fmaxf(fabsf(lo), fabsf(hi)), range = hi - lo;
-  // the accumulator starts at ||b||^2 <= Kp mabs^2 and then takes the terms -2 q_i b_i: it stays within
-  // [-2 Kp mabs^2, Kp mabs^2 + 2 Kp |lo hi|], the upper end only when the values take both signs
-  const float negprod = (lo < 0.f && hi > 0.f) ? -lo * hi : 0.f;
-  const bool exact_regime = !p.bst->not_integer && !p.qst->not_integer && !p.bst->not_finite && !p.qst->not_finite &&
-                            mabs <= (p.bf16 ? 256.f : 2048.f) && float(p.Kp) * mabs * mabs <= 8388608.f &&
-                            float(p.Kp) * (mabs * mabs + 2.f * negprod) <= 16777216.f &&
-                            float(p.Kp) * range * range < 16777216.f;
+  // how far a score can be from the reference distance (minus ||q||^2 for L2): 0 in the exact-arithmetic regime, inf for
+  // a query that cannot be scored
+  const float eps = p.eps[q];
+  const bool exact_regime = eps == 0.f, q_in_range = eps < INFINITY;
   const float qn2 = p.qnorm2[q];
-  // error bound of a score against the reference distance (minus ||q||^2 for L2) outside that regime
-  const float u16 = p.bf16 ? 0.00390625f : 0.00048828125f;
-  const float qn = sqrtf(p.is_l2 ? qn2 : 0.f), bn = sqrtf(p.bst->max_norm2);
-  float eps;
-  // The query operand of the GEMM is this row times -2 (L2) or -1 in the 16-bit type.  A component that leaves that
-  // type's range (fp16: 65504) turns every score of the query into +-inf or NaN, so no row is a candidate and the
-  // reasoning below ("a row that is not a candidate scores above the bound") says nothing: such a query is never
-  // certified here and goes to the full-precision scan, which returns the reference's k finite neighbours.
-  bool q_in_range;
-  {
-    // inner-product case needs the query norm too; it is recomputed here from the staged query
-    float s = 0.f, qmax = 0.f;
-    bool fin = true;
-    for (int c = lane; c < p.pd; c += 32) {
-      s = __fmaf_rn(sq[c], sq[c], s);
-      qmax = fmaxf(qmax, fabsf(sq[c]));
-      fin = fin && fabsf(sq[c]) <= 3.0e38f;  // false for inf and NaN
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      s += __shfl_xor_sync(FV_FULL, s, o);
-      qmax = fmaxf(qmax, __shfl_xor_sync(FV_FULL, qmax, o));
-    }
-    fin = __all_sync(FV_FULL, fin);
-    const float scale = p.is_l2 ? 2.f : 1.f;
-    q_in_range = fin && (p.bf16 ? qmax <= 1.0e38f : qmax * scale <= 65504.f);
-    const float qnorm = p.is_l2 ? qn : sqrtf(s);
-    const float kf = float(p.Kp);
-    const float e_dot = (2.f * u16 * (1.f + u16) + kf * 4.7683716e-7f + kf * 1.1920929e-7f) * qnorm * bn +
-                        5.9604645e-8f * sqrtf(kf) * (qnorm + bn);
-    // L2: the norm is added inside the MMA (its split loses < 2^-24 of the largest norm, the accumulation
-    // about 2^-21 per step of a partial sum that now includes it), then the reference chain's own rounding
-    const float e_norm = (kf + 16.f) * 4.7683716e-7f * bn * bn + 1.1920929e-7f * bn * bn;
-    eps = p.is_l2 ? 2.f * e_dot + e_norm + kf * 2.3841858e-7f * (qnorm * qnorm + bn * bn) * 2.f : e_dot;
-    eps = exact_regime ? 0.f : eps * 1.01f + 1e-30f;
-  }
 
   const bool is8 = IS_L2 && p.shapes.is8();
   const PassShape& sh = p.shapes.taken();
@@ -1934,7 +1959,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   // statistics
   const size_t a16_bytes = (nq_pad * size_t(Kp) * 2 + 255) & ~size_t(255);
   FV_TRY(ctx->scratch[3].reserve(a16_bytes + (tc->i8 ? nq_pad * size_t(tc->Kp8) : 0)));
-  FV_TRY(ctx->scratch[5].reserve(3 * nq_pad * sizeof(float) + nlists * sizeof(unsigned int)));  // (nq_pad is a multiple of 128: the counts are aligned)
+  FV_TRY(ctx->scratch[5].reserve(4 * nq_pad * sizeof(float) + nlists * sizeof(unsigned int)));  // (nq_pad is a multiple of 128: the counts are aligned)
   // Sample pass: the minima of 1, 8, 32 or 64 sampled rows, so that there are hundreds of groups and two of a query's R best
   // seldom share one (their number times R (R - 1) / 2 is what the rank slips by), for at most 512 MB of queries at a time.
   const int group = ns <= 1024 ? 1 : ns <= 16384 ? 8 : ns <= 65536 ? 32 : 64;
@@ -1948,7 +1973,8 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   float* qn2 = ctx->scratch[5].as<float>();
   float* tau = qn2 + nq_pad;
   float* const8 = tau + nq_pad;
-  unsigned int* ccnt = reinterpret_cast<unsigned int*>(const8 + nq_pad);
+  float* eps = const8 + nq_pad;
+  unsigned int* ccnt = reinterpret_cast<unsigned int*>(eps + nq_pad);
   RangeStats* bst = tc->stats.as<RangeStats>();
   RangeStats* qst = bst + 1;
   unsigned int* words = side_words(tc);
@@ -2003,8 +2029,25 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
     }
     FV_TRY(launch_gemm<true>(ctx, ts[0], way[0].sample, ts[1], tc->i8 ? &way[1].sample : nullptr, q8_bad));
     const size_t with_bound = std::min(slice, nq_pad - q0);
-    sample_tau_kernel<<<unsigned((with_bound + 7) / 8), 256, 0, ctx->stream>>>(
-        ctx->scratch[6].as<float>(), int(smin_ld), int((ns + group - 1) / group), int(with_bound), R, tau + q0);
+    TauParams tp{};
+    tp.smin = ctx->scratch[6].as<float>();
+    tp.ld = int(smin_ld);
+    tp.groups = int((ns + group - 1) / group);
+    tp.nq = int(with_bound);
+    tp.R = R;
+    tp.queries = d_queries + q0 * size_t(pd);
+    tp.real = int(nqs);
+    tp.pd = pd;
+    tp.Kp = Kp;
+    tp.is_l2 = is_l2 ? 1 : 0;
+    tp.bf16 = tc->bf16 ? 1 : 0;
+    tp.qnorm2 = qn2 + q0;
+    tp.bst = bst;
+    tp.qst = qst;
+    tp.q8_bad = q8_bad;
+    tp.tau = tau + q0;
+    tp.eps = eps + q0;
+    sample_tau_kernel<<<unsigned((with_bound + 7) / 8), 256, 0, ctx->stream>>>(tp);
     ctx->stats.launches++;
     FV_CUDA(cudaGetLastError());
   }
@@ -2033,15 +2076,11 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   rp.rows = d_rows;
   rp.queries = d_queries;
   rp.qnorm2 = qn2;
-  rp.bst = bst;
-  rp.qst = qst;
+  rp.eps = eps;
   rp.n = int(n);
   rp.nq = int(nq);
   rp.pd = pd;
-  rp.Kp = Kp;
   rp.k = k;
-  rp.is_l2 = metric == FV_L2 ? 1 : 0;
-  rp.bf16 = tc->bf16 ? 1 : 0;
   rp.id_base = id_base;
   rp.out_keys = d_out_keys;
   rp.retry_ids = ctx->scratch[7].as<uint32_t>();
