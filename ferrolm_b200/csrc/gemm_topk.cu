@@ -1525,6 +1525,12 @@ struct TcSide {
   int ext_e = 0;           // the pieces hold ||b||^2 / 2^ext_e
   bool ext_valid = false;
   RangeStats h_stats{};
+  // The maps of the base, the sample and their norm steps, by operand form and by CTAs per tile: made by the first search
+  // that needs them (3 us each; ten of them in every call were a sixth of 1,000 queries at 100k x 128).
+  struct Maps {
+    bool valid = false;
+    CUtensorMap base, sample, base_norm, sample_norm;
+  } maps[2][2];
 };
 
 void tc_free(TcSide* tc) { delete tc; }
@@ -1665,6 +1671,8 @@ int tc_append(fv_ctx* ctx, TcSide** ptc, int metric, const float* d_rows_new, si
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   tc->n = total;
+  for (auto& form : tc->maps)
+    for (TcSide::Maps& m : form) m.valid = false;
   if (metric == FV_L2) {
     // norm pieces: ||b||^2 / 2^e with the largest quotient in (128, 256] when e was chosen, re-split when it outgrows 2^15
     FV_TRY(tc->ext.grow(npad * size_t(EXT_K) * 2, n_old * size_t(EXT_K) * 2, ctx->stream));
@@ -1747,13 +1755,14 @@ static int make_tiling(fv_ctx* ctx, int row_bytes, size_t nq, size_t rows, Tilin
   t->MT = int((nq + rows_per_tile - 1) / rows_per_tile);
   t->NT = int((rows + TILE_N - 1) / TILE_N);
   t->grid = int(std::min<long long>(ctx->sm_count / t->ctas, (long long)t->MT * t->NT));
+  // for a number of waves the most parts that fit are the best: shorter chunks at the same cost of each
   long long best = -1;
-  for (int P = 1; P <= t->NT && P <= 4096; ++P) {
+  const long long units = (long long)t->MT * t->NT;
+  for (long long waves = (t->MT + t->grid - 1) / t->grid; best < 0 || units / t->grid + 3 * waves < best; ++waves) {
+    const int P = int(std::max<long long>(1, std::min<long long>(std::min(t->NT, 4096), waves * t->grid / t->MT)));
     const int cpn = (t->NT + P - 1) / P;
     const int parts = (t->NT + cpn - 1) / cpn;
-    const long long chunks = (long long)t->MT * parts;
-    const long long waves = (chunks + t->grid - 1) / t->grid;
-    const long long cost = waves * (cpn + 3);
+    const long long cost = ((long long)t->MT * parts + t->grid - 1) / t->grid * (cpn + 3);
     if (best < 0 || cost < best) {
       best = cost;
       t->cpn = cpn;
@@ -1980,13 +1989,22 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   unsigned int* words = side_words(tc);
   unsigned int* retry_count = words + W_RETRY;
   unsigned int* q8_bad = tc->i8 ? words + W_Q8_BAD : nullptr;
-  const size_t n_pad = (n + TILE_N - 1) / TILE_N * TILE_N, ns_pad = (ns + TILE_N - 1) / TILE_N * TILE_N;
   for (int i = 0; i < ways; ++i) {
     Way& w = way[i];
     const CUtensorMapDataType type = i ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : type16(tc->bf16);
-    const int K = i ? tc->Kp8 : Kp, box = TILE_N / w.tm.ctas;
+    const int K = i ? tc->Kp8 : Kp;
+    TcSide::Maps& maps = tc->maps[i][pairs ? 1 : 0];
+    if (!maps.valid) {
+      const int box = TILE_N / w.tm.ctas;
+      FV_TRY(make_tmap(&maps.base, type, (i ? tc->rows8 : tc->half).p, n, K, box));
+      FV_TRY(make_tmap(&maps.sample, type, (i ? tc->samp8 : tc->samp).p, tc->ns, K, box));  // (a coarser sample: the kernel's n)
+      if (is_l2 && pairs) {
+        FV_TRY(make_norm_tmap(&maps.base_norm, (i ? tc->ext8 : tc->ext).p, (n + TILE_N - 1) / TILE_N * TILE_N));
+        FV_TRY(make_norm_tmap(&maps.sample_norm, (i ? tc->samp_ext8 : tc->samp_ext).p, (tc->ns + TILE_N - 1) / TILE_N * TILE_N));
+      }
+      maps.valid = true;
+    }
     FV_TRY(make_tmap(&w.main.tmA, type, i ? static_cast<void*>(dA8) : dA, nq_pad, K, 128));
-    FV_TRY(make_tmap(&w.main.tmB, type, (i ? tc->rows8 : tc->half).p, n, K, box));
     GemmParams& g = w.main.p;
     g = GemmParams{};
     g.has_ext = is_l2 ? 1 : 0;
@@ -1994,13 +2012,12 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
     g.idesc = i ? make_idesc_i8(128 * w.tm.ctas, TILE_N) : make_idesc(128 * w.tm.ctas, TILE_N, tc->bf16);
     g.err = tc_error_word(tc);
     w.sample = w.main;
-    FV_TRY(make_tmap(&w.sample.tmB, type, (i ? tc->samp8 : tc->samp).p, ns, K, box));
-    if (is_l2) {
-      g.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
-      w.sample.p.ext = (i ? tc->samp_ext8 : tc->samp_ext).as<uint16_t>();
-      FV_TRY(make_norm_tmap(&w.main.tmE, (i ? tc->ext8 : tc->ext).p, n_pad));
-      FV_TRY(make_norm_tmap(&w.sample.tmE, (i ? tc->samp_ext8 : tc->samp_ext).p, ns_pad));
-    }
+    w.main.tmB = maps.base;
+    w.main.tmE = maps.base_norm;
+    w.sample.tmB = maps.sample;
+    w.sample.tmE = maps.sample_norm;
+    g.ext = (i ? tc->ext8 : tc->ext).as<uint16_t>();
+    w.sample.p.ext = (i ? tc->samp_ext8 : tc->samp_ext).as<uint16_t>();
   }
 
   init_search_kernel<<<1, 1, 0, ctx->stream>>>(qst, words);
