@@ -36,8 +36,8 @@ struct HnswDev {
 // their distances, the team's job, and the beam where it is not in registers.
 static constexpr int SEARCH_BLOCKS_PER_SM = 3;  // of 256 threads
 template <int R>
-__host__ __device__ __forceinline__ size_t search_smem(int pd, int ef, int sbits) {
-  return size_t(pd) * 4 + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + sizeof(TeamJob) +
+__host__ __device__ __forceinline__ size_t search_smem(int pd, int m0, int ef, int sbits, bool team) {
+  return size_t(pd) * 4 + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + (team ? team_smem(m0) : 0) +
          (R == 0 ? ((size_t(ef) * 8 + 15) & ~size_t(15)) : 0);
 }
 
@@ -50,27 +50,27 @@ __host__ __device__ __forceinline__ size_t search_smem(int pd, int ef, int sbits
 // overflow[] and left for a re-run).  NW = 1: one warp per query, blockDim / 32 queries per block; NW > 1: a query
 // per block (Team in hnsw.cuh).
 template <bool IS_L2, int R, int NW>
-__global__ void __launch_bounds__(256, SEARCH_BLOCKS_PER_SM)
+__global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
     hnsw_search_kernel(HnswDev g, const float* __restrict__ queries, const uint32_t* __restrict__ qids, size_t nq, int k,
                        int ef, int sbits, int log2slots, uint32_t* __restrict__ tables, fv_neighbor* __restrict__ out,
                        uint32_t* __restrict__ counts, uint32_t* __restrict__ overflow,
                        unsigned long long* __restrict__ work, unsigned int* __restrict__ next_query) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int searcher = NW == 1 ? w : 0, per_block = NW == 1 ? int(blockDim.x >> 5) : 1;
-  unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, ef, sbits);
+  unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, g.m0, ef, sbits, NW > 1);
   float* sq = reinterpret_cast<float*>(mine);
   uint32_t* small = reinterpret_cast<uint32_t*>(sq + g.pd);
   uint32_t* tied = small + visit_smem(sbits) / 4;
+  const size_t gw = size_t(blockIdx.x) * per_block + searcher;
+  VisitSet seen;
+  visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
   Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + 32),
-                reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64)};
-  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + sizeof(TeamJob));
+                reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64), slot_links(g.m0), uint32_t(g.n), seen, 0u};
+  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + (NW > 1 ? team_smem(g.m0) : 0));
   if (NW > 1 && w > 0) {
     team_serve<IS_L2, NW>(team);
     return;
   }
-  const size_t gw = size_t(blockIdx.x) * per_block + searcher;
-  VisitSet seen;
-  visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
   unsigned long long n_dist = 0, n_exp = 0, n_tie_lost = 0, n_over = 0;
   auto upper = [&](uint32_t x, int layer) {
     size_t p = g.upper_off[x];
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256, SEARCH_BLOCKS_PER_SM)
     best.insert(beam_key(curd, cur));
     visit_warp(seen, lane == 0, cur);
     bool over = false, tie_lost = false;
-    beam_search<IS_L2, R, NW>(team, g.n, layer0, g.m0, sq, best, tied, seen, over, tie_lost, n_dist, n_exp);
+    beam_search<IS_L2, R, NW>(team, g.n, layer0, g.m0, sq, best, tied, seen, over, tie_lost, n_dist, n_exp, g.links0);
     if (tie_lost && !over) n_tie_lost += 1;
     if (lane == 0) overflow[qi] = over ? 1 : 0;
     if (over) {
@@ -384,13 +384,13 @@ static SearchKernel pick_search(bool is_l2, int R) {
 static int search_shape(fv_ctx* ctx, bool is_l2, size_t n, int pd, int m0, int ef, size_t active, SearchShape* s) {
   const int R = ef <= 32 ? 1 : ef <= 64 ? 2 : ef <= 128 ? 4 : ef <= 256 ? 8 : 0;
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
-  const bool team = active <= size_t(ctx->sm_count) * team_searches_per_sm(pd, m0, ef);
+  const bool team = active <= size_t(ctx->sm_count) * team_searches_per_sm(pd, m0, ef), scouts = team && scouts_pay(ctx->sm_count, m0, ef, active);
   s->sbits = team ? visit_sbits(ef) : visit_sbits_single(n, ef);
-  size_t per = R == 0 ? search_smem<0>(pd, ef, s->sbits) : search_smem<1>(pd, ef, s->sbits);
+  size_t per = R == 0 ? search_smem<0>(pd, m0, ef, s->sbits, team) : search_smem<1>(pd, m0, ef, s->sbits, team);
   int W = 8;
   if (team) {
     s->searchers = 1;
-    s->threads = TEAM_WARPS * 32;
+    s->threads = (scouts ? SCOUT_WARPS : TEAM_WARPS) * 32;
     while (s->sbits > 7 && per > budget) {
       per -= size_t(2) << s->sbits;
       s->sbits--;
@@ -402,10 +402,10 @@ static int search_shape(fv_ctx* ctx, bool is_l2, size_t n, int pd, int m0, int e
   }
   s->smem = per * s->searchers;
   if (s->smem > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "dimension and ef too large for shared memory");
-  const size_t by_warps = 8 * SEARCH_BLOCKS_PER_SM / (s->threads / 32);
+  const size_t by_warps = scouts ? team_blocks(SCOUT_WARPS) : 8 * SEARCH_BLOCKS_PER_SM / (s->threads / 32);
   const size_t per_sm = std::max<size_t>(1, std::min(size_t(227 * 1024) / (s->smem + 1024), by_warps));
   s->blocks = std::min<size_t>((active + s->searchers - 1) / s->searchers, size_t(ctx->sm_count) * per_sm);
-  s->kern = team ? pick_search<TEAM_WARPS>(is_l2, R) : pick_search<1>(is_l2, R);
+  s->kern = scouts ? pick_search<SCOUT_WARPS>(is_l2, R) : team ? pick_search<TEAM_WARPS>(is_l2, R) : pick_search<1>(is_l2, R);
   FV_TRY(allow_smem(ctx, s->kern, s->smem));
   return FV_OK;
 }

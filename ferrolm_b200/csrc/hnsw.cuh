@@ -50,6 +50,17 @@ static constexpr int TIED_CAP = 64;
 // 11 at 32 and 64, 6 to 10, 4 to 8; of 128 and more 10 to 20, 11 to 15, 7 to 9 (with m = 24 and 200 dimensions 7 and 5 from
 // ef 100 on); with the beam in shared memory (ef 400 and 1,000) 2 to 4 at any dimension.
 static constexpr int TEAM_WARPS = 8;
+// Up to two searches per SM run by scouting teams: a warp with the beam and eight that work out the links and distances of
+// the node that is next in line while the first is still busy with the one before.  80 to 93 % of the expansions find theirs
+// done or under way; what is left of one is mostly the first warp's own part (1,900 cycles of 2,200 at 96 dimensions and 200
+// entries).  us with teams of eight and with scouts, 20 queries: 5,183 x 384, ef 64 203 and 176, ef 200 526 and 387; 100,000
+// x 128 154 and 141, 333 and 268; 20,000 x 200 with m = 24 248 and 161, 659 and 361.  Not with the beam in shared memory (100,000
+// x 128, ef 400: 1,090 and 1,216).  Construction, 20,000 x 96: 122 ms of kernels and 106.
+static constexpr int SCOUT_WARPS = 9;
+static constexpr int SCOUT_LINKS = 64;  // links of a node, at most
+static inline bool scouts_pay(int sm_count, int m0, int ef, size_t searches) {
+  return m0 <= SCOUT_LINKS && ef <= 256 && searches <= size_t(sm_count) * 2;
+}
 static inline size_t team_searches_per_sm(int pd, int m0, int ef) {
   static constexpr size_t most[5][3] = {{6, 14, 16}, {6, 10, 16}, {6, 8, 14}, {3, 6, 8}, {2, 2, 2}};
   const size_t line = most[ef <= 16 ? 0 : ef <= 64 ? 1 : ef <= 160 ? 2 : ef <= 256 ? 3 : 4][pd < 64 ? 0 : pd < 128 ? 1 : 2];
@@ -198,6 +209,13 @@ __device__ __forceinline__ bool visit_warp(VisitSet& v, bool on, uint32_t x) {
   }
   return fresh;
 }
+// whether x was in its home bucket a moment ago (it stays then); anyone may ask while the set's warp adds to it
+__device__ __forceinline__ bool visit_seen(const VisitSet& v, uint32_t x) {
+  if (v.sbits < 0 || v.probes <= 0) return false;
+  const uint32_t h = (x * 0x9E3779B1u) & v.idmask, rem = h & ((1u << v.rb) - 1u);
+  const uint32_t w = *reinterpret_cast<volatile uint32_t*>(v.small + (h >> v.rb));
+  return (w & 0xFFFFu) == rem || (w >> 16) == rem;
+}
 __device__ __forceinline__ bool visit_overflow(const VisitSet& v) { return v.in_big > (1 << (v.log2slots - 1)); }
 
 // ---- the beam: the ef nearest entries seen so far, ascending, each with its "expanded" bit.
@@ -215,13 +233,13 @@ struct Beam {
     for (int r = 0; r < R; ++r) e[r] = r * 32 + lane_id() < off ? 1ull : FV_EMPTY_KEY;
   }
   __device__ __forceinline__ u64 last() const { return __shfl_sync(FV_FULL, e[R - 1], 31); }
-  __device__ __forceinline__ int last_pos() const { return 32 * R - 1; }
   __device__ __forceinline__ void insert(u64 key) {  // key < last()
 #pragma unroll
     for (int r = R - 1; r >= 0; --r) {
-      u64 prev = __shfl_up_sync(FV_FULL, e[r], 1);
-      const u64 carry = r > 0 ? __shfl_sync(FV_FULL, e[r > 0 ? r - 1 : 0], 31) : 0ull;
-      if (lane_id() == 0) prev = carry;
+      // the entry one place before: lane 31 passes on its entry of the row below, which lane 0 is the one to read
+      const u64 own = e[r], below = e[r > 0 ? r - 1 : 0];
+      u64 prev = __shfl_sync(FV_FULL, lane_id() == 31 ? below : own, (lane_id() + 31) & 31);
+      if (r == 0 && lane_id() == 0) prev = 0;
       if (!(e[r] < key)) e[r] = prev < key ? key : prev;
     }
   }
@@ -244,23 +262,22 @@ struct Beam {
     bound = now;
     pending = 0;
   }
-  // the first entry that is not expanded: its position (-1: none) and key
-  __device__ __forceinline__ int first_open(u64& key) const {
-    int pos = -1;
-    u64 v = 0;
+  // the first entry that is not expanded (FV_EMPTY_KEY: none); marking one
+  __device__ __forceinline__ u64 first_open() const {
+    unsigned pos = 0x7FFFFFFFu;
+    u64 v = FV_EMPTY_KEY;
 #pragma unroll
-    for (int r = R - 1; r >= 0; --r) {
-      const unsigned mk = __ballot_sync(FV_FULL, !(e[r] & 1ull));
-      pos = mk ? r * 32 + __ffs(mk) - 1 : pos;
-      v = mk ? e[r] : v;
-    }
-    key = __shfl_sync(FV_FULL, v, pos & 31);
-    return pos;
+    for (int r = R - 1; r >= 0; --r)
+      if (!(e[r] & 1ull)) {
+        pos = unsigned(r * 32 + lane_id());
+        v = e[r];
+      }
+    return __shfl_sync(FV_FULL, v, int(__reduce_min_sync(FV_FULL, pos) & 31));  // (none: any lane's)
   }
-  __device__ __forceinline__ void mark(int pos) {
+  __device__ __forceinline__ void mark(u64 key) {
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (pos == r * 32 + lane_id()) e[r] |= 1ull;
+      if (e[r] == key) e[r] |= 1ull;
   }
   __device__ __forceinline__ int filled() const {
     int c = 0;
@@ -299,7 +316,6 @@ struct Beam<0> {
     warp_list_init(e, ef);
   }
   __device__ __forceinline__ u64 last() const { return e[ef - 1]; }
-  __device__ __forceinline__ int last_pos() const { return ef - 1; }
   __device__ __forceinline__ void insert(u64 key) {
     int below = 0;
     for (int e0 = 0; e0 < n; e0 += 32) {
@@ -313,21 +329,22 @@ struct Beam<0> {
     if (below < cursor) cursor = below;
   }
   __device__ __forceinline__ void take(unsigned&, u64, u64&, int&) {}
-  __device__ __forceinline__ int first_open(u64& key) const {
+  __device__ __forceinline__ u64 first_open() {  // (the cursor comes to stand on it)
     for (int e0 = cursor & ~31; e0 < n; e0 += 32) {
       const int i = e0 + lane_id();
       const unsigned mk = __ballot_sync(FV_FULL, i >= cursor && i < n && !(e[i] & 1ull));
       if (mk) {
-        key = e[e0 + __ffs(mk) - 1];
-        return e0 + __ffs(mk) - 1;
+        cursor = e0 + __ffs(mk) - 1;
+        return e[cursor];
       }
     }
-    return -1;
+    cursor = n;
+    return FV_EMPTY_KEY;
   }
-  __device__ __forceinline__ void mark(int pos) {
+  __device__ __forceinline__ void mark(u64) {  // the one first_open has just found
     __syncwarp();
-    if (lane_id() == 0) e[pos] |= 1ull;
-    cursor = pos + 1;
+    if (lane_id() == 0) e[cursor] |= 1ull;
+    cursor++;
     __syncwarp();
   }
   __device__ __forceinline__ int filled() const { return n; }
@@ -352,20 +369,61 @@ struct Beam<0> {
 };
 
 // Who computes a run of distances.  NW = 1: the warp itself.  NW > 1: the block's NW warps together; warp 0 runs the
-// search and posts each run (team_eval), the others wait for it in team_serve.  A single search is a chain of memory
-// trips, and when there are fewer searches than warps the rest of the SM can only help by shortening each link.
+// search and posts jobs, the others wait for them in team_serve.  A single search is a chain of memory trips, and when there
+// are fewer searches than warps the rest of the SM can only help by shortening each link.
+// Two kinds of jobs: a run of rows, which warp 0 takes part in (team_eval), and the links of a node with the distances of
+// those that are not visited yet, which the others work out while warp 0 goes on (post_node).  Jobs are done in the order
+// they are posted; two may be under way.
 struct TeamJob {
-  const float* from;  // shared memory: the vector the distances are from
-  int count;          // rows; -1: no more work
+  const float* from;    // shared memory: the vector the distances are from
+  const uint32_t* row;  // a node's link block (count, ids), or null: a run of rows
+  int count;            // rows of the run, or the most links to read; -1: no more work
+  int slot;             // where a node's links go
+  const uint32_t* flat; // link blocks of all nodes, count_max + 1 words each, or null
 };
+static_assert(sizeof(TeamJob) == 32, "");
+static constexpr int NODE_SLOTS = 4;  // nodes whose links and distances are kept
+static constexpr uint32_t NO_LINK = 0xFFFFFFFFu;
+__host__ __device__ __forceinline__ int slot_links(int m0) { return (m0 + 31) & ~31; }
+__host__ __device__ __forceinline__ size_t team_smem(int m0) {  // bytes: the job, the slots
+  return 2 * sizeof(TeamJob) + 2 * (SCOUT_LINKS + 4) * 4 + NODE_SLOTS * (size_t(slot_links(m0)) * 8 + 4);  // a multiple of 16
+}
+// blocks of 256 threads per SM; those of scouting teams have 288
+__host__ __device__ constexpr int team_threads(int nw) { return nw == 1 ? 256 : nw * 32; }
+__host__ __device__ constexpr int team_blocks(int nw) { return nw == SCOUT_WARPS ? 2 : 3; }
 template <int NW>
 struct Team {
+  static constexpr bool SCOUTS = NW == SCOUT_WARPS;
   const float* data;
   int pd;
   uint32_t* ids;  // shared memory: the rows of a run ...
   float* out;     // ... and their distances
-  TeamJob* job;   // NW > 1
+  TeamJob* job;   // NW > 1, like the rest: one for even and one for odd jobs
+  int links;      // slot_links
+  uint32_t n;     // nodes
+  VisitSet seen;  // as it was set up: for visit_seen
+  mutable unsigned posted;  // jobs so far
+  // of an even and an odd job: the places of the new links, their number in front
+  __device__ __forceinline__ uint32_t* fresh(unsigned j) const { return reinterpret_cast<uint32_t*>(job + 2) + (j & 1) * (SCOUT_LINKS + 4); }
+  __device__ __forceinline__ uint32_t* slot_cnt() const { return reinterpret_cast<uint32_t*>(job + 2) + 2 * (SCOUT_LINKS + 4); }
+  __device__ __forceinline__ uint32_t* slot_ids(int s) const { return slot_cnt() + NODE_SLOTS + s * 2 * links; }  // NO_LINK: visited
+  __device__ __forceinline__ float* slot_out(int s) const { return reinterpret_cast<float*>(slot_ids(s) + links); }
 };
+// Named barriers, one for even and one for odd jobs: 1, 2 a job is posted; 3, 4 a node's links are there; 5, 6 it is done;
+// 7 the warps of a job among themselves.
+__device__ __forceinline__ void team_arrive(int bar, int threads) {
+  __syncwarp();
+  asm volatile("fence.acq_rel.cta;" ::: "memory");
+  asm volatile("bar.arrive %0, %1;" ::"r"(bar), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void team_sync(int bar, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory"); }
+template <int NW>
+__device__ __forceinline__ unsigned team_post(const Team<NW>& t, const TeamJob& job) {  // the job's number
+  const unsigned j = t.posted++;
+  if (lane_id() == 0) t.job[j & 1] = job;
+  team_arrive(1 + int(j & 1), NW * 32);
+  return j;
+}
 template <bool IS_L2, int LPR>
 __device__ __forceinline__ void team_rows(const float* __restrict__ data, int pd, const uint32_t* ids, float* out,
                                           const float* from, int count, int first, int step) {
@@ -387,32 +445,68 @@ __device__ __forceinline__ void team_eval(const Team<NW>& t, const float* from, 
     team_rows<IS_L2, 8>(t.data, t.pd, t.ids, t.out, from, count, 0, 4);
     __syncwarp();
   } else {
-    if (lane_id() == 0) {
-      t.job->from = from;
-      t.job->count = count;
-    }
-    __syncthreads();
+    const unsigned j = team_post<NW>(t, TeamJob{from, nullptr, count, 0, nullptr});
     team_rows<IS_L2, 8>(t.data, t.pd, t.ids, t.out, from, count, 0, 4 * NW);
-    __syncthreads();
+    team_sync(5 + int(j & 1), NW * 32);
   }
 }
 template <bool IS_L2, int NW>
 __device__ __forceinline__ void team_serve(const Team<NW>& t) {  // warps 1 .. NW - 1
-  for (;;) {
-    __syncthreads();
-    const int count = t.job->count;
-    if (count < 0) return;
-    team_rows<IS_L2, 8>(t.data, t.pd, t.ids, t.out, t.job->from, count, 4 * int(threadIdx.x >> 5), 4 * NW);
-    __syncthreads();
+  const int w = int(threadIdx.x >> 5), sub = lane_id() & 7, g = lane_id() >> 3;
+  for (unsigned j = 0;; ++j) {
+    const int odd = int(j & 1);
+    team_sync(1 + odd, NW * 32);
+    const TeamJob job = t.job[odd];
+    if (job.count < 0) return;
+    if (!Team<NW>::SCOUTS || !job.row) {
+      team_rows<IS_L2, 8>(t.data, t.pd, t.ids, t.out, job.from, job.count, 4 * w, 4 * NW);
+    } else {
+      uint32_t* ids = t.slot_ids(job.slot);
+      float* out = t.slot_out(job.slot);
+      uint32_t* fresh = t.fresh(j);
+      if (w == 1) {
+        const int lane = lane_id();
+        // (rows of the searched graph are not written while a search runs: the non-coherent path is safe)
+        const uint32_t x0 = lane < job.count ? __ldg(job.row + 1 + lane) : 0u;  // requested together with the count
+        const uint32_t x1 = lane + 32 < job.count ? __ldg(job.row + 33 + lane) : 0u;
+        const int cnt = min(int(__ldg(job.row)), job.count);
+        const bool on0 = lane < cnt && FV_IDX_OK(x0, t.n, 2) && !visit_seen(t.seen, x0);
+        const unsigned mask0 = __ballot_sync(FV_FULL, on0), below = (1u << lane) - 1u;
+        int n = __popc(mask0);
+        ids[lane] = on0 ? x0 : NO_LINK;
+        if (on0) fresh[4 + __popc(mask0 & below)] = uint32_t(lane);
+        if (cnt > 32) {
+          const bool on1 = lane + 32 < cnt && FV_IDX_OK(x1, t.n, 2) && !visit_seen(t.seen, x1);
+          const unsigned mask1 = __ballot_sync(FV_FULL, on1);
+          ids[32 + lane] = on1 ? x1 : NO_LINK;
+          if (on1) fresh[4 + n + __popc(mask1 & below)] = uint32_t(32 + lane);
+          n += __popc(mask1);
+        }
+        if (lane == 0) {
+          t.slot_cnt()[job.slot] = uint32_t(cnt);
+          fresh[0] = uint32_t(n);
+        }
+        team_arrive(3 + odd, 64);
+      }
+      team_sync(7, (NW - 1) * 32);
+      const int n = int(fresh[0]);
+      for (int k0 = 4 * (w - 1); k0 < n; k0 += 4 * (NW - 1)) {
+        const uint32_t at = fresh[4 + min(k0 + g, n - 1)], y = ids[at];  // (rows past the end: the last one again)
+        const float d = group_distance_ahead<IS_L2>(job.from, t.data + size_t(y) * t.pd, t.pd);
+        if (sub == 0) out[at] = d;
+        // its own links, should it be expanded, are brought into L1: one word of each 32 bytes
+        if (job.flat && sub * 8 <= job.count) {
+          uint32_t word;
+          asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(word) : "l"(job.flat + size_t(y) * (job.count + 1) + sub * 8));
+        }
+      }
+    }
+    team_arrive(5 + odd, NW * 32);
   }
 }
 template <int NW>
 __device__ __forceinline__ void team_dismiss(const Team<NW>& t) {
-  if (NW > 1) {
-    __syncwarp();
-    if (lane_id() == 0) t.job->count = -1;
-    __syncthreads();
-  }
+  if (NW > 1) team_post<NW>(t, TeamJob{nullptr, nullptr, -1, 0, nullptr});
 }
 
 // The greedy descent through layers top .. bottom + 1 (hnsw.rs:254-268, :334-347).  `rows(c, layer)` is a node's link
@@ -464,19 +558,50 @@ __device__ __forceinline__ void greedy_descent(const Team<NW>& t, size_t n, Rows
 // trips the stop test (hnsw.rs:203-205) unless its distance ties the current worst exactly -- see TIED_CAP.
 // The unvisited neighbours of the expanded node are offered to the list in stored order, so the admission test
 // (hnsw.rs:214) sees the same evolving bound as the sequential loop.  A search that fills more than half of the
-// visited set's part in global memory stops with `over`.  n_dist and n_exp grow by the distances evaluated and the nodes
+// visited set's part in global memory stops with `over`.  `flat`: where the link blocks of all nodes lie one behind the other,
+// width + 1 words each, if they do.  n_dist and n_exp grow by the distances evaluated and the nodes
 // expanded.
 template <bool IS_L2, int R, int NW, class Rows>
 __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows rows, int width, const float* sq, Beam<R>& best,
                                             uint32_t* tied, VisitSet& seen, bool& over, bool& tie_lost,
-                                            unsigned long long& n_dist, unsigned long long& n_exp) {
+                                            unsigned long long& n_dist, unsigned long long& n_exp,
+                                            const uint32_t* flat = nullptr) {
   const int lane = lane_id();
   int ntied = 0;  // pushed-out entries still tied with the worst kept distance
   over = false;
+  // scouting teams: the nodes whose links are in the slots (lane s: slot s); the slots of the jobs under way (the older
+  // first, -1: none), whether the links of the older have been waited for, and its number; the next slot to take
+  uint32_t kept = NO_LINK;
+  int busy0 = -1, busy1 = -1, next_slot = 0;
+  bool links_here = false;
+  unsigned oldest = t.posted;
+  auto links_done = [&]() {  // of the older job
+    if (!links_here) team_sync(3 + int(oldest & 1), 64);
+    links_here = true;
+  };
+  auto job_done = [&]() {
+    links_done();
+    team_sync(5 + int(oldest & 1), NW * 32);
+    busy0 = busy1;
+    busy1 = -1;
+    links_here = false;
+    ++oldest;
+  };
+  auto ask = [&](uint32_t node, int current) {  // returns the slot; one job at most is under way
+    while (next_slot == current || next_slot == busy0) next_slot = (next_slot + 1) & (NODE_SLOTS - 1);
+    const int slot = next_slot;
+    next_slot = (slot + 1) & (NODE_SLOTS - 1);
+    if (lane == slot) kept = node;
+    team_post<NW>(t, TeamJob{sq, rows(node), width, slot, flat});
+    (busy0 < 0 ? busy0 : busy1) = slot;
+    return slot;
+  };
   u64 bound = best.last();
+  constexpr bool CARRY = R > 0 && Team<NW>::SCOUTS;  // (the other forms have no registers for it, or a cursor)
+  u64 next = best.first_open();  // the nearest entry that is not expanded
   for (;;) {
-    u64 ck = 0;
-    int pos = best.first_open(ck);
+    const u64 ck = next;
+    bool in_beam = ck != FV_EMPTY_KEY;
     uint32_t c = beam_id(ck);
     if (ntied > 0) {
       // the smallest id among the tied entries; it goes first if the beam has nothing open or only a larger key
@@ -484,53 +609,88 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
       for (int i = lane; i < ntied; i += 32) tmin = min(tmin, tied[i]);
       tmin = __reduce_min_sync(FV_FULL, tmin);
       const u64 tkey = (bound & 0xFFFFFFFF00000000ull) | (u64(tmin) << 1);
-      if (pos < 0 || tkey < ck) {
+      if (!in_beam || tkey < ck) {
         __syncwarp();
         for (int i = lane; i < ntied; i += 32)
           if (tied[i] == tmin) tied[i] = tied[ntied - 1];  // ids are unique: one match
         __syncwarp();
         ntied--;
-        pos = -2;
+        in_beam = false;
         c = tmin;
+      } else {
+        in_beam = true;
       }
+    } else if (!in_beam) {
+      break;
     }
-    if (pos == -1) break;
-    if (pos >= 0) {
-      best.mark(pos);
-      if (pos == best.last_pos()) bound |= 1ull;
+    if (in_beam) {
+      best.mark(ck);
+      if (ck == bound) bound |= 1ull;
+      if (R > 0) next = best.first_open();
     }
     if (!FV_IDX_OK(c, n, 1)) break;
-    const uint32_t* row = rows(c);
-    // the first 32 links are requested together with the count: one round trip, not two
-    // (rows of the searched graph are not written while a search runs: the non-coherent path is safe)
-    const uint32_t x_first = lane < width ? __ldg(row + 1 + lane) : 0u;
-    const int cnt = min(int(__ldg(row)), width);
     n_exp += 1;
-    if (R > 0) {
-      // the entry that is next in line now is expanded next unless a nearer one is found: its links are on their way
-      // (with the beam in shared memory finding it costs what this saves, and 1 to 3 % more)
-      u64 nk = 0;
-      if (best.first_open(nk) >= 0) {
-        const uint32_t* nrow = rows(beam_id(nk));
+    const uint32_t* row = rows(c);
+    uint32_t x_first = 0;
+    int cnt, slot = 0;
+    if (Team<NW>::SCOUTS) {
+      const unsigned known = __ballot_sync(FV_FULL, kept == c);
+      if (known) {
+        slot = __ffs(known) - 1;
+      } else {
+        if (busy1 >= 0) job_done();
+        slot = ask(c, -1);
+      }
+      // the entry that is next in line now is expanded next unless a nearer one is found
+      if (busy1 < 0 && next != FV_EMPTY_KEY && FV_IDX_OK(beam_id(next), n, 1) && !__any_sync(FV_FULL, kept == beam_id(next)))
+        ask(beam_id(next), slot);
+      if (busy1 == slot) job_done();
+      if (busy0 == slot) links_done();
+      cnt = int(t.slot_cnt()[slot]);
+    } else {
+      // the first 32 links are requested together with the count: one round trip, not two
+      // (rows of the searched graph are not written while a search runs: the non-coherent path is safe)
+      x_first = lane < width ? __ldg(row + 1 + lane) : 0u;
+      cnt = min(int(__ldg(row)), width);
+      if (R > 0 && next != FV_EMPTY_KEY) {
+        // the entry that is next in line now is expanded next unless a nearer one is found: its links are on their way
+        // (with the beam in shared memory finding it costs what this saves, and 1 to 3 % more)
+        const uint32_t* nrow = rows(beam_id(next));
         if (lane * 32 <= width) asm volatile("prefetch.global.L1 [%0];" ::"l"(nrow + min(lane * 32, width)));
       }
     }
     for (int c0 = 0; c0 < cnt; c0 += 32) {
       const int i = c0 + lane;
-      uint32_t x = 0;
-      if (i < cnt) x = c0 == 0 ? x_first : __ldg(row + 1 + i);
-      const bool fresh = visit_warp(seen, i < cnt && FV_IDX_OK(x, n, 2), x);
-      const unsigned fmask = __ballot_sync(FV_FULL, fresh);
-      const int nfresh = __popc(fmask);
-      if (nfresh == 0) continue;
-      n_dist += nfresh;
-      if (fresh) t.ids[__popc(fmask & ((1u << lane) - 1u))] = x;  // stored order
-      team_eval<IS_L2, NW>(t, sq, nfresh);
+      u64 key = FV_EMPTY_KEY;  // a new link's, in the lane of its place
+      if (Team<NW>::SCOUTS) {
+        const uint32_t x = i < cnt ? t.slot_ids(slot)[i] : NO_LINK;
+        const bool fresh = visit_warp(seen, x != NO_LINK, x);
+        n_dist += __popc(__ballot_sync(FV_FULL, fresh));
+        if (busy0 == slot) job_done();
+        if (fresh) key = beam_key(t.slot_out(slot)[i], x);
+      } else {
+        uint32_t x = 0;
+        if (i < cnt) x = c0 == 0 ? x_first : __ldg(row + 1 + i);
+        const bool fresh = visit_warp(seen, i < cnt && FV_IDX_OK(x, n, 2), x);
+        const unsigned fmask = __ballot_sync(FV_FULL, fresh);
+        const int nfresh = __popc(fmask);
+        if (nfresh == 0) continue;
+        n_dist += nfresh;
+        if (fresh) t.ids[__popc(fmask & ((1u << lane) - 1u))] = x;  // stored order
+        team_eval<IS_L2, NW>(t, sq, nfresh);
+        if (lane < nfresh) key = beam_key(t.out[lane], t.ids[lane]);
+        __syncwarp();
+      }
       // offered in stored order: admitted while the list is not full, or on a strictly smaller distance
-      const u64 key = lane < nfresh ? beam_key(t.out[lane], t.ids[lane]) : FV_EMPTY_KEY;
-      __syncwarp();
       const uint32_t hi = uint32_t(key >> 32);
-      unsigned pending = __ballot_sync(FV_FULL, lane < nfresh && hi < uint32_t(bound >> 32));
+      unsigned pending = __ballot_sync(FV_FULL, hi < uint32_t(bound >> 32));
+      // the nearest of them is admitted whatever happens to the others, unless the worst kept distance comes down to its own
+      u64 nearest = FV_EMPTY_KEY;
+      if (CARRY && pending) {
+        const uint32_t near = __reduce_min_sync(FV_FULL, hi);
+        const uint32_t low = __reduce_min_sync(FV_FULL, hi == near ? uint32_t(key) : 0xFFFFFFFFu);
+        nearest = (u64(near) << 32) | low;
+      }
       if (R > 0 && __popc(pending) > (R == 1 ? 8 : R == 2 ? 6 : R == 4 ? 5 : 4))
         best.take(pending, key, bound, ntied);  // (leaves them pending if ties at the cut need the order they came in)
       while (pending) {
@@ -538,7 +698,7 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
         const u64 pushed = bound;  // the entry that falls off the end, if the beam is full
         best.insert(__shfl_sync(FV_FULL, key, src));
         bound = best.last();
-        pending = __ballot_sync(FV_FULL, lane > src && lane < nfresh && hi < uint32_t(bound >> 32));
+        pending = __ballot_sync(FV_FULL, lane > src && hi < uint32_t(bound >> 32));
         // once the worst distance has gone down, nothing pushed out so far can tie with it any more
         const bool lower = uint32_t(bound >> 32) < uint32_t(pushed >> 32);
         ntied = lower ? 0 : ntied;
@@ -553,12 +713,19 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
           }
         }
       }
+      if (CARRY && nearest != FV_EMPTY_KEY) {
+        if (uint32_t(nearest >> 32) == uint32_t(bound >> 32)) next = best.first_open();
+        else next = nearest < next ? nearest : next;
+      }
     }
     if (visit_overflow(seen)) {
       over = true;
       break;
     }
+    if (!CARRY) next = best.first_open();
   }
+  if (Team<NW>::SCOUTS)
+    while (busy0 >= 0) job_done();
   __syncwarp();
 }
 #endif

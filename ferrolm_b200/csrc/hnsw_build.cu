@@ -3,7 +3,7 @@
 //
 // The reference hands nodes out in id order to the pool's threads; what each thread's search sees of the others'
 // half-made links depends on timing.  Here nodes go in in id order in BATCHES:
-//   1. hnsw_insert_kernel, a warp per node of the batch (a team of eight in batches of up to 16 nodes per SM): the
+//   1. hnsw_insert_kernel, a warp per node of the batch (a team of eight or nine in batches of up to 16 nodes per SM): the
 //      greedy descent and the per-layer search_layer of insert() against the graph as it stood when the batch began
 //      (no node of the batch is visible to another), then select() over what was found; the node's own lists are
 //      written and one edge (target, layer, source) per chosen neighbour is pushed on a chain headed at (target, layer);
@@ -124,13 +124,14 @@ __device__ __forceinline__ int select_links(const BuildDev& g, const Team<NW>& t
 // list, a run of rows and their distances, the chosen links, the bits of select_links, the team's job, the found list.
 __host__ __device__ __forceinline__ size_t insert_smem(int pd, int m0, int ef, int sbits) {
   const size_t run = size_t(run_rows(ef));
-  return size_t(pd) * 8 + visit_smem(sbits) + (TIED_CAP + 2 * run + ((m0 + 3) & ~3) + 128) * 4 + sizeof(TeamJob) +
+  return size_t(pd) * 8 + visit_smem(sbits) + (TIED_CAP + 2 * run + ((m0 + 3) & ~3) + 128) * 4 + (sbits >= 0 ? team_smem(m0) : 0) +  // (only teams have a shared part)
+        
          ((size_t(ef) * 8 + 15) & ~size_t(15));
 }
 
 // flags: [0] visited-table overflows, [1] tie lists that overflowed, [2] edges that did not fit
 template <bool IS_L2, int R, int NW>
-__global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
+__global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
     hnsw_insert_kernel(BuildDev g, uint32_t lo, uint32_t hi, uint32_t ep, int top, int ef, int sbits, int log2slots,
                        uint32_t* __restrict__ tables, Edge* __restrict__ edges, uint32_t* __restrict__ edge_cnt,
                        uint32_t* __restrict__ next_node, uint32_t edge_cap, uint32_t* __restrict__ head,
@@ -145,16 +146,16 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
   uint32_t* tied = small + visit_smem(sbits) / 4;
   uint32_t* sel = tied + TIED_CAP + 2 * run;
   uint32_t* gone = sel + ((g.m0 + 3) & ~3);
+  const size_t gw = size_t(blockIdx.x) * per_block + searcher;
+  VisitSet seen;
+  visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
   Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + run),
-                reinterpret_cast<TeamJob*>(gone + 128)};
-  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + sizeof(TeamJob));
+                reinterpret_cast<TeamJob*>(gone + 128), slot_links(g.m0), g.n, seen, 0u};
+  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + (NW > 1 ? team_smem(g.m0) : 0));
   if (NW > 1 && w > 0) {
     team_serve<IS_L2, NW>(team);
     return;
   }
-  const size_t gw = size_t(blockIdx.x) * per_block + searcher;
-  VisitSet seen;
-  visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
 
   // nodes are drawn from a counter: a search takes anything from a few to a few hundred expansions, and which warp
   // inserts which node changes nothing in the result
@@ -187,7 +188,8 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
       best.reopen([&](bool on, uint32_t x) { visit_warp(seen, on, x); });
       bool over = false;
       beam_search<IS_L2, R, NW>(team, g.n, [&](uint32_t c) { return (const uint32_t*)link_row(g, c, layer); },
-                                layer == 0 ? g.m0 : g.m, sq, best, tied, seen, over, tie_lost, n_dist, n_exp);
+                                layer == 0 ? g.m0 : g.m, sq, best, tied, seen, over, tie_lost, n_dist, n_exp,
+                                layer == 0 ? g.links0 : nullptr);
       if (over) {
         if (lane == 0) atomicAdd(flags, 1ull);
         break;
@@ -253,7 +255,7 @@ __global__ void __launch_bounds__(256, BUILD_BLOCKS_PER_SM)
   uint32_t* srcs = sel + cap_max;
   uint32_t* srcs_sorted = srcs + SRC_CAP;
   uint32_t* gone = srcs_sorted + SRC_CAP;
-  const Team<1> team{g.data, g.pd, gone + 8, reinterpret_cast<float*>(gone + 8 + run_rows(nc)), nullptr};
+  const Team<1> team{g.data, g.pd, gone + 8, reinterpret_cast<float*>(gone + 8 + run_rows(nc)), nullptr, 0, g.n, VisitSet{}, 0u};
   const uint32_t count = min(*edge_cnt, edge_cap);
   const uint32_t gw = blockIdx.x * W + w, total_warps = gridDim.x * W;
 
@@ -452,10 +454,12 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
     return fail(FV_ERR_UNSUPPORTED, "dimension and ef_construction too large for shared memory");
   const size_t resident_blocks = size_t(ctx->sm_count) * BUILD_BLOCKS_PER_SM;
   const size_t searchers_max = std::min(resident_blocks * W, std::max<size_t>(widest, 1));  // (a team is one searcher)
-  InsertKernel ins = pick_insert<1>(is_l2, R), ins_team = pick_insert<TEAM_WARPS>(is_l2, R);
+  InsertKernel ins = pick_insert<1>(is_l2, R), ins_team = pick_insert<TEAM_WARPS>(is_l2, R),
+               ins_scouts = pick_insert<SCOUT_WARPS>(is_l2, R);
   auto lnk = is_l2 ? hnsw_link_kernel<true> : hnsw_link_kernel<false>;
   FV_TRY(allow_smem(ctx, ins, ins_warp * W));
   FV_TRY(allow_smem(ctx, ins_team, team_bytes(sbits)));
+  FV_TRY(allow_smem(ctx, ins_scouts, team_bytes(sbits)));
   FV_TRY(allow_smem(ctx, lnk, link_warp * LW));
 
   int log2slots = 11;
@@ -473,8 +477,9 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
     while (inserted < n) {
       const size_t b = next_batch(h->levels, inserted, top, max_batch, divisor);
       FV_CUDA(cudaMemsetAsync(d_edge_cnt, 0, 8, st));  // and the node counter
+      const bool scouts = scouts_pay(ctx->sm_count, int(m0), int(ef), b);
       if (b <= size_t(ctx->sm_count) * TEAM_INSERTS_PER_SM)
-        ins_team<<<unsigned(std::min(b, resident_blocks)), TEAM_WARPS * 32, team_bytes(sbits), st>>>(
+        (scouts ? ins_scouts : ins_team)<<<unsigned(std::min(b, resident_blocks)), (scouts ? SCOUT_WARPS : TEAM_WARPS) * 32, team_bytes(sbits), st>>>(
             g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), sbits, log2slots, d_tables.as<uint32_t>(),
             d_edges.as<Edge>(), d_edge_cnt, d_next_node, uint32_t(edge_cap), d_head.as<uint32_t>(), d_flags);
       else
