@@ -750,7 +750,8 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
           // Threshold mode.  The accumulator IS the score (the norm step and the scaled query side put
           // ||b||^2 - 2<q,b> there), so a chunk of 64 columns costs a minimum tree and one vote.  Every column
           // below the bound is appended to this thread's private list: a plain store and a register counter.
-          auto chunk = [&](const uint32_t* r) {
+          // the runs of eight columns in which some row of the warp has a hit
+          auto runs_with_hits = [&](const uint32_t* r) -> uint32_t {
             T g8[8];
 #pragma unroll
             for (int gi = 0; gi < 8; ++gi) {
@@ -760,11 +761,14 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
               g8[gi] = S::min2(S::min3(t0, t1, S::of(q[6])), S::of(q[7]));
             }
             const T m = S::min2(S::min3(g8[0], g8[1], g8[2]), S::min3(S::min3(g8[3], g8[4], g8[5]), g8[6], g8[7]));
-            if (!__any_sync(FV_FULL, m < w.thr)) return;
-            uint32_t groups = 0;  // the runs of eight columns in which some row of the warp has a hit
+            if (!__any_sync(FV_FULL, m < w.thr)) return 0u;
+            uint32_t runs = 0;
 #pragma unroll
-            for (int gi = 0; gi < 8; ++gi) groups |= g8[gi] < w.thr ? 1u << gi : 0u;
-            groups = __reduce_or_sync(FV_FULL, groups);
+            for (int gi = 0; gi < 8; ++gi) runs |= g8[gi] < w.thr ? 1u << gi : 0u;
+            return __reduce_or_sync(FV_FULL, runs);
+          };
+          auto chunk = [&](const uint32_t* r) {
+            uint32_t groups = runs_with_hits(r);
             // One run at a time: its eight scores are moved to the same registers, so that there is one copy of the code
             // that looks at them (with eight the loop outgrew the instruction cache: 3 times the time at MH = 2).
             while (groups) {
@@ -806,14 +810,21 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
           // as two bit masks, the warp reserves room for all of them with ONE atomic on the CTA's counter, and each
           // thread stores its own.
           auto chunk_tasks = [&](const uint32_t* r) {
-            T m = S::of(r[0]);
-#pragma unroll
-            for (int i = 1; i < 64; ++i) m = S::min2(m, S::of(r[i]));
-            if (!__any_sync(FV_FULL, m < w.thr)) return;
+            const uint32_t runs = runs_with_hits(r);
+            if (!runs) return;
             uint32_t mk[2] = {0u, 0u};
 #pragma unroll
-            for (int i = 0; i < 64; ++i)
-              if (S::of(r[i]) < w.thr && row_base + uint32_t(i) < n_rows) mk[i >> 5] |= 1u << (i & 31);
+            for (int gi = 0; gi < 8; ++gi) {
+              if (!(runs & (1u << gi))) continue;
+#pragma unroll
+              for (int i = gi * 8; i < gi * 8 + 8; ++i)
+                if (S::of(r[i]) < w.thr) mk[i >> 5] |= 1u << (i & 31);
+            }
+            if (row_base + 64u > n_rows) {  // the run ends within these columns
+              const uint32_t left = row_base < n_rows ? n_rows - row_base : 0u;
+              mk[0] &= left >= 32u ? ~0u : (1u << left) - 1u;
+              mk[1] &= left >= 64u ? ~0u : left > 32u ? (1u << (left - 32u)) - 1u : 0u;
+            }
             const int mine = __popc(mk[0]) + __popc(mk[1]);
             int incl = mine;  // inclusive prefix sum over the warp
 #pragma unroll

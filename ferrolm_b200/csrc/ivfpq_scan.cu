@@ -748,27 +748,59 @@ __global__ void pair_kernel(PairArgs a) {
   }
 }
 
-// The same for ALL probed lists of this shard (no row budget), one thread per (query, probe); the counting pass
-// remembers the place its atomic handed out, so the filing pass needs none.  The threads are numbered probe rank
+// The same for ALL probed lists of this shard (no row budget), a (query, probe) per thread and turn; the counting pass
+// remembers the place each pair got, so the filing pass needs no atomics.  The pairs are numbered probe rank
 // first (all queries' nearest cell, then all second nearest, ...), so that a list's pairs come out roughly in order of
 // probe rank: the pairs that will let many rows through (a query meeting one of its nearest lists) sit together in
 // the first operand tiles and warps of a list, and the epilogue warps that hold only far pairs keep to their fast
 // path (with the pairs in query order the tensor-core pass measured 0.51 instead of 0.41 ms).
+// Counting is bound by the atomics on the lists' counters: a block counts PAIRS_PER_BLOCK pairs in shared memory and takes
+// their places with one atomic per list it met (10,000 queries x 64 probes of 1,024 lists, an atomic per pair: 55 us).
+static constexpr int PAIRS_PER_BLOCK = 4096;
 template <bool FILL>
-__global__ void pair_flat_kernel(PairArgs a) {
-  const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  if (i >= a.nq * size_t(a.nprobe)) return;
-  const size_t p = i / a.nq, q = i - p * a.nq;
-  const u64 c = a.cells[q * size_t(a.nprobe) + p];
-  if (c == FV_EMPTY_KEY) return;
-  const uint32_t l = key_id(c);
-  if (a.shard_world > 1 && int(l % uint32_t(a.shard_world)) != a.shard_rank) return;
-  if (!FV_IDX_OK(l, a.nlist, 4)) return;
+__global__ void __launch_bounds__(1024) pair_flat_kernel(PairArgs a, bool in_smem) {
+  uint32_t* count = reinterpret_cast<uint32_t*>(dyn_smem());  // in_smem: a word per list, pairs of this block, then their first place
+  const size_t total = a.nq * size_t(a.nprobe), first = blockIdx.x * size_t(PAIRS_PER_BLOCK);
+  auto list_of = [&](size_t i, u64& c) -> uint32_t {  // 0xFFFFFFFF: none of this shard's
+    if (i >= total) return 0xFFFFFFFFu;
+    const size_t p = i / a.nq, q = i - p * a.nq;
+    c = a.cells[q * size_t(a.nprobe) + p];
+    if (c == FV_EMPTY_KEY) return 0xFFFFFFFFu;
+    const uint32_t l = key_id(c);
+    if (a.shard_world > 1 && int(l % uint32_t(a.shard_world)) != a.shard_rank) return 0xFFFFFFFFu;
+    return FV_IDX_OK(l, a.nlist, 4) ? l : 0xFFFFFFFFu;
+  };
+  u64 c = 0;
   if (FILL) {
-    a.pairs[a.pair_off[l] + a.slot_of[i]] = make_uint2(uint32_t(q), __float_as_uint(key_distance(c)));
-  } else {
-    a.slot_of[i] = atomicAdd(a.pair_cnt + l, 1u);
+#pragma unroll
+    for (int t = 0; t < PAIRS_PER_BLOCK / 1024; ++t) {
+      const size_t i = first + t * 1024 + threadIdx.x;
+      const uint32_t l = list_of(i, c);
+      if (l != 0xFFFFFFFFu) a.pairs[a.pair_off[l] + a.slot_of[i]] = make_uint2(uint32_t(i % a.nq), __float_as_uint(key_distance(c)));
+    }
+    return;
   }
+  uint32_t l[PAIRS_PER_BLOCK / 1024], at[PAIRS_PER_BLOCK / 1024];
+  if (in_smem) {
+    for (uint32_t j = threadIdx.x; j < a.nlist; j += 1024) count[j] = 0;
+    __syncthreads();
+  }
+#pragma unroll
+  for (int t = 0; t < PAIRS_PER_BLOCK / 1024; ++t) {
+    l[t] = list_of(first + t * 1024 + threadIdx.x, c);
+    if (l[t] != 0xFFFFFFFFu) at[t] = atomicAdd((in_smem ? count : a.pair_cnt) + l[t], 1u);
+  }
+  if (in_smem) {
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < a.nlist; j += 1024) {
+      const uint32_t n = count[j];
+      if (n) count[j] = atomicAdd(a.pair_cnt + j, n);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int t = 0; t < PAIRS_PER_BLOCK / 1024; ++t)
+    if (l[t] != 0xFFFFFFFFu) a.slot_of[first + t * 1024 + threadIdx.x] = at[t] + (in_smem ? count[l[t]] : 0u);
 }
 
 // One block: exclusive prefix sums over the lists of the pair counts and of the task counts.
@@ -1873,10 +1905,14 @@ static int bucket_pairs(fv_ctx* ctx, const ScanIndex& ix, const u64* cells, size
   pa.pairs = pairs;
   pa.slot_of = slot_of;
   if (min_rows == 0 && slot_of) {
-    const unsigned fblocks = unsigned((nq * size_t(nprobe) + 255) / 256);
-    pair_flat_kernel<false><<<fblocks, 256, 0, ctx->stream>>>(pa);
+    const unsigned fblocks = unsigned((nq * size_t(nprobe) + PAIRS_PER_BLOCK - 1) / PAIRS_PER_BLOCK);
+    // a block meets as many lists as it has pairs at the most: beyond a few times that clearing its counters is the work
+    const bool in_smem = ix.nlist <= 16384;
+    const size_t csmem = in_smem ? ix.nlist * sizeof(uint32_t) : 0;
+    FV_TRY(allow_smem(ctx, pair_flat_kernel<false>, csmem));
+    pair_flat_kernel<false><<<fblocks, 1024, csmem, ctx->stream>>>(pa, in_smem);
     pair_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(ps.pair_cnt, ix.list_off, ix.nlist, ps.pair_off, ps.task_off, ps.counters);
-    pair_flat_kernel<true><<<fblocks, 256, 0, ctx->stream>>>(pa);
+    pair_flat_kernel<true><<<fblocks, 1024, 0, ctx->stream>>>(pa, false);
   } else {
     const unsigned qblocks = unsigned((nq + 255) / 256);
     pair_kernel<false><<<qblocks, 256, 0, ctx->stream>>>(pa);
