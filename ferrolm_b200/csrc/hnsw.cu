@@ -24,6 +24,8 @@ namespace fv {
 
 struct HnswDev {
   const float* data;
+  const uint8_t* bytes;        // or null (fv_hnsw::d_bytes)
+  float byte_lo;
   const uint32_t* links0;
   const uint32_t* upper_off;   // n + 1 offsets into upper_flat
   const uint32_t* upper_flat;
@@ -37,7 +39,7 @@ struct HnswDev {
 static constexpr int SEARCH_BLOCKS_PER_SM = 3;  // of 256 threads
 template <int R>
 __host__ __device__ __forceinline__ size_t search_smem(int pd, int m0, int ef, int sbits, bool team) {
-  return size_t(pd) * 4 + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + (team ? team_smem(m0) : 0) +
+  return size_t(pd) * 4 + row_bytes(pd) + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + (team ? team_smem(m0) : 0) +
          (R == 0 ? ((size_t(ef) * 8 + 15) & ~size_t(15)) : 0);
 }
 
@@ -59,13 +61,14 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
   const int searcher = NW == 1 ? w : 0, per_block = NW == 1 ? int(blockDim.x >> 5) : 1;
   unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, g.m0, ef, sbits, NW > 1);
   float* sq = reinterpret_cast<float*>(mine);
-  uint32_t* small = reinterpret_cast<uint32_t*>(sq + g.pd);
+  uint8_t* q_bytes = reinterpret_cast<uint8_t*>(sq + g.pd);
+  uint32_t* small = reinterpret_cast<uint32_t*>(q_bytes + row_bytes(g.pd));
   uint32_t* tied = small + visit_smem(sbits) / 4;
   const size_t gw = size_t(blockIdx.x) * per_block + searcher;
   VisitSet seen;
   visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
   Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + 32),
-                reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64), slot_links(g.m0), uint32_t(g.n), seen, 0u};
+                reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64), slot_links(g.m0), uint32_t(g.n), seen, 0u, IS_L2 ? g.bytes : nullptr, -1};
   u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + (NW > 1 ? team_smem(g.m0) : 0));
   if (NW > 1 && w > 0) {
     team_serve<IS_L2, NW>(team);
@@ -88,7 +91,23 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
     if (qi >= nq) break;
     const size_t qsrc = qids ? size_t(qids[qi]) : qi;
     const unsigned long long n_dist0 = n_dist, n_exp0 = n_exp;  // a query that overflows its table is re-run: its work counts once
-    for (int c = lane; c < g.pd; c += 32) sq[c] = queries[qsrc * size_t(g.pd) + c];
+    team.q_norm = -1;
+    if (IS_L2 && g.bytes) {  // the query in bytes too, if it is of the rows' kind
+      bool fits = true;
+      int norm = 0;
+      for (int c = lane; c < row_bytes(g.pd); c += 32) {
+        const float x = c < g.pd ? queries[qsrc * size_t(g.pd) + c] : 0.f, v = c < g.pd ? x - g.byte_lo : 0.f;
+        if (c < g.pd) sq[c] = x;
+        fits = fits && v >= 0.f && v <= 255.f && v == rintf(v);
+        const int u = fits ? int(v) : 0;
+        q_bytes[c] = uint8_t(u);
+        norm += u * u;
+      }
+      norm = __reduce_add_sync(FV_FULL, norm);
+      if (__all_sync(FV_FULL, fits)) team.q_norm = norm;
+    } else {
+      for (int c = lane; c < g.pd; c += 32) sq[c] = queries[qsrc * size_t(g.pd) + c];
+    }
     visit_clear(seen);
 
     // entry point and greedy descent (hnsw.rs:329-347)
@@ -183,6 +202,64 @@ static void flatten_upper(const fv_hnsw* h, std::vector<uint32_t>& off, std::vec
   off[n] = uint32_t(flat.size());
 }
 
+// Smallest and largest value (as order bits), whether all are whole.
+__global__ void value_range_kernel(const float* __restrict__ x, size_t n, uint32_t* __restrict__ words) {
+  uint32_t lo = 0xFFFFFFFFu, hi = 0u;
+  bool whole = true;
+  for (size_t i = (blockIdx.x * size_t(blockDim.x) + threadIdx.x) * 4; i < n; i += size_t(gridDim.x) * blockDim.x * 4) {  // (n is a multiple of 8)
+    const float4 v = *reinterpret_cast<const float4*>(x + i);
+    const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      whole = whole && f[j] == rintf(f[j]) && fabsf(f[j]) <= 65536.f;
+      lo = min(lo, order_bits(f[j]));
+      hi = max(hi, order_bits(f[j]));
+    }
+  }
+  lo = __reduce_min_sync(FV_FULL, lo);
+  hi = __reduce_max_sync(FV_FULL, hi);
+  whole = __all_sync(FV_FULL, whole);
+  if (lane_id() == 0) {
+    atomicMin(words, lo);
+    atomicMax(words + 1, hi);
+    if (!whole) words[2] = 1u;
+  }
+}
+// one warp per row
+__global__ void row_bytes_kernel(const float* __restrict__ x, size_t n, int pd, float lo, uint8_t* __restrict__ out) {
+  const size_t row = blockIdx.x * size_t(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= n) return;
+  for (int c = lane_id(); c < row_bytes(pd); c += 32)
+    out[row * row_bytes(pd) + c] = c < pd ? uint8_t(x[row * size_t(pd) + c] - lo) : uint8_t(0);
+}
+
+// The rows as bytes, where they qualify.  (-0 counts as a whole number: it makes the same distances as 0.)
+static int make_bytes(fv_hnsw* h) {
+  fv_ctx* ctx = h->ctx;
+  h->d_bytes.release();
+  const size_t n = h->n();
+  if (h->metric != FV_L2 || n == 0) return FV_OK;
+  DevBuf words;
+  FV_TRY(words.reserve(16));
+  const uint32_t init[4] = {0xFFFFFFFFu, 0u, 0u, 0u};
+  uint32_t got[4];
+  FV_CUDA(cudaMemcpyAsync(words.p, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
+  value_range_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(h->d_data.as<float>(), n * h->pd, words.as<uint32_t>());
+  FV_CUDA(cudaGetLastError());
+  FV_CUDA(cudaMemcpyAsync(got, words.p, sizeof(got), cudaMemcpyDeviceToHost, ctx->stream));
+  FV_CUDA(cudaStreamSynchronize(ctx->stream));
+  words.release();
+  if (got[2]) return FV_OK;
+  const float lo = order_bits_to_float(got[0]), hi = order_bits_to_float(got[1]);
+  // queries may lie a little beyond the rows' values: bytes above 0 or -128 where those hold all rows
+  h->byte_lo = lo >= 0.f && hi <= 255.f ? 0.f : lo >= -128.f && hi <= 127.f ? -128.f : lo;
+  if (!(hi - h->byte_lo <= 255.f) || double(h->pd) * 255.0 * 255.0 >= 16777216.0) return FV_OK;
+  if (h->d_bytes.reserve(n * size_t(row_bytes(int(h->pd)))) != FV_OK) return FV_OK;  // (no room: the searches do without)
+  row_bytes_kernel<<<unsigned((n + 7) / 8), 256, 0, ctx->stream>>>(h->d_data.as<float>(), n, int(h->pd), h->byte_lo, h->d_bytes.as<uint8_t>());
+  FV_CUDA(cudaGetLastError());
+  return FV_OK;
+}
+
 int upload_graph(fv_hnsw* h, bool with_data) {
   fv_ctx* ctx = h->ctx;
   std::vector<uint32_t> off, flat;
@@ -197,6 +274,7 @@ int upload_graph(fv_hnsw* h, bool with_data) {
   FV_CUDA(cudaMemcpyAsync(h->d_upper_off.p, off.data(), off.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
   if (!flat.empty())
     FV_CUDA(cudaMemcpyAsync(h->d_upper_flat.p, flat.data(), flat.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+  FV_TRY(make_bytes(h));
   FV_CUDA(cudaStreamSynchronize(ctx->stream));
   return FV_OK;
 }
@@ -447,6 +525,8 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   unsigned int* d_next = reinterpret_cast<unsigned int*>(ctx->d_flags + 24);
   HnswDev g{};
   g.data = h->d_data.as<float>();
+  g.bytes = h->d_bytes.as<uint8_t>();
+  g.byte_lo = h->byte_lo;
   g.links0 = h->d_links0.as<uint32_t>();
   g.upper_off = h->d_upper_off.as<uint32_t>();
   g.upper_flat = h->d_upper_flat.as<uint32_t>();
