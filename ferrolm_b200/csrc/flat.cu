@@ -708,18 +708,19 @@ int fv_flat_set_mode(fv_flat* ix, int mode) {
   return FV_OK;
 }
 
-// The one-launch scan against the tensor-core path.  Fitted to calls timed at 5,183 x 384, 100,000 x 128 and 1M x 128
-// (1 to 64 queries, k = 10): the scan takes about 60 us and, for every four queries, the time to read the rows at
-// 5 TB/s; the tensor-core path 130 us and the time to read its 16-bit rows at 2 TB/s.  (100,000 rows: 16 queries 122
-// against 150 us, 64 queries 239 against 151; 1M rows: 4 queries 209 against 269, 8 queries 298 against 272.)  With more
-// than 32 results the scan takes two queries at a time and its merge costs more; so does the other path's re-rank
-// (1 query 287 against 410 us on 1M rows, 2 queries 488 against 409; 100,000 rows: 16 queries 367 against 400).
+// The one-launch scan against the tensor-core path, microseconds of a call.  Fitted to calls timed at 5,183 x 384, 20,000 and
+// 100,000 x 128, 100,000 x 384, 400,000 x 256, 1M x 128 and 4M x 64 (1 to 64 queries, 10, 33 and 100 results): the scan takes
+// about 55 us (one query 40) and, for every four queries, the time to read the rows at 4.8 TB/s; the tensor-core path 85 us and
+// the time to read its rows.  (Scan / tensor cores: 100,000 x 128, 8 queries 82 / 96, 32 queries 132 / 99; 1M x 128, 2 queries
+// 171 / 155, 8 queries 280 / 164; 5,183 x 384, 64 queries 74 / 125.)  With more than 32 results the scan takes two queries at a
+// time and its merge costs more; the other path's re-rank grows with the results (100,000 x 128, 16 queries, 33 results 132 /
+// 100, 100 results 146 / 113; 4 queries 89 / 97 and 91 / 114).
 static bool flat_prefers_few(size_t n, int pd, size_t nq, int L) {
   const double mb = double(n) * pd * 4e-6;
   const size_t qt = nq == 1 ? 1 : (L <= 32 ? 4 : 2);
   const double passes = double((nq + qt - 1) / qt);
-  const double few = (L <= 32 ? 60.0 : (nq == 1 ? 160.0 : 280.0)) + passes * mb / 5.0;
-  const double tc = (L <= 32 ? 130.0 : 370.0) + mb / 4.0;
+  const double few = L <= 32 ? (nq == 1 ? 40.0 + mb / 6.6 : 55.0 + passes * mb / 4.8) : (nq == 1 ? 48.0 + mb / 5.5 : 75.0 + passes * mb / 6.5);
+  const double tc = (L <= 32 ? 85.0 : 95.0 + 0.25 * (L - 32)) + 0.14 * mb;
   return few < tc;
 }
 
