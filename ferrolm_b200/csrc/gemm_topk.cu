@@ -359,7 +359,6 @@ struct GemmParams {
   const uint32_t* ntasks;      // device word: number of tasks
   unsigned int* next_task;     // device word, zero at launch: the next task nobody has taken yet
   u64* pool;                   // [grid][pool_cap] survivors: (A row << 32) | B row relative to y
-  float* pool_score;           // [grid][pool_cap] their scores
   unsigned int* pool_cnt;      // [grid] entries each CTA produced (may exceed pool_cap: overflow)
   unsigned int pool_cap;
   // A survivor that finds its CTA's pool full is dropped, and the owner of its operand row (row_owner[A row], a
@@ -768,35 +767,28 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
             for (int gi = 0; gi < 8; ++gi) runs |= g8[gi] < w.thr ? 1u << gi : 0u;
             return __reduce_or_sync(FV_FULL, runs);
           };
-          // A run's eight scores are moved to the same registers, so that there is one copy of the code that looks at them
-          // (with eight the loop outgrew the instruction cache: 3 times the time at MH = 2).
-          auto move_run = [&](const uint32_t* r, int gi, T* v) {
-            auto run = [&](int k) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) v[i] = S::of(r[k * 8 + i]);
-            };
-            switch (gi) {
-              case 0: run(0); break;
-              case 1: run(1); break;
-              case 2: run(2); break;
-              case 3: run(3); break;
-              case 4: run(4); break;
-              case 5: run(5); break;
-              case 6: run(6); break;
-              default: run(7); break;
-            }
-          };
-          auto of_run = [](const T* v, int i) {
-            const T a = i & 1 ? v[1] : v[0], b = i & 1 ? v[3] : v[2], c = i & 1 ? v[5] : v[4], d = i & 1 ? v[7] : v[6];
-            return i & 4 ? (i & 2 ? d : c) : (i & 2 ? b : a);
-          };
           auto chunk = [&](const uint32_t* r) {
             uint32_t groups = runs_with_hits(r);
+            // One run at a time: its eight scores are moved to the same registers, so that there is one copy of the code
+            // that looks at them (with eight the loop outgrew the instruction cache: 3 times the time at MH = 2).
             while (groups) {
               const int gi = __ffs(groups) - 1;
               groups &= groups - 1;
               T v[8];
-              move_run(r, gi, v);
+              auto run = [&](int k) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = S::of(r[k * 8 + i]);
+              };
+              switch (gi) {
+                case 0: run(0); break;
+                case 1: run(1); break;
+                case 2: run(2); break;
+                case 3: run(3); break;
+                case 4: run(4); break;
+                case 5: run(5); break;
+                case 6: run(6); break;
+                default: run(7); break;
+              }
               const uint32_t row0 = row_base + uint32_t(gi * 8);
               uint32_t hits = 0;
 #pragma unroll
@@ -805,7 +797,9 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
               while (hits) {
                 const int i = __ffs(hits) - 1;
                 hits &= hits - 1;
-                if (w.ncand < unsigned(p.ccap)) w.list[w.ncand] = make_key(float(of_run(v, i)), row0 + uint32_t(i));
+                const T a = i & 1 ? v[1] : v[0], b = i & 1 ? v[3] : v[2], c = i & 1 ? v[5] : v[4], d = i & 1 ? v[7] : v[6];
+                const T x = i & 4 ? (i & 2 ? d : c) : (i & 2 ? b : a);
+                if (w.ncand < unsigned(p.ccap)) w.list[w.ncand] = make_key(float(x), row0 + uint32_t(i));
                 w.ncand++;
               }
               __syncwarp();
@@ -845,24 +839,15 @@ __device__ __forceinline__ void gemm_topk_body(const CUtensorMap& tmA, const CUt
             base = __shfl_sync(FV_FULL, base, 31);
             unsigned int pos = base + unsigned(incl - mine);
             u64* dst = p.pool + size_t(blockIdx.x) * p.pool_cap;
-            float* dst_score = p.pool_score + size_t(blockIdx.x) * p.pool_cap;
-            uint32_t todo = runs;
-            while (todo) {
-              const int gi = __ffs(todo) - 1;
-              todo &= todo - 1;
-              T v[8];
-              move_run(r, gi, v);
-              uint32_t bits = ((gi & 4 ? mk[1] : mk[0]) >> ((gi & 3) * 8)) & 0xFFu;
-              while (bits) {
-                const int i = __ffs(bits) - 1;
-                bits &= bits - 1;
-                if (pos < p.pool_cap) {
-                  dst[pos] = (u64(w.a_row) << 32) | u64(row_base + uint32_t(gi * 8 + i));
-                  dst_score[pos] = float(of_run(v, i));
-                }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t mm = mk[h];
+              while (mm) {
+                const int i = __ffs(mm) - 1;
+                mm &= mm - 1;
+                if (pos < p.pool_cap) dst[pos] = (u64(w.a_row) << 32) | u64(row_base + uint32_t(h * 32 + i));
                 ++pos;
               }
-              __syncwarp();
             }
             if (mine && pos > p.pool_cap) p.owner_dropped[p.row_owner[w.a_row]] = 1u;  // some of this row's did not fit
           };
@@ -1923,7 +1908,6 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
   gp.ntasks = d_ntasks;
   gp.next_task = d_next_task;
   gp.pool = d_pool;
-  gp.pool_score = reinterpret_cast<float*>(d_pool + size_t(ctx->sm_count) * pool_cap);
   gp.pool_cnt = d_pool_cnt;
   gp.pool_cap = pool_cap;
   gp.row_owner = d_row_owner;

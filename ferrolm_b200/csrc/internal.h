@@ -239,8 +239,7 @@ int* tc_error_word(TcSide* tc);
 // Scores the tile_rows (256 or 128) operand rows of every task against its run of side rows: d_tasks[t] = {first operand row, first side
 // row (a multiple of 8), units of 256 side rows, valid side rows}.  Every (operand row, side row) whose score
 // ||b||^2 - 2<a, b> (L2; -<a, b> for inner product, operand rows being pre-scaled) is below d_thr[operand row] goes to
-// the survivor pool as (operand row << 32 | side row relative to the task's first), its score to the float array behind
-// the pool's *grid_out * pool_cap entries: CTA c of *grid_out fills
+// the survivor pool as (operand row << 32 | side row relative to the task's first): CTA c of *grid_out fills
 // d_pool[c * pool_cap ..] and writes its count (which may exceed pool_cap: overflow) to d_pool_cnt[c]; a survivor
 // that does not fit is dropped and d_dropped[d_row_owner[operand row]] set to 1.  The CTAs draw the tasks in table
 // order from the counter *d_next_task (which this call zeroes): sort the table longest first.  Asynchronous.

@@ -1195,128 +1195,6 @@ __global__ void __launch_bounds__(128) tc_bound_select_kernel(const float* __res
   if (lane == 0) tau_bits[q] = lo;
 }
 
-struct RescoreArgs {
-  const u64* pool;
-  const unsigned int* pool_cnt;
-  unsigned int pool_cap;
-  int npools;
-  const uint32_t* g_q;
-  const uint32_t* g_l;
-  const float* g_base;
-  const uint32_t* list_off;
-  const uint8_t* codes;
-  const uint32_t* ids;
-  const float* qtab;
-  const float* pre;  // or null (inner product)
-  int m;
-  const uint32_t* tau_bits;
-  u64* cand;
-  uint32_t* cand_cnt;
-  int cap;
-  const float* pool_score;  // first round: the survivors' scores, and of the gathered rows
-  const float* thr;         // threshold,
-  const float* eps;         // margin,
-  const uint32_t* q_eps;    // largest margin per query (bits)
-  const uint32_t* only;  // second round: only survivors of queries with only[q] != 0 (null: all)
-  const uint32_t* gate;  // second round: the device word that counts its queries; the kernel leaves at once if it is 0
-  size_t a_rows;         // extents (gathered operand rows, lists, rows in all lists), for the checks of the debug build
-  uint32_t nlist, nrows;
-};
-
-// The reference's compressed distance of a survivor (ivfpq.rs:256-262, :272-276), bit for bit, with its id as a key
-// (FV_EMPTY_KEY: not a number below inf).
-__device__ __forceinline__ u64 survivor_key(const RescoreArgs& a, u64 e, uint32_t q) {
-  const uint32_t arow = uint32_t(e >> 32), row = uint32_t(e);
-  const uint32_t l = a.g_l[arow];
-  if (!FV_IDX_OK(l, a.nlist, 6)) return FV_EMPTY_KEY;
-  const size_t r = size_t(a.list_off[l]) + row;
-  if (!FV_IDX_OK(r, a.nrows, 7)) return FV_EMPTY_KEY;
-  const size_t tab = size_t(a.m) * KSUB;
-  const uint8_t* code = a.codes + r * a.m;
-  const float* qt = a.qtab + size_t(q) * tab;
-  const float* pt = a.pre ? a.pre + size_t(l) * tab : nullptr;
-  float d = a.g_base[arow];
-  if (a.m == 16) {  // all 32 table reads in flight before the chain of additions starts
-    const uint4 cw = *reinterpret_cast<const uint4*>(code);
-    const uint32_t cws[4] = {cw.x, cw.y, cw.z, cw.w};
-    float t[16], pv[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int cj = int((cws[j >> 2] >> ((j & 3) * 8)) & 0xFFu);
-      t[j] = __ldg(qt + j * 256 + cj);
-      pv[j] = pt ? __ldg(pt + j * 256 + cj) : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) d = __fadd_rn(d, pt ? __fadd_rn(pv[j], t[j]) : t[j]);
-  } else {
-    for (int j = 0; j < a.m; ++j) {
-      const int cj = code[j];
-      float t = __ldg(qt + j * 256 + cj);
-      if (pt) t = __fadd_rn(__ldg(pt + j * 256 + cj), t);
-      d = __fadd_rn(d, t);
-    }
-  }
-  return d < INFINITY ? make_key(d, __ldg(a.ids + r)) : FV_EMPTY_KEY;
-}
-
-// One thread per survivor, in two forms.
-// FILE (first round): the survivor's place in the pools goes to its query's buffer, under an upper bound of its compressed
-// distance less the query's bound: score - threshold + 2 eps (the margin of tc_gather_kernel).  The finishing kernel works
-// the distance out for those that can be among the best `keep` only, about a third (10,000 queries, keep 100: 320 survivors
-// per query; with every one worked out here, as it was, this kernel took 320 us for its 32 scattered table reads each).
-// Otherwise (second round): the compressed distance itself, kept if at or below the query's bound.
-// The pools are very unequal (a CTA that drew the lists of a dense region holds several times the average), so the
-// blocks split the concatenation of all pools evenly instead of a pool each.
-template <bool FILE>
-__global__ void __launch_bounds__(128) rescore_kernel(RescoreArgs a) {
-  if (a.gate && *a.gate == 0) return;
-  uint32_t* start = reinterpret_cast<uint32_t*>(dyn_smem());  // npools + 1: first global index of every pool
-  if (threadIdx.x < 32) {  // prefix sums of the pools' counts
-    uint32_t s = 0;
-    for (int c0 = 0; c0 < a.npools; c0 += 32) {
-      const int c = c0 + lane_id();
-      const uint32_t v = c < a.npools ? min(a.pool_cnt[c], a.pool_cap) : 0u;
-      uint32_t incl = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(FV_FULL, incl, o);
-        if (lane_id() >= o) incl += t;
-      }
-      if (c < a.npools) start[c] = s + incl - v;
-      s += __shfl_sync(FV_FULL, incl, 31);
-    }
-    if (threadIdx.x == 0) start[a.npools] = s;
-  }
-  __syncthreads();
-  const uint32_t total = start[a.npools];
-  const uint32_t per = ((total + gridDim.x - 1) / gridDim.x + 127u) & ~127u;
-  const uint32_t i0 = min(total, blockIdx.x * per), i1 = min(total, i0 + per);
-  for (uint32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-    int lo = 0, hi = a.npools - 1;  // the pool holding global index i: the last one starting at or before it
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (start[mid] <= i) lo = mid;
-      else hi = mid - 1;
-    }
-    const size_t at = size_t(lo) * a.pool_cap + (i - start[lo]);
-    const u64 e = a.pool[at];
-    const uint32_t arow = uint32_t(e >> 32);
-    if (!FV_IDX_OK(arow, a.a_rows, 5)) continue;
-    const uint32_t q = a.g_q[arow];
-    u64 key;
-    if (FILE) {
-      const float over = __fadd_ru(__fsub_ru(a.pool_score[at], a.thr[arow]), 2.f * a.eps[arow]);
-      key = make_key(over, uint32_t(at));
-    } else {
-      if (a.only && !a.only[q]) continue;
-      key = survivor_key(a, e, q);
-      if (key == FV_EMPTY_KEY || uint32_t(key >> 32) > a.tau_bits[q]) continue;
-    }
-    const uint32_t slot = atomicAdd(a.cand_cnt + q, 1u);
-    if (slot < uint32_t(a.cap)) a.cand[size_t(q) * a.cap + slot] = key;
-  }
-}
-
 struct FinishArgs {
   const u64* cand;
   uint32_t* cand_cnt;
@@ -1337,21 +1215,13 @@ struct FinishArgs {
   uint32_t* over_ids;
   uint32_t* rerun_ids;
   const uint32_t* dropped;  // or null; dropped[q] != 0: the scan lost survivors of q (a full pool): to rerun_ids
-  // The buffers hold places in the survivor pools under upper bounds (rescore_kernel<true>), not keys: the keep-th of them
-  // bounds the keep-th best distance, and whatever lies within twice the query's largest margin above that is worked out.
-  int filed;
 };
-// the word up to which filed survivors can be among the best, when the keep-th of their upper bounds is `word`
-__device__ __forceinline__ uint32_t filed_cut(uint32_t word, float eps) {
-  const float t = order_bits_to_float(word);
-  return t < INFINITY ? order_bits(__fadd_ru(t, 2.f * eps)) : 0xFFFFFFFFu;
-}
 
 // One block per query: the best `keep` of the appended candidates, then the common tail.  With f.qids the blocks
 // walk that list (*f.nqids entries: a count only the device knows when the kernel is launched) instead of taking
 // query blockIdx.x.
-__device__ __forceinline__ void finish_block_query(const ScanArgs& a, const FinishArgs& f, const RescoreArgs& s, size_t q, u64* lists,
-                                                   u64* rerank, float* sq) {
+__device__ __forceinline__ void finish_block_query(const ScanArgs& a, const FinishArgs& f, size_t q, u64* lists, u64* rerank,
+                                                   float* sq) {
   const int tid = threadIdx.x;
   const uint32_t cnt = f.cand_cnt[q];
   if (cnt == 0xFFFFFFFFu || (cnt > uint32_t(f.cap) && !f.tighten) || (f.dropped && f.dropped[q])) {
@@ -1367,30 +1237,12 @@ __device__ __forceinline__ void finish_block_query(const ScanArgs& a, const Fini
   block_sort(lists, n);
   if (cnt > uint32_t(f.cap)) {  // ran over: a tighter bound from what was stored, and a second round
     if (tid == 0) {
-      const uint32_t kth = uint32_t(lists[a.keep - 1] >> 32);  // cap >= keep entries are stored
-      if (!f.filed) {
-        f.tau_bits[q] = kth;
-      } else {  // an upper bound less the query's bound, which it may tighten (not where fewer than `keep` were stored)
-        const float tau = order_bits_to_float(f.tau_bits[q]);
-        const float tighter = kth < 0xFF800000u ? __fadd_ru(tau, order_bits_to_float(kth)) : tau;
-        if (tighter < tau) f.tau_bits[q] = order_bits(tighter);
-      }
+      f.tau_bits[q] = uint32_t(lists[a.keep - 1] >> 32);  // cap >= keep entries are stored
       f.cand_cnt[q] = 0;
       f.redo[q] = 1;
       f.over_ids[atomicAdd(f.counters + LS_C_OVER, 1u)] = uint32_t(q);
     }
     return;
-  }
-  if (f.filed) {
-    const uint32_t cut = have > a.keep ? filed_cut(uint32_t(lists[a.keep - 1] >> 32), __uint_as_float(s.q_eps[q])) : 0xFFFFFFFFu;
-    __syncthreads();
-    for (int e = tid; e < n; e += blockDim.x) {
-      const u64 c = lists[e];
-      const bool in = e < have && uint32_t(c >> 32) <= cut;
-      lists[e] = in ? survivor_key(s, s.pool[uint32_t(c)], uint32_t(q)) : FV_EMPTY_KEY;
-    }
-    __syncthreads();
-    block_sort(lists, n);
   }
   scan_tail(a, q, lists, rerank, sq);
 }
@@ -1402,42 +1254,38 @@ __device__ __forceinline__ void finish_block_query(const ScanArgs& a, const Fini
 // Bound by those reads, 512 bytes at random.  10,000 queries, 100 candidates re-ranked at 128 dimensions: 113 us (the
 // block kernel, whose sort alone is 36 to 45 passes over shared memory: 325).
 static constexpr int FW_NPL = 16;
-__host__ __device__ __forceinline__ size_t finish_warp_words(int pd, int keep, int filed) {  // of shared memory, per query
-  return size_t(pd) + ((keep + 7) & ~7) + (filed ? 64 * FW_NPL : 0);
-}
 template <bool IS_L2>
-__global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishArgs f, RescoreArgs s, size_t nq,
-                                                             uint32_t* __restrict__ large_ids) {
+__global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishArgs f, size_t nq, uint32_t* __restrict__ large_ids) {
   const int w = threadIdx.x >> 5, lane = lane_id();
   const size_t q = size_t(blockIdx.x) * 8 + w;
   if (q >= nq) return;
-  float* sq = reinterpret_cast<float*>(dyn_smem()) + size_t(w) * finish_warp_words(a.pd, a.keep, f.filed);
+  float* sq = reinterpret_cast<float*>(dyn_smem()) + size_t(w) * (a.pd + ((a.keep + 7) & ~7));
   uint32_t* sel = reinterpret_cast<uint32_t*>(sq + a.pd);
-  u64* keys = reinterpret_cast<u64*>(sel + ((a.keep + 7) & ~7));  // filed: 32 * FW_NPL
   const uint32_t cnt = f.cand_cnt[q];
   if (cnt > uint32_t(min(f.cap, 32 * FW_NPL)) || (f.dropped && f.dropped[q])) {
     if (lane == 0) large_ids[atomicAdd(f.counters + LS_C_LARGE, 1u)] = uint32_t(q);
     return;
   }
-  int have = int(cnt);
+  const int have = int(cnt);
   uint32_t hi[FW_NPL], lo[FW_NPL];
-  auto take_in = [&](const u64* src) {
 #pragma unroll
-    for (int j = 0; j < FW_NPL; ++j) {
-      const int i = j * 32 + lane;
-      const u64 key = i < have ? src[i] : FV_EMPTY_KEY;
-      hi[j] = uint32_t(key >> 32);
-      lo[j] = uint32_t(key);
-    }
-  };
-  auto count_le = [&](uint32_t x) {
-    int c = 0;
+  for (int j = 0; j < FW_NPL; ++j) {
+    const int i = j * 32 + lane;
+    const u64 key = i < have ? f.cand[q * size_t(f.cap) + i] : FV_EMPTY_KEY;
+    hi[j] = uint32_t(key >> 32);
+    lo[j] = uint32_t(key);
+  }
+  for (int c = lane; c < a.pd; c += 32) sq[c] = a.queries[q * size_t(a.pd) + c];
+  // The best `keep`: the rows whose word is below T, those at T with ids below id_cut, and `room` of those at both.
+  uint32_t T = 0xFFFFFFFFu, id_cut = 0xFFFFFFFFu;
+  int room = 0;  // rows AT the cut that belong to the best `keep`: one, unless a file holds an id more than once
+  if (have > a.keep) {
+    auto count_le = [&](uint32_t x) {
+      int c = 0;
 #pragma unroll
-    for (int j = 0; j < FW_NPL; ++j) c += (j * 32 + lane < have && hi[j] <= x) ? 1 : 0;
-    return __reduce_add_sync(FV_FULL, c);
-  };
-  // the keep-th smallest word, or any below the next one; `at`: the entries up to it, -1 if they are not counted yet
-  auto cut_of = [&](int& at) {
+      for (int j = 0; j < FW_NPL; ++j) c += (j * 32 + lane < have && hi[j] <= x) ? 1 : 0;
+      return __reduce_add_sync(FV_FULL, c);
+    };
     uint32_t lo_w = 0xFFFFFFFFu, hi_w = 0;
 #pragma unroll
     for (int j = 0; j < FW_NPL; ++j)
@@ -1447,7 +1295,7 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
       }
     lo_w = __reduce_min_sync(FV_FULL, lo_w);
     hi_w = __reduce_max_sync(FV_FULL, hi_w);
-    at = -1;
+    int at = -1;  // rows at or below lo_w, once known
     while (lo_w < hi_w) {
       const uint32_t mid = lo_w + ((hi_w - lo_w) >> 1);
       const int c = count_le(mid);
@@ -1459,44 +1307,7 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
       if (c > a.keep) hi_w = mid;
       else lo_w = mid + 1;
     }
-    return lo_w;
-  };
-  take_in(f.cand + q * size_t(f.cap));
-  for (int c = lane; c < a.pd; c += 32) sq[c] = a.queries[q * size_t(a.pd) + c];
-  if (f.filed) {
-    uint32_t cut = 0xFFFFFFFFu;
-    if (have > a.keep) {
-      int at;
-      cut = filed_cut(cut_of(at), __uint_as_float(s.q_eps[q]));
-    }
-    int need = 0;
-#pragma unroll
-    for (int j = 0; j < FW_NPL; ++j) {
-      const bool in = j * 32 + lane < have && hi[j] <= cut;
-      const unsigned m = __ballot_sync(FV_FULL, in);
-      if (in) keys[need + __popc(m & ((1u << lane) - 1u))] = lo[j];
-      need += __popc(m);
-    }
-    __syncwarp();
-    have = 0;
-#pragma unroll 1
-    for (int i0 = 0; i0 < need; i0 += 32) {
-      u64 key = FV_EMPTY_KEY;
-      if (i0 + lane < need) key = survivor_key(s, s.pool[uint32_t(keys[i0 + lane])], uint32_t(q));
-      __syncwarp();
-      const unsigned m = __ballot_sync(FV_FULL, key != FV_EMPTY_KEY);
-      if (key != FV_EMPTY_KEY) keys[have + __popc(m & ((1u << lane) - 1u))] = key;  // (behind what is still to be read)
-      have += __popc(m);
-      __syncwarp();
-    }
-    take_in(keys);
-  }
-  // The best `keep`: the rows whose word is below T, those at T with ids below id_cut, and `room` of those at both.
-  uint32_t T = 0xFFFFFFFFu, id_cut = 0xFFFFFFFFu;
-  int room = 0;  // rows AT the cut that belong to the best `keep`: one, unless a file holds an id more than once
-  if (have > a.keep) {
-    int at;
-    T = cut_of(at);
+    T = lo_w;
     if (at < 0) at = count_le(T);
     if (at > a.keep) {  // rows tie at the cut: the smallest ids among them
       const int want = a.keep - (T ? count_le(T - 1) : 0);
@@ -1552,17 +1363,17 @@ __global__ void __launch_bounds__(256, 3) finish_warp_kernel(ScanArgs a, FinishA
 // keys for the re-rank: an even number, so that the query behind them is read 16 bytes at a time
 __host__ __device__ __forceinline__ int rerank_keys(int keep, int k) { return (keep + k + 1) & ~1; }
 
-__global__ void __launch_bounds__(256) ivfpq_finish_kernel(ScanArgs a, FinishArgs f, RescoreArgs s, int n2max) {
+__global__ void __launch_bounds__(256) ivfpq_finish_kernel(ScanArgs a, FinishArgs f, int n2max) {
   u64* lists = reinterpret_cast<u64*>(dyn_smem());  // n2max keys, a power of two from 32 on
   u64* rerank = lists + n2max;                      // keep + k
   float* sq = reinterpret_cast<float*>(rerank + rerank_keys(a.keep, a.k));
   if (!f.qids) {
-    finish_block_query(a, f, s, blockIdx.x, lists, rerank, sq);
+    finish_block_query(a, f, blockIdx.x, lists, rerank, sq);
     return;
   }
   const uint32_t n = *f.nqids;
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    finish_block_query(a, f, s, f.qids[i], lists, rerank, sq);
+    finish_block_query(a, f, f.qids[i], lists, rerank, sq);
     __syncthreads();  // the shared buffers are reused by the next query
   }
 }
@@ -1766,8 +1577,6 @@ struct GatherArgs {
   float kf, bn, cw2, c1;      // Kp; largest codeword-row norm; max ||centroid||^2 + max ||codewords||^2; rounding count of the chain
   uint16_t* qg;               // gathered operand rows
   float* thr;                 // per gathered row
-  float* eps;                 // main pass: per gathered row, the margin in it
-  uint32_t* q_eps;            // ... and per query the largest of its rows' (the bits of a float that is not negative; zeroed)
   uint32_t* g_q;
   uint32_t* g_l;
   float* g_base;
@@ -1882,8 +1691,6 @@ __global__ void __launch_bounds__(256) tc_gather_kernel(GatherArgs a) {
         if (!(thr == thr)) thr = INFINITY;
       } else {
         thr = a.is_l2 ? (tau - a2) + eps : (tau - base) + eps;
-        a.eps[arow] = eps;
-        atomicMax(a.q_eps + q, __float_as_uint(eps));
         if (!(thr == thr) || thr == INFINITY) thr = -INFINITY;  // a margin that is not a number: leave it to the other kernel
       }
     } else if (bound_pass) {
@@ -1899,6 +1706,104 @@ __global__ void __launch_bounds__(256) tc_gather_kernel(GatherArgs a) {
     a.g_q[arow] = q;
     a.g_l[arow] = uint32_t(l);
     a.g_base[arow] = base;
+  }
+}
+
+struct RescoreArgs {
+  const u64* pool;
+  const unsigned int* pool_cnt;
+  unsigned int pool_cap;
+  int npools;
+  const uint32_t* g_q;
+  const uint32_t* g_l;
+  const float* g_base;
+  const uint32_t* list_off;
+  const uint8_t* codes;
+  const uint32_t* ids;
+  const float* qtab;
+  const float* pre;  // or null (inner product)
+  int m;
+  const uint32_t* tau_bits;
+  u64* cand;
+  uint32_t* cand_cnt;
+  int cap;
+  const uint32_t* only;  // second round: only survivors of queries with only[q] != 0 (null: all)
+  const uint32_t* gate;  // second round: the device word that counts its queries; the kernel leaves at once if it is 0
+  size_t a_rows;         // extents (gathered operand rows, lists, rows in all lists), for the checks of the debug build
+  uint32_t nlist, nrows;
+};
+
+// One thread per survivor: the reference's compressed distance (ivfpq.rs:256-262, :272-276), bit for bit; kept if
+// at or below the query's bound.
+// The pools are very unequal (a CTA that drew the lists of a dense region holds several times the average), so the
+// blocks split the concatenation of all pools evenly instead of a pool each.
+__global__ void __launch_bounds__(128) rescore_kernel(RescoreArgs a) {
+  if (a.gate && *a.gate == 0) return;
+  uint32_t* start = reinterpret_cast<uint32_t*>(dyn_smem());  // npools + 1: first global index of every pool
+  if (threadIdx.x < 32) {  // prefix sums of the pools' counts
+    uint32_t s = 0;
+    for (int c0 = 0; c0 < a.npools; c0 += 32) {
+      const int c = c0 + lane_id();
+      const uint32_t v = c < a.npools ? min(a.pool_cnt[c], a.pool_cap) : 0u;
+      uint32_t incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(FV_FULL, incl, o);
+        if (lane_id() >= o) incl += t;
+      }
+      if (c < a.npools) start[c] = s + incl - v;
+      s += __shfl_sync(FV_FULL, incl, 31);
+    }
+    if (threadIdx.x == 0) start[a.npools] = s;
+  }
+  __syncthreads();
+  const uint32_t total = start[a.npools];
+  const uint32_t per = ((total + gridDim.x - 1) / gridDim.x + 127u) & ~127u;
+  const uint32_t i0 = min(total, blockIdx.x * per), i1 = min(total, i0 + per);
+  const size_t tab = size_t(a.m) * KSUB;
+  for (uint32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    int lo = 0, hi = a.npools - 1;  // the pool holding global index i: the last one starting at or before it
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (start[mid] <= i) lo = mid;
+      else hi = mid - 1;
+    }
+    const u64 e = a.pool[size_t(lo) * a.pool_cap + (i - start[lo])];
+    const uint32_t arow = uint32_t(e >> 32), row = uint32_t(e);
+    if (!FV_IDX_OK(arow, a.a_rows, 5)) continue;
+    const uint32_t q = a.g_q[arow], l = a.g_l[arow];
+    if (!FV_IDX_OK(l, a.nlist, 6)) continue;
+    if (a.only && !a.only[q]) continue;
+    const size_t r = size_t(a.list_off[l]) + row;
+    if (!FV_IDX_OK(r, a.nrows, 7)) continue;
+    const uint8_t* code = a.codes + r * a.m;
+    const float* qt = a.qtab + size_t(q) * tab;
+    const float* pt = a.pre ? a.pre + size_t(l) * tab : nullptr;
+    float d = a.g_base[arow];
+    if (a.m == 16) {  // all 32 table reads in flight before the chain of additions starts
+      const uint4 cw = *reinterpret_cast<const uint4*>(code);
+      const uint32_t cws[4] = {cw.x, cw.y, cw.z, cw.w};
+      float t[16], pv[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int cj = int((cws[j >> 2] >> ((j & 3) * 8)) & 0xFFu);
+        t[j] = __ldg(qt + j * 256 + cj);
+        pv[j] = pt ? __ldg(pt + j * 256 + cj) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) d = __fadd_rn(d, pt ? __fadd_rn(pv[j], t[j]) : t[j]);
+    } else {
+      for (int j = 0; j < a.m; ++j) {
+        const int cj = code[j];
+        float t = __ldg(qt + j * 256 + cj);
+        if (pt) t = __fadd_rn(__ldg(pt + j * 256 + cj), t);
+        d = __fadd_rn(d, t);
+      }
+    }
+    if (d < INFINITY && order_bits(d) <= a.tau_bits[q]) {
+      const uint32_t slot = atomicAdd(a.cand_cnt + q, 1u);
+      if (slot < uint32_t(a.cap)) a.cand[size_t(q) * a.cap + slot] = make_key(d, __ldg(a.ids + r));
+    }
   }
 }
 
@@ -2184,8 +2089,7 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
     uint32_t *g_q = nullptr, *g_l = nullptr, *a_off = nullptr, *ntasks = nullptr, *task_moff = nullptr, *task_rows = nullptr;
     uint32_t* tile_task0 = nullptr;
     uint32_t tr_a = 256u, tr_b = 256u;  // operand tile rows of the bound pass and of the main pass
-    float *g_base = nullptr, *g_eps = nullptr;
-    uint32_t* q_eps = nullptr;
+    float* g_base = nullptr;
     uint4* tasks = nullptr;
     unsigned int* pool_cnt = nullptr;
     unsigned int pool_cap = 0;
@@ -2203,23 +2107,21 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       if (max_tasks > 0x7FFFFFF0u) return fail(FV_ERR_UNSUPPORTED, "too many tasks for one tensor-core pass");
       const int q_slots = std::min(nprobe, 64);
       FV_TRY(ctx->scratch[12].reserve(a_rows * Kp * sizeof(uint16_t)));
-      FV_TRY(ctx->scratch[13].reserve((a_rows * 5 + nq * size_t(q_slots + 3)) * sizeof(uint32_t) + 64));
+      FV_TRY(ctx->scratch[13].reserve((a_rows * 4 + nq * size_t(q_slots + 2)) * sizeof(uint32_t) + 64));
       FV_TRY(ctx->scratch[14].reserve(max_tasks * (sizeof(uint4) + 2 * sizeof(uint32_t)) +
                                       (ix.nlist + 8 + size_t(ctx->sm_count) + max_tiles + 2) * sizeof(uint32_t)));
       // per CTA; the fullest pool measured holds four to six times the average
       pool_cap = unsigned(std::min<size_t>(size_t(1) << 21, std::max<size_t>(65536, nq * 4096 / size_t(ctx->sm_count))));
       if (ix.survivor_slots) pool_cap = unsigned(ix.survivor_slots);
-      FV_TRY(ctx->scratch[15].reserve(size_t(ctx->sm_count) * pool_cap * (sizeof(u64) + sizeof(float))));
+      FV_TRY(ctx->scratch[15].reserve(size_t(ctx->sm_count) * pool_cap * sizeof(u64)));
       qg = ctx->scratch[12].as<uint16_t>();
       thr = ctx->scratch[13].as<float>();
       g_q = reinterpret_cast<uint32_t*>(thr + a_rows);
       g_l = g_q + a_rows;
       g_base = reinterpret_cast<float*>(g_l + a_rows);
-      g_eps = g_base + a_rows;
-      uint32_t* q_rows = reinterpret_cast<uint32_t*>(g_eps + a_rows);
+      uint32_t* q_rows = reinterpret_cast<uint32_t*>(g_base + a_rows);
       uint32_t* q_cnt = q_rows + nq * size_t(q_slots);
       dropped = q_cnt + nq;
-      q_eps = dropped + nq;
       tasks = ctx->scratch[14].as<uint4>();
       task_moff = reinterpret_cast<uint32_t*>(tasks + max_tasks);
       task_rows = task_moff + max_tasks;
@@ -2247,8 +2149,6 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       ga.g_q = g_q;
       ga.g_l = g_l;
       ga.g_base = g_base;
-      ga.eps = g_eps;
-      ga.q_eps = q_eps;
       // Operand tiles of 128 rows instead of 256 when a list has few pairs: the pass costs a tile's multiplications
       // whatever the tile holds.  Estimated from the averages (pairs per list), per pass.
       const double avg_len = double(ix.nrows) / double(std::max<size_t>(1, ix.nlist));
@@ -2340,7 +2240,6 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
     } else {
       tc_tasks_kernel<<<1, 1024, 0, ctx->stream>>>(pb_set.pair_off, ix.list_off, ix.roff8, ix.roff8 + ix.nlist + 1, ix.nlist, tasks,
                                                    a_off, tile_task0, uint32_t(max_tasks), ntasks, d_rows + 1, nullptr, nullptr, 0u, tr_b);
-      FV_CUDA(cudaMemsetAsync(dropped, 0, 2 * nq * sizeof(uint32_t), ctx->stream));  // and q_eps
       ga.tile_rows = tr_b;
       ga.pair_off = pb_set.pair_off;
       ga.pairs = pairs_b;
@@ -2348,6 +2247,7 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       ctx->stats.launches += 2;
       FV_CUDA(cudaGetLastError());
       stage_mark(ctx);  // 2
+      FV_CUDA(cudaMemsetAsync(dropped, 0, nq * sizeof(uint32_t), ctx->stream));
       FV_TRY(tc_list_pass(ctx, ix.recon, ix.metric, qg, a_rows, thr, tasks, ntasks, ntasks + 1, ctx->scratch[15].as<u64>(), pool_cnt,
                           pool_cap, g_q, dropped, &tc_grid, int(tr_b)));
       stage_mark(ctx);  // 3
@@ -2371,11 +2271,7 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       ra.cand = cand;
       ra.cand_cnt = cand_cnt;
       ra.cap = cap;
-      ra.pool_score = reinterpret_cast<const float*>(ra.pool + size_t(tc_grid) * pool_cap);
-      ra.thr = thr;
-      ra.eps = g_eps;
-      ra.q_eps = q_eps;
-      rescore_kernel<true><<<unsigned(tc_grid) * 16, 128, size_t(tc_grid + 1) * sizeof(uint32_t), ctx->stream>>>(ra);
+      rescore_kernel<<<unsigned(tc_grid) * 16, 128, size_t(tc_grid + 1) * sizeof(uint32_t), ctx->stream>>>(ra);
       ctx->stats.launches++;
       FV_CUDA(cudaGetLastError());
     }
@@ -2394,27 +2290,26 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
     fa.over_ids = pb_set.extra;
     fa.rerun_ids = pb_set.extra2;
     fa.dropped = dropped;
-    fa.filed = path == LIST_TENSOR ? 1 : 0;
     int n2max = 32;
     while (n2max < cap || n2max < keep) n2max <<= 1;
     const size_t fsmem = (size_t(n2max) + size_t(rerank_keys(keep, k))) * sizeof(u64) + size_t(ix.pd) * sizeof(float);
     if (fsmem + 256 > ctx->smem_optin) return fail(FV_ERR_UNSUPPORTED, "k * refine too large for shared memory");
     FV_TRY(allow_smem(ctx, ivfpq_finish_kernel, fsmem));
     // eight queries' vectors and selected ids per block: up to about 7,200 dimensions
-    const size_t wsmem = size_t(8) * finish_warp_words(ix.pd, keep, fa.filed) * sizeof(float);
+    const size_t wsmem = size_t(8) * (ix.pd + ((keep + 7) & ~7)) * sizeof(float);
     if (!candidates && !ix.owned_ids && k <= 32 && keep <= 256 && wsmem + 256 <= ctx->smem_optin) {
       FV_TRY(ctx->scratch[18].reserve(nq * sizeof(uint32_t)));
       uint32_t* large = ctx->scratch[18].as<uint32_t>();
       auto fw = ix.metric == FV_L2 ? finish_warp_kernel<true> : finish_warp_kernel<false>;
       FV_TRY(allow_smem(ctx, fw, wsmem));
-      fw<<<unsigned((nq + 7) / 8), 256, wsmem, ctx->stream>>>(a, fa, ra, nq, large);
+      fw<<<unsigned((nq + 7) / 8), 256, wsmem, ctx->stream>>>(a, fa, nq, large);
       FinishArgs fl = fa;  // (a count only the device knows; nearly always none)
       fl.qids = large;
       fl.nqids = pb_set.counters + LS_C_LARGE;
-      ivfpq_finish_kernel<<<unsigned(std::min<size_t>(nq, size_t(ctx->sm_count) * 4)), 256, fsmem, ctx->stream>>>(a, fl, ra, n2max);
+      ivfpq_finish_kernel<<<unsigned(std::min<size_t>(nq, size_t(ctx->sm_count) * 4)), 256, fsmem, ctx->stream>>>(a, fl, n2max);
       ctx->stats.launches++;
     } else {
-      ivfpq_finish_kernel<<<unsigned(nq), 256, fsmem, ctx->stream>>>(a, fa, ra, n2max);
+      ivfpq_finish_kernel<<<unsigned(nq), 256, fsmem, ctx->stream>>>(a, fa, n2max);
     }
     ctx->stats.launches++;
     FV_CUDA(cudaGetLastError());
@@ -2424,13 +2319,12 @@ int ivfpq_scan(fv_ctx* ctx, const ScanIndex& ix, const float* q, size_t nq, cons
       // round left.  Both kernels leave at once when there are none.
       ra.only = redo;
       ra.gate = pb_set.counters + LS_C_OVER;
-      rescore_kernel<false><<<unsigned(tc_grid) * 16, 128, size_t(tc_grid + 1) * sizeof(uint32_t), ctx->stream>>>(ra);
+      rescore_kernel<<<unsigned(tc_grid) * 16, 128, size_t(tc_grid + 1) * sizeof(uint32_t), ctx->stream>>>(ra);
       FinishArgs f2 = fa;
-      f2.filed = 0;
       f2.qids = fa.over_ids;
       f2.nqids = pb_set.counters + LS_C_OVER;
       f2.tighten = 0;
-      ivfpq_finish_kernel<<<unsigned(std::min<size_t>(nq, size_t(ctx->sm_count) * 4)), 256, fsmem, ctx->stream>>>(a, f2, ra, n2max);
+      ivfpq_finish_kernel<<<unsigned(std::min<size_t>(nq, size_t(ctx->sm_count) * 4)), 256, fsmem, ctx->stream>>>(a, f2, n2max);
       ctx->stats.launches += 2;
       FV_CUDA(cudaGetLastError());
     }
