@@ -10,7 +10,7 @@
 // into three 16-bit pieces, inside the MMA.  The epilogue reads the accumulators back with
 // tcgen05.ld (one query row per thread) and only compares.
 //
-// Two passes.  A sample pass over 1 base row in 32 leaves, per query, the smallest score of every few
+// Two passes.  A sample pass over 1 base row in 8 to 128 leaves, per query, the smallest score of every few
 // rows; about the fifth smallest of those is that query's bound.  The main pass appends every row scoring below
 // the bound to a candidate list.  A third kernel recomputes the reference's exact fp32 distance
 // chain (src/kernels.rs:200-231) for those candidates, picks the k best by (distance, id) and
@@ -1938,7 +1938,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   FV_TRY(pin_ready(ctx));
   const int Kp = tc->Kp;
   const bool is_l2 = metric == FV_L2;
-  // The rank R of the sampled bound has to fit the epilogue's register lists: a long result takes a coarser sample (a
+  // The rank R of the sampled bound is kept to SAMPLE_R_MAX: a long result takes a coarser sample (a
   // prefix of the stored one), where fewer of its rows are sampled.  k = 100 over 50,000 rows: 1 row in 32 instead of
   // 1 in 8, R = 13 (at 1 in 8 the bound would have to be about the 29th).  Results of up to 32 keep their own rate even
   // where R = 13 misses the aim by a factor of two (32 results at 1 in 8: one query in 25,000 is re-run): the coarser
