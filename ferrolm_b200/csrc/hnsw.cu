@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
       for (int c = lane; c < row_bytes(g.pd); c += 32) {
         const float x = c < g.pd ? queries[qsrc * size_t(g.pd) + c] : 0.f, v = c < g.pd ? x - g.byte_lo : 0.f;
         if (c < g.pd) sq[c] = x;
-        fits = fits && v >= 0.f && v <= 255.f && v == rintf(v);
+        fits = fits && x == rintf(x) && v >= 0.f && v <= 255.f;  // (x itself: the subtraction can round what is not whole, 5e-6 + 128 is 128)
         const int u = fits ? int(v) : 0;
         q_bytes[c] = uint8_t(u);
         norm += u * u;

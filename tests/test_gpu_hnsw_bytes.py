@@ -57,3 +57,18 @@ def test_values_that_are_not_whole(oracle, ctx):
     base = whole(2000, 40, 0, 255, 7)
     base[1999, 39] += 0.25
     check(oracle, ctx, base, whole(3000, 40, 0, 255, 8), 33)
+
+
+@pytest.mark.parametrize("lo,span", [(-128, 255), (-7, 255), (-250, 120)])
+def test_queries_a_little_off_whole_numbers(oracle, ctx, lo, span):
+    # the difference to the rows' lowest value rounds to a whole number where the components are none
+    base, q = whole(1500, 40, lo, span, 11), whole(3000, 40, lo, span, 12)
+    base[200:240], base[240:280] = -1, 1
+    rng = np.random.default_rng(13)
+    little = q * np.float32(1 + 2.0**-22)
+    little[q == 0] = 5e-6
+    at = rng.random(q.shape) < 0.1
+    q[at] = little[at]
+    q[:, 7] = little[:, 7]
+    q[1], q[2], q[3], q[4], q[1000] = 5e-6, 3.0000002, 0.99999994, 1e-6, 1e-6
+    check(oracle, ctx, base, q, 24)
