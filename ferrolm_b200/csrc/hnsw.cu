@@ -24,7 +24,7 @@ namespace fv {
 
 struct HnswDev {
   const float* data;
-  const uint8_t* bytes;        // or null (fv_hnsw::d_bytes)
+  const uint8_t* bytes;        // fv_hnsw::d_bytes
   float byte_lo;
   const uint32_t* links0;
   const uint32_t* upper_off;   // n + 1 offsets into upper_flat
@@ -34,12 +34,12 @@ struct HnswDev {
   size_t n;
 };
 
-// Shared memory of one search, in bytes: the query, the visited set's first part, the tie list, a run of rows and
+// Shared memory of one search, in bytes: the query (BYTES: as bytes too), the visited set's first part, the tie list, a run of rows and
 // their distances, the team's job, and the beam where it is not in registers.
 static constexpr int SEARCH_BLOCKS_PER_SM = 3;  // of 256 threads
 template <int R>
-__host__ __device__ __forceinline__ size_t search_smem(int pd, int m0, int ef, int sbits, bool team) {
-  return size_t(pd) * 4 + row_bytes(pd) + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + (team ? team_smem(m0) : 0) +
+__host__ __device__ __forceinline__ size_t search_smem(int pd, bool bytes, int m0, int ef, int sbits, bool team) {
+  return size_t(pd) * 4 + (bytes ? row_bytes(pd) : 0) + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + (team ? team_smem(m0) : 0) +
          (R == 0 ? ((size_t(ef) * 8 + 15) & ~size_t(15)) : 0);
 }
 
@@ -51,7 +51,7 @@ __host__ __device__ __forceinline__ size_t search_smem(int pd, int m0, int ef, i
 // work: distances, expansions, queries whose tie list overflowed, queries whose visited set overflowed (marked in
 // overflow[] and left for a re-run).  NW = 1: one warp per query, blockDim / 32 queries per block; NW > 1: a query
 // per block (Team in hnsw.cuh).
-template <bool IS_L2, int R, int NW>
+template <bool IS_L2, bool BYTES, int R, int NW>
 __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
     hnsw_search_kernel(HnswDev g, const float* __restrict__ queries, const uint32_t* __restrict__ qids, size_t nq, int k,
                        int ef, int sbits, int log2slots, uint32_t* __restrict__ tables, fv_neighbor* __restrict__ out,
@@ -59,16 +59,16 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
                        unsigned long long* __restrict__ work, unsigned int* __restrict__ next_query) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int searcher = NW == 1 ? w : 0, per_block = NW == 1 ? int(blockDim.x >> 5) : 1;
-  unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, g.m0, ef, sbits, NW > 1);
+  unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, BYTES, g.m0, ef, sbits, NW > 1);
   float* sq = reinterpret_cast<float*>(mine);
   uint8_t* q_bytes = reinterpret_cast<uint8_t*>(sq + g.pd);
-  uint32_t* small = reinterpret_cast<uint32_t*>(q_bytes + row_bytes(g.pd));
+  uint32_t* small = reinterpret_cast<uint32_t*>(q_bytes + (BYTES ? row_bytes(g.pd) : 0));
   uint32_t* tied = small + visit_smem(sbits) / 4;
   const size_t gw = size_t(blockIdx.x) * per_block + searcher;
   VisitSet seen;
   visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
-  Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + 32),
-                reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64), slot_links(g.m0), uint32_t(g.n), seen, 0u, IS_L2 ? g.bytes : nullptr, -1};
+  Team<NW, BYTES> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + 32),
+                reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64), slot_links(g.m0), uint32_t(g.n), seen, 0u, g.bytes, -1};
   u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + (NW > 1 ? team_smem(g.m0) : 0));
   if (NW > 1 && w > 0) {
     team_serve<IS_L2, NW>(team);
@@ -91,8 +91,7 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
     if (qi >= nq) break;
     const size_t qsrc = qids ? size_t(qids[qi]) : qi;
     const unsigned long long n_dist0 = n_dist, n_exp0 = n_exp;  // a query that overflows its table is re-run: its work counts once
-    team.q_norm = -1;
-    if (IS_L2 && g.bytes) {  // the query in bytes too, if it is of the rows' kind
+    if (BYTES) {  // the query in bytes too, if it is of the rows' kind
       bool fits = true;
       int norm = 0;
       for (int c = lane; c < row_bytes(g.pd); c += 32) {
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
         norm += u * u;
       }
       norm = __reduce_add_sync(FV_FULL, norm);
-      if (__all_sync(FV_FULL, fits)) team.q_norm = norm;
+      team.q_norm = __all_sync(FV_FULL, fits) ? norm : -1;
     } else {
       for (int c = lane; c < g.pd; c += 32) sq[c] = queries[qsrc * size_t(g.pd) + c];
     }
@@ -448,23 +447,27 @@ struct SearchShape {
   int threads, sbits;
 };
 
-template <int NW>
-static SearchKernel pick_search(bool is_l2, int R) {
+template <bool IS_L2, bool BYTES, int NW>
+static SearchKernel pick_search_of(int R) {
   switch (R) {
-    case 1: return is_l2 ? hnsw_search_kernel<true, 1, NW> : hnsw_search_kernel<false, 1, NW>;
-    case 2: return is_l2 ? hnsw_search_kernel<true, 2, NW> : hnsw_search_kernel<false, 2, NW>;
-    case 4: return is_l2 ? hnsw_search_kernel<true, 4, NW> : hnsw_search_kernel<false, 4, NW>;
-    case 8: return is_l2 ? hnsw_search_kernel<true, 8, NW> : hnsw_search_kernel<false, 8, NW>;
-    default: return is_l2 ? hnsw_search_kernel<true, 0, NW> : hnsw_search_kernel<false, 0, NW>;
+    case 1: return hnsw_search_kernel<IS_L2, BYTES, 1, NW>;
+    case 2: return hnsw_search_kernel<IS_L2, BYTES, 2, NW>;
+    case 4: return hnsw_search_kernel<IS_L2, BYTES, 4, NW>;
+    case 8: return hnsw_search_kernel<IS_L2, BYTES, 8, NW>;
+    default: return hnsw_search_kernel<IS_L2, BYTES, 0, NW>;
   }
 }
+template <int NW>
+static SearchKernel pick_search(bool is_l2, bool bytes, int R) {
+  return bytes ? pick_search_of<true, true, NW>(R) : is_l2 ? pick_search_of<true, false, NW>(R) : pick_search_of<false, false, NW>(R);
+}
 
-static int search_shape(fv_ctx* ctx, bool is_l2, size_t n, int pd, int m0, int ef, size_t active, SearchShape* s) {
+static int search_shape(fv_ctx* ctx, bool is_l2, bool bytes, size_t n, int pd, int m0, int ef, size_t active, SearchShape* s) {
   const int R = ef <= 32 ? 1 : ef <= 64 ? 2 : ef <= 128 ? 4 : ef <= 256 ? 8 : 0;
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
   const bool team = active <= size_t(ctx->sm_count) * team_searches_per_sm(pd, m0, ef), scouts = team && scouts_pay(ctx->sm_count, m0, ef, active);
   s->sbits = team ? visit_sbits(ef) : visit_sbits_single(n, ef);
-  size_t per = R == 0 ? search_smem<0>(pd, m0, ef, s->sbits, team) : search_smem<1>(pd, m0, ef, s->sbits, team);
+  size_t per = R == 0 ? search_smem<0>(pd, bytes, m0, ef, s->sbits, team) : search_smem<1>(pd, bytes, m0, ef, s->sbits, team);
   int W = 8;
   if (team) {
     s->searchers = 1;
@@ -483,7 +486,7 @@ static int search_shape(fv_ctx* ctx, bool is_l2, size_t n, int pd, int m0, int e
   const size_t by_warps = scouts ? team_blocks(SCOUT_WARPS) : 8 * SEARCH_BLOCKS_PER_SM / (s->threads / 32);
   const size_t per_sm = std::max<size_t>(1, std::min(size_t(227 * 1024) / (s->smem + 1024), by_warps));
   s->blocks = std::min<size_t>((active + s->searchers - 1) / s->searchers, size_t(ctx->sm_count) * per_sm);
-  s->kern = scouts ? pick_search<SCOUT_WARPS>(is_l2, R) : team ? pick_search<TEAM_WARPS>(is_l2, R) : pick_search<1>(is_l2, R);
+  s->kern = scouts ? pick_search<SCOUT_WARPS>(is_l2, bytes, R) : team ? pick_search<TEAM_WARPS>(is_l2, bytes, R) : pick_search<1>(is_l2, bytes, R);
   FV_TRY(allow_smem(ctx, s->kern, s->smem));
   return FV_OK;
 }
@@ -554,7 +557,7 @@ static int hnsw_search_dev(fv_hnsw* h, const float* d_queries, size_t nq, size_t
   bool fetched = false;
   for (int attempt = 0; attempt < 8 && active; ++attempt) {
     SearchShape sh{};
-    FV_TRY(search_shape(ctx, h->metric == FV_L2, n, pd, int(h->m0), int(ef), active, &sh));
+    FV_TRY(search_shape(ctx, h->metric == FV_L2, g.bytes != nullptr, n, pd, int(h->m0), int(ef), active, &sh));
     const size_t tables = sh.blocks * sh.searchers;
     FV_TRY(ctx->scratch[7].reserve((tables << log2slots) * 4));
     FV_CUDA(cudaMemsetAsync(d_work, 0, 4 * sizeof(unsigned long long) + sizeof(unsigned int), ctx->stream));

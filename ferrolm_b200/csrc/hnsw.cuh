@@ -398,7 +398,10 @@ __host__ __device__ __forceinline__ size_t team_smem(int m0) {  // bytes: the jo
 // blocks of 256 threads per SM; those of scouting teams have 288
 __host__ __device__ constexpr int team_threads(int nw) { return nw == 1 ? 256 : nw * 32; }
 __host__ __device__ constexpr int team_blocks(int nw) { return nw == SCOUT_WARPS ? 2 : 3; }
-template <int NW>
+// BYTES: the index has its rows as bytes too (a parameter, because the registers of the code for them cost searches without
+// any 3 to 9 %: 10,000 queries of 20,000 x 128 floats, ef 64 674 us with it, 629 without; and the room for a query's bytes an
+// SM's third block where rows are long: 2,000 queries of 4,000 x 4,096, ef 200 16.4 and 10.9 ms).
+template <int NW, bool BYTES = false>
 struct Team {
   static constexpr bool SCOUTS = NW == SCOUT_WARPS;
   const float* data;
@@ -410,8 +413,8 @@ struct Team {
   uint32_t n;     // nodes
   VisitSet seen;  // as it was set up: for visit_seen
   mutable unsigned posted;  // jobs so far
-  // the rows' bytes; those of a query lie behind its floats.  q_norm: the sum of the query's squares, -1 where it or the rows
-  // have no bytes and distances come from the floats
+  // BYTES: the rows' bytes; those of a query lie behind its floats.  q_norm: the sum of the query's squares, -1 where it has
+  // no bytes and distances come from the floats
   const uint8_t* bytes = nullptr;
   int q_norm = -1;
   // of an even and an odd job: the places of the new links, their number in front
@@ -428,8 +431,8 @@ __device__ __forceinline__ void team_arrive(int bar, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(bar), "r"(threads) : "memory");
 }
 __device__ __forceinline__ void team_sync(int bar, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory"); }
-template <int NW>
-__device__ __forceinline__ unsigned team_post(const Team<NW>& t, const TeamJob& job) {  // the job's number
+template <int NW, bool BYTES>
+__device__ __forceinline__ unsigned team_post(const Team<NW, BYTES>& t, const TeamJob& job) {  // the job's number
   const unsigned j = t.posted++;
   if (lane_id() == 0) t.job[j & 1] = job;
   team_arrive(1 + int(j & 1), NW * 32);
@@ -458,20 +461,20 @@ __device__ __forceinline__ float byte_distance(const uint4* __restrict__ q, cons
   return float(v + q_norm);
 }
 
-template <bool IS_L2, int LPR, int NW>
-__device__ __forceinline__ void team_rows(const Team<NW>& t, const float* from, int q_norm, int count, int first, int step) {
+template <bool IS_L2, int LPR, int NW, bool BYTES>
+__device__ __forceinline__ void team_rows(const Team<NW, BYTES>& t, const float* from, int q_norm, int count, int first, int step) {
   const int sub = lane_id() & (LPR - 1), g = lane_id() / LPR;
   for (int i0 = first; i0 < count; i0 += step) {
     const int i = i0 + g;
     const size_t x = t.ids[min(i, count - 1)];  // (rows past the end: the last one again)
-    const float d = IS_L2 && q_norm >= 0
+    const float d = BYTES && q_norm >= 0
                         ? byte_distance<LPR>(reinterpret_cast<const uint4*>(from + t.pd), t.bytes + x * row_bytes(t.pd), t.pd, q_norm)
                         : group_distance<IS_L2, LPR>(from, t.data + x * t.pd, t.pd);
     if (sub == 0 && i < count) t.out[i] = d;
   }
 }
-template <bool IS_L2, int NW>
-__device__ __forceinline__ void team_eval(const Team<NW>& t, const float* from, int count) {
+template <bool IS_L2, int NW, bool BYTES>
+__device__ __forceinline__ void team_eval(const Team<NW, BYTES>& t, const float* from, int count) {
   __syncwarp();
   if (NW == 1) {
     team_rows<IS_L2, 4>(t, from, t.q_norm, count, 0, 8);
@@ -480,20 +483,20 @@ __device__ __forceinline__ void team_eval(const Team<NW>& t, const float* from, 
     team_rows<IS_L2, 8>(t, from, t.q_norm, count, 0, 4);
     __syncwarp();
   } else {
-    const unsigned j = team_post<NW>(t, TeamJob{from, nullptr, count, 0, nullptr, IS_L2 ? t.q_norm : -1});
+    const unsigned j = team_post(t, TeamJob{from, nullptr, count, 0, nullptr, t.q_norm});
     team_rows<IS_L2, 8>(t, from, t.q_norm, count, 0, 4 * NW);
     team_sync(5 + int(j & 1), NW * 32);
   }
 }
-template <bool IS_L2, int NW>
-__device__ __forceinline__ void team_serve(const Team<NW>& t) {  // warps 1 .. NW - 1
+template <bool IS_L2, int NW, bool BYTES>
+__device__ __forceinline__ void team_serve(const Team<NW, BYTES>& t) {  // warps 1 .. NW - 1
   const int w = int(threadIdx.x >> 5), sub = lane_id() & 7, g = lane_id() >> 3;
   for (unsigned j = 0;; ++j) {
     const int odd = int(j & 1);
     team_sync(1 + odd, NW * 32);
     const TeamJob job = t.job[odd];
     if (job.count < 0) return;
-    if (!Team<NW>::SCOUTS || !job.row) {
+    if (!Team<NW, BYTES>::SCOUTS || !job.row) {
       team_rows<IS_L2, 8>(t, job.from, job.q_norm, job.count, 4 * w, 4 * NW);
     } else {
       uint32_t* ids = t.slot_ids(job.slot);
@@ -527,7 +530,7 @@ __device__ __forceinline__ void team_serve(const Team<NW>& t) {  // warps 1 .. N
       const int n = int(fresh[0]);
       for (int k0 = 4 * (w - 1); k0 < n; k0 += 4 * (NW - 1)) {
         const uint32_t at = fresh[4 + min(k0 + g, n - 1)], y = ids[at];  // (rows past the end: the last one again)
-        const float d = IS_L2 && job.q_norm >= 0
+        const float d = BYTES && job.q_norm >= 0
                             ? byte_distance<8>(reinterpret_cast<const uint4*>(job.from + t.pd), t.bytes + size_t(y) * row_bytes(t.pd), t.pd, job.q_norm)
                             : group_distance_ahead<IS_L2>(job.from, t.data + size_t(y) * t.pd, t.pd);
         if (sub == 0) out[at] = d;
@@ -541,15 +544,15 @@ __device__ __forceinline__ void team_serve(const Team<NW>& t) {  // warps 1 .. N
     team_arrive(5 + odd, NW * 32);
   }
 }
-template <int NW>
-__device__ __forceinline__ void team_dismiss(const Team<NW>& t) {
-  if (NW > 1) team_post<NW>(t, TeamJob{nullptr, nullptr, -1, 0, nullptr, -1});
+template <int NW, bool BYTES>
+__device__ __forceinline__ void team_dismiss(const Team<NW, BYTES>& t) {
+  if (NW > 1) team_post(t, TeamJob{nullptr, nullptr, -1, 0, nullptr, -1});
 }
 
 // The greedy descent through layers top .. bottom + 1 (hnsw.rs:254-268, :334-347).  `rows(c, layer)` is a node's link
 // block on a layer (count, then at most `width` ids).
-template <bool IS_L2, int NW, class Rows>
-__device__ __forceinline__ void greedy_descent(const Team<NW>& t, size_t n, Rows rows, int width, const float* sq, int top,
+template <bool IS_L2, int NW, bool BYTES, class Rows>
+__device__ __forceinline__ void greedy_descent(const Team<NW, BYTES>& t, size_t n, Rows rows, int width, const float* sq, int top,
                                                int bottom, uint32_t& cur, float& curd, unsigned long long& n_dist,
                                                unsigned long long& n_exp) {
   const int lane = lane_id();
@@ -598,8 +601,8 @@ __device__ __forceinline__ void greedy_descent(const Team<NW>& t, size_t n, Rows
 // visited set's part in global memory stops with `over`.  `flat`: where the link blocks of all nodes lie one behind the other,
 // width + 1 words each, if they do.  n_dist and n_exp grow by the distances evaluated and the nodes
 // expanded.
-template <bool IS_L2, int R, int NW, class Rows>
-__device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows rows, int width, const float* sq, Beam<R>& best,
+template <bool IS_L2, int R, int NW, bool BYTES, class Rows>
+__device__ __forceinline__ void beam_search(const Team<NW, BYTES>& t, size_t n, Rows rows, int width, const float* sq, Beam<R>& best,
                                             uint32_t* tied, VisitSet& seen, bool& over, bool& tie_lost,
                                             unsigned long long& n_dist, unsigned long long& n_exp,
                                             const uint32_t* flat = nullptr) {
@@ -629,12 +632,12 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
     const int slot = next_slot;
     next_slot = (slot + 1) & (NODE_SLOTS - 1);
     if (lane == slot) kept = node;
-    team_post<NW>(t, TeamJob{sq, rows(node), width, slot, flat, IS_L2 ? t.q_norm : -1});
+    team_post(t, TeamJob{sq, rows(node), width, slot, flat, t.q_norm});
     (busy0 < 0 ? busy0 : busy1) = slot;
     return slot;
   };
   u64 bound = best.last();
-  constexpr bool CARRY = R > 0 && Team<NW>::SCOUTS;  // (the other forms have no registers for it, or a cursor)
+  constexpr bool CARRY = R > 0 && Team<NW, BYTES>::SCOUTS;  // (the other forms have no registers for it, or a cursor)
   u64 next = best.first_open();  // the nearest entry that is not expanded
   for (;;) {
     const u64 ck = next;
@@ -670,7 +673,7 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
     const uint32_t* row = rows(c);
     uint32_t x_first = 0;
     int cnt, slot = 0;
-    if (Team<NW>::SCOUTS) {
+    if (Team<NW, BYTES>::SCOUTS) {
       const unsigned known = __ballot_sync(FV_FULL, kept == c);
       if (known) {
         slot = __ffs(known) - 1;
@@ -699,7 +702,7 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
     for (int c0 = 0; c0 < cnt; c0 += 32) {
       const int i = c0 + lane;
       u64 key = FV_EMPTY_KEY;  // a new link's, in the lane of its place
-      if (Team<NW>::SCOUTS) {
+      if (Team<NW, BYTES>::SCOUTS) {
         const uint32_t x = i < cnt ? t.slot_ids(slot)[i] : NO_LINK;
         const bool fresh = visit_warp(seen, x != NO_LINK, x);
         n_dist += __popc(__ballot_sync(FV_FULL, fresh));
@@ -761,7 +764,7 @@ __device__ __forceinline__ void beam_search(const Team<NW>& t, size_t n, Rows ro
     }
     if (!CARRY) next = best.first_open();
   }
-  if (Team<NW>::SCOUTS)
+  if (Team<NW, BYTES>::SCOUTS)
     while (busy0 >= 0) job_done();
   __syncwarp();
 }
