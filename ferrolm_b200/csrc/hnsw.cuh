@@ -376,9 +376,11 @@ struct Beam<0> {
 // Who computes a run of distances.  NW = 1: the warp itself.  NW > 1: the block's NW warps together; warp 0 runs the
 // search and posts jobs, the others wait for them in team_serve.  A single search is a chain of memory trips, and when there
 // are fewer searches than warps the rest of the SM can only help by shortening each link.
-// Two kinds of jobs: a run of rows, which warp 0 takes part in (team_eval), and the links of a node with the distances of
-// those that are not visited yet, which the others work out while warp 0 goes on (post_node).  Jobs are done in the order
-// they are posted; two may be under way.
+// A run of rows is a job that warp 0 takes part in (team_eval): all warps meet before and after it.  Scouting teams have a
+// second kind, the links of a node with the distances of those that are not visited yet, which the others work out while
+// warp 0 goes on (ask in beam_search).  Their jobs are done in the order they are posted; two may be under way; named barriers
+// keep them apart.  (Those and their fences cost teams of eight 3 to 6 %: 600 queries of 4,000 x 1,536, ef 200 2,550 us with
+// them, 2,400 with __syncthreads.)
 struct TeamJob {
   const float* from;    // shared memory: the vector the distances are from
   const uint32_t* row;  // a node's link block (count, ids), or null: a run of rows
@@ -423,7 +425,7 @@ struct Team {
   __device__ __forceinline__ uint32_t* slot_ids(int s) const { return slot_cnt() + NODE_SLOTS + s * 2 * links; }  // NO_LINK: visited
   __device__ __forceinline__ float* slot_out(int s) const { return reinterpret_cast<float*>(slot_ids(s) + links); }
 };
-// Named barriers, one for even and one for odd jobs: 1, 2 a job is posted; 3, 4 a node's links are there; 5, 6 it is done;
+// Named barriers of scouting teams, one for even and one for odd jobs: 1, 2 a job is posted; 3, 4 a node's links are there; 5, 6 it is done;
 // 7 the warps of a job among themselves.
 __device__ __forceinline__ void team_arrive(int bar, int threads) {
   __syncwarp();
@@ -482,21 +484,38 @@ __device__ __forceinline__ void team_eval(const Team<NW, BYTES>& t, const float*
   } else if (count <= 4) {  // one step of this warp: not worth the two barriers
     team_rows<IS_L2, 8>(t, from, t.q_norm, count, 0, 4);
     __syncwarp();
-  } else {
+  } else if (Team<NW, BYTES>::SCOUTS) {
     const unsigned j = team_post(t, TeamJob{from, nullptr, count, 0, nullptr, t.q_norm});
     team_rows<IS_L2, 8>(t, from, t.q_norm, count, 0, 4 * NW);
     team_sync(5 + int(j & 1), NW * 32);
+  } else {
+    if (lane_id() == 0) {
+      t.job->from = from;
+      t.job->count = count;
+      if (BYTES) t.job->q_norm = t.q_norm;
+    }
+    __syncthreads();
+    team_rows<IS_L2, 8>(t, from, t.q_norm, count, 0, 4 * NW);
+    __syncthreads();
   }
 }
 template <bool IS_L2, int NW, bool BYTES>
 __device__ __forceinline__ void team_serve(const Team<NW, BYTES>& t) {  // warps 1 .. NW - 1
   const int w = int(threadIdx.x >> 5), sub = lane_id() & 7, g = lane_id() >> 3;
   for (unsigned j = 0;; ++j) {
+    if (!Team<NW, BYTES>::SCOUTS) {
+      __syncthreads();
+      const int count = t.job->count;
+      if (count < 0) return;
+      team_rows<IS_L2, 8>(t, t.job->from, BYTES ? t.job->q_norm : -1, count, 4 * w, 4 * NW);
+      __syncthreads();
+      continue;
+    }
     const int odd = int(j & 1);
     team_sync(1 + odd, NW * 32);
     const TeamJob job = t.job[odd];
     if (job.count < 0) return;
-    if (!Team<NW, BYTES>::SCOUTS || !job.row) {
+    if (!job.row) {
       team_rows<IS_L2, 8>(t, job.from, job.q_norm, job.count, 4 * w, 4 * NW);
     } else {
       uint32_t* ids = t.slot_ids(job.slot);
@@ -546,7 +565,13 @@ __device__ __forceinline__ void team_serve(const Team<NW, BYTES>& t) {  // warps
 }
 template <int NW, bool BYTES>
 __device__ __forceinline__ void team_dismiss(const Team<NW, BYTES>& t) {
-  if (NW > 1) team_post(t, TeamJob{nullptr, nullptr, -1, 0, nullptr, -1});
+  if (Team<NW, BYTES>::SCOUTS) {
+    team_post(t, TeamJob{nullptr, nullptr, -1, 0, nullptr, -1});
+  } else if (NW > 1) {
+    __syncwarp();
+    if (lane_id() == 0) t.job->count = -1;
+    __syncthreads();
+  }
 }
 
 // The greedy descent through layers top .. bottom + 1 (hnsw.rs:254-268, :334-347).  `rows(c, layer)` is a node's link
