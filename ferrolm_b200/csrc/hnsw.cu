@@ -38,8 +38,8 @@ struct HnswDev {
 // their distances, the team's job, and the beam where it is not in registers.
 static constexpr int SEARCH_BLOCKS_PER_SM = 3;  // of 256 threads
 template <int R>
-__host__ __device__ __forceinline__ size_t search_smem(int pd, bool bytes, int m0, int ef, int sbits, bool team) {
-  return size_t(pd) * 4 + (bytes ? row_bytes(pd) : 0) + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + (team ? team_smem(m0) : 0) +
+__host__ __device__ __forceinline__ size_t search_smem(int pd, bool bytes, int m0, int ef, int sbits, int nw) {
+  return size_t(pd) * 4 + (bytes ? row_bytes(pd) : 0) + visit_smem(sbits) + (TIED_CAP + 32 + 32) * 4 + team_smem(nw, m0) +
          (R == 0 ? ((size_t(ef) * 8 + 15) & ~size_t(15)) : 0);
 }
 
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
                        unsigned long long* __restrict__ work, unsigned int* __restrict__ next_query) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int searcher = NW == 1 ? w : 0, per_block = NW == 1 ? int(blockDim.x >> 5) : 1;
-  unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, BYTES, g.m0, ef, sbits, NW > 1);
+  unsigned char* mine = dyn_smem() + size_t(searcher) * search_smem<R>(g.pd, BYTES, g.m0, ef, sbits, NW);
   float* sq = reinterpret_cast<float*>(mine);
   uint8_t* q_bytes = reinterpret_cast<uint8_t*>(sq + g.pd);
   uint32_t* small = reinterpret_cast<uint32_t*>(q_bytes + (BYTES ? row_bytes(g.pd) : 0));
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
   visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
   Team<NW, BYTES> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + 32),
                 reinterpret_cast<TeamJob*>(tied + TIED_CAP + 64), slot_links(g.m0), uint32_t(g.n), seen, 0u, g.bytes, -1};
-  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + (NW > 1 ? team_smem(g.m0) : 0));
+  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + team_smem(NW, g.m0));
   if (NW > 1 && w > 0) {
     team_serve<IS_L2, NW>(team);
     return;
@@ -465,9 +465,12 @@ static SearchKernel pick_search(bool is_l2, bool bytes, int R) {
 static int search_shape(fv_ctx* ctx, bool is_l2, bool bytes, size_t n, int pd, int m0, int ef, size_t active, SearchShape* s) {
   const int R = ef <= 32 ? 1 : ef <= 64 ? 2 : ef <= 128 ? 4 : ef <= 256 ? 8 : 0;
   const size_t budget = std::min<size_t>(ctx->smem_optin, 200 * 1024);
-  const bool team = active <= size_t(ctx->sm_count) * team_searches_per_sm(pd, m0, ef), scouts = team && scouts_pay(ctx->sm_count, m0, ef, active);
+  auto bytes_of = [&](int sbits, int nw) { return R == 0 ? search_smem<0>(pd, bytes, m0, ef, sbits, nw) : search_smem<1>(pd, bytes, m0, ef, sbits, nw); };
+  const bool team = active <= size_t(ctx->sm_count) * team_searches_per_sm(pd, m0, ef);
+  // (rows too long for a scouting team's slots beside the smallest first part of the visited set: a team of eight)
+  const bool scouts = team && scouts_pay(ctx->sm_count, m0, ef, active) && bytes_of(7, SCOUT_WARPS) <= ctx->smem_optin;
   s->sbits = team ? visit_sbits(ef) : visit_sbits_single(n, ef);
-  size_t per = R == 0 ? search_smem<0>(pd, bytes, m0, ef, s->sbits, team) : search_smem<1>(pd, bytes, m0, ef, s->sbits, team);
+  size_t per = bytes_of(s->sbits, scouts ? SCOUT_WARPS : team ? TEAM_WARPS : 1);
   int W = 8;
   if (team) {
     s->searchers = 1;

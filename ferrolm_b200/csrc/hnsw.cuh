@@ -383,19 +383,24 @@ struct Beam<0> {
 // them, 2,400 with __syncthreads.)
 struct TeamJob {
   const float* from;    // shared memory: the vector the distances are from
-  const uint32_t* row;  // a node's link block (count, ids), or null: a run of rows
   int count;            // rows of the run, or the most links to read; -1: no more work
-  int slot;             // where a node's links go
-  const uint32_t* flat; // link blocks of all nodes, count_max + 1 words each, or null
   int q_norm;           // Team::q_norm
+  // of scouting teams only (TEAM_JOB_BYTES)
+  const uint32_t* row;  // a node's link block (count, ids), or null: a run of rows
+  const uint32_t* flat; // link blocks of all nodes, count_max + 1 words each, or null
+  int slot;             // where a node's links go
   int unused[3];
 };
 static_assert(sizeof(TeamJob) == 48, "");
+static constexpr size_t TEAM_JOB_BYTES = 16;  // what a team of eight has room for
 static constexpr int NODE_SLOTS = 4;  // nodes whose links and distances are kept
 static constexpr uint32_t NO_LINK = 0xFFFFFFFFu;
 __host__ __device__ __forceinline__ int slot_links(int m0) { return (m0 + 31) & ~31; }
-__host__ __device__ __forceinline__ size_t team_smem(int m0) {  // bytes: the job, the slots
-  return 2 * sizeof(TeamJob) + 2 * (SCOUT_LINKS + 4) * 4 + NODE_SLOTS * (size_t(slot_links(m0)) * 8 + 4);  // a multiple of 16
+// bytes, a multiple of 16: the job of a run of rows; a scouting team's two jobs, the places of new links and the slots (lists of
+// more than SCOUT_LINKS have none: a file may hold some of thousands)
+__host__ __device__ __forceinline__ size_t team_smem(int nw, int m0) {
+  return nw != SCOUT_WARPS ? TEAM_JOB_BYTES
+                           : 2 * sizeof(TeamJob) + 2 * (SCOUT_LINKS + 4) * 4 + NODE_SLOTS * (size_t(slot_links(m0)) * 8 + 4);
 }
 // blocks of 256 threads per SM; those of scouting teams have 288
 __host__ __device__ constexpr int team_threads(int nw) { return nw == 1 ? 256 : nw * 32; }
@@ -485,7 +490,7 @@ __device__ __forceinline__ void team_eval(const Team<NW, BYTES>& t, const float*
     team_rows<IS_L2, 8>(t, from, t.q_norm, count, 0, 4);
     __syncwarp();
   } else if (Team<NW, BYTES>::SCOUTS) {
-    const unsigned j = team_post(t, TeamJob{from, nullptr, count, 0, nullptr, t.q_norm});
+    const unsigned j = team_post(t, TeamJob{from, count, t.q_norm, nullptr, nullptr, 0});
     team_rows<IS_L2, 8>(t, from, t.q_norm, count, 0, 4 * NW);
     team_sync(5 + int(j & 1), NW * 32);
   } else {
@@ -566,7 +571,7 @@ __device__ __forceinline__ void team_serve(const Team<NW, BYTES>& t) {  // warps
 template <int NW, bool BYTES>
 __device__ __forceinline__ void team_dismiss(const Team<NW, BYTES>& t) {
   if (Team<NW, BYTES>::SCOUTS) {
-    team_post(t, TeamJob{nullptr, nullptr, -1, 0, nullptr, -1});
+    team_post(t, TeamJob{nullptr, -1, -1, nullptr, nullptr, 0});
   } else if (NW > 1) {
     __syncwarp();
     if (lane_id() == 0) t.job->count = -1;
@@ -657,7 +662,7 @@ __device__ __forceinline__ void beam_search(const Team<NW, BYTES>& t, size_t n, 
     const int slot = next_slot;
     next_slot = (slot + 1) & (NODE_SLOTS - 1);
     if (lane == slot) kept = node;
-    team_post(t, TeamJob{sq, rows(node), width, slot, flat, t.q_norm});
+    team_post(t, TeamJob{sq, width, t.q_norm, rows(node), flat, slot});
     (busy0 < 0 ? busy0 : busy1) = slot;
     return slot;
   };

@@ -122,10 +122,9 @@ __device__ __forceinline__ int select_links(const BuildDev& g, const Team<NW>& t
 
 // Shared memory of one insertion: the node's row and a kept candidate's, the visited set's first part (a team's), the tie
 // list, a run of rows and their distances, the chosen links, the bits of select_links, the team's job, the found list.
-__host__ __device__ __forceinline__ size_t insert_smem(int pd, int m0, int ef, int sbits) {
+__host__ __device__ __forceinline__ size_t insert_smem(int pd, int m0, int ef, int sbits, int nw) {
   const size_t run = size_t(run_rows(ef));
-  return size_t(pd) * 8 + visit_smem(sbits) + (TIED_CAP + 2 * run + ((m0 + 3) & ~3) + 128) * 4 + (sbits >= 0 ? team_smem(m0) : 0) +  // (only teams have a shared part)
-        
+  return size_t(pd) * 8 + visit_smem(sbits) + (TIED_CAP + 2 * run + ((m0 + 3) & ~3) + 128) * 4 + team_smem(nw, m0) +
          ((size_t(ef) * 8 + 15) & ~size_t(15));
 }
 
@@ -139,7 +138,7 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int searcher = NW == 1 ? w : 0, per_block = NW == 1 ? int(blockDim.x >> 5) : 1;
   const int run = run_rows(ef);
-  unsigned char* mine = dyn_smem() + size_t(searcher) * insert_smem(g.pd, g.m0, ef, sbits);
+  unsigned char* mine = dyn_smem() + size_t(searcher) * insert_smem(g.pd, g.m0, ef, sbits, NW);
   float* sq = reinterpret_cast<float*>(mine);
   float* sc = sq + g.pd;
   uint32_t* small = reinterpret_cast<uint32_t*>(sc + g.pd);
@@ -151,7 +150,7 @@ __global__ void __launch_bounds__(team_threads(NW), team_blocks(NW))
   visit_setup(seen, small, sbits, tables + (gw << log2slots), log2slots, g.n);
   Team<NW> team{g.data, g.pd, tied + TIED_CAP, reinterpret_cast<float*>(tied + TIED_CAP + run),
                 reinterpret_cast<TeamJob*>(gone + 128), slot_links(g.m0), g.n, seen, 0u};
-  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + (NW > 1 ? team_smem(g.m0) : 0));
+  u64* list = reinterpret_cast<u64*>(reinterpret_cast<unsigned char*>(team.job) + team_smem(NW, g.m0));
   if (NW > 1 && w > 0) {
     team_serve<IS_L2, NW>(team);
     return;
@@ -445,12 +444,14 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
   const bool is_l2 = h->metric == FV_L2;
   const size_t link_warp = link_smem(pd, int(m0));
   int sbits = visit_sbits(int(ef)), W = 8, LW = 8;
-  const size_t ins_warp = insert_smem(pd, int(m0), int(ef), -1);  // a single warp's visited set is in global memory
-  auto team_bytes = [&](int bits) { return insert_smem(pd, int(m0), int(ef), bits); };
+  const size_t ins_warp = insert_smem(pd, int(m0), int(ef), -1, 1);  // a single warp's visited set is in global memory
+  auto team_bytes = [&](int bits, int nw) { return insert_smem(pd, int(m0), int(ef), bits, nw); };
+  // (rows too long for a scouting team's slots beside the smallest first part of the visited set: teams of eight)
+  const bool scouting = team_bytes(7, SCOUT_WARPS) <= ctx->smem_optin;
   while (W > 1 && ins_warp * W > budget / BUILD_BLOCKS_PER_SM) W >>= 1;
   while (LW > 1 && link_warp * LW > budget / BUILD_BLOCKS_PER_SM) LW >>= 1;
-  while (sbits > 7 && team_bytes(sbits) > ctx->smem_optin) sbits--;
-  if (std::max({ins_warp * W, team_bytes(sbits), link_warp * LW}) > ctx->smem_optin)
+  while (sbits > 7 && team_bytes(sbits, scouting ? SCOUT_WARPS : TEAM_WARPS) > ctx->smem_optin) sbits--;
+  if (std::max({ins_warp * W, team_bytes(sbits, TEAM_WARPS), link_warp * LW}) > ctx->smem_optin)
     return fail(FV_ERR_UNSUPPORTED, "dimension and ef_construction too large for shared memory");
   const size_t resident_blocks = size_t(ctx->sm_count) * BUILD_BLOCKS_PER_SM;
   const size_t searchers_max = std::min(resident_blocks * W, std::max<size_t>(widest, 1));  // (a team is one searcher)
@@ -458,8 +459,8 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
                ins_scouts = pick_insert<SCOUT_WARPS>(is_l2, R);
   auto lnk = is_l2 ? hnsw_link_kernel<true> : hnsw_link_kernel<false>;
   FV_TRY(allow_smem(ctx, ins, ins_warp * W));
-  FV_TRY(allow_smem(ctx, ins_team, team_bytes(sbits)));
-  FV_TRY(allow_smem(ctx, ins_scouts, team_bytes(sbits)));
+  FV_TRY(allow_smem(ctx, ins_team, team_bytes(sbits, TEAM_WARPS)));
+  if (scouting) FV_TRY(allow_smem(ctx, ins_scouts, team_bytes(sbits, SCOUT_WARPS)));
   FV_TRY(allow_smem(ctx, lnk, link_warp * LW));
 
   int log2slots = 11;
@@ -477,9 +478,10 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
     while (inserted < n) {
       const size_t b = next_batch(h->levels, inserted, top, max_batch, divisor);
       FV_CUDA(cudaMemsetAsync(d_edge_cnt, 0, 8, st));  // and the node counter
-      const bool scouts = scouts_pay(ctx->sm_count, int(m0), int(ef), b);
+      const bool scouts = scouting && scouts_pay(ctx->sm_count, int(m0), int(ef), b);
+      const int nw = scouts ? SCOUT_WARPS : TEAM_WARPS;
       if (b <= size_t(ctx->sm_count) * TEAM_INSERTS_PER_SM)
-        (scouts ? ins_scouts : ins_team)<<<unsigned(std::min(b, resident_blocks)), (scouts ? SCOUT_WARPS : TEAM_WARPS) * 32, team_bytes(sbits), st>>>(
+        (scouts ? ins_scouts : ins_team)<<<unsigned(std::min(b, resident_blocks)), nw * 32, team_bytes(sbits, nw), st>>>(
             g, uint32_t(inserted), uint32_t(inserted + b), ep, int(top), int(ef), sbits, log2slots, d_tables.as<uint32_t>(),
             d_edges.as<Edge>(), d_edge_cnt, d_next_node, uint32_t(edge_cap), d_head.as<uint32_t>(), d_flags);
       else
