@@ -468,7 +468,7 @@ static int search_shape(fv_ctx* ctx, bool is_l2, bool bytes, size_t n, int pd, i
   auto bytes_of = [&](int sbits, int nw) { return R == 0 ? search_smem<0>(pd, bytes, m0, ef, sbits, nw) : search_smem<1>(pd, bytes, m0, ef, sbits, nw); };
   const bool team = active <= size_t(ctx->sm_count) * team_searches_per_sm(pd, m0, ef);
   // (rows too long for a scouting team's slots beside the smallest first part of the visited set: a team of eight)
-  const bool scouts = team && scouts_pay(ctx->sm_count, m0, ef, active) && bytes_of(7, SCOUT_WARPS) <= ctx->smem_optin;
+  const bool scouts = team && scouts_pay(ctx->sm_count, pd, m0, ef, active) && bytes_of(7, SCOUT_WARPS) <= ctx->smem_optin;
   s->sbits = team ? visit_sbits(ef) : visit_sbits_single(n, ef);
   size_t per = bytes_of(s->sbits, scouts ? SCOUT_WARPS : team ? TEAM_WARPS : 1);
   int W = 8;

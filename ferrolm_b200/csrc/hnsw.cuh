@@ -60,11 +60,14 @@ static constexpr int TEAM_WARPS = 8;
 // done or under way; what is left of one is mostly the first warp's own part (1,900 cycles of 2,200 at 96 dimensions and 200
 // entries).  us with teams of eight and with scouts, 20 queries: 5,183 x 384, ef 64 203 and 176, ef 200 526 and 387; 100,000
 // x 128 154 and 141, 333 and 268; 20,000 x 200 with m = 24 248 and 161, 659 and 361.  Not with the beam in shared memory (100,000
-// x 128, ef 400: 1,090 and 1,216).  Construction, 20,000 x 96: 122 ms of kernels and 106.
+// x 128, ef 400: 1,090 and 1,216), nor where the rows are so long and the beam so short that working out what turns out not to
+// be next takes longer than it saves (4,000 x 2,048, ef 10: 1 query 108 and 116, 20 141 and 165, 296 189 and 207; ef 32 311 and
+// 327; ef 64 510 and 517, 20 queries 451 and 425; 5,000 x 768 the same at ef 10 and 32, 240 and 214 at 64).  Construction,
+// 20,000 x 96: 122 ms of kernels and 106.
 static constexpr int SCOUT_WARPS = 9;
 static constexpr int SCOUT_LINKS = 64;  // links of a node, at most
-static inline bool scouts_pay(int sm_count, int m0, int ef, size_t searches) {
-  return m0 <= SCOUT_LINKS && ef <= 256 && searches <= size_t(sm_count) * 2;
+static inline bool scouts_pay(int sm_count, int pd, int m0, int ef, size_t searches) {
+  return m0 <= SCOUT_LINKS && ef <= 256 && (pd < 1024 || ef > 32) && searches <= size_t(sm_count) * 2;
 }
 static inline size_t team_searches_per_sm(int pd, int m0, int ef) {
   static constexpr size_t most[5][3] = {{6, 14, 16}, {6, 10, 16}, {6, 8, 14}, {3, 6, 8}, {2, 2, 2}};

@@ -478,7 +478,7 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
     while (inserted < n) {
       const size_t b = next_batch(h->levels, inserted, top, max_batch, divisor);
       FV_CUDA(cudaMemsetAsync(d_edge_cnt, 0, 8, st));  // and the node counter
-      const bool scouts = scouting && scouts_pay(ctx->sm_count, int(m0), int(ef), b);
+      const bool scouts = scouting && scouts_pay(ctx->sm_count, pd, int(m0), int(ef), b);
       const int nw = scouts ? SCOUT_WARPS : TEAM_WARPS;
       if (b <= size_t(ctx->sm_count) * TEAM_INSERTS_PER_SM)
         (scouts ? ins_scouts : ins_team)<<<unsigned(std::min(b, resident_blocks)), nw * 32, team_bytes(sbits, nw), st>>>(

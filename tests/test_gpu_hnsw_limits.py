@@ -64,3 +64,16 @@ def test_files_with_long_link_lists(oracle, ctx, m):
     assert g.save() == data
     for nq, ef in ((3, 20), (900, 20), (20, 300)):
         same(g.search_batch(q[:nq], 10, ef), o.search_batch(q[:nq], 10, ef))
+
+
+@pytest.mark.parametrize("dim", [1016, 1024])
+def test_short_beams_over_long_rows(oracle, ctx, dim):
+    # scouting teams up to 1,023 dimensions or from beams of 33 on, teams of eight otherwise
+    import ferrolm_b200 as fv
+
+    base, q = oracle.testdata(900, dim, 6), oracle.testdata(40, dim, 7)
+    g = fv.Hnsw.build_batched(ctx, IP, dim, base, fv.HnswParams(8, 32, 1))
+    assert g.save() == oracle.Hnsw.build_batched(IP, dim, base, m=8, ef_construction=32, seed=1).save()
+    o = oracle.Hnsw.load(g.save())
+    for ef in (10, 32, 33):
+        same(g.search_batch(q, 10, ef), o.search_batch(q, 10, ef))
