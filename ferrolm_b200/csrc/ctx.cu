@@ -18,7 +18,14 @@ int fail(int status, const std::string& msg) {
 }
 
 static thread_local size_t g_alloc_limit = 0;
-bool alloc_refused(size_t bytes) { return g_alloc_limit && bytes > g_alloc_limit; }
+static thread_local int g_alloc_count = -1;
+bool alloc_refused(size_t bytes) {
+  if (g_alloc_limit && bytes > g_alloc_limit) return true;
+  if (g_alloc_count < 0) return false;
+  if (g_alloc_count == 0) return true;
+  --g_alloc_count;
+  return false;
+}
 
 static std::mutex g_ctx_mutex;
 }  // namespace fv
@@ -152,6 +159,11 @@ extern "C" {
 
 int fv_debug_alloc_limit(size_t bytes) {
   fv::g_alloc_limit = bytes;
+  return FV_OK;
+}
+
+int fv_debug_alloc_count(int allocations) {
+  fv::g_alloc_count = allocations;
   return FV_OK;
 }
 

@@ -1628,6 +1628,9 @@ int tc_append(fv_ctx* ctx, TcSide** ptc, int metric, const float* d_rows_new, si
     (*ptc)->Kp = Kp;
   }
   TcSide* tc = *ptc;
+  // before any buffer moves: should this call fail halfway, the rows of before are searched on, where they lie then
+  for (auto& form : tc->maps)
+    for (TcSide::Maps& m : form) m.valid = false;
   const size_t total = n_old + n_new;
   if (!tc->stats.p) {
     FV_TRY(tc->stats.reserve(256));
@@ -1682,8 +1685,6 @@ int tc_append(fv_ctx* ctx, TcSide** ptc, int metric, const float* d_rows_new, si
   ctx->stats.launches++;
   FV_CUDA(cudaGetLastError());
   tc->n = total;
-  for (auto& form : tc->maps)
-    for (TcSide::Maps& m : form) m.valid = false;
   if (metric == FV_L2) {
     // norm pieces: ||b||^2 / 2^e with the largest quotient in (128, 256] when e was chosen, re-split when it outgrows 2^15
     FV_TRY(tc->ext.grow(npad * size_t(EXT_K) * 2, n_old * size_t(EXT_K) * 2, ctx->stream));

@@ -13,7 +13,7 @@
 #include "common.cuh"
 
 namespace fv {
-bool alloc_refused(size_t bytes);  // the test hook fv_debug_alloc_limit
+bool alloc_refused(size_t bytes);  // the test hooks fv_debug_alloc_limit and fv_debug_alloc_count; asked once per allocation
 }
 
 // A growable device allocation (raw bytes).
@@ -48,11 +48,11 @@ struct DevBuf {
     if (bytes <= cap) return FV_OK;
     size_t want = bytes > 2 * cap ? bytes : 2 * cap;
     void* np = nullptr;
-    cudaError_t e = cudaMalloc(&np, want);
+    cudaError_t e = fv::alloc_refused(want) ? cudaErrorMemoryAllocation : cudaMalloc(&np, want);
     if (e != cudaSuccess && want > bytes) {
       (void)cudaGetLastError();
       want = bytes;
-      e = cudaMalloc(&np, want);
+      e = fv::alloc_refused(want) ? cudaErrorMemoryAllocation : cudaMalloc(&np, want);
     }
     if (e != cudaSuccess) {
       (void)cudaGetLastError();

@@ -180,9 +180,11 @@ int fv_debug_bounds_build(void);
  * tensor memory and returns, and the search that launched it fails with FV_ERR_TIMEOUT; the context stays usable.
  * Nothing on the device faults or spins without bound.  (0, -1) disarms.  Not for production callers. */
 int fv_debug_tc_fault(long long wait_limit_cycles, int skip_unit);
-/* Test hook for what a search or a training does when the device has little room: workspaces of more than `bytes` bytes
- * that the calling thread asks for are refused as cudaMalloc would refuse them (0: no limit, the default). */
+/* Test hooks for what a call does when the device has little room: device memory in pieces of more than `bytes` bytes that
+ * the calling thread asks for is refused as cudaMalloc would refuse it (0: no limit, the default); ... */
 int fv_debug_alloc_limit(size_t bytes);
+/* ... all that it asks for once it has got `allocations` more pieces (-1: no end, the default). */
+int fv_debug_alloc_count(int allocations);
 size_t fv_ivfpq_save_size(const fv_ivfpq* ix);
 int fv_ivfpq_save(const fv_ivfpq* ix, uint8_t* buf, size_t cap, size_t* written);      /* save :332 ("FLIVFPQ1") */
 int fv_ivfpq_load(fv_ctx* ctx, const uint8_t* bytes, size_t len, fv_ivfpq** out);      /* load :354 */

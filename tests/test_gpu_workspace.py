@@ -79,3 +79,49 @@ def test_what_cannot_be_done_without_is_an_error(oracle, ctx):
         fv.IvfPq.train(ctx, L2, 64, oracle.testdata(6000, 64, 1), fv.IvfPqParams(20, 16, 2, True, 1))
     assert e.value.status == FV_ERR_NOMEM
     assert len(fv.IvfPq.train(ctx, L2, 64, oracle.testdata(6000, 64, 1), fv.IvfPqParams(20, 16, 2, True, 1))) == 0
+
+
+@contextlib.contextmanager
+def allocations(count):
+    from ferrolm_b200._lib import check, lib
+
+    check(lib().fv_debug_alloc_count(count))
+    try:
+        yield
+    finally:
+        check(lib().fv_debug_alloc_count(-1))
+
+
+def rows(oracle, kind, n, seed):
+    x = oracle.testdata(n, 40, seed)
+    return np.rint(x * 8).clip(-100, 100).astype(np.float32) if kind == "whole" else x
+
+
+@pytest.mark.parametrize("metric,kind", [(L2, "any"), (L2, "whole"), (IP, "any")])
+def test_an_add_that_is_refused_at_any_of_its_allocations(oracle, ctx, metric, kind):
+    import ferrolm_b200 as fv
+    from ferrolm_b200._lib import FV_ERR_NOMEM
+
+    a, b, q = rows(oracle, kind, 5000, 1), rows(oracle, kind, 6000, 2), rows(oracle, kind, 300, 3)
+    o = oracle.FlatIndex(metric, 40)
+    o.add(a)
+    before, _ = o.search_batch(q, 10)
+    o.add(b)
+    after, _ = o.search_batch(q, 10)
+    for count in range(40):
+        ix = fv.FlatIndex(ctx, metric, 40)
+        ix.add(a)
+        assert ix.search_batch(q, 10)[0].tobytes() == before.tobytes()
+        try:
+            with allocations(count):
+                ix.add(b)
+        except fv.FerrovecError as e:
+            assert e.status == FV_ERR_NOMEM
+            assert len(ix) == 5000 and ix.search_batch(q, 10)[0].tobytes() == before.tobytes(), count
+            ix.add(b)
+            assert len(ix) == 11000 and ix.search_batch(q, 10)[0].tobytes() == after.tobytes(), count
+            continue
+        assert count > 5 and ix.search_batch(q, 10)[0].tobytes() == after.tobytes()
+        break
+    else:
+        raise AssertionError("the add was never taken")
