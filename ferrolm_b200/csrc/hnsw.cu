@@ -239,7 +239,7 @@ static int make_bytes(fv_hnsw* h) {
   const size_t n = h->n();
   if (h->metric != FV_L2 || n == 0) return FV_OK;
   DevBuf words;
-  FV_TRY(words.reserve(16));
+  if (words.reserve(16) != FV_OK) return FV_OK;  // (no room: the searches do without)
   const uint32_t init[4] = {0xFFFFFFFFu, 0u, 0u, 0u};
   uint32_t got[4];
   FV_CUDA(cudaMemcpyAsync(words.p, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
@@ -253,7 +253,7 @@ static int make_bytes(fv_hnsw* h) {
   // queries may lie a little beyond the rows' values: bytes above 0 or -128 where those hold all rows
   h->byte_lo = lo >= 0.f && hi <= 255.f ? 0.f : lo >= -128.f && hi <= 127.f ? -128.f : lo;
   if (!(hi - h->byte_lo <= 255.f) || double(h->pd) * 255.0 * 255.0 >= 16777216.0) return FV_OK;
-  if (h->d_bytes.reserve(n * size_t(row_bytes(int(h->pd)))) != FV_OK) return FV_OK;  // (no room: the searches do without)
+  if (h->d_bytes.reserve(n * size_t(row_bytes(int(h->pd)))) != FV_OK) return FV_OK;
   row_bytes_kernel<<<unsigned((n + 7) / 8), 256, 0, ctx->stream>>>(h->d_data.as<float>(), n, int(h->pd), h->byte_lo, h->d_bytes.as<uint8_t>());
   FV_CUDA(cudaGetLastError());
   return FV_OK;

@@ -125,3 +125,30 @@ def test_an_add_that_is_refused_at_any_of_its_allocations(oracle, ctx, metric, k
         break
     else:
         raise AssertionError("the add was never taken")
+
+
+def test_an_add_does_without_room_for_bytes(oracle, ctx):
+    import ferrolm_b200 as fv
+
+    def taken(kind, count):
+        a, b = rows(oracle, kind, 5000, 1), rows(oracle, kind, 6000, 2)
+        ix = fv.FlatIndex(ctx, L2, 40)
+        ix.add(a)
+        try:
+            with allocations(count):
+                ix.add(b)
+        except fv.FerrovecError:
+            return None
+        return ix, np.concatenate([a, b])
+
+    least = next(count for count in range(40) if taken("any", count))
+    q = rows(oracle, "whole", 300, 3)
+    for count in range(least, least + 7):  # none to all of the five pieces that the bytes take
+        ix, both = taken("whole", count)
+        o = oracle.FlatIndex(L2, 40)
+        o.add(both)
+        assert ix.search_batch(q, 10)[0].tobytes() == o.search_batch(q, 10)[0].tobytes(), count
+        more = rows(oracle, "whole", 700, 4)  # with room again
+        ix.add(more)
+        o.add(more)
+        assert ix.search_batch(q, 10)[0].tobytes() == o.search_batch(q, 10)[0].tobytes(), count
