@@ -1532,6 +1532,7 @@ struct TcSide {
   bool i8 = false;         // the base has 8-bit operands too
   int Kp8 = 0;             // their row length: pd rounded up to 128
   float lo8 = 0.f;         // the value they store as -128
+  float refused_lo8 = NAN; // above this value some row is too far from the middle: rows only come, so no add need look again
   DevBuf rows8, ext8, parity8, samp8, samp_ext8;
   int ext_e = 0;           // the pieces hold ||b||^2 / 2^ext_e
   bool ext_valid = false;
@@ -1589,11 +1590,12 @@ static int split_norms(fv_ctx* ctx, bool bf16, const float* norm2, size_t first,
 
 // The 8-bit form of rows n_old .. total, or of all of them where the rows before have none or another `lo`, and room for the
 // sample's; none for a base that does not qualify, nor where the device has no room for it: the 16-bit form does alone.
-// Costs 128 ceil(pd / 128) + 33 bytes per row and the sample's, and time: 100,000 x 128 in one add from the device 2.0 -> 2.6 ms.
+// Costs 128 ceil(pd / 128) + 33 bytes per row and the sample's, and time: 100,000 x 128 in one add from the device 1.6 -> 2.7 ms, mostly the allocations.
 static int append8(fv_ctx* ctx, TcSide* tc, const float* all_rows, size_t n_old, size_t total, size_t npad, size_t nspad) {
   const RangeStats& st = tc->h_stats;
   const float lo = st.min_v >= 0.f && st.max_v <= 255.f ? 0.f : st.min_v >= -128.f && st.max_v <= 127.f ? -128.f : st.min_v;
-  bool fits = !st.not_integer && !st.not_finite && tc->pd <= I8_MAX_PD && std::fabs(lo) <= 65536.f && st.max_v - lo <= 255.f;
+  bool fits = !st.not_integer && !st.not_finite && tc->pd <= I8_MAX_PD && std::fabs(lo) <= 65536.f && st.max_v - lo <= 255.f &&
+              lo != tc->refused_lo8;
   const size_t first = tc->i8 && tc->lo8 == lo ? n_old : 0;
   if (fits) {
     tc->Kp8 = round_up(tc->pd, 2 * KBLK);
@@ -1620,6 +1622,7 @@ static int append8(fv_ctx* ctx, TcSide* tc, const float* all_rows, size_t n_old,
     FV_CUDA(cudaMemcpyAsync(&h_large, too_large, sizeof(h_large), cudaMemcpyDeviceToHost, ctx->stream));
     FV_CUDA(cudaStreamSynchronize(ctx->stream));
     fits = h_large == 0;
+    if (!fits) tc->refused_lo8 = lo;
   }
   tc->i8 = fits;
   tc->lo8 = lo;

@@ -88,3 +88,23 @@ def test_rows_added_in_pieces(oracle, ctx):
     check(oracle, ctx, [a, whole(300, 72, -100, 90, 13)], q, 10)  # another offset: the old rows are converted again
     check(oracle, ctx, [a, b + 0.25], q, 10)                      # no longer whole numbers
     check(oracle, ctx, [b[:200] + 0.25, a], q, 10)
+
+
+def test_pieces_added_to_rows_that_do_not_fit(oracle, ctx):
+    import ferrolm_b200 as fv
+
+    dark = whole(4500, 128, 0, 100, 14)
+    dark[5] = 0  # 128 x 127^2 is beyond the norm's bytes above 0, not above -128
+    piece, q = whole(300, 128, 0, 100, 15), whole(200, 128, 0, 100, 16)
+    check(oracle, ctx, [dark, piece, piece[:9]], q, 10)
+    check(oracle, ctx, [dark, piece, whole(100, 128, -28, 100, 17), piece], q, 10)
+
+    def launches(base):  # of the second and third add: the rows of before are not converted again
+        ix = fv.FlatIndex(ctx, fv.Metric.L2, 128)
+        ix.add(base)
+        before = ctx.stats()["launches"]
+        ix.add(piece)
+        ix.add(piece)
+        return ctx.stats()["launches"] - before
+
+    assert launches(dark) == launches(dark + 0.5)
