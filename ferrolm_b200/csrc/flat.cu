@@ -10,6 +10,7 @@
 // lines per load instruction, and the L1 data pipe -- not the FMAs -- sets the pace (measured: 78 % of its peak
 // on the coarse step of an IVF-PQ search).
 #include <algorithm>
+#include <cmath>
 
 #include "internal.h"
 
@@ -708,19 +709,27 @@ int fv_flat_set_mode(fv_flat* ix, int mode) {
   return FV_OK;
 }
 
-// The one-launch scan against the tensor-core path, microseconds of a call.  Fitted to calls timed at 5,183 x 384, 20,000 and
-// 100,000 x 128, 100,000 x 384, 400,000 x 256, 1M x 128 and 4M x 64 (1 to 64 queries, 10, 33 and 100 results): the scan takes
-// about 55 us (one query 40) and, for every four queries, the time to read the rows at 4.8 TB/s; the tensor-core path 85 us and
-// the time to read its rows.  (Scan / tensor cores: 100,000 x 128, 8 queries 82 / 96, 32 queries 132 / 99; 1M x 128, 2 queries
-// 171 / 155, 8 queries 280 / 164; 5,183 x 384, 64 queries 74 / 125.)  With more than 32 results the scan takes two queries at a
-// time and its merge costs more; the other path's re-rank grows with the results (100,000 x 128, 16 queries, 33 results 132 /
-// 100, 100 results 146 / 113; 4 queries 89 / 97 and 91 / 114).
-static bool flat_prefers_few(size_t n, int pd, size_t nq, int L) {
-  const double mb = double(n) * pd * 4e-6;
-  const size_t qt = nq == 1 ? 1 : (L <= 32 ? 4 : 2);
-  const double passes = double((nq + qt - 1) / qt);
-  const double few = L <= 32 ? (nq == 1 ? 40.0 + mb / 6.6 : 55.0 + passes * mb / 4.8) : (nq == 1 ? 48.0 + mb / 5.5 : 75.0 + passes * mb / 6.5);
-  const double tc = (L <= 32 ? 85.0 : 95.0 + 0.25 * (L - 32)) + 0.14 * mb;
+// The one-launch scan against the tensor-core path: microseconds of a call, fitted to 1,680 calls timed both ways (4,100 x 32 to
+// 3M x 64 and 1M x 128, 1 to 64 queries, 1 to 128 results).  The scan takes a launch, more where the rows have to come from
+// memory, and per group of four queries (two with more than 32 results) the time to read the rows at 6.5 TB/s and to offer them;
+// the tensor-core path its short kernels, the reading of its operands and a re-rank that grows with results, queries and
+// dimensions.  Scan / tensor cores: 5,183 x 384, 64 queries 75 / 110; 20,000 x 128, 64 queries 83 / 89, 33 results 116 / 88;
+// 20,000 x 384, 24 queries 87 / 101, 100 results 107 / 125; 100,000 x 128, 8 queries 81 / 99, 32 queries 133 / 101; 1M x 128, 2
+// queries 172 / 173, 8 queries 277 / 175 (bytes 161).  One call of 67 takes the way that is 5 % slower or more, the worst one
+// 20 %.
+static bool flat_prefers_few(const fv::TcInfo& side, size_t n_rows, int pd, size_t nq, int L) {
+  const double n = double(n_rows), mb = n * pd * 4e-6, g = std::log2(double(nq)), kp = side.Kp;
+  const size_t qt = L <= 32 ? 4 : 2;
+  const double groups = double((nq + qt - 1) / qt);
+  double few, tc;
+  if (L <= 32) {
+    few = nq == 1 ? 34 + 0.16 * mb + 3.3e-8 * n * L : 43.5 + 29 * mb / (mb + 62) + groups * (0.15 * mb + (13 + 0.54 * L) * 1e-6 * n);
+    tc = 81 + (side.bytes ? 0.13 : 0.19) * mb + 0.26 * L + 0.015 * kp + g * (0.8 + 3.9e-4 * L * kp);
+  } else {
+    few = nq == 1 ? 43 + 0.17 * mb + 1.3e-7 * n * L
+                  : 47 + 112 * mb / (mb + 168) + groups * (0.14 * mb + (2.4 + 0.027 * L) * 1e-3 * std::sqrt(n));
+    tc = 77 + (side.bytes ? 0.1 : 0.14) * mb + 0.37 * L - 0.029 * kp + g * (1 + 1.6e-4 * L * kp);
+  }
   return few < tc;
 }
 
@@ -750,8 +759,12 @@ static int flat_search_impl(fv_flat* ix, const float* d_queries, size_t nq, size
     fv::stage_end(ctx);
     return FV_OK;
   };
-  if (ix->mode == 0 && fv::few_scan_usable(ctx, ix->n, pd, nq, L) &&
-      (!fv::tc_usable(ix->tc, ix->n, nq, L) || flat_prefers_few(ix->n, pd, nq, L))) {
+  auto prefers_few = [&]() {
+    fv::TcInfo side{};
+    fv::tc_info(ix->tc, &side);
+    return flat_prefers_few(side, ix->n, pd, nq, L);
+  };
+  if (ix->mode == 0 && fv::few_scan_usable(ctx, ix->n, pd, nq, L) && (!fv::tc_usable(ix->tc, ix->n, nq, L) || prefers_few())) {
     FV_TRY(fv::few_scan(ctx, ix->metric, ix->data.as<float>(), ix->n, pd, q, size_t(pd), nullptr, nq, L, true, ix->id_base,
                         nullptr, d_out, d_counts, 2));
     return finish();

@@ -1890,6 +1890,7 @@ void tc_info(const TcSide* tc, TcInfo* out) {
   out->min_v = tc->h_stats.min_v;
   out->max_v = tc->h_stats.max_v;
   out->not_finite = tc->h_stats.not_finite != 0;
+  out->bytes = tc->i8;
 }
 
 int* tc_error_word(TcSide* tc) {

@@ -231,6 +231,7 @@ struct TcInfo {
   size_t n;          // rows of the side
   float max_norm2, min_v, max_v;
   bool not_finite;
+  bool bytes;        // it has 8-bit operands too
 };
 void tc_info(const TcSide* tc, TcInfo* out);
 // Device word that a bounded wait inside the kernel sets when it runs out.  tc_list_pass does not clear it: a caller
