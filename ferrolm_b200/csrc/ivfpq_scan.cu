@@ -755,12 +755,15 @@ __global__ void pair_kernel(PairArgs a) {
 // the first operand tiles and warps of a list, and the epilogue warps that hold only far pairs keep to their fast
 // path (with the pairs in query order the tensor-core pass measured 0.51 instead of 0.41 ms).
 // Counting is bound by the atomics on the lists' counters: a block counts PAIRS_PER_BLOCK pairs in shared memory and takes
-// their places with one atomic per list it met (10,000 queries x 64 probes of 1,024 lists, an atomic per pair: 55 us).
-static constexpr int PAIRS_PER_BLOCK = 4096;
-template <bool FILL>
-__global__ void __launch_bounds__(1024) pair_flat_kernel(PairArgs a, bool in_smem) {
+// their places with one atomic per list it met (10,000 queries x 64 probes of 1,024 lists, an atomic per pair: 55 us).  Up to
+// PAIRS_FOR_SMEM pairs, which blocks of that size would leave to a few SMs, go by an atomic each, one per thread (TURNS = 1): 256
+// queries x 64 probes of 64 lists, the whole search 222 us, 226 to 231 with four turns.
+static constexpr int PAIR_TURNS = 4, PAIRS_PER_BLOCK = PAIR_TURNS * 1024, PAIRS_FOR_SMEM = 32768;
+template <bool FILL, int TURNS>
+__global__ void __launch_bounds__(1024) pair_flat_kernel(PairArgs a) {
+  constexpr bool in_smem = !FILL && TURNS > 1;
   uint32_t* count = reinterpret_cast<uint32_t*>(dyn_smem());  // in_smem: a word per list, pairs of this block, then their first place
-  const size_t total = a.nq * size_t(a.nprobe), first = blockIdx.x * size_t(PAIRS_PER_BLOCK);
+  const size_t total = a.nq * size_t(a.nprobe), first = blockIdx.x * size_t(TURNS * 1024);
   auto list_of = [&](size_t i, u64& c) -> uint32_t {  // 0xFFFFFFFF: none of this shard's
     if (i >= total) return 0xFFFFFFFFu;
     const size_t p = i / a.nq, q = i - p * a.nq;
@@ -773,20 +776,20 @@ __global__ void __launch_bounds__(1024) pair_flat_kernel(PairArgs a, bool in_sme
   u64 c = 0;
   if (FILL) {
 #pragma unroll
-    for (int t = 0; t < PAIRS_PER_BLOCK / 1024; ++t) {
+    for (int t = 0; t < TURNS; ++t) {
       const size_t i = first + t * 1024 + threadIdx.x;
       const uint32_t l = list_of(i, c);
       if (l != 0xFFFFFFFFu) a.pairs[a.pair_off[l] + a.slot_of[i]] = make_uint2(uint32_t(i % a.nq), __float_as_uint(key_distance(c)));
     }
     return;
   }
-  uint32_t l[PAIRS_PER_BLOCK / 1024], at[PAIRS_PER_BLOCK / 1024];
+  uint32_t l[TURNS], at[TURNS];
   if (in_smem) {
     for (uint32_t j = threadIdx.x; j < a.nlist; j += 1024) count[j] = 0;
     __syncthreads();
   }
 #pragma unroll
-  for (int t = 0; t < PAIRS_PER_BLOCK / 1024; ++t) {
+  for (int t = 0; t < TURNS; ++t) {
     l[t] = list_of(first + t * 1024 + threadIdx.x, c);
     if (l[t] != 0xFFFFFFFFu) at[t] = atomicAdd((in_smem ? count : a.pair_cnt) + l[t], 1u);
   }
@@ -799,7 +802,7 @@ __global__ void __launch_bounds__(1024) pair_flat_kernel(PairArgs a, bool in_sme
     __syncthreads();
   }
 #pragma unroll
-  for (int t = 0; t < PAIRS_PER_BLOCK / 1024; ++t)
+  for (int t = 0; t < TURNS; ++t)
     if (l[t] != 0xFFFFFFFFu) a.slot_of[first + t * 1024 + threadIdx.x] = at[t] + (in_smem ? count[l[t]] : 0u);
 }
 
@@ -1905,14 +1908,20 @@ static int bucket_pairs(fv_ctx* ctx, const ScanIndex& ix, const u64* cells, size
   pa.pairs = pairs;
   pa.slot_of = slot_of;
   if (min_rows == 0 && slot_of) {
-    const unsigned fblocks = unsigned((nq * size_t(nprobe) + PAIRS_PER_BLOCK - 1) / PAIRS_PER_BLOCK);
     // a block meets as many lists as it has pairs at the most: beyond a few times that clearing its counters is the work
-    const bool in_smem = ix.nlist <= 16384;
-    const size_t csmem = in_smem ? ix.nlist * sizeof(uint32_t) : 0;
-    FV_TRY(allow_smem(ctx, pair_flat_kernel<false>, csmem));
-    pair_flat_kernel<false><<<fblocks, 1024, csmem, ctx->stream>>>(pa, in_smem);
+    const size_t pairs = nq * size_t(nprobe);
+    const bool in_smem = ix.nlist <= 16384 && pairs > PAIRS_FOR_SMEM;
+    const unsigned per_block = in_smem ? PAIRS_PER_BLOCK : 1024, fblocks = unsigned((pairs + per_block - 1) / per_block);
+    if (in_smem) {
+      const size_t csmem = ix.nlist * sizeof(uint32_t);
+      FV_TRY(allow_smem(ctx, pair_flat_kernel<false, PAIR_TURNS>, csmem));
+      pair_flat_kernel<false, PAIR_TURNS><<<fblocks, 1024, csmem, ctx->stream>>>(pa);
+    } else {
+      pair_flat_kernel<false, 1><<<fblocks, 1024, 0, ctx->stream>>>(pa);
+    }
     pair_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(ps.pair_cnt, ix.list_off, ix.nlist, ps.pair_off, ps.task_off, ps.counters);
-    pair_flat_kernel<true><<<fblocks, 1024, 0, ctx->stream>>>(pa, false);
+    if (in_smem) pair_flat_kernel<true, PAIR_TURNS><<<fblocks, 1024, 0, ctx->stream>>>(pa);
+    else pair_flat_kernel<true, 1><<<fblocks, 1024, 0, ctx->stream>>>(pa);
   } else {
     const unsigned qblocks = unsigned((nq + 255) / 256);
     pair_kernel<false><<<qblocks, 256, 0, ctx->stream>>>(pa);

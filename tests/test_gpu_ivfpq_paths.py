@@ -143,3 +143,17 @@ def test_many_probes_of_many_lists(oracle, metric):
         # tables, scan and conversion; the coarse step's passes besides
         assert (launches >= 8) == (nprobe <= 128), launches
     ctx.close()
+
+
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("nq,nprobe", [(341, 3), (1024, 1), (4096, 8), (4097, 8), (1725, 19)])
+def test_pairs_are_filed_by_one_thread_each_and_by_blocks(made, metric, nq, nprobe):
+    # up to 32,768 pairs and beyond; whole and partial blocks
+    ix, _, q = made(metric, 16)
+    q = np.concatenate([q] * 6)[:nq]
+    ix.set_scan_mode(1)
+    want, wc = ix.search_batch(q, 10, nprobe, 0)
+    ix.set_scan_mode(3)
+    got, gc = ix.search_batch(q, 10, nprobe, 0)
+    ix.set_scan_mode(1)
+    assert np.array_equal(gc, wc) and np.array_equal(got, want)
