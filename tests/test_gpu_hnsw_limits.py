@@ -77,3 +77,19 @@ def test_short_beams_over_long_rows(oracle, ctx, dim):
     o = oracle.Hnsw.load(g.save())
     for ef in (10, 32, 33):
         same(g.search_batch(q, 10, ef), o.search_batch(q, 10, ef))
+
+
+@pytest.mark.parametrize("metric,m", [(L2, 17), (IP, 24), (L2, 32), (L2, 33)])
+def test_links_of_scouting_teams(oracle, ctx, metric, m):
+    # 34 to 64 links per node are looked at in two turns, 66 are beyond scouting teams; batches and queries on both sides of two
+    # per SM (148 SMs), beams on both sides of registers
+    import ferrolm_b200 as fv
+
+    base, q = oracle.testdata(2600, 40, 8), oracle.testdata(297, 40, 9)
+    g = fv.Hnsw.build_batched(ctx, metric, 40, base, fv.HnswParams(m, 60, 1), max_batch=600, divisor=4)
+    assert g.save() == oracle.Hnsw.build_batched(metric, 40, base, m=m, ef_construction=60, seed=1, max_batch=600, divisor=4).save()
+    o = oracle.Hnsw.load(g.save())
+    for ef in (20, 100, 256, 257):
+        want, wc = o.search_batch(q, 10, ef)
+        for nq in (1, 296, 297):
+            same(g.search_batch(q[:nq], 10, ef), (want[:nq], wc[:nq]))
