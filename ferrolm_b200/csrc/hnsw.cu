@@ -454,7 +454,9 @@ static SearchKernel pick_search_of(int R) {
     case 2: return hnsw_search_kernel<IS_L2, BYTES, 2, NW>;
     case 4: return hnsw_search_kernel<IS_L2, BYTES, 4, NW>;
     case 8: return hnsw_search_kernel<IS_L2, BYTES, 8, NW>;
-    default: return hnsw_search_kernel<IS_L2, BYTES, 0, NW>;
+    default:
+      if constexpr (NW == SCOUT_WARPS) return nullptr;  // (scouts_pay)
+      else return hnsw_search_kernel<IS_L2, BYTES, 0, NW>;
   }
 }
 template <int NW>

@@ -380,7 +380,9 @@ static InsertKernel pick_insert(bool is_l2, int R) {
     case 2: return is_l2 ? hnsw_insert_kernel<true, 2, NW> : hnsw_insert_kernel<false, 2, NW>;
     case 4: return is_l2 ? hnsw_insert_kernel<true, 4, NW> : hnsw_insert_kernel<false, 4, NW>;
     case 8: return is_l2 ? hnsw_insert_kernel<true, 8, NW> : hnsw_insert_kernel<false, 8, NW>;
-    default: return is_l2 ? hnsw_insert_kernel<true, 0, NW> : hnsw_insert_kernel<false, 0, NW>;
+    default:
+      if constexpr (NW == SCOUT_WARPS) return nullptr;  // (scouts_pay)
+      else return is_l2 ? hnsw_insert_kernel<true, 0, NW> : hnsw_insert_kernel<false, 0, NW>;
   }
 }
 
@@ -447,7 +449,7 @@ static int build_on_device(fv_hnsw* h, size_t ef, size_t max_batch, size_t divis
   const size_t ins_warp = insert_smem(pd, int(m0), int(ef), -1, 1);  // a single warp's visited set is in global memory
   auto team_bytes = [&](int bits, int nw) { return insert_smem(pd, int(m0), int(ef), bits, nw); };
   // (rows too long for a scouting team's slots beside the smallest first part of the visited set: teams of eight)
-  const bool scouting = team_bytes(7, SCOUT_WARPS) <= ctx->smem_optin;
+  const bool scouting = R > 0 && team_bytes(7, SCOUT_WARPS) <= ctx->smem_optin;
   while (W > 1 && ins_warp * W > budget / BUILD_BLOCKS_PER_SM) W >>= 1;
   while (LW > 1 && link_warp * LW > budget / BUILD_BLOCKS_PER_SM) LW >>= 1;
   while (sbits > 7 && team_bytes(sbits, scouting ? SCOUT_WARPS : TEAM_WARPS) > ctx->smem_optin) sbits--;
