@@ -1259,9 +1259,10 @@ struct RerankParams {
   unsigned int* retry_count;
 };
 
-// Bound by gathering the candidates' rows (about 160 per query at k = 10, 420 at k = 100): eight rows at a time, four
+// Bound by gathering the candidates' rows (56 to 112 per query at k = 10, 420 at k = 100): eight rows at a time, four
 // lanes to a row (group_distance), the result list in registers (32 * KR places).  With four rows of eight lanes staged
-// through shared memory and the list there too 10,000 queries at 1M x 128 took 274 us (201 now).  A batch that leaves
+// through shared memory and the list there too 10,000 queries at 1M x 128 took 274 us (201 this way, with 160 candidates
+// each).  Bytes have no rows to gather: 48 us.  A batch that leaves
 // the SMs short of warps and has long results is given `wpq` warps per query, which share its candidates and merge
 // their lists: 501 queries with k = 100 over 50,001 x 100, the whole search 455 us in the old form, 315 with a warp per
 // query, 217 with eight.
@@ -1942,8 +1943,8 @@ int tc_list_pass(fv_ctx* ctx, TcSide* tc, int metric, const uint16_t* d_A, size_
 }
 
 // Stages (fv_stats.stage_ms): 0 query conversion, 1 sample pass, 2 main pass, 3 re-rank + certificate, 4 fallback.
-// scratch slots: 2 scan partials (fallback), 3 A operand, 5 query norms + bounds + candidate counters, 6 sample lists,
-// 7 retry ids, 8 fallback keys, 9 candidate buffers
+// scratch slots: 2 scan partials (fallback), 3 A operands (16 bits, then bytes), 5 query norms + bounds + constants of the byte
+// form + error bounds + candidate counters, 6 group minima of the sample, 7 retry ids, 8 fallback keys, 9 candidate buffers
 int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n, int pd, const float* d_queries,
               size_t nq, int k, uint32_t id_base, u64* d_out_keys, bool mark_stages, bool prefilter_inf,
               const std::function<int()>& then) {
@@ -1961,7 +1962,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   R = std::min(R, SAMPLE_R_MAX);
   const size_t ns = sample_prefix(tc->ns, level);
   // One way through both passes, or two: over the 8-bit operands where the base has them and, should a query of the batch
-  // not fit them (known on the device only), over the 16-bit ones.  The kernels of the way that is not taken leave at once.
+  // not fit them (known on the device only), over the 16-bit ones: one launch that takes either (gemm_topk_either_kernel).
   const int ways = tc->i8 ? 2 : 1;
   // Pairs of CTAs where the batch has queries for both: more than one CTA's tile of the taller of the two ways.
   const bool pairs = nq > (Kp <= 2 * KBLK || tc->i8 ? 256u : 128u);
@@ -1978,7 +1979,7 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
     nq_pad = std::max(nq_pad, way[i].nq_pad);
     Tiling& t = way[i].tm;
     // Candidate slots per list, 4 lists per query and chunk: 256 (128 with the twice as many lists of MH = 2) unless the
-    // buffers would pass 2 GB (they are written sparsely: about 160 entries per query in all).  A base stored cluster by
+    // buffers would pass 2 GB (they are written sparsely: 56 to 112 entries per query in all).  A base stored cluster by
     // cluster puts most of a query's candidates into one or two chunks, so the slots must hold more than the average.
     t.nlists = size_t(t.grid) * t.ctas * t.segmax * (128 * t.MH * 4);
     t.ccap = t.MH == 2 ? 128 : 256;

@@ -45,9 +45,8 @@ __host__ __device__ __forceinline__ size_t search_smem(int pd, bool bytes, int m
 
 // Bound by the latency of a chain: link row, visited set, rows, insertions, about 65 times per query at ef 64, and by the
 // longest of a batch's queries (twice the average) at its end.  24 warps of 80 registers per SM hold a lane's 16
-// pieces of a row in flight: 2.02 ms per 10,000 queries at 200k x 128, ef 64 (32 warps of 64 registers, where the
-// loads are issued a few at a time: 2.46; 16 warps of 128: 2.28; before, with a row per lane, the beam in shared
-// memory and the visited set in L2: 2.35).
+// pieces of a row in flight (10,000 queries at 200k x 128, ef 64, in an earlier form 2.02 ms; 32 warps of 64 registers, where
+// the loads are issued a few at a time, 2.46; 16 warps of 128 2.28): now 1.52 ms from floats, 1.03 from bytes.
 // work: distances, expansions, queries whose tie list overflowed, queries whose visited set overflowed (marked in
 // overflow[] and left for a re-run).  NW = 1: one warp per query, blockDim / 32 queries per block; NW > 1: a query
 // per block (Team in hnsw.cuh).
