@@ -236,6 +236,28 @@ def time_gpu(fn, stream, reps: int, warm: int = 3):
     return e0.elapsed_time(e1) / reps
 
 
+def whole_bytes(rows):
+    """Whether rows are whole numbers in 0..255 (the graph search reads such rows as bytes), and whether exact search scores
+    them in 8-bit integers as well: the sum that stands for a row's norm has to fit (convert8_rows_kernel)."""
+    whole, norms_fit = True, True
+    for a in range(0, len(rows), 100_000):
+        x = rows[a:a + 100_000]
+        whole = whole and bool((x == np.rint(x)).all() and x.min() >= 0 and x.max() <= 255)
+        norms_fit = norms_fit and bool((((x - 127.0) ** 2).sum(axis=1) // 2).max() <= 30 * 255 * 127 + 126)
+    return whole, whole and norms_fit
+
+
+def exact_roofline(nq, n, dim, kernel_ms, pk, i8):
+    """Rate of the main pass against the measured 16-bit peak, or twice that for 8-bit operands."""
+    flops = 2.0 * nq * n * dim
+    rate, peak = flops / (kernel_ms * 1e-3) / 1e12, pk["tflops"] * (2 if i8 else 1)
+    return {"kernel": "gemm_topk_either_kernel" if i8 else "gemm_topk_kernel", "bound": "tensor", "achieved": rate, "peak": peak,
+            "unit": "TOP/s" if i8 else "TFLOP/s", "frac": rate / peak, "traffic": None, "peak_source": pk["source"],
+            "peak_note": "twice the 16-bit rate: 8-bit operands" if i8 else "16-bit rate",
+            "algorithmic_flops_per_launch": flops, "kernel_ms": kernel_ms,
+            "frac_of_sustained_peak": rate / (pk["tflops_sustained"] * (2 if i8 else 1))}
+
+
 def also_section(fv, oracle, ctx, stream, ix, base, queries, dq, pk, nprobe, refine, threads):
     """The other benchmark configurations at a glance (N=1 only): each entry carries its own time, recall against
     exact search on the same data and, where the oracle is cheap enough, a parity sample."""
@@ -255,10 +277,11 @@ def also_section(fv, oracle, ctx, stream, ix, base, queries, dq, pk, nprobe, ref
     # exact search on the same data (recall 1.0 by construction), same timing method
     ms_f = time_gpu(lambda: flat.search_batch(dq, K), stream, 10)
     st = ctx.stats()
-    gemm_ms = st["stage_ms"][2]
-    tf = 2.0 * NQ * N_BASE * DIM / (gemm_ms * 1e-3) / 1e12
+    i8 = whole_bytes(base)[1]
+    rl = exact_roofline(NQ, N_BASE, DIM, st["stage_ms"][2], pk, i8)
     out["exact_search_same_data"] = {"value": NQ / (ms_f * 1e-3), "unit": "queries/s", "recall_at_10": 1.0, "ms_per_step": ms_f,
-                                     "gemm_topk_kernel_ms": gemm_ms, "tensor_tflops": tf, "frac_of_measured_peak": tf / pk["tflops"],
+                                     "gemm_topk_kernel_ms": rl["kernel_ms"], "tensor_tflops": rl["achieved"],
+                                     "operands": "i8" if i8 else "f16", "frac_of_measured_peak": rl["frac"],
                                      "uncertified": st["uncertified"]}
     del flat
     # the sweep of the reference's driver (src/main.rs:553-565) on this index, with a parity sample each
@@ -307,7 +330,7 @@ def also_section(fv, oracle, ctx, stream, ix, base, queries, dq, pk, nprobe, ref
     got = h.search_batch(dqh, K, HNSW["ef"])
     want, wc = oh.search_batch(queries[:nsub], K, HNSW["ef"], threads)[:2]
     g = fv.neighbors_from_tensor(got[0])
-    alg = st["dist_evals"] * DIM * 4 + st["expansions"] * (2 * HNSW["m"] + 1) * 4
+    alg = st["dist_evals"] * DIM * (1 if whole_bytes(base[:hn])[0] else 4) + st["expansions"] * (2 * HNSW["m"] + 1) * 4
     out["hnsw_ef64_200k_nodes"] = {
         "value": hq / (ms_h * 1e-3), "unit": "queries/s", "ms_per_step": ms_h, "queries": hq,
         "recall_at_10": fv.recall(g, got[1].cpu().numpy().astype(np.uint32), ht, K),
@@ -579,11 +602,20 @@ def run_ours(args):
         names = FLAT_SHARDED_STAGES if world > 1 else FLAT_STAGES
     else:
         names = ["beam search"]
+    # (rows that were made on the GPU in chunks are judged by the first million)
+    bytes_rows = i8 = False
+    dtype = "f16 operands, f32 accumulate, f32 exact re-score"
+    if args.workload != "ivfpq":
+        bytes_rows, i8 = whole_bytes(base if base is not None else fv.datagen(0, 1, 1_000_000, DIM, CLUSTERS))
+    if args.workload == "hnsw":
+        dtype = "u8 rows, exact integer distances" if bytes_rows else "f32"
+    elif i8:
+        dtype = "i8 operands, i32 accumulate, exact distances"
     line = {
         "metric": METRIC, "value": NQ / (ms * 1e-3), "unit": "queries/s",
         "n_gpus": world, "steps": args.steps, "warmup": n_warm, "ms_per_step": ms,
         "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "data": "synthetic",
-        "dtype": "f32" if args.workload == "hnsw" else "f16 operands, f32 accumulate, f32 exact re-score",
+        "dtype": dtype,
         "config": workload_config(args.workload, world, nprobe, refine, list_shards),
         "e2e": {"value": NQ / (e2e_ms * 1e-3), "unit": "queries/s", "h2d_bytes_per_step": int((q_hi - q_lo) * DIM * 4),
                 "d2h_bytes_per_step": int(h_out.numel() * 4), "ms_per_step": e2e_ms,
@@ -630,16 +662,10 @@ def run_ours(args):
                                 "traffic": None, "peak_source": pk["source"], "algorithmic_bytes_per_launch": int(alg),
                                 "kernel_ms": kms}
     elif args.workload == "flat":
-        kms = float(src["stage_ms"][2])
-        alg = 2.0 * NQ * (hi - lo) * DIM
-        ach = alg / (kms * 1e-3) / 1e12
-        line["roofline"] = {"kernel": "gemm_topk_kernel", "bound": "tensor", "achieved": ach, "peak": pk["tflops"],
-                            "unit": "TFLOP/s", "frac": ach / pk["tflops"], "traffic": None, "peak_source": pk["source"],
-                            "algorithmic_flops_per_launch": alg, "kernel_ms": kms,
-                            "frac_of_sustained_peak": ach / pk["tflops_sustained"]}
+        line["roofline"] = exact_roofline(NQ, hi - lo, DIM, float(src["stage_ms"][2]), pk, i8)
     else:
         kms = float(stages[0])
-        alg = last["dist_evals"] * DIM * 4 + last["expansions"] * (2 * HNSW["m"] + 1) * 4
+        alg = last["dist_evals"] * DIM * (1 if bytes_rows else 4) + last["expansions"] * (2 * HNSW["m"] + 1) * 4
         ach = alg / (kms * 1e-3) / 1e9
         line["roofline"] = {"kernel": "hnsw_search_kernel", "bound": "hbm", "achieved": ach, "peak": pk["hbm_gbs"],
                             "unit": "GB/s", "frac": ach / pk["hbm_gbs"], "traffic": None, "peak_source": pk["source"],
