@@ -757,9 +757,10 @@ __global__ void pair_kernel(PairArgs a) {
 // Counting is bound by the atomics on the lists' counters: a block counts PAIRS_PER_BLOCK pairs in shared memory and takes
 // their places with one atomic per list it met (10,000 queries x 64 probes of 1,024 lists, an atomic per pair: 55 us).  Up to
 // PAIRS_FOR_SMEM pairs, which blocks of that size would leave to a few SMs, go by an atomic each, one per thread (TURNS = 1): 256
-// queries x 64 probes of 64 lists, the whole search 222 us, 226 to 231 with four turns.  Filing is always a pair per thread (13.9 us
+// queries x 64 probes of 64 lists, the whole search 222 us, 226 to 231 with four turns; 300 x 64 of 256 lists 246 and 252, 512 x 64
+// 587 and 578.  Filing is always a pair per thread (13.9 us
 // of 640,000 pairs in four turns, 10.5 in one).
-static constexpr int PAIR_TURNS = 4, PAIRS_PER_BLOCK = PAIR_TURNS * 1024, PAIRS_FOR_SMEM = 32768;
+static constexpr int PAIR_TURNS = 4, PAIRS_PER_BLOCK = PAIR_TURNS * 1024, PAIRS_FOR_SMEM = 20480;
 template <bool FILL, int TURNS>
 __global__ void __launch_bounds__(1024) pair_flat_kernel(PairArgs a) {
   constexpr bool in_smem = !FILL && TURNS > 1;

@@ -146,9 +146,9 @@ def test_many_probes_of_many_lists(oracle, metric):
 
 
 @pytest.mark.parametrize("metric", [L2, IP])
-@pytest.mark.parametrize("nq,nprobe", [(341, 3), (1024, 1), (4096, 8), (4097, 8), (1725, 19)])
+@pytest.mark.parametrize("nq,nprobe", [(341, 3), (1024, 1), (2560, 8), (2561, 8), (4096, 8), (4097, 8), (1725, 19)])
 def test_pairs_are_filed_by_one_thread_each_and_by_blocks(made, metric, nq, nprobe):
-    # up to 32,768 pairs and beyond; whole and partial blocks
+    # up to 20,480 pairs and beyond; whole and partial blocks
     ix, _, q = made(metric, 16)
     q = np.concatenate([q] * 6)[:nq]
     ix.set_scan_mode(1)
