@@ -1997,8 +1997,13 @@ int tc_search(fv_ctx* ctx, TcSide* tc, int metric, const float* d_rows, size_t n
   // seldom share one (their number times R (R - 1) / 2 is what the rank slips by), for at most 512 MB of queries at a time.
   const int group = ns <= 1024 ? 1 : ns <= 16384 ? 8 : ns <= 65536 ? 32 : 64;
   const size_t smin_ld = (ns + TILE_N - 1) / TILE_N * TILE_N / group;
-  const size_t slice = std::min(nq_pad, std::max<size_t>(512, ((size_t(512) << 20) / (smin_ld * sizeof(float))) & ~size_t(511)));
-  FV_TRY(ctx->scratch[6].reserve(slice * smin_ld * sizeof(float)));
+  size_t slice = std::min(nq_pad, std::max<size_t>(512, ((size_t(512) << 20) / (smin_ld * sizeof(float))) & ~size_t(511)));
+  for (;;) {  // (fewer at a time where the device has no room for those of so many)
+    const int got = ctx->scratch[6].reserve(slice * smin_ld * sizeof(float));
+    if (got == FV_OK) break;
+    if (got != FV_ERR_NOMEM || slice <= 512) return got;
+    slice = std::max<size_t>(512, slice / 2 & ~size_t(511));
+  }
   FV_TRY(ctx->scratch[7].reserve(nq * sizeof(uint32_t)));
   FV_TRY(ctx->scratch[9].reserve(cand_slots * sizeof(u64)));
   uint16_t* dA = ctx->scratch[3].as<uint16_t>();

@@ -152,3 +152,20 @@ def test_an_add_does_without_room_for_bytes(oracle, ctx):
         ix.add(more)
         o.add(more)
         assert ix.search_batch(q, 10)[0].tobytes() == o.search_batch(q, 10)[0].tobytes(), count
+
+
+@pytest.mark.parametrize("kind", ["any", "whole"])
+def test_search_without_room_for_the_samples_minima(oracle, ctx, kind):
+    import ferrolm_b200 as fv
+
+    base, q = rows(oracle, kind, 40_000, 5), rows(oracle, kind, 2900, 6)
+    ix = fv.FlatIndex(ctx, L2, 40)
+    ix.add(base)
+    ix.search_batch(q, 100)  # everything but the minima, which are a quarter of those below (a coarser sample)
+    with at_most(3_000_000):  # 3,072 queries' minima take 7.9 MB
+        got, gc = ix.search_batch(q, 10)
+    want, wc = ix.search_batch(q, 10)
+    assert got.tobytes() == want.tobytes() and (gc == wc).all()
+    o = oracle.FlatIndex(L2, 40)
+    o.add(base)
+    assert o.search_batch(q[:200], 10)[0].tobytes() == want[:200].tobytes()
